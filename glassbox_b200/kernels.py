@@ -66,6 +66,8 @@ _SIGNATURES = {
     "gb_kv_prefetch": [_P, _P, _P, _I, _P, _P, _I, _I, _I, _LL, _LL, _I, _I, _P],
     "gb_attention_prefill": [_P, _LL, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P],
     "gb_attention_prefill_supported": [_I, _I, _I, _I],
+    "gb_attention_prefill_f32": [_P, _LL, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P],
+    "gb_attention_prefill_f32_supported": [_I, _I, _I],
     "gb_gemm_tcgen05_qkv": [_P, _P, _P, _I, _I, _LL, _LL, _LL, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _LL, _I, _P, _P,
                             _P, _I, _F],
     "gb_gemm_tcgen05_qkv_supported": [_I],
@@ -922,6 +924,28 @@ def attention_prefill(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, 
     S = block_tables.shape[0]
     assert seq_first_row.numel() == S + 1 and seq_start_pos.numel() == S
     _call("gb_attention_prefill", _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(kcache), _ptr(vcache),
+          _ptr(block_tables), block_tables.shape[1], _ptr(seq_first_row), _ptr(seq_start_pos), S, int(max_rows_per_seq),
+          nh, nkv, hd, page_size, kcache.shape[0], float(scale), int(window or 0), _ptr(status), _stream())
+
+
+def attention_prefill_f32_supported(q: torch.Tensor, out: torch.Tensor, nh: int, nkv: int, hd: int) -> bool:
+    """Whether the float32 flash-attention kernel takes these operands (head size 16, 32, 64, 96 or 128, aligned rows)."""
+    return (q.dtype == torch.float32 and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0
+            and out.data_ptr() % 16 == 0 and bool(lib().gb_attention_prefill_f32_supported(nh, nkv, hd)))
+
+
+def attention_prefill_f32(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
+                          block_tables: torch.Tensor, seq_first_row: torch.Tensor, seq_start_pos: torch.Tensor,
+                          max_rows_per_seq: int, nh: int, nkv: int, hd: int, page_size: int, scale: float,
+                          window: Optional[int], status: torch.Tensor) -> None:
+    """float32 flash attention (FMA only) for batches whose requests bring runs of consecutive rows; arguments as
+    ``attention_prefill``."""
+    _cuda(q, out, kcache, vcache, block_tables, seq_first_row, seq_start_pos, status)
+    assert q.dtype == out.dtype == kcache.dtype == vcache.dtype == torch.float32 and q.stride(1) == 1 and out.stride(1) == 1
+    assert block_tables.dtype == torch.int32 and block_tables.is_contiguous()
+    S = block_tables.shape[0]
+    assert seq_first_row.numel() == S + 1 and seq_start_pos.numel() == S
+    _call("gb_attention_prefill_f32", _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(kcache), _ptr(vcache),
           _ptr(block_tables), block_tables.shape[1], _ptr(seq_first_row), _ptr(seq_start_pos), S, int(max_rows_per_seq),
           nh, nkv, hd, page_size, kcache.shape[0], float(scale), int(window or 0), _ptr(status), _stream())
 

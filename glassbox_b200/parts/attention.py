@@ -148,7 +148,8 @@ class GqaAttention(Mixer):
 
     def _has_flash(self, q, att, cache) -> bool:
         return (kernels.attention_prefill_tc_supported(q, att, self.nh, self.nkv, self.hd, cache.page_size)
-                or kernels.attention_prefill_supported(q.dtype, self.nh, self.nkv, self.hd, cache.page_size))
+                or kernels.attention_prefill_supported(q.dtype, self.nh, self.nkv, self.hd, cache.page_size)
+                or kernels.attention_prefill_f32_supported(q, att, self.nh, self.nkv, self.hd))
 
     def _attend_flash(self, ctx, q, att, cache, first_seq: int) -> bool:
         """The requests from ``first_seq`` on (runs of consecutive rows); False if no flash kernel takes the shape."""
@@ -163,6 +164,11 @@ class GqaAttention(Mixer):
             kernels.attention_prefill(q, att, cache.k, cache.v, tables, first_row, start_pos, ctx.max_rows_per_seq,
                                       self.nh, self.nkv, self.hd, cache.page_size, self.spec.scale, self.spec.window,
                                       ctx.status)
+            return True
+        if kernels.attention_prefill_f32_supported(q, att, self.nh, self.nkv, self.hd):
+            kernels.attention_prefill_f32(q, att, cache.k, cache.v, tables, first_row, start_pos, ctx.max_rows_per_seq,
+                                          self.nh, self.nkv, self.hd, cache.page_size, self.spec.scale, self.spec.window,
+                                          ctx.status)
             return True
         return False
 

@@ -1236,3 +1236,67 @@ def test_a_wait_at_the_programs_barrier_that_runs_out_is_reported_and_harms_noth
     chain(prog, st)
     ref = (a.double() @ w.double().T).to(torch.bfloat16).double() @ w.double().T
     assert int(st) == 0 and (out.double() - ref).abs().max() <= 1e-2 * ref.abs().max()
+
+
+PREFILL_F32_CASES = [  # the float32 flash kernel: 64-row query tiles over 64-key tiles
+    (9, 3, 64, 16, None, [(0, 200), (0, 64), (0, 1), (0, 65)]),
+    (9, 3, 64, 16, None, [(100, 31), (640, 2), (63, 130), (1, 1)]),       # portions that continue a cache
+    (4, 4, 64, 32, 100, [(0, 300), (250, 77)]),                          # a window that ends inside tiles
+    (4, 2, 16, 5, None, [(0, 130), (7, 9)]),                             # pages of no power of two
+    (3, 1, 32, 8, 17, [(0, 140), (300, 65)]),
+    (2, 1, 96, 16, None, [(0, 129), (70, 3)]),
+    (2, 1, 128, 64, 64, [(0, 150), (129, 64)]),
+]
+
+
+@pytest.mark.parametrize("case", PREFILL_F32_CASES)
+def test_attention_prefill_float32(case):
+    """Against the float64 formula, and the garbage that masked keys may hold (pages behind a window, tokens after the row)
+    must not reach a row: every key and value that no row of the step sees is infinite."""
+    from glassbox_b200 import kernels
+    nh, nkv, hd, ps, window, seqs = case
+    lens = [c + n for c, n in seqs]
+    k, v, tables, dense = make_cache(torch.float32, len(lens), lens, nkv, hd, ps, seed=4)
+    first, row_seq, positions = [0], [], []
+    for s_i, (c, n) in enumerate(seqs):
+        row_seq += [s_i] * n
+        positions += list(range(c, c + n))
+        first.append(first[-1] + n)
+        host = tables[s_i].tolist()
+        for key in list(range(0, max(0, c + 1 - window) if window else 0)) + list(range(c + n, -(-(c + n) // ps) * ps)):
+            k[host[key // ps], :, key % ps] = float("inf")
+            v[host[key // ps], :, key % ps] = float("nan")
+    n = len(row_seq)
+    q = torch.randn(n, nh, hd)
+    wide = torch.zeros(n, nh * hd + 2 * nkv * hd, device=DEV)                # q sits inside a wider qkv buffer
+    wide[:, :nh * hd] = q.reshape(n, -1).to(DEV)
+    out = torch.full((n, nh * hd), 7.0, device=DEV)
+    assert kernels.attention_prefill_f32_supported(wide[:, :nh * hd], out, nh, nkv, hd)
+    st = status()
+    kernels.attention_prefill_f32(wide[:, :nh * hd], out, k, v, tables, torch.tensor(first, dtype=torch.int32, device=DEV),
+                                  torch.tensor([c for c, _ in seqs], dtype=torch.int32, device=DEV), max(nn for _, nn in seqs),
+                                  nh, nkv, hd, ps, hd ** -0.5, window, st)
+    ref = ref_attention(q, dense, row_seq, positions, nh, nkv, hd ** -0.5, window)
+    assert int(st) == 0
+    diff = (out.cpu().double().reshape(n, nh, hd) - ref).abs()
+    worst = int(diff.amax(dim=(1, 2)).argmax())
+    assert diff.max() <= tol(torch.float32), f"row {worst} (sequence, position) = {row_seq[worst], positions[worst]}"
+
+
+def test_attention_prefill_float32_rows_beyond_the_table_and_padding_read_nothing():
+    from glassbox_b200 import kernels
+    nh, nkv, hd, ps = 2, 1, 64, 16
+    k, v, tables, dense = make_cache(torch.float32, 3, [32, 16, 40], nkv, hd, ps, seed=5)
+    tables = tables[:, :2].contiguous()                                     # reaches 32 positions
+    q = torch.randn(70, nh, hd)
+    out = torch.full((70, nh * hd), 7.0, device=DEV)
+    st = status()
+    args = (nh, nkv, hd, ps, hd ** -0.5, None, st)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    kernels.attention_prefill_f32(q.to(DEV).reshape(70, -1), out, k, v, tables, i32([0, 20, 30, 70]), i32([12, -1, 0]), 40, *args)
+    got = out.cpu().double().reshape(70, nh, hd)
+    assert int(st) == 4                                                      # the third request's rows 32 .. 39 are beyond the table
+    assert not got[20:30].any() and not got[62:].any()
+    ref = ref_attention(torch.cat([q[:20], q[30:62]]), dense, [0] * 20 + [2] * 32, list(range(12, 32)) + list(range(32)), nh, nkv,
+                        hd ** -0.5, None)
+    assert (torch.cat([got[:20], got[30:62]]) - ref).abs().max() <= tol(torch.float32)
