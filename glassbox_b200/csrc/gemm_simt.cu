@@ -1,12 +1,14 @@
 // C[M, N] (+)= A[M, K] * W[N, K]^T on the CUDA cores with float32 FMA only.
 //
 // This is the true 32-bit matrix product (no TF32, no tensor cores) and also the generic
-// fallback for any mix of float32 / bfloat16 operands at any size. Two kernels:
-//   * a 64x64x16 register-tiled kernel for M > 8,
+// fallback for any mix of float32 / bfloat16 operands at any size. Three kernels:
+//   * a register-tiled kernel with tiles of 128 x 128 or 128 x 64 and packed FMA where such tiles fill the chip (float32
+//     activations, rows aligned to 16 bytes),
+//   * a 64x64x16 register-tiled kernel for every other M > 8,
 //   * a weight-streaming kernel for M <= 8 (one warp per output column), which is what a
 //     decode step needs: every weight is read once, coalesced along K.
-// Each output element is reduced over K in an order that depends only on K (and on which of
-// the two kernels runs), never on M or on the element's place in the batch.
+// Each output element is reduced over K in an order that depends only on K (and on whether M > 8: both tiled kernels
+// add one product after the other from k = 0, so they give the same bits), never on M or on the element's place in the batch.
 // Row-major [out, in] weights as in crates/glassbox-core/src/kernels.rs:381, 586-655.
 #include "common.cuh"
 
@@ -103,6 +105,122 @@ __global__ void __launch_bounds__(256) gemm_tiled_kernel(const TA* __restrict__ 
     }
 }
 
+// -------------------------------------------------------------------------- wide tiled kernel
+// Tiles of 128 x WN outputs, 256 threads, 8 x (WN / 16) outputs each, k in slices of 16 double-buffered in shared memory (the
+// next slice's loads are in flight while one is worked on; one barrier per slice). Bound by the FMA pipe: a packed FMA does
+// two neighbouring rows, so a k costs 8 x (WN / 16) / 2 packed FMAs against 2 + WN / 64 16-byte loads and the copies of W's
+// numbers into both halves, where the 64 x 64 tile paid 8 loads for 16 scalar FMAs. Shared-memory bandwidth comes next: 8 x 4
+// outputs a thread read 3 x 16 bytes per 16 packed FMAs. Measured, 2,047 rows (64 x 64 tiles -> these): 960 x 576
+// 87 -> 66 us, 576 x 576 58 -> 41, 3072 x 576 228 -> 184 (39 TFLOP/s), 576 x 1536 139 -> 100.
+typedef unsigned long long simt_pair;
+constexpr int WIDE_M = 128, WIDE_K = 16;
+
+template <typename TA, typename TW, typename TC, int WN>
+__global__ void __launch_bounds__(256, 2) gemm_wide_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, int M,
+                                                           int N, int K, long long lda, long long ldw, long long ldc, int mode) {
+    constexpr int NQ = WN / 64;                          // groups of four columns of a thread, 64 apart
+    __shared__ __align__(16) float As[2][WIDE_K][WIDE_M + 4];
+    __shared__ __align__(16) float Ws[2][WIDE_K][WN + 4];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.y * WIDE_M, n0 = blockIdx.x * WN;
+    const int lr = tid >> 2, lk = (tid & 3) * 4;         // the row (and those 64 further on) and the k's that this thread fetches
+    simt_pair acc[4][NQ * 4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < NQ * 4; ++j) acc[i][j] = 0ull;
+    float fa[2][4], fw[NQ][4];
+    auto fetch = [&](int k0) {
+        const int gk = k0 + lk;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int gm = m0 + lr + 64 * h;
+            if (gm < M && gk < K) Vec4Load<TA>::load(A + (size_t)gm * lda + gk, fa[h]);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e) fa[h][e] = 0.f;
+        }
+#pragma unroll
+        for (int h = 0; h < NQ; ++h) {
+            const int gn = n0 + lr + 64 * h;
+            if (gn < N && gk < K) Vec4Load<TW>::load(W + (size_t)gn * ldw + gk, fw[h]);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e) fw[h][e] = 0.f;
+        }
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) As[buf][lk + e][lr + 64 * h] = fa[h][e];
+#pragma unroll
+            for (int h = 0; h < NQ; ++h) Ws[buf][lk + e][lr + 64 * h] = fw[h][e];
+        }
+    };
+    fetch(0);
+    put(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += WIDE_K, buf ^= 1) {
+        const bool more = k0 + WIDE_K < K;
+        if (more) fetch(k0 + WIDE_K);
+#pragma unroll
+        for (int kk = 0; kk < WIDE_K; ++kk) {
+            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][ty * 8]);
+            const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][ty * 8 + 4]);
+            const simt_pair a[4] = {a0.x, a0.y, a1.x, a1.y};
+#pragma unroll
+            for (int g = 0; g < NQ; ++g) {
+                const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][kk][g * 64 + tx * 4]);
+                const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    simt_pair both;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(both) : "f"(w[j]));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][g * 4 + j]) : "l"(a[i]), "l"(both));
+                }
+            }
+        }
+        if (more) put(buf ^ 1);
+        __syncthreads();
+    }
+    const bool whole = N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)C & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int gm = m0 + ty * 8 + i;
+        if (gm >= M) continue;
+#pragma unroll
+        for (int g = 0; g < NQ; ++g) {
+            const int gn = n0 + g * 64 + tx * 4;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i / 2][g * 4 + j]));
+                v[j] = i & 1 ? hi : lo;
+            }
+            TC* dst = C + (size_t)gm * ldc + gn;
+            if (sizeof(TC) == 4 && whole) {
+                if (gn >= N) continue;
+                float4* d4 = reinterpret_cast<float4*>(dst);
+                float4 r = make_float4(v[0], v[1], v[2], v[3]);
+                if (mode == OUT_ACCUMULATE) {
+                    const float4 o = *d4;
+                    r = make_float4(o.x + r.x, o.y + r.y, o.z + r.z, o.w + r.w);
+                }
+                *d4 = r;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (gn + j < N) store_out<TC>(dst + j, v[j], mode);
+            }
+        }
+    }
+}
+
 // ------------------------------------------------------------------- weight-streaming kernel
 // One warp per output column n. Lanes stride over K four elements at a time; up to 8 rows of A
 // are reduced against the same weight row, so the weight matrix is read exactly once.
@@ -160,6 +278,20 @@ static int launch_gemm(const void* a, const void* w, void* c, int M, int N, int 
         if (vec) gemm_skinny_kernel<TA, TW, TC, true><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
         else gemm_skinny_kernel<TA, TW, TC, false><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
     } else {
+        // The tile whose rounds over the SMs end soonest; a wide tile has a quarter more than an SM's share of the outputs at
+        // most before the 64 x 64 tiles, which run at half its rate, would be level.
+        if constexpr (sizeof(TA) == 4 && sizeof(TC) == 4) {
+            const long long rows = gb_ceil_div(M, WIDE_M);
+            const long long t128 = rows * gb_ceil_div(N, 128), t64 = rows * gb_ceil_div(N, 64);
+            const long long small = (long long)gb_ceil_div(M, BM) * gb_ceil_div(N, BN);
+            const long long c128 = 4 * ((t128 + 147) / 148), c64 = 2 * ((t64 + 147) / 148);        // in 64 x 64 outputs an SM
+            const long long c_small = 2 * ((small + 147) / 148);
+            if (vec && M > 64 && (c64 <= c_small || c128 <= c_small)) {
+                if (c128 < c64) gemm_wide_kernel<TA, TW, TC, 128><<<dim3(gb_ceil_div(N, 128), rows), 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
+                else gemm_wide_kernel<TA, TW, TC, 64><<<dim3(gb_ceil_div(N, 64), rows), 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
+                return gb_check_launch("gb_gemm_simt");
+            }
+        }
         dim3 grid(gb_ceil_div(N, BN), gb_ceil_div(M, BM));
         if (vec) gemm_tiled_kernel<TA, TW, TC, true><<<grid, 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
         else gemm_tiled_kernel<TA, TW, TC, false><<<grid, 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);

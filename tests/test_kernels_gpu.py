@@ -1300,3 +1300,25 @@ def test_attention_prefill_float32_rows_beyond_the_table_and_padding_read_nothin
     ref = ref_attention(torch.cat([q[:20], q[30:62]]), dense, [0] * 20 + [2] * 32, list(range(12, 32)) + list(range(32)), nh, nkv,
                         hd ** -0.5, None)
     assert (torch.cat([got[:20], got[30:62]]) - ref).abs().max() <= tol(torch.float32)
+
+
+@pytest.mark.parametrize("w_dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M, N, K", [(2048, 576, 576), (1025, 960, 100), (2047, 2500, 36), (4000, 577, 20)])
+def test_gemm_simt_wide_tiles_give_the_bits_of_the_small_ones(M, N, K, w_dt):
+    """Both tiled kernels add one product after the other: the wide tiles' bits are those of a call small enough for the
+    64 x 64 tiles, at sizes with ragged edges in every direction, stored and added."""
+    from glassbox_b200 import kernels
+    torch.manual_seed(M + N)
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV).to(w_dt)
+    c = torch.randn(M, N, device=DEV)
+    got, added = torch.empty(M, N, device=DEV), c.clone()
+    kernels.gemm_simt(a, w, got)
+    kernels.gemm_simt(a, w, added, accumulate=True)
+    small = torch.empty(M, N, device=DEV)
+    for lo in range(0, M, 40):
+        hi = min(M, lo + 40) if M - lo >= 49 else M
+        kernels.gemm_simt(a[lo:hi], w, small[lo:hi])
+        if hi == M:
+            break
+    assert torch.equal(got, small) and torch.equal(added, c + small)
+    assert (got.double() - a.double() @ w.double().T).abs().max() <= 1e-5 * K ** 0.5 * 4
