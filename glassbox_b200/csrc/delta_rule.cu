@@ -50,6 +50,53 @@ __global__ void __launch_bounds__(256) short_conv_kernel(const float* __restrict
     y[(size_t)row * ldy + ch] = acc / (1.0f + expf(-acc));
 }
 
+// The same for steps of many rows: a thread takes a channel of STRIP rows one after the other, every input once (the form above
+// reads each of them `taps` times and the channel's taps per row: bound by its loads' latency, a seventh of the copy rate).
+// Measured, 2,048 rows x 3,072 channels, four taps: 52 -> 23 us.
+constexpr int SC_STRIP = 16;
+
+template <int TAPS>
+__global__ void __launch_bounds__(256) short_conv_strip_kernel(const float* __restrict__ x, long long ldx, const float* __restrict__ w,
+                                                               float* __restrict__ y, long long ldy, const float* __restrict__ state,
+                                                               long long state_stride, long long state_off, const int* __restrict__ row_seq,
+                                                               const int* __restrict__ positions, const int* __restrict__ seq_first_row,
+                                                               const int* __restrict__ seq_slots, int n, int C, int num_slots,
+                                                               int* __restrict__ status) {
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    const int row0 = blockIdx.x * SC_STRIP;
+    const int ch = blockIdx.y * blockDim.x + threadIdx.x;
+    if (ch >= C) return;
+    float in[SC_STRIP + TAPS - 1];                 // rows row0 - (TAPS - 1) .. row0 + STRIP - 1
+#pragma unroll
+    for (int i = 0; i < SC_STRIP + TAPS - 1; ++i) {
+        const int row = row0 - (TAPS - 1) + i;
+        in[i] = row >= 0 && row < n ? x[(size_t)row * ldx + ch] : 0.f;
+    }
+    float tap[TAPS];
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) tap[j] = w[(size_t)ch * TAPS + j];
+#pragma unroll
+    for (int t = 0; t < SC_STRIP; ++t) {
+        const int row = row0 + t;
+        if (row >= n || positions[row] < 0) continue;
+        const int seq = row_seq[row], r0 = seq_first_row[seq], slot = seq_slots[seq];
+        if (slot < 0 || slot >= num_slots) {
+            atomicOr(status, GB_STATUS_BAD_SLOT);
+            continue;
+        }
+        const float* st = state + (size_t)slot * state_stride + state_off;
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const int src = row - (TAPS - 1) + j;
+            const float v = src >= r0 ? in[t + j] : st[(size_t)(TAPS - 1 - (r0 - src)) * C + ch];
+            acc = fmaf(tap[j], v, acc);
+        }
+        y[(size_t)row * ldy + ch] = acc / (1.0f + expf(-acc));
+    }
+}
+
 // One thread per (sequence, channel): shift what the slot holds by the portion's length and append the portion's last inputs.
 __global__ void __launch_bounds__(256) short_conv_state_kernel(const float* __restrict__ x, long long ldx, float* __restrict__ state,
                                                                long long state_stride, long long state_off,
@@ -78,9 +125,19 @@ GB_EXPORT int gb_short_conv(const float* x, long long ldx, const float* w, float
                             int num_slots, int update_state, int* status, cudaStream_t stream) {
     GB_REQUIRE(n >= 0 && S >= 0 && C > 0 && taps >= 1 && taps <= 64, "gb_short_conv: bad sizes (taps %d)", taps);
     if (n == 0 || S == 0) return 0;
-    dim3 grid(n, gb_ceil_div(C, 256));
-    gb_launch(GB_PDL_ELEMENTWISE, short_conv_kernel, grid, dim3(256), 0, stream, x, ldx, w, y, ldy, (const float*)state, state_stride,
-              state_off, row_seq, positions, seq_first_row, seq_slots, n, C, taps, num_slots, status);
+    // strips only where they fill the chip (half a block of 256 channels an SM or more) and for the taps they are built for
+    const dim3 strips(gb_ceil_div(n, SC_STRIP), gb_ceil_div(C, 256)), grid(n, gb_ceil_div(C, 256));
+#define SC_STRIPS(TAPS)                                                                                                            \
+    gb_launch(GB_PDL_ELEMENTWISE, short_conv_strip_kernel<TAPS>, strips, dim3(256), 0, stream, x, ldx, w, y, ldy, (const float*)state, \
+              state_stride, state_off, row_seq, positions, seq_first_row, seq_slots, n, C, num_slots, status)
+    const bool many = (long long)strips.x * strips.y >= 74;
+    if (many && taps == 4) SC_STRIPS(4);
+    else if (many && taps == 3) SC_STRIPS(3);
+    else if (many && taps == 2) SC_STRIPS(2);
+    else
+        gb_launch(GB_PDL_ELEMENTWISE, short_conv_kernel, grid, dim3(256), 0, stream, x, ldx, w, y, ldy, (const float*)state, state_stride,
+                  state_off, row_seq, positions, seq_first_row, seq_slots, n, C, taps, num_slots, status);
+#undef SC_STRIPS
     int rc = gb_check_launch("gb_short_conv");
     if (rc || !update_state || taps == 1) return rc;
     dim3 grid2(S, gb_ceil_div(C, 256));

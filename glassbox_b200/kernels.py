@@ -122,6 +122,9 @@ _SIGNATURES = {
     "gb_talk_combine": [_P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _P],
     "gb_short_conv": [_P, _LL, _P, _P, _LL, _P, _LL, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "gb_channel_delta": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P],
+    "gb_channel_delta_chunks": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P],
+    "gb_delta_chunk_rows": [],
+    "gb_delta_chunk_floats": [],
     "gb_channel_delta_decode_supported": [_I, _I],
     "gb_channel_delta_decode": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _LL, _P, _F, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I,
                                 _I, _I, _P, _P, _LL, _P, _LL, _I, _I, _I, _I, _P, _P, _I, _I, _I, _P],
@@ -1436,6 +1439,53 @@ def channel_delta(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bia
     _call("gb_channel_delta", _ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(a), a.stride(0), _ptr(dt_bias),
           _ptr(a_log), _ptr(state), state.stride(0), _ptr(out), _ptr(seq_first_row), _ptr(seq_start_pos), _ptr(seq_slots),
           seq_start_pos.shape[0], heads, kv_heads, dk, dv, state.shape[0], 1 if write_state else 0, _ptr(status), dc, 0, _stream())
+
+
+#: from how many rows of the longest portion on the delta rule runs in chunks of tokens instead of token by token, and how
+#: many rows more for every further request of the step
+DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 80, 8
+
+
+def delta_chunks_chosen(longest: int, num_seqs: int, dk: int) -> bool:
+    """Whether the delta rule takes a step of ``num_seqs`` requests, of which the longest brings ``longest`` rows, in chunks of 32
+    tokens (key sizes up to 128). The walk's time is its longest portion's; the chunks cost a further request more (its state
+    goes through shared memory). Whole mixer at 8 heads x 128 x 128, chunks / walk: one request of 48 rows 64 / 59 us, 64 rows
+    68 / 68, 96 rows 78 / 84, 256 rows 101 / 144; 36 requests of which the longest brings 19 rows 154 / 133; at 16 heads 88 / 83,
+    94 / 92, 100 / 108, 123 / 167 and 306 / 234."""
+    return dk <= 128 and longest >= DELTA_CHUNKS_FROM + DELTA_CHUNKS_PER_REQUEST * (num_seqs - 1)
+
+
+def delta_chunks_needed(n: int, num_seqs: int) -> int:
+    """How many chunks ``channel_delta_chunks`` may need for a step of ``n`` rows in ``num_seqs`` sequences."""
+    return n // lib().gb_delta_chunk_rows() + num_seqs
+
+
+def delta_chunk_floats() -> int:
+    return lib().gb_delta_chunk_floats()
+
+
+def channel_delta_chunks(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
+                         state: torch.Tensor, out: torch.Tensor, seq_first_row: torch.Tensor, seq_start_pos: torch.Tensor,
+                         seq_slots: torch.Tensor, max_rows_per_seq: int, heads: int, kv_heads: int, dk: int, dv: int, write_state: bool,
+                         status: torch.Tensor, workspace: torch.Tensor, decay_per_head: bool = False) -> None:
+    """``channel_delta`` with the tokens of a request taken 32 at a time (the same sums in another order, float32
+    throughout). ``workspace`` float32 [chunks, heads * delta_chunk_floats()] is scratch, chunks = ``delta_chunks_needed``;
+    no request may bring more than ``max_rows_per_seq`` rows."""
+    _cuda(qkv, beta, a, dt_bias, a_log, state, out, seq_first_row, seq_start_pos, seq_slots, status, workspace)
+    n, S = qkv.shape[0], seq_start_pos.shape[0]
+    dc = 1 if decay_per_head else dk
+    for t in (qkv, beta, a, dt_bias, a_log, state, out, workspace):
+        assert t.dtype == torch.float32
+    assert qkv.shape[1] == 2 * kv_heads * dk + heads * dv and qkv.stride(1) == 1 and beta.shape == (n, heads)
+    assert a.shape == (n, heads * dc) and a.stride(1) == 1 and beta.stride(1) == 1 and out.shape == (n, heads * dv)
+    assert out.is_contiguous() and state.dim() == 2 and state.is_contiguous() and state.shape[1] >= heads * dk * dv
+    assert dt_bias.numel() == heads * dc and a_log.numel() == heads
+    assert workspace.is_contiguous() and workspace.numel() >= delta_chunks_needed(n, S) * heads * delta_chunk_floats()
+    _call("gb_channel_delta_chunks", _ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(a), a.stride(0), _ptr(dt_bias),
+          _ptr(a_log), _ptr(state), state.stride(0), _ptr(out), _ptr(seq_first_row), _ptr(seq_start_pos), _ptr(seq_slots), S,
+          int(max_rows_per_seq), heads, kv_heads, dk, dv, state.shape[0], 1 if write_state else 0, _ptr(status), dc, _ptr(workspace), _stream())
+    global launch_count
+    launch_count += 1
 
 
 CD_SILU_INPUTS, CD_PLAIN, CD_GATE_SILU, CD_NO_NORM = 1, 2, 4, 8

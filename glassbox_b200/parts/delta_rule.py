@@ -24,6 +24,19 @@ from .base import Mixer, StateSpec, register_part
 from .linear import linear
 
 
+def run_delta(ctx, qkv, beta, decay, params, state, out, heads: int, kv_heads: int, dk: int, dv: int, writes_cache: bool,
+              decay_per_head: bool = False) -> None:
+    """The recurrence over the step's runs of rows: in chunks of tokens where a portion is long enough, else token by token."""
+    args = (qkv, beta, decay, params["dt_bias"], params["a_log"], state, out, ctx.seq_first_row, ctx.seq_start_pos, ctx.seq_slots)
+    if not kernels.delta_chunks_chosen(ctx.max_rows_per_seq, ctx.seq_start_pos.shape[0], dk):
+        kernels.channel_delta(*args, heads, kv_heads, dk, dv, writes_cache, ctx.status, decay_per_head=decay_per_head)
+        return
+    chunks = kernels.delta_chunks_needed(qkv.shape[0], ctx.seq_start_pos.shape[0])
+    work = ctx.scratch("delta_chunks", (chunks, heads * kernels.delta_chunk_floats()), torch.float32, grow=True)
+    kernels.channel_delta_chunks(*args, ctx.max_rows_per_seq, heads, kv_heads, dk, dv, writes_cache, ctx.status, work,
+                                 decay_per_head=decay_per_head)
+
+
 #: With few requests a decode step is a chain of short kernels and every launch saved counts: the fused form (three
 #: launches fewer per layer) wins. With many, every block of the fused form reads its head's slice of the two low-rank
 #: matrices again, half as many bytes as S itself, and the products done once for all rows win. Measured, ms per step
@@ -114,8 +127,7 @@ class ChannelDelta(Mixer):
                                              ctx.seq_slots, self.H, self.KH, self.dk, self.dv, writes_cache, ctx.status)
             else:
                 o = ctx.scratch("delta_o", (n, self.v_cols), f32)
-                kernels.channel_delta(qkv, beta, decay, self.params["dt_bias"], self.params["a_log"], state, o, ctx.seq_first_row,
-                                      ctx.seq_start_pos, ctx.seq_slots, self.H, self.KH, self.dk, self.dv, writes_cache, ctx.status)
+                run_delta(ctx, qkv, beta, decay, self.params, state, o, self.H, self.KH, self.dk, self.dv, writes_cache)
                 kernels.gated_head_norm(o, gate, self.params["out_norm"], att, self.H, s.norm_eps)
         linear(ctx, att, self.params["wo"], residual, accumulate=not getattr(ctx, "overwrite_output", False))
 
@@ -194,8 +206,7 @@ class HeadDelta(Mixer):
                                          writes_cache, ctx.status, decay_per_head=True, gate_silu=silu)
         else:
             o = ctx.scratch("delta_o", (n, self.v_cols), f32)
-            kernels.channel_delta(qkv, beta, decay, p["dt_bias"], p["a_log"], state, o, ctx.seq_first_row, ctx.seq_start_pos,
-                                  ctx.seq_slots, self.H, self.KH, self.dk, self.dv, writes_cache, ctx.status, decay_per_head=True)
+            run_delta(ctx, qkv, beta, decay, p, state, o, self.H, self.KH, self.dk, self.dv, writes_cache, decay_per_head=True)
             kernels.gated_head_norm(o, gate, p["out_norm"], att, self.H, s.norm_eps, gate_silu=silu)
         linear(ctx, att, p["wo"], residual, accumulate=not getattr(ctx, "overwrite_output", False))
 

@@ -1,0 +1,100 @@
+"""The delta rule in chunks of tokens against the recurrence in float64, and its error beside that of the walk token by token."""
+import numpy as np
+import pytest
+import torch
+
+from plain import zurerax_plain as plain
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _inputs(lens, H, KH, D, V, per_head, seed):
+    rng = np.random.default_rng(seed)
+    n, dc = sum(lens), 1 if per_head else D
+    qkv = rng.standard_normal((n, 2 * KH * D + H * V))
+    beta, a = 2 * rng.standard_normal((n, H)), 2 * rng.standard_normal((n, H * dc))
+    # decays from next to none to more than a float32 can hold over a chunk
+    dt_bias, a_log = rng.uniform(-6, 1, H * dc), rng.uniform(-3, 3, H)
+    states = rng.standard_normal((len(lens), H, D, V))
+    return [np.float32(x) for x in (qkv, beta, a, dt_bias, a_log, states)]
+
+
+def _truth(lens, H, KH, D, V, per_head, qkv, beta, a, dt_bias, a_log, states):
+    outs, after, row = [], [], 0
+    for s, n in enumerate(lens):
+        x = qkv[row:row + n].astype(np.float64)
+        q, k = x[:, :KH * D].reshape(n, KH, D), x[:, KH * D:2 * KH * D].reshape(n, KH, D)
+        q = q / np.sqrt((q * q).sum(-1, keepdims=True) + 1e-6) * D ** -0.5
+        k = k / np.sqrt((k * k).sum(-1, keepdims=True) + 1e-6)
+        q, k = np.repeat(q, H // KH, 1), np.repeat(k, H // KH, 1)
+        z = plain.softplus(a[row:row + n].astype(np.float64) + dt_bias).reshape(n, H, -1)
+        g = np.broadcast_to(np.exp(-np.exp(a_log.astype(np.float64))[None, :, None] * z), (n, H, D))
+        b = plain.sigmoid(beta[row:row + n].astype(np.float64))
+        v = x[:, 2 * KH * D:].reshape(n, H, V)
+        S, o = states[s].astype(np.float64), np.zeros((n, H, V))
+        for t in range(n):
+            S = g[t][:, :, None] * S
+            u = b[t][:, None] * (v[t] - np.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            o[t] = np.einsum("hdv,hd->hv", S, q[t])
+        outs.append(o.reshape(n, H * V))
+        after.append(S)
+        row += n
+    return np.concatenate(outs), np.stack(after)
+
+
+def _run(chunked, lens, H, KH, D, V, per_head, qkv, beta, a, dt_bias, a_log, states, padding=False):
+    """Requests in slots in reverse order; with ``padding`` a padding sequence of two rows in front."""
+    from glassbox_b200 import kernels
+    f = lambda x: torch.tensor(x.copy(), dtype=torch.float32, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    S, lead = len(lens), [2] if padding else []
+    state = torch.full((S + 1, H * D * V + 3), 3.0, device=DEV)
+    state[:S, :H * D * V] = f(states[::-1]).reshape(S, -1)
+    rows = lead + list(lens)
+    pad = lambda x: f(np.concatenate([np.full((sum(lead), x.shape[1]), np.nan, np.float32), x])) if padding else f(x)
+    first = i32([0] + list(np.cumsum(rows)))
+    start = i32(([-1] if padding else []) + [0] * S)
+    slots = i32(([0] if padding else []) + list(range(S - 1, -1, -1)))
+    out = torch.zeros((sum(rows), H * V), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    args = (pad(qkv), pad(beta), pad(a), f(dt_bias), f(a_log), state, out, first, start, slots)
+    if chunked:
+        work = torch.full((kernels.delta_chunks_needed(sum(rows), len(rows)), H * kernels.delta_chunk_floats()), float("nan"), device=DEV)
+        kernels.channel_delta_chunks(*args, max(rows), H, KH, D, V, True, status, work, decay_per_head=per_head)
+    else:
+        kernels.channel_delta(*args, H, KH, D, V, True, status, decay_per_head=per_head)
+    assert int(status) == 0 and torch.all(state[S] == 3.0) and torch.all(state[:, H * D * V:] == 3.0)
+    assert torch.all(out[:sum(lead)] == 0)
+    return out[sum(lead):].double().cpu().numpy(), state[:S, :H * D * V].reshape(S, H, D, V).double().cpu().numpy()[::-1]
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("H, KH, D, V, lens", [(2, 1, 128, 128, [31, 32, 33, 1, 96]), (1, 1, 64, 20, [100, 65]), (4, 2, 40, 9, [7, 200])])
+def test_chunks_against_the_recurrence(H, KH, D, V, lens, per_head):
+    data = _inputs(lens, H, KH, D, V, per_head, D + V)
+    want = _truth(lens, H, KH, D, V, per_head, *data)
+    for got in (_run(True, lens, H, KH, D, V, per_head, *data), _run(True, lens, H, KH, D, V, per_head, *data, padding=True)):
+        for g, w in zip(got, want):
+            # sums of up to 128 products of unit vectors with entries near one: 1e-5 is some 80 roundings
+            np.testing.assert_allclose(g, w, atol=1e-5 * max(1.0, np.abs(w).max()), rtol=1e-5)
+
+
+def test_chunks_are_as_exact_as_the_walk():
+    lens, H, KH, D, V = [700], 2, 2, 128, 128
+    data = _inputs(lens, H, KH, D, V, False, 5)
+    want = _truth(lens, H, KH, D, V, False, *data)
+    rel = lambda got: [np.linalg.norm(g - w) / np.linalg.norm(w) for g, w in zip(got, want)]
+    walk, chunks = rel(_run(False, lens, H, KH, D, V, False, *data)), rel(_run(True, lens, H, KH, D, V, False, *data))
+    assert all(c <= 1.2 * w + 1e-7 for c, w in zip(chunks, walk)), (chunks, walk)
+
+
+def test_a_token_does_not_reach_the_ones_before_it():
+    lens, H, KH, D, V = [80], 1, 1, 128, 16
+    data = _inputs(lens, H, KH, D, V, False, 6)
+    clean, _ = _run(True, lens, H, KH, D, V, False, *data)
+    data[0][45] = np.inf
+    data[1][45] = np.nan
+    spoiled, _ = _run(True, lens, H, KH, D, V, False, *data)
+    assert np.array_equal(clean[:45], spoiled[:45]) and not np.isfinite(spoiled[45:]).any()
