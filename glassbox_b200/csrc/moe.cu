@@ -167,18 +167,88 @@ __global__ void __launch_bounds__(RB > 1 ? MOE_ROUTE_THREADS / 2 : MOE_ROUTE_THR
     gb_pdl_wait();
     const int row0 = blockIdx.x * RB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5);
-    bool any = false;
+    int pos[RB];                                // every row's position asked for before the first is used
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-        const int row = row0 + r;
-        const bool live = row < n && positions[row] >= 0;
-        any = any || live;
-        const T* src = h + (size_t)(live ? row : 0) * d;
-        for (int i = threadIdx.x; i < d; i += blockDim.x) hx[r * ldh + i] = live ? gb_to_float(src[i]) : 0.f;
+    for (int r = 0; r < RB; ++r) pos[r] = row0 + r < n ? positions[row0 + r] : -1;
+    unsigned live = 0;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) live |= (pos[r] >= 0 ? 1u : 0u) << r;
+    if (!live) return;
+    constexpr int PIECE = 16 / sizeof(T);
+    if (RB > 1 && d % PIECE == 0 && ((uintptr_t)h & 15) == 0) {
+        // 16 bytes a load, four of them in flight (one number a load and a row after the other: 37 us for 2,048 rows of 1,024 and
+        // 16 experts, now 21)
+        const int per_row = d / PIECE, total = RB * per_row;
+        for (int i0 = threadIdx.x; i0 < total; i0 += 4 * blockDim.x) {
+            uint4 raw[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * blockDim.x, r = i / per_row;
+                raw[u] = i < total && (live >> r & 1) ? *reinterpret_cast<const uint4*>(h + (size_t)(row0 + r) * d + (i % per_row) * PIECE)
+                                                      : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * blockDim.x;
+                if (i >= total) break;
+                const T* v = reinterpret_cast<const T*>(&raw[u]);
+                float* dst = hx + (i / per_row) * ldh + (i % per_row) * PIECE;
+#pragma unroll
+                for (int c = 0; c < PIECE; c += 4)
+                    *reinterpret_cast<float4*>(dst + c) = make_float4(gb_to_float(v[c]), gb_to_float(v[c + 1]), gb_to_float(v[c + 2]), gb_to_float(v[c + 3]));
+            }
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            const bool on = live >> r & 1;
+            const T* src = h + (size_t)(on ? row0 + r : 0) * d;
+            for (int i = threadIdx.x; i < d; i += blockDim.x) hx[r * ldh + i] = on ? gb_to_float(src[i]) : 0.f;
+        }
     }
-    if (!any) return;
     __syncthreads();
-    for (int e = warp; e < E + (w_gate ? 1 : 0); e += warps) {
+    auto settle = [&](int e, const float (&acc)[RB]) {      // a logit per row, or the shared gate's
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            const float z = gb_warp_sum(acc[r]);
+            const int row = row0 + r;
+            if (lane == 0 && (live >> r & 1)) {
+                const float sg = moe_sigmoid(z);
+                if (e < E && scoring != MOE_SIGMOID) {
+                    score[r][e] = choice[r][e] = z + (router_bias ? router_bias[e] : 0.f);
+                } else if (e < E) {
+                    score[r][e] = sg;
+                    choice[r][e] = sg + (correction ? correction[e] : 0.f);
+                } else {
+                    gate_out[row] = sg;
+                }
+            }
+        }
+    };
+    int e_from = 0;
+    if (RB > 1 && d % 4 == 0 && ((uintptr_t)w_router & 15) == 0) {
+        // two experts a warp: the rows come out of shared memory half as often
+        for (int e = 2 * warp; e + 1 < E; e += 2 * warps) {
+            const float* w0 = w_router + (size_t)e * d;
+            float a0[RB], a1[RB];
+#pragma unroll
+            for (int r = 0; r < RB; ++r) a0[r] = a1[r] = 0.f;
+#pragma unroll 4
+            for (int i = lane * 4; i < d; i += 128) {
+                const float4 v = *reinterpret_cast<const float4*>(w0 + i), u = *reinterpret_cast<const float4*>(w0 + d + i);
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    const float4 x = *reinterpret_cast<const float4*>(hx + r * ldh + i);
+                    a0[r] = fmaf(v.x, x.x, a0[r]); a0[r] = fmaf(v.y, x.y, a0[r]); a0[r] = fmaf(v.z, x.z, a0[r]); a0[r] = fmaf(v.w, x.w, a0[r]);
+                    a1[r] = fmaf(u.x, x.x, a1[r]); a1[r] = fmaf(u.y, x.y, a1[r]); a1[r] = fmaf(u.z, x.z, a1[r]); a1[r] = fmaf(u.w, x.w, a1[r]);
+                }
+            }
+            settle(e, a0);
+            settle(e + 1, a1);
+        }
+        e_from = E & ~1;
+    }
+    for (int e = e_from + warp; e < E + (w_gate ? 1 : 0); e += warps) {
         const float* wrow = e < E ? w_router + (size_t)e * d : w_gate;
         float acc[RB];
 #pragma unroll
@@ -201,27 +271,12 @@ __global__ void __launch_bounds__(RB > 1 ? MOE_ROUTE_THREADS / 2 : MOE_ROUTE_THR
                 for (int r = 0; r < RB; ++r) acc[r] = fmaf(v, hx[r * ldh + i], acc[r]);
             }
         }
-#pragma unroll
-        for (int r = 0; r < RB; ++r) {
-            const float z = gb_warp_sum(acc[r]);
-            const int row = row0 + r;
-            if (lane == 0 && row < n && positions[row] >= 0) {
-                const float sg = moe_sigmoid(z);
-                if (e < E && scoring != MOE_SIGMOID) {
-                    score[r][e] = choice[r][e] = z + (router_bias ? router_bias[e] : 0.f);
-                } else if (e < E) {
-                    score[r][e] = sg;
-                    choice[r][e] = sg + (correction ? correction[e] : 0.f);
-                } else {
-                    gate_out[row] = sg;
-                }
-            }
-        }
+        settle(e, acc);
     }
     __syncthreads();
     for (int r = warp; r < RB; r += warps) {
         const int row = row0 + r;
-        if (row < n && positions[row] >= 0) {
+        if (live >> r & 1) {
             if (scoring == MOE_SOFTMAX) {        // the row's logits become its softmax over all experts, by this row's warp
                 float m = -INFINITY, sum = 0.f;
                 for (int e = lane; e < E; e += 32) m = fmaxf(m, score[r][e]);
@@ -244,7 +299,7 @@ static void moe_route_launch(const void* h, int d, const float* w_router, const 
                              float* weight_out, float* gate_out, const float* router_bias, int scoring, int run_best, float renorm_eps,
                              cudaStream_t stream) {
     const size_t smem = (size_t)RB * ((d + 3) & ~3) * 4;
-    int warps = E + (w_gate ? 1 : 0);
+    int warps = RB > 1 ? (E + 1) / 2 : E + (w_gate ? 1 : 0);
     const int most = (RB > 1 ? MOE_ROUTE_THREADS / 2 : MOE_ROUTE_THREADS) / 32, least = RB > 4 ? RB : 4;
     warps = warps < least ? least : (warps > most ? most : warps);
     if (smem > 32 * 1024) cudaFuncSetAttribute(moe_route_kernel<T, RB, EMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -350,12 +405,40 @@ GB_EXPORT int gb_moe_expert_rows(const void* h, int dtype, int d, const void* w_
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ pair, const float* __restrict__ weight, int top,
                                                           const float* __restrict__ shared, long long lds, const float* __restrict__ gate,
                                                           const int* __restrict__ positions, float* __restrict__ out, long long ldo,
-                                                          int n, int d, int accumulate) {
+                                                          int n, int d, int accumulate, int vec) {
     gb_pdl_launch_dependents();
     gb_pdl_wait();
     const int row = blockIdx.x;
     if (row >= n || positions[row] < 0) return;
     const float g = gate ? gate[row] : 1.f;
+    if (vec) {         // four columns a thread, four choices' loads in flight (8,192 pairs of 1,024: 15 -> 7.5 us)
+        for (int j = threadIdx.x * 4; j < d; j += blockDim.x * 4) {
+            const float* src = pair + (size_t)row * top * d + j;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4* o = reinterpret_cast<float4*>(out + (size_t)row * ldo + j);
+            const float4 old = accumulate ? *o : a, s = shared ? *reinterpret_cast<const float4*>(shared + (size_t)row * lds + j) : a;
+            for (int k0 = 0; k0 < top; k0 += 4) {
+                float4 v[4];
+                float w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k0 + k < top) {
+                        v[k] = *reinterpret_cast<const float4*>(src + (size_t)(k0 + k) * d);
+                        w[k] = weight[(size_t)row * top + k0 + k];
+                    }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k0 + k < top) {
+                        a.x = fmaf(w[k], v[k].x, a.x); a.y = fmaf(w[k], v[k].y, a.y);
+                        a.z = fmaf(w[k], v[k].z, a.z); a.w = fmaf(w[k], v[k].w, a.w);
+                    }
+            }
+            if (shared) { a.x = fmaf(g, s.x, a.x); a.y = fmaf(g, s.y, a.y); a.z = fmaf(g, s.z, a.z); a.w = fmaf(g, s.w, a.w); }
+            if (accumulate) { a.x = old.x + a.x; a.y = old.y + a.y; a.z = old.z + a.z; a.w = old.w + a.w; }
+            *o = a;
+        }
+        return;
+    }
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
         float a = 0.f;
         for (int k = 0; k < top; ++k) a = fmaf(weight[(size_t)row * top + k], pair[((size_t)row * top + k) * d + j], a);
@@ -369,8 +452,9 @@ GB_EXPORT int gb_moe_combine(const float* pair, const float* weight, int top, co
                              const int* positions, float* out, long long ldo, int n, int d, int accumulate, cudaStream_t stream) {
     GB_REQUIRE(n >= 0 && d > 0 && top > 0, "gb_moe_combine: bad sizes");
     if (n == 0) return 0;
+    const bool vec = d % 4 == 0 && ldo % 4 == 0 && lds % 4 == 0 && (((uintptr_t)pair | (uintptr_t)out | (uintptr_t)shared) & 15) == 0;
     gb_launch(GB_PDL_ELEMENTWISE, moe_combine_kernel, dim3(n), dim3(256), 0, stream, pair, weight, top, shared, lds, gate, positions, out,
-              ldo, n, d, accumulate);
+              ldo, n, d, accumulate, vec ? 1 : 0);
     return gb_check_launch("gb_moe_combine");
 }
 
@@ -453,214 +537,67 @@ GB_EXPORT int gb_moe_expert_halves(const void* h, int dtype, int d, const void* 
 
 // ----------------------------------------------------------------------------------------------
 // Many rows (prompt portions, large batches), bfloat16: the (row, choice) pairs are sorted by expert, and the experts'
-// products run as ONE grouped product per half on the tensor cores.
-//   moe_sort            one block: counts per expert, where each expert's pairs start (offsets [E + 1]), where its 64-row
-//                       tiles start (tile_start [E + 1]), and sorted[slot] = pair. The order of an expert's pairs is not
-//                       fixed from run to run; no result depends on it (a pair's numbers do not depend on its slot).
-//   moe_grouped_gemm    a block = 64 slots of one expert x 128 outputs, 8 warps of mma.sync m16n8k16 (bf16, float32 sums),
-//                       operands staged by cp.async in a ring of three buffers of 64 columns. UP: rows of h gathered by pair, epilogue relu^2, act
-//                       [slot, ff] bfloat16. DOWN: rows of act, float32 out scattered to pair[pair, :].
+// products run as one grouped product per half on the tensor cores (moe_tcgen05.cu).
+//   moe_sort            one block: counts per expert, where each expert's pairs start (offsets [E + 1]) and sorted[slot] = pair.
+//                       The order of an expert's pairs is not fixed from run to run; no result depends on it (a pair's
+//                       numbers do not depend on its slot).
+// A thread keeps up to 16 pairs' experts in registers, asked for together: the two passes over the pairs cost one trip to
+// memory between them.
 // ----------------------------------------------------------------------------------------------
-constexpr int MG_BM = 64, MG_BN = 128, MG_BK = 64, MG_STAGES = 3;
-constexpr int MG_LD = MG_BK + 8;             // (rows padded by 16 bytes: ldmatrix meets no bank twice)
-constexpr int MG_SMEM = MG_STAGES * (MG_BM + MG_BN) * MG_LD * 2;
-constexpr int MG_THREADS = 256;
+constexpr int MS_THREADS = 1024, MS_KEEP = 16;
 
-__global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ choice, const int* __restrict__ positions, int n, int E,
-                                                        int top, int* __restrict__ offsets, int* __restrict__ tile_start,
-                                                        int* __restrict__ sorted) {
+__global__ void __launch_bounds__(MS_THREADS) moe_sort_kernel(const int* __restrict__ choice, const int* __restrict__ positions, int n, int E,
+                                                              int top, int* __restrict__ offsets, int* __restrict__ sorted) {
     __shared__ int count[MOE_MAX_EXPERTS], cursor[MOE_MAX_EXPERTS];
     gb_pdl_launch_dependents();
     gb_pdl_wait();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
-    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += MS_THREADS) count[e] = 0;
     const int pairs = n * top;
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+    auto expert_of = [&](int p) {
+        if (p >= pairs) return -1;
         const int e = positions[p / top] >= 0 ? choice[p] : -1;
-        if (e >= 0 && e < E) atomicAdd(&count[e], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0, tiles = 0;
-        for (int e = 0; e < E; ++e) {
-            offsets[e] = at;
-            tile_start[e] = tiles;
-            cursor[e] = at;
-            at += count[e];
-            tiles += (count[e] + MG_BM - 1) / MG_BM;
-        }
-        offsets[E] = at;
-        tile_start[E] = tiles;
-    }
-    __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int e = positions[p / top] >= 0 ? choice[p] : -1;
-        if (e >= 0 && e < E) sorted[atomicAdd(&cursor[e], 1)] = p;
-    }
-}
-
-__device__ __forceinline__ void mg_cp_async16(void* smem, const void* gmem, bool valid) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    const int bytes = valid ? 16 : 0;        // 0: the 16 bytes are filled with zeros, nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes));
-}
-
-template <bool UP>
-__global__ void __launch_bounds__(MG_THREADS) moe_grouped_gemm_kernel(const __nv_bfloat16* __restrict__ A, long long lda,
-                                                               const __nv_bfloat16* __restrict__ W, int N, int K,
-                                                               const int* __restrict__ sorted, const int* __restrict__ offsets,
-                                                               const int* __restrict__ tile_start, int E, int top,
-                                                               void* __restrict__ C, long long ldc, int unit, float limit,
-                                                               float slope) {
-    extern __shared__ __align__(16) unsigned char mg_smem[];
-    __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(mg_smem);                 // [stages][BM][LD]
-    __nv_bfloat16* sb = sa + MG_STAGES * MG_BM * MG_LD;                            // [stages][BN][LD]
-    __shared__ int src_row[MG_BM];           // where each slot's input row is (UP: the token's row; DOWN: the slot), -1: none
-    __shared__ int dst_row[MG_BM];           // where its output goes (UP: the slot; DOWN: the pair)
-    gb_pdl_launch_dependents();
-    gb_pdl_wait();
-    const int tile = blockIdx.x;
-    if (tile >= tile_start[E]) return;
-    int lo = 0, hi = E;                      // the expert whose tiles hold this one: the last e with tile_start[e] <= tile
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (tile_start[mid] <= tile) lo = mid; else hi = mid;
-    }
-    const int e = lo;
-    const int m0 = offsets[e] + (tile - tile_start[e]) * MG_BM, m_end = offsets[e + 1];
-    const int n0 = blockIdx.y * MG_BN;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid < MG_BM) {
-        const int slot = m0 + tid;
-        const bool live = slot < m_end;
-        const int pair = live ? sorted[slot] : -1;
-        src_row[tid] = !live ? -1 : (UP ? pair / top : slot);
-        dst_row[tid] = !live ? -1 : (UP ? slot : pair);
-    }
-    __syncthreads();
-    const __nv_bfloat16* Wb = W + (size_t)e * N * K;
-    const int steps = (K + MG_BK - 1) / MG_BK;
-    // staging: rows of BK = 64 columns are 8 chunks of 16 bytes; 256 threads take 2 chunks of A and 4 of W each
-    auto stage = [&](int st) {
-        if (st < steps) {
-            const int buf = st % MG_STAGES, k0 = st * MG_BK;
-#pragma unroll
-            for (int i = 0; i < (MG_BM * 8) / MG_THREADS; ++i) {
-                const int chunk = tid + i * MG_THREADS, r = chunk >> 3, c = (chunk & 7) * 8;
-                const int ar = src_row[r];
-                const bool ka = k0 + c < K;
-                mg_cp_async16(sa + (buf * MG_BM + r) * MG_LD + c, A + (size_t)(ar < 0 ? 0 : ar) * lda + (ka ? k0 + c : 0), ar >= 0 && ka);
-            }
-#pragma unroll
-            for (int i = 0; i < (MG_BN * 8) / MG_THREADS; ++i) {
-                const int chunk = tid + i * MG_THREADS, r = chunk >> 3, c = (chunk & 7) * 8;
-                const int br = n0 + r;
-                const bool ka = k0 + c < K;
-                mg_cp_async16(sb + (buf * MG_BN + r) * MG_LD + c, Wb + (size_t)(br < N ? br : 0) * K + (ka ? k0 + c : 0), br < N && ka);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");      // (a group per round, empty past the end: the count stays in step)
+        return e >= 0 && e < E ? e : -1;
     };
-    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 32;       // this warp's 32 x 32 piece of the tile (8 warps: 2 x 4)
-    float acc[2][4][4];
+    int own[MS_KEEP];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < MS_KEEP; ++i) own[i] = expert_of(threadIdx.x + i * MS_THREADS);
+    __syncthreads();
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int t = 0; t < 4; ++t) acc[i][j][t] = 0.f;
-#pragma unroll
-    for (int st = 0; st < MG_STAGES - 1; ++st) stage(st);
-    for (int s = 0; s < steps; ++s) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(MG_STAGES - 2) : "memory");
-        __syncthreads();                     // round s has landed for everyone, and everyone is done with round s - 1's buffer
-        stage(s + MG_STAGES - 1);
-        const __nv_bfloat16* ta = sa + (s % MG_STAGES) * MG_BM * MG_LD;
-        const __nv_bfloat16* tb = sb + (s % MG_STAGES) * MG_BN * MG_LD;
-#pragma unroll
-        for (int kk = 0; kk < MG_BK; kk += 16) {
-            unsigned a[2][4], b[4][2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const unsigned addr = (unsigned)__cvta_generic_to_shared(ta + (wm + i * 16 + (lane & 15)) * MG_LD + kk + (lane >> 4) * 8);
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(a[i][0]), "=r"(a[i][1]), "=r"(a[i][2]), "=r"(a[i][3]) : "r"(addr));
-            }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {      // two 8-column tiles of W per ldmatrix.x4: rows n, columns k
-                const int nrow = wn + j * 16 + (lane & 7) + ((lane >> 4) << 3), kcol = kk + ((lane >> 3) & 1) * 8;
-                const unsigned addr = (unsigned)__cvta_generic_to_shared(tb + nrow * MG_LD + kcol);
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(b[2 * j][0]), "=r"(b[2 * j][1]), "=r"(b[2 * j + 1][0]), "=r"(b[2 * j + 1][1]) : "r"(addr));
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                                 : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
-                                 : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[j][0]), "r"(b[j][1]));
-        }
+    for (int i = 0; i < MS_KEEP; ++i)
+        if (own[i] >= 0) atomicAdd(&count[own[i]], 1);
+    for (int p = threadIdx.x + MS_KEEP * MS_THREADS; p < pairs; p += MS_THREADS) {
+        const int e = expert_of(p);
+        if (e >= 0) atomicAdd(&count[e], 1);
     }
-    // epilogue: thread holds rows (lane / 4) and (lane / 4 + 8) of each 16-row tile, columns 2 * (lane % 4), + 1
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + threadIdx.x, c = e < E ? count[e] : 0;
+            int sum = c;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int r = wm + i * 16 + (lane >> 2) + half * 8;
-            const int out_row = dst_row[r];
-            if (out_row < 0) continue;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int col = n0 + wn + j * 8 + (lane & 3) * 2;
-                float v0 = acc[i][j][half * 2], v1 = acc[i][j][half * 2 + 1];
-                if (UP && unit) {
-                    // neighbouring outputs are the gate sum and the up sum of one unit: N / 2 units per row
-                    if (col + 1 < N) ((__nv_bfloat16*)C)[(size_t)out_row * ldc + (col >> 1)] = __float2bfloat16_rn(gb_gated_unit(v0, v1, limit, slope));
-                } else if (UP) {
-                    v0 = fmaxf(v0, 0.f); v0 *= v0;
-                    v1 = fmaxf(v1, 0.f); v1 *= v1;
-                    __nv_bfloat16* o = (__nv_bfloat16*)C + (size_t)out_row * ldc + col;
-                    if (col + 1 < N && (ldc & 1) == 0) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(v0, v1);
-                    else {
-                        if (col < N) o[0] = __float2bfloat16_rn(v0);
-                        if (col + 1 < N) o[1] = __float2bfloat16_rn(v1);
-                    }
-                } else {
-                    float* o = (float*)C + (size_t)out_row * ldc + col;
-                    if (col < N) o[0] = v0;
-                    if (col + 1 < N) o[1] = v1;
-                }
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                if ((int)threadIdx.x >= o) sum += v;
             }
+            if (e < E) offsets[e] = cursor[e] = before + sum - c;
+            before += __shfl_sync(0xffffffffu, sum, 31);
         }
+        if (threadIdx.x == 0) offsets[E] = before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MS_KEEP; ++i)
+        if (own[i] >= 0) sorted[atomicAdd(&cursor[own[i]], 1)] = threadIdx.x + i * MS_THREADS;
+    for (int p = threadIdx.x + MS_KEEP * MS_THREADS; p < pairs; p += MS_THREADS) {
+        const int e = expert_of(p);
+        if (e >= 0) sorted[atomicAdd(&cursor[e], 1)] = p;
+    }
 }
 
-GB_EXPORT int gb_moe_sort(const int* choice, const int* positions, int n, int E, int top, int* offsets, int* tile_start, int* sorted,
-                          cudaStream_t stream) {
+GB_EXPORT int gb_moe_sort(const int* choice, const int* positions, int n, int E, int top, int* offsets, int* sorted, cudaStream_t stream) {
     GB_REQUIRE(n >= 0 && E > 0 && E <= MOE_MAX_EXPERTS && top > 0, "gb_moe_sort: bad sizes");
     if (n == 0) return 0;
-    gb_launch(GB_PDL_ELEMENTWISE, moe_sort_kernel, dim3(1), dim3(1024), 0, stream, choice, positions, n, E, top, offsets, tile_start, sorted);
+    gb_launch(GB_PDL_ELEMENTWISE, moe_sort_kernel, dim3(1), dim3(MS_THREADS), 0, stream, choice, positions, n, E, top, offsets, sorted);
     return gb_check_launch("gb_moe_sort");
-}
-
-// 1 if the grouped tensor-core products take these sizes (rows of 16-byte pieces)
-GB_EXPORT int gb_moe_grouped_supported(int d, int ff) { return d % 8 == 0 && ff % 8 == 0 ? 1 : 0; }
-
-GB_EXPORT int gb_moe_grouped_gemm(const void* a, long long lda, const void* w, int N, int K, const int* sorted, const int* offsets,
-                                  const int* tile_start, int E, int top, int pairs, void* c, long long ldc, int up, int unit, float limit,
-                                  float slope, cudaStream_t stream) {
-    GB_REQUIRE(!unit || (up && N % 2 == 0), "gb_moe_grouped_gemm: the gated unit belongs to the up half and needs pairs of rows");
-    GB_REQUIRE(N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && pairs >= 0, "gb_moe_grouped_gemm: rows must be whole 16-byte pieces (K=%d)", K);
-    GB_REQUIRE(((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0, "gb_moe_grouped_gemm: operands must be 16-byte aligned");
-    if (pairs == 0) return 0;
-    dim3 grid(gb_ceil_div(pairs, MG_BM) + E, gb_ceil_div(N, MG_BN));      // (at most this many tiles: blocks beyond the last return)
-    cudaFuncSetAttribute(moe_grouped_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM);
-    cudaFuncSetAttribute(moe_grouped_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM);
-    if (up)
-        gb_launch(GB_PDL_GEMM, moe_grouped_gemm_kernel<true>, grid, dim3(MG_THREADS), MG_SMEM, stream, (const __nv_bfloat16*)a, lda,
-                  (const __nv_bfloat16*)w, N, K, sorted, offsets, tile_start, E, top, c, ldc, unit, limit, slope);
-    else
-        gb_launch(GB_PDL_GEMM, moe_grouped_gemm_kernel<false>, grid, dim3(MG_THREADS), MG_SMEM, stream, (const __nv_bfloat16*)a, lda,
-                  (const __nv_bfloat16*)w, N, K, sorted, offsets, tile_start, E, top, c, ldc, 0, 0.f, 0.f);
-    return gb_check_launch("gb_moe_grouped_gemm");
 }

@@ -1,0 +1,325 @@
+// The experts' products of many rows on the 5th-generation tensor cores: the (row, choice) pairs sorted by expert (moe_sort in
+// moe.cu), one persistent grouped product per half.
+//
+// A tile is 128 of an expert's pairs x BN of its outputs; a block (one per SM) walks the tiles of all experts in turn, an
+// expert's tiles next to each other and its rows innermost, so that a piece of its matrix is read from memory once and from L2
+// by the expert's other row tiles. Six warps, as in the dense product (gemm_tcgen05.cu):
+//   warp 0     producer: per 64-wide k-block a TMA box of the expert's matrix and the 128 input rows. UP: the rows of h lie
+//              anywhere (sorted[slot] / top); every lane fetches four of them by TMA gather, straight into the swizzled tile.
+//              DOWN: the rows are the slots themselves, one box.
+//   warp 1     issues tcgen05.mma (M 128, N BN, K 16) into one of two accumulators in tensor memory
+//   warps 2-5  epilogue: UP stores bfloat16 relu(c)^2, or one gated unit of every two neighbouring outputs; DOWN scatters
+//              float32 rows to pair[pair, :].
+// Rows past an expert's last pair are loaded (another row's numbers) and never stored. Bound by the tensor pipe and, with few
+// pairs per expert, by reading every expert's matrices once; the mma.sync kernel that this replaced was bound by that
+// instruction's rate and by its operands' way through registers. Measured, 2,048 rows, 16 experts, four per token
+// (1024 -> 2 x 1024 -> 1024): up half 167 -> 102 us, down half 86 -> 40 us.
+//
+// Every wait is bounded, as in the dense product: on a timeout the block records GB_STATUS_WAIT_TIMEOUT, waits (bounded) for its
+// copies, frees its tensor memory and returns. No multicast.
+#include "tcgen05.cuh"
+
+constexpr int ME_BM = 128, ME_BK = 64, ME_THREADS = 192, ME_MAX_EXPERTS = 512, ME_MAX_STAGES = 8;
+
+struct __align__(8) MeShared {
+    uint64_t full[ME_MAX_STAGES], empty[ME_MAX_STAGES], tfull[2], tempty[2];
+    uint32_t tmem_base;
+    int abort_flag, issued, consumed;
+    int row_tiles[ME_MAX_EXPERTS + 1];        // row tiles of the experts before each one
+    int offset[ME_MAX_EXPERTS + 1];           // where each expert's slots start
+};
+
+template <int BN> struct MeGeometry {
+    static constexpr int A_BYTES = ME_BM * ME_BK * 2, W_BYTES = BN * ME_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
+    static constexpr int STAGES = (192 * 1024 / STAGE_BYTES) < ME_MAX_STAGES ? (192 * 1024 / STAGE_BYTES) : ME_MAX_STAGES;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 4 * 32 * 33 * 4 + 1024;
+};
+
+// four rows of the tensor map's matrix (box: one row of 64), 128 bytes each, one behind the other
+__device__ __forceinline__ void me_gather4(void* dst, const CUtensorMap* map, uint64_t* bar, int col, int r0, int r1, int r2, int r3) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
+
+// One gated unit as gb_gated_unit forms it, with the hardware's division (two units in the last place of float32, in front of
+// a rounding to bfloat16).
+__device__ __forceinline__ float me_unit(float gate, float up, float limit, float slope) {
+    if (slope > 0.f) {
+        const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
+        return __fdividef(g, 1.0f + expf(-slope * g)) * (u + 1.0f);
+    }
+    return slope < 0.f ? gb_gelu_tanh(gate) * up : __fdividef(gate, 1.0f + expf(-gate)) * up;
+}
+
+template <int BN, bool UP>
+__global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                                                                 const int* __restrict__ sorted, const int* __restrict__ offsets, int E,
+                                                                 int top, int N, int K, void* __restrict__ C, long long ldc, int unit,
+                                                                 float limit, float slope, int* __restrict__ status) {
+    using G = MeGeometry<BN>;
+    constexpr int STAGES = G::STAGES;
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* tiles = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);      // swizzled tiles: 1024-byte aligned
+    float* epi = reinterpret_cast<float*>(tiles + STAGES * G::STAGE_BYTES);
+    __shared__ MeShared sh;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int kblocks = (K + ME_BK - 1) / ME_BK;
+    const int tiles_n = (N + BN - 1) / BN;
+
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&sh.full[s], 1);
+            mbar_init(&sh.empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&sh.tfull[b], 1);
+            mbar_init(&sh.tempty[b], 4);
+        }
+        sh.abort_flag = sh.issued = sh.consumed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(2 * BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    // every block adds up the experts' row tiles for itself (one warp, 32 experts a round)
+    if (warp == 1) {
+        int before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            const int from = offsets[e < E ? e : E], to = offsets[e < E ? e + 1 : E];
+            const int own = (to - from + ME_BM - 1) / ME_BM;
+            int sum = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += v;
+            }
+            if (e < E) {
+                sh.row_tiles[e] = before + sum - own;
+                sh.offset[e] = from;
+            }
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) {
+            sh.row_tiles[E] = before;
+            sh.offset[E] = offsets[E];
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem_base;
+    volatile int* abort_flag = &sh.abort_flag;
+    const int ntiles = sh.row_tiles[E] * tiles_n;
+
+    // a tile: its expert, its first slot, the end of the expert's slots, its first output
+    struct Place { int e, m0, m_end, n0; };
+    auto place = [&](int tile) {
+        int lo = 0, hi = E;                                       // the expert: the last e whose tiles start at or before this one
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (sh.row_tiles[mid] * tiles_n <= tile) lo = mid; else hi = mid;
+        }
+        // (an expert without pairs shares its start with the next one; the last of equals is the one that has them)
+        const int rows = sh.row_tiles[lo + 1] - sh.row_tiles[lo], t = tile - sh.row_tiles[lo] * tiles_n;
+        return Place{lo, sh.offset[lo] + (t % rows) * ME_BM, sh.offset[lo + 1], (t / rows) * BN};
+    };
+
+    if (warp == 0) {
+        int it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            const Place p = place(tile);
+            int r[4];
+            if (UP) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int slot = p.m0 + 4 * lane + i;
+                    r[i] = sorted[slot < p.m_end ? slot : p.m0] / top;        // (past the expert's pairs: any row that exists)
+                }
+            }
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const int s = it % STAGES;
+                if (it >= STAGES && !mbar_wait_warp(&sh.empty[s], ((it / STAGES) - 1) & 1, abort_flag, status)) { ok = false; break; }
+                unsigned char* a_dst = tiles + s * G::STAGE_BYTES;
+                if (lane == 0) {
+                    mbar_expect_tx(&sh.full[s], G::STAGE_BYTES);
+                    tma_load_2d(a_dst + G::A_BYTES, &map_w, &sh.full[s], kb * ME_BK, p.e * N + p.n0);
+                    if (!UP) tma_load_2d(a_dst, &map_a, &sh.full[s], kb * ME_BK, p.m0);
+                    sh.issued = it + 1;
+                }
+                __syncwarp();
+                if (UP) me_gather4(a_dst + lane * 512, &map_a, &sh.full[s], kb * ME_BK, r[0], r[1], r[2], r[3]);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = umma_idesc(ME_BM, BN);
+            int it = 0, tcount = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
+                const int acc = tcount & 1;
+                if (tcount >= 2 && !mbar_wait(&sh.tempty[acc], ((tcount >> 1) - 1) & 1, abort_flag, status)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem + (uint32_t)(acc * BN);
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (!mbar_wait(&sh.full[s], (it / STAGES) & 1, abort_flag, status)) { ok = false; break; }
+                    sh.consumed = it + 1;
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(tiles + s * G::STAGE_BYTES), w_addr = a_addr + G::A_BYTES;
+#pragma unroll
+                    for (int k = 0; k < ME_BK / 16; ++k)
+                        umma_bf16(d_tmem, umma_desc(a_addr + k * 32), umma_desc(w_addr + k * 32), idesc, (kb | k) ? 1u : 0u);
+                    umma_commit(&sh.empty[s]);
+                }
+                if (ok) umma_commit(&sh.tfull[acc]);
+            }
+        }
+    } else {
+        const int q = warp & 3;                                   // the quarter of the tensor-memory lanes this warp may read
+        float* stage = epi + q * (32 * 33);
+        int tcount = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
+            const Place p = place(tile);
+            const int acc = tcount & 1, slot = p.m0 + q * 32 + lane;
+            const bool live = slot < p.m_end;
+            const int out_row = UP ? slot : (live ? sorted[slot] : -1);
+            const int rows = min(32, p.m_end - (p.m0 + q * 32));              // (may be negative: no row of this warp is live)
+            if (!mbar_wait_warp(&sh.tfull[acc], (tcount >> 1) & 1, abort_flag, status)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t t_base = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                const int col0 = p.n0 + c0;
+                if (col0 >= N) break;                                         // (uniform for the block)
+                uint32_t v[32];
+                tmem_load32(t_base + (uint32_t)c0, v);
+                if (UP && unit) {
+                    // neighbouring outputs are the gate sum and the up sum of one unit
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)out_row * ldc + (col0 >> 1);
+                    if (live) {
+                        float u[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) u[j] = me_unit(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), limit, slope);
+                        if (col0 + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
+#pragma unroll
+                            for (int j = 0; j < 16; j += 8) {
+                                uint4 w;
+                                w.x = pack2(__float_as_uint(u[j]), __float_as_uint(u[j + 1])); w.y = pack2(__float_as_uint(u[j + 2]), __float_as_uint(u[j + 3]));
+                                w.z = pack2(__float_as_uint(u[j + 4]), __float_as_uint(u[j + 5])); w.w = pack2(__float_as_uint(u[j + 6]), __float_as_uint(u[j + 7]));
+                                *reinterpret_cast<uint4*>(dst + j) = w;
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (col0 + 2 * j + 1 < N) dst[j] = __float2bfloat16_rn(u[j]);
+                        }
+                    }
+                } else if (UP) {
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)out_row * ldc + col0;
+                    if (live) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const float g = fmaxf(__uint_as_float(v[j]), 0.f);
+                            v[j] = __float_as_uint(g * g);
+                        }
+                        if (col0 + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
+#pragma unroll
+                            for (int j = 0; j < 32; j += 8) {
+                                uint4 w;
+                                w.x = pack2(v[j], v[j + 1]); w.y = pack2(v[j + 2], v[j + 3]);
+                                w.z = pack2(v[j + 4], v[j + 5]); w.w = pack2(v[j + 6], v[j + 7]);
+                                *reinterpret_cast<uint4*>(dst + j) = w;
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (col0 + j < N) dst[j] = __float2bfloat16_rn(__uint_as_float(v[j]));
+                        }
+                    }
+                } else {
+                    // float32 through shared memory, so that one instruction writes 128 contiguous bytes of one pair's row
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(v[j]);
+                    __syncwarp();
+                    const int col = col0 + lane;
+#pragma unroll 8
+                    for (int rr = 0; rr < 32; ++rr) {
+                        const int row = __shfl_sync(0xffffffffu, out_row, rr);
+                        if (rr < rows && col < N) reinterpret_cast<float*>(C)[(size_t)row * ldc + col] = stage[rr * 33 + lane];
+                    }
+                    __syncwarp();
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.tempty[acc]);
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        if (lane == 0 && sh.abort_flag) {
+            for (int it = sh.consumed; it < sh.issued; ++it) {                // copies that nobody consumed may still be in flight
+                const long long t0 = clock64();
+                while (!mbar_try_wait(&sh.full[it % STAGES], (it / STAGES) & 1) && clock64() - t0 < TC_WAIT_CYCLES) {}
+            }
+        }
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+    }
+}
+
+template <int BN, bool UP>
+static int me_launch(const CUtensorMap& ma, const CUtensorMap& mw, const int* sorted, const int* offsets, int E, int top, int N, int K, void* c,
+                     long long ldc, int unit, float limit, float slope, int* status, long long most_tiles, cudaStream_t stream) {
+    auto kernel = moe_tcgen05_kernel<BN, UP>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MeGeometry<BN>::SMEM);
+    GB_REQUIRE(e == cudaSuccess, "gb_moe_grouped_gemm: %d bytes of shared memory refused: %s", MeGeometry<BN>::SMEM, cudaGetErrorString(e));
+    const int grid = most_tiles < 148 ? (int)most_tiles : 148;                // one block per SM walks the tiles
+    e = gb_launch(GB_PDL_GEMM, kernel, dim3(grid), dim3(ME_THREADS), MeGeometry<BN>::SMEM, stream, ma, mw, sorted, offsets, E, top, N, K, c, ldc,
+                  unit, limit, slope, status);
+    GB_REQUIRE(e == cudaSuccess, "gb_moe_grouped_gemm: launch failed: %s", cudaGetErrorString(e));
+    return gb_check_launch("gb_moe_grouped_gemm");
+}
+
+// 1 if the grouped tensor-core products take these sizes (rows of 16-byte pieces)
+GB_EXPORT int gb_moe_grouped_supported(int d, int ff) { return d % 8 == 0 && ff % 8 == 0 ? 1 : 0; }
+
+// up: a = h [rows, K] (row stride lda), c bfloat16 [pairs, ldc] in slot order; otherwise a = the up half's output [pairs, K] and c
+// float32 [pairs, ldc] in pair order. w: the experts' matrices [E * N, K]. sorted, offsets: as moe_sort leaves them.
+GB_EXPORT int gb_moe_grouped_gemm(const void* a, long long lda, int rows, const void* w, int N, int K, const int* sorted, const int* offsets,
+                                  int E, int top, int pairs, void* c, long long ldc, int up, int unit, float limit, float slope, int* status,
+                                  cudaStream_t stream) {
+    GB_REQUIRE(!unit || (up && N % 2 == 0), "gb_moe_grouped_gemm: the gated unit belongs to the up half and needs pairs of rows");
+    GB_REQUIRE(N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && pairs >= 0 && E > 0 && E <= ME_MAX_EXPERTS && status != nullptr,
+               "gb_moe_grouped_gemm: rows must be whole 16-byte pieces (K=%d), at most %d experts (%d)", K, ME_MAX_EXPERTS, E);
+    GB_REQUIRE(((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0, "gb_moe_grouped_gemm: operands must be 16-byte aligned");
+    GB_REQUIRE((long long)E * N <= 0x7fffffff, "gb_moe_grouped_gemm: too many rows of weights");
+    if (pairs == 0) return 0;
+    // The width whose rounds of tiles end soonest, as in the dense product: a k-block takes about as long whatever the width.
+    // How many row tiles there are is known on the device alone: every expert's last one is taken to be half full.
+    const long long used = pairs < E ? pairs : E;
+    const long long likely = pairs / ME_BM + used / 2, row_tiles = likely > used ? likely : used;
+    const float main_us = 0.33f * (float)gb_ceil_div(K, ME_BK);
+    const float epi[2] = {up ? 2.5f : 5.5f, up ? 4.5f : 11.0f};
+    const long long t128 = row_tiles * gb_ceil_div(N, 128), t256 = row_tiles * gb_ceil_div(N, 256);
+    const bool wide = (float)((t256 + 147) / 148) * (main_us + epi[1]) <= (float)((t128 + 147) / 148) * (main_us + epi[0]);
+    CUtensorMap ma, mw;
+    if (tc_make_map_2d(&ma, a, rows, K, lda, up ? 1 : ME_BM, ME_BK, "gb_moe_grouped_gemm")) return 1;
+    if (tc_make_map_2d(&mw, w, (long long)E * N, K, K, wide ? 256 : 128, ME_BK, "gb_moe_grouped_gemm")) return 1;
+#define ME_CASE(BN_, UP_) me_launch<BN_, UP_>(ma, mw, sorted, offsets, E, top, N, K, c, ldc, unit, limit, slope, status, \
+                                              (pairs / ME_BM + used) * gb_ceil_div(N, BN_), stream)
+    if (up) return wide ? ME_CASE(256, true) : ME_CASE(128, true);
+    return wide ? ME_CASE(256, false) : ME_CASE(128, false);
+#undef ME_CASE
+}

@@ -148,9 +148,9 @@ _SIGNATURES = {
     "gb_moe_route": [_P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P, _P, _P, _P, _I, _I, _F, _P],
     "gb_moe_expert_rows": [_P, _I, _I, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P],
     "gb_moe_expert_halves": [_P, _I, _I, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _F, _F, _P],
-    "gb_moe_sort": [_P, _P, _I, _I, _I, _P, _P, _P, _P],
+    "gb_moe_sort": [_P, _P, _I, _I, _I, _P, _P, _P],
     "gb_moe_grouped_supported": [_I, _I],
-    "gb_moe_grouped_gemm": [_P, _LL, _P, _I, _I, _P, _P, _P, _I, _I, _I, _P, _LL, _I, _I, _F, _F, _P],
+    "gb_moe_grouped_gemm": [_P, _LL, _I, _P, _I, _I, _P, _P, _I, _I, _I, _P, _LL, _I, _I, _F, _F, _P, _P],
     "gb_moe_combine": [_P, _P, _I, _P, _LL, _P, _P, _P, _LL, _I, _I, _I, _P],
     "gb_post_norm": [_P, _LL, _P, _F, _F, _I, _P, _P, _P, _P, _F, _F, _F, _P, _P, _I, _P, _P, _P, _I, _P, _I, _I, _P],
     "gb_gate_group_norm": [_P, _P, _LL, _P, _P, _I, _P, _I, _I, _I, _F, _P],
@@ -2007,13 +2007,17 @@ def moe_grouped_supported(dtype: torch.dtype, d: int, ff: int) -> bool:
 
 
 def moe_experts_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, choice: torch.Tensor,
-                        positions: torch.Tensor, tables: torch.Tensor, act: torch.Tensor, pair: torch.Tensor, unit=None) -> None:
+                        positions: torch.Tensor, tables: torch.Tensor, act: torch.Tensor, pair: torch.Tensor, unit=None,
+                        status: Optional[torch.Tensor] = None) -> None:
     """The chosen experts of many rows as grouped products on the tensor cores (bfloat16): the (row, choice) pairs are
     sorted by expert (``tables`` int32 [2 * (experts + 1) + n * top] is the sort's scratch), then one launch computes
     act = relu(W_up[e] h)^2 for all pairs (bfloat16 [n, top * ff], in sorted order) and one pair = W_down[e] act
     (float32 [n, top * d], in pair order). ``unit`` as in ``moe_expert_halves``: the up product then has 2 ff outputs per
-    expert, and its epilogue forms one unit from every two neighbours."""
-    _cuda(h, w_up, w_down, choice, positions, tables, act, pair)
+    expert, and its epilogue forms one unit from every two neighbours. ``status``: the word in which a wait that gives up is
+    recorded (``check_status``)."""
+    if status is None:
+        status = torch.zeros(1, dtype=torch.int32, device=h.device)
+    _cuda(h, w_up, w_down, choice, positions, tables, act, pair, status)
     n, d = h.shape
     top = choice.shape[1]
     up_rows = w_up.shape[0] // experts
@@ -2024,12 +2028,12 @@ def moe_experts_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tenso
     assert w_up.shape == (experts * up_rows, d) and w_down.shape == (experts * d, ff) and choice.is_contiguous()
     assert act.shape == (n, top * ff) and pair.shape == (n, top * d)
     assert tables.dtype == torch.int32 and tables.is_contiguous() and tables.numel() >= 2 * (experts + 1) + P
-    offsets, tile_start, order = tables[:experts + 1], tables[experts + 1:2 * (experts + 1)], tables[2 * (experts + 1):]
-    _call("gb_moe_sort", _ptr(choice), _ptr(positions), n, experts, top, _ptr(offsets), _ptr(tile_start), _ptr(order), _stream())
-    _call("gb_moe_grouped_gemm", _ptr(h), d, _ptr(w_up), up_rows, d, _ptr(order), _ptr(offsets), _ptr(tile_start), experts, top, P,
-          _ptr(act), ff, 1, 1 if unit else 0, float(unit[0]) if unit else 0.0, float(unit[1]) if unit else 0.0, _stream())
-    _call("gb_moe_grouped_gemm", _ptr(act), ff, _ptr(w_down), d, ff, _ptr(order), _ptr(offsets), _ptr(tile_start), experts, top, P,
-          _ptr(pair), d, 0, 0, 0.0, 0.0, _stream())
+    offsets, order = tables[:experts + 1], tables[2 * (experts + 1):]
+    _call("gb_moe_sort", _ptr(choice), _ptr(positions), n, experts, top, _ptr(offsets), _ptr(order), _stream())
+    _call("gb_moe_grouped_gemm", _ptr(h), d, n, _ptr(w_up), up_rows, d, _ptr(order), _ptr(offsets), experts, top, P,
+          _ptr(act), ff, 1, 1 if unit else 0, float(unit[0]) if unit else 0.0, float(unit[1]) if unit else 0.0, _ptr(status), _stream())
+    _call("gb_moe_grouped_gemm", _ptr(act), ff, P, _ptr(w_down), d, ff, _ptr(order), _ptr(offsets), experts, top, P,
+          _ptr(pair), d, 0, 0, 0.0, 0.0, _ptr(status), _stream())
 
 
 def moe_combine(pair: torch.Tensor, weight: torch.Tensor, shared: Optional[torch.Tensor], gate: Optional[torch.Tensor],

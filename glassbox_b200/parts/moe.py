@@ -113,7 +113,8 @@ class RoutedExperts(FeedForward):
             # many rows: the pairs sorted by expert, one grouped product per half on the tensor cores
             tables = ctx.zeros_once(f"moe_tables_{self.E}_{self.top}", 2 * (self.E + 1) + ctx.max_rows * self.top, torch.int32)
             act = ctx.scratch("moe_act", (n, self.top * self.ff))
-            kernels.moe_experts_grouped(h, p["w_up"], p["w_down"], self.E, choice, ctx.positions, tables, act, pair, unit=unit)
+            kernels.moe_experts_grouped(h, p["w_up"], p["w_down"], self.E, choice, ctx.positions, tables, act, pair, unit=unit,
+                                        status=ctx.status)
         else:
             # few rows (or float32): the chosen experts' matrices streamed once per (row, choice), many blocks each
             act = ctx.scratch("moe_act32", (n, self.top * self.ff), torch.float32)
