@@ -1,0 +1,471 @@
+// Flash attention for prompt portions whose values are wider than a head (sm_100a, tcgen05): the talking-heads attention, whose
+// every query head is applied to the values of all key/value heads (up to 256 channels a block), and attention over a latent
+// cache, whose keys are a latent and a rotated part (up to 192 numbers) and whose values are the latents themselves.
+//
+// One block = 128 consecutive rows of one request for one query head, over tiles of 128 keys. Tensor memory holds two score
+// buffers of 128 columns and one accumulator of DV columns; the weights P_j take the place of the scores S_j they come from
+// (bfloat16, 64 columns), so nothing else has to fit.
+//   warp 0     producer of the query tile and of the keys: page by page through the request's block table, in 64-channel
+//              column blocks of 128 rows x 128 bytes (128-byte swizzle; channels past the row are zero-filled)
+//   warp 1     issues S_0, S_1, then in turn O += P_j V_j (as soon as P_j is written) and, when that is done, S_(j+2) into the
+//              buffer that P_j leaves; meanwhile the softmax warps work on S_(j+1)
+//   warps 2-9  softmax, two threads per row: a thread reads 64 of its row's 128 scores, caps and masks them, exchanges its
+//              maximum with its partner, and writes its half of P_j. The running maximum is raised (and O rescaled) only when
+//              exceeded by more than 2^8 in the exponent, as in attention_prefill_tc.cu.
+//   warp 10    producer of the values (not for the latent cache, whose key tile serves both products)
+// Bound by the softmax warps' exponentials (with a cap two and a quarter special-function operations a score: 2,300 cycles a
+// tile against 1,280 of the tensor pipe); the mma.sync kernels that this replaced formed the scores once per 128 value
+// channels and fed both products through ldmatrix. Measured: see gb_talking_attention_flash, gb_latent_flash.
+//
+// Every wait is bounded: on a timeout the block records GB_STATUS_WAIT_TIMEOUT, waits (bounded) for its copies, frees its tensor
+// memory and returns. No multicast.
+#include "tcgen05.cuh"
+
+constexpr int FW_BM = 128, FW_BN = 128, FW_WARPS = 11;
+constexpr float FW_NEG_BIG = -1.0e30f, FW_LOG2E = 1.4426950408889634f;
+constexpr int FW_BLOCK = FW_BM * 128;        // bytes of a column block: 128 rows of 64 bfloat16
+
+struct FwArgs {
+    void* out;                 // LATENT: bfloat16 [n, H, DV]; else float32 [n, H, wide]
+    const int* block_tables;
+    int max_pages;
+    const int* seq_first_row;
+    const int* seq_start_pos;
+    const float* sink;         // LATENT: a logit per head in the denominator, or nullptr
+    int H, kv_heads, page_size, page_shift;
+    long long num_pages;
+    float scale, cap;          // cap > 0: cap * tanh(score / cap)
+    int unit;                  // a key of score 0 without a value in the denominator
+    int window, wide, vdim;    // channels of a row's output in all; of a value head
+    int key_steps;             // 16-channel steps of a key row
+    int col_blocks;            // blocks of DV channels that a row's output is cut into
+    int* status;
+};
+
+struct __align__(8) FwShared {
+    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, x_bar[4];
+    float stat[2][2][FW_BM];   // [parity of the tile][half][row]: a half's maximum, at the end its sum
+    uint32_t tmem_base;
+    int abort_flag, issued[2], consumed[2], q_issued, q_consumed;
+};
+
+// KB: column blocks of a key row; DV: value channels of the block
+template <int KB, int DV, bool LATENT> struct FwGeometry {
+    static constexpr int K_STAGES = 3, V_STAGES = 2, K_BYTES = KB * FW_BLOCK, V_BYTES = LATENT ? 0 : (DV / 64) * FW_BLOCK;
+    static constexpr int K_OFF = KB * FW_BLOCK, V_OFF = K_OFF + K_STAGES * K_BYTES, SH_OFF = V_OFF + V_STAGES * V_BYTES;
+    static constexpr int SMEM = SH_OFF + (int)sizeof(FwShared) + 1024, O_COL = 2 * FW_BN;
+    static_assert(O_COL + DV <= 512 && SMEM <= 227 * 1024, "the block does not fit");
+};
+
+__device__ __forceinline__ float fw_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float fw_rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// two non-negative floats to a bfloat16 pair, rounding half up (integer instructions: the conversion shares ex2's pipe)
+__device__ __forceinline__ uint32_t fw_pack(float lo, float hi) {
+    return __byte_perm(__float_as_uint(lo) + 0x8000u, __float_as_uint(hi) + 0x8000u, 0x7632);
+}
+// MN-major B operand (rows are keys, 64-channel column blocks FW_BLOCK apart), 128-byte-swizzled rows
+__device__ __forceinline__ uint64_t fw_desc_mn(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)(FW_BLOCK >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
+           (uint64_t)2 << 61;
+}
+__device__ __forceinline__ void fw_tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+                 "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+
+template <int KB, int DV, bool LATENT>
+__global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                                                                   const __grid_constant__ CUtensorMap map_v, const FwArgs a) {
+    using G = FwGeometry<KB, DV, LATENT>;
+    extern __shared__ __align__(16) unsigned char fw_dyn[];
+    unsigned char* smem = fw_dyn + ((1024u - (smem_u32(fw_dyn) & 1023u)) & 1023u);        // swizzled tiles: 1024-byte aligned
+    unsigned char* Qs = smem, *Ks = smem + G::K_OFF, *Vs = LATENT ? Ks : smem + G::V_OFF;
+    FwShared& sh = *reinterpret_cast<FwShared*>(smem + G::SH_OFF);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // later tiles see more keys: the longest blocks start first (the row tile is the slowest dimension of the grid)
+    const int qt = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, seq = blockIdx.y / a.col_blocks, col0 = (blockIdx.y % a.col_blocks) * DV;
+    const int row0 = a.seq_first_row[seq], nrows = a.seq_first_row[seq + 1] - row0, q_lo = qt * FW_BM;
+    const int start_pos = a.seq_start_pos[seq];
+    if (q_lo >= nrows || start_pos < 0) return;                 // (uniform for the block, before anything is allocated)
+    const int pos_lo = start_pos + q_lo, pos_hi = start_pos + min(nrows, q_lo + FW_BM) - 1;
+    if ((pos_hi >> a.page_shift) >= a.max_pages) {
+        if (tid == 0) atomicOr(a.status, GB_STATUS_BAD_POSITION);
+        return;
+    }
+    const int kvh = head / (a.H / a.kv_heads);
+    const int key_lo = gb_first_key(pos_lo, a.window);
+    const int kt_begin = key_lo / FW_BN, ntiles = pos_hi / FW_BN - kt_begin + 1;
+    const int* table = a.block_tables + (size_t)seq * a.max_pages;
+
+    if (tid == 0) {
+        mbar_init(&sh.q_full, 1);
+        for (int i = 0; i < 3; ++i) { mbar_init(&sh.k_full[i], 1); mbar_init(&sh.k_empty[i], 1); }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh.v_full[i], 1);
+            mbar_init(&sh.v_empty[i], 1);
+            mbar_init(&sh.s_full[i], 1);
+            mbar_init(&sh.p_ready[i], 8);                       // one arrival per softmax warp
+        }
+        mbar_init(&sh.pv_done, 1);
+        for (int i = 0; i < 4; ++i) mbar_init(&sh.x_bar[i], 2);   // the two warps of a quarter of the rows
+        sh.abort_flag = sh.issued[0] = sh.issued[1] = sh.consumed[0] = sh.consumed[1] = sh.q_issued = sh.q_consumed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+        if (!LATENT) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem_base;
+    volatile int* abort_flag = &sh.abort_flag;
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+
+    if (warp == 0 || (!LATENT && warp == FW_WARPS - 1)) {
+        // ------------------------------------------------------------------------- producers
+        const int what = warp == 0 ? 0 : 1;                     // keys, values
+        if (what == 0 && lane == 0) {
+            mbar_expect_tx(&sh.q_full, KB * FW_BLOCK);
+            for (int c = 0; c < KB; ++c) fw_tma_3d(Qs + c * FW_BLOCK, &map_q, &sh.q_full, c * 64, head, row0 + q_lo);
+            sh.q_issued = 1;
+        }
+        const int ppt = FW_BN >> a.page_shift;                  // pages per key tile (1 .. 16): a lane each
+        const int boxes = what == 0 ? KB : DV / 64, stages = what == 0 ? G::K_STAGES : G::V_STAGES;
+        const int bytes = boxes * FW_BLOCK;
+        uint64_t* full = what == 0 ? sh.k_full : sh.v_full;
+        uint64_t* empty = what == 0 ? sh.k_empty : sh.v_empty;
+        unsigned char* ring = what == 0 ? Ks : Vs;
+        int bad = 0;
+        auto page_of = [&](int kt) -> long long {               // this lane's page of key tile kt
+            long long page = 0;
+            if (lane < ppt) {
+                const int pi = ((kt * FW_BN) >> a.page_shift) + lane;
+                page = pi < a.max_pages ? table[pi] : -1;
+                if (page < 0 || page >= a.num_pages) {
+                    // only a page that holds a key some row can see is missed; page 0, finite, is read in the place of others
+                    const int first = pi << a.page_shift;
+                    if (first <= pos_hi && first + a.page_size - 1 >= key_lo) bad = 1;
+                    page = 0;
+                }
+            }
+            return page;
+        };
+        long long page = page_of(kt_begin);
+        int s = 0, round = 0;
+        for (int j = 0; j < ntiles; ++j) {
+            const long long next_page = j + 1 < ntiles ? page_of(kt_begin + j + 1) : 0;   // in flight during the wait
+            int ok = 1;
+            if (lane == 0 && round > 0) ok = mbar_wait(&empty[s], (round - 1) & 1, abort_flag, a.status) ? 1 : 0;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            if (lane == 0) mbar_expect_tx(&full[s], bytes);
+            __syncwarp();
+            if (lane < ppt) {
+                unsigned char* dst = ring + s * bytes + lane * a.page_size * 128;
+                for (int b = 0; b < boxes; ++b) {
+                    if (what == 0) {
+                        tma_load_2d(dst + b * FW_BLOCK, &map_k, &full[s], b * 64, (int)((page * a.kv_heads + kvh) * a.page_size));
+                    } else {
+                        const int col = col0 + b * 64;          // of the wide value row
+                        tma_load_2d(dst + b * FW_BLOCK, &map_v, &full[s], col % a.vdim, (int)((page * a.kv_heads + col / a.vdim) * a.page_size));
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) sh.issued[what] = j + 1;
+            page = next_page;
+            if (++s == stages) { s = 0; ++round; }
+        }
+        if (bad && what == 0) atomicOr(a.status, GB_STATUS_BAD_SLOT);
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------------- MMA issuer
+        if (lane == 0) {
+            const uint32_t idesc_qk = umma_idesc(FW_BM, FW_BN), idesc_pv = umma_idesc(FW_BM, DV) | (1u << 16);     // (B is MN-major)
+            const uint32_t q_addr = smem_u32(Qs), k_addr = smem_u32(Ks), v_addr = smem_u32(Vs);
+            bool ok = mbar_wait(&sh.q_full, 0, abort_flag, a.status);
+            if (ok) sh.q_consumed = 1;
+            auto scores = [&](int j) {
+                const int s = j % G::K_STAGES;
+                if (!mbar_wait(&sh.k_full[s], (j / G::K_STAGES) & 1, abort_flag, a.status)) return false;
+                sh.consumed[0] = j + 1;
+                tc_fence_after();
+                const uint32_t kb = k_addr + (uint32_t)(s * G::K_BYTES);
+                for (int k = 0; k < a.key_steps; ++k) {
+                    const uint32_t at = (uint32_t)((k >> 2) * FW_BLOCK + (k & 3) * 32);
+                    umma_bf16(tmem + (uint32_t)((j & 1) * FW_BN), umma_desc(q_addr + at), umma_desc(kb + at), idesc_qk, k ? 1u : 0u);
+                }
+                umma_commit(&sh.s_full[j & 1]);
+                if (!LATENT) umma_commit(&sh.k_empty[s]);
+                return true;
+            };
+            for (int j = 0; j < 2 && j < ntiles && ok; ++j) ok = scores(j);
+            for (int j = 0; j < ntiles && ok; ++j) {
+                const int s = LATENT ? j % G::K_STAGES : j % G::V_STAGES;
+                if (!LATENT && !(ok = mbar_wait(&sh.v_full[s], (j / G::V_STAGES) & 1, abort_flag, a.status))) break;
+                if (!LATENT) sh.consumed[1] = j + 1;
+                if (!(ok = mbar_wait(&sh.p_ready[j & 1], (j >> 1) & 1, abort_flag, a.status))) break;
+                tc_fence_after();
+                const uint32_t vb = v_addr + (uint32_t)(s * (LATENT ? G::K_BYTES : G::V_BYTES));
+#pragma unroll
+                for (int kk = 0; kk < FW_BN / 16; ++kk)         // 16 keys an instruction: 8 columns of P, 16 rows of the values
+                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + kk * 8), fw_desc_mn(vb + kk * 16 * 128), idesc_pv,
+                                 (j | kk) ? 1u : 0u);
+                umma_commit(&sh.pv_done);
+                umma_commit(LATENT ? &sh.k_empty[s] : &sh.v_empty[s]);
+                // S_(j+2) goes where P_j is: only once the product that reads it is done
+                if (j + 2 < ntiles) ok = mbar_wait(&sh.pv_done, j & 1, abort_flag, a.status) && scores(j + 2);
+            }
+        }
+    } else if (warp < FW_WARPS - 1) {
+        // ------------------------------------------------------------------------- softmax
+        const int q = warp & 3, h = (warp - 2) >> 2;            // the quarter of the rows this warp may read; its half of the keys
+        const int r = q * 32 + lane, pos = pos_lo + r;
+        const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
+        const float sl2 = a.scale * FW_LOG2E;                   // scores are brought into the base-2 domain
+        const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? 2.0f * sl2 / a.cap : 0.f;
+        const float slx = cap2 > 0.f ? 1.0f : sl2;              // what is left to scale once capped
+        const int first = gb_first_key(pos, a.window), first_last = gb_first_key(pos_lo + FW_BM - 1, a.window);
+        float m_run = FW_NEG_BIG, l_run = 0.f;
+        bool ok = true;
+        for (int j = 0; j < ntiles; ++j) {
+            const int b = j & 1, key0 = (kt_begin + j) * FW_BN + h * 64;
+            if (!mbar_wait_warp(&sh.s_full[b], (j >> 1) & 1, abort_flag, a.status)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t sv[64];
+            tmem_load64(lane_base + (uint32_t)(b * FW_BN + h * 64), sv);
+            tc_fence_before();
+            if (cap2 > 0.f) {
+                // cap tanh(s / cap) = cap - 2 cap / (1 + exp(2 s / cap)); four scores share a reciprocal, of the product of their
+                // denominators (each at most 1 + 2^30, where the tanh is 1 to the last bit)
+                const float2 in2 = make_float2(cap_in, cap_in), one2 = make_float2(1.f, 1.f);
+                const float2 top2 = make_float2(cap2, cap2), down2 = make_float2(-2.0f * cap2, -2.0f * cap2);
+#pragma unroll
+                for (int k = 0; k < 64; k += 4) {
+                    const float2 ya = __fmul2_rn(make_float2(__uint_as_float(sv[k]), __uint_as_float(sv[k + 1])), in2);
+                    const float2 yb = __fmul2_rn(make_float2(__uint_as_float(sv[k + 2]), __uint_as_float(sv[k + 3])), in2);
+                    const float2 ea = __fadd2_rn(make_float2(fw_exp2(fminf(ya.x, 30.f)), fw_exp2(fminf(ya.y, 30.f))), one2);
+                    const float2 eb = __fadd2_rn(make_float2(fw_exp2(fminf(yb.x, 30.f)), fw_exp2(fminf(yb.y, 30.f))), one2);
+                    const float2 both = __fmul2_rn(ea, eb);
+                    const float rc = fw_rcp(both.x * both.y);
+                    const float2 rb = __fmul2_rn(make_float2(both.y, both.x), make_float2(rc, rc));
+                    const float2 sa = __ffma2_rn(__fmul2_rn(eb, rb), down2, top2), sb = __ffma2_rn(__fmul2_rn(ea, rb), down2, top2);
+                    sv[k] = __float_as_uint(sa.x);
+                    sv[k + 1] = __float_as_uint(sa.y);
+                    sv[k + 2] = __float_as_uint(sb.x);
+                    sv[k + 3] = __float_as_uint(sb.y);
+                }
+            }
+            if (key0 + 63 > pos_lo || key0 < first_last) {      // the tile crosses the diagonal, the window's edge or the last key
+#pragma unroll
+                for (int k = 0; k < 64; ++k)
+                    if (!(key0 + k <= pos && key0 + k >= first)) sv[k] = __float_as_uint(FW_NEG_BIG);
+            }
+            float mx4[4] = {FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG};
+#pragma unroll
+            for (int k = 0; k < 64; k += 8)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) asm("max.f32 %0, %0, %1, %2;" : "+f"(mx4[u]) : "f"(__uint_as_float(sv[k + 2 * u])), "f"(__uint_as_float(sv[k + 2 * u + 1])));
+            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            // the partner's maximum. Once both have met here, both have also read their scores: P may take their place
+            sh.stat[b][h][r] = mx;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.x_bar[q]);
+            if (!mbar_wait_warp(&sh.x_bar[q], j & 1, abort_flag, a.status)) { ok = false; break; }
+            mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
+            const bool raise = (mx - m_run) * slx > 8.0f;
+            if (j == 0) {
+                if (raise) m_run = mx;                          // nothing is accumulated yet
+            } else if (__any_sync(0xffffffffu, raise)) {
+                // (S_j was issued after O += P_(j-2) V_(j-2) was done: the phase of P_(j-1) V_(j-1) is the one to wait for)
+                if (!mbar_wait_warp(&sh.pv_done, (j - 1) & 1, abort_flag, a.status)) { ok = false; break; }
+                tc_fence_after();
+                const float corr = raise ? fw_exp2((m_run - mx) * slx) : 1.0f;
+                if (raise) m_run = mx;
+                l_run *= corr;
+#pragma unroll 1
+                for (int c = 0; c < DV / 2; c += 32) {
+                    uint32_t ov[32];
+                    const uint32_t at = lane_base + (uint32_t)(G::O_COL + h * (DV / 2) + c);
+                    tmem_load32(at, ov);
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * corr);
+                    tmem_store32(at, ov);
+                }
+            }
+            // a masked key holds -1e30 and comes out as exactly 0; a row that has seen no key yet must not cancel that
+            const float msl = m_run <= FW_NEG_BIG ? 0.f : m_run * slx;
+            const float2 scale2 = make_float2(slx, slx), off2 = make_float2(-msl, -msl);
+            float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            uint32_t pw[32];
+#pragma unroll
+            for (int c = 0; c < 64; c += 2) {
+                const float2 y = __ffma2_rn(make_float2(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), scale2, off2);
+                const float2 pp = make_float2(fw_exp2(y.x), fw_exp2(y.y));
+                // the denominator sums what the product uses: the weights as rounded to bfloat16
+                const uint32_t both = pw[c >> 1] = fw_pack(pp.x, pp.y);
+                l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
+            }
+            l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
+            tmem_store32(lane_base + (uint32_t)(b * FW_BN + h * 32), pw);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.p_ready[b]);
+        }
+        if (ok) {                                               // the halves' sums
+            sh.stat[ntiles & 1][h][r] = l_run;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.x_bar[q]);
+            ok = mbar_wait_warp(&sh.x_bar[q], ntiles & 1, abort_flag, a.status);
+            // the last two products may both be under way: their phases one after the other (a wait for a parity passes while the
+            // phase before it is still open)
+            for (int j = max(ntiles - 2, 0); j < ntiles && ok; ++j) ok = mbar_wait_warp(&sh.pv_done, j & 1, abort_flag, a.status);
+        }
+        if (ok) {
+            tc_fence_after();
+            float l = l_run + sh.stat[ntiles & 1][h ^ 1][r], m2 = m_run <= FW_NEG_BIG ? FW_NEG_BIG : m_run * slx;
+            float sink2 = FW_NEG_BIG;
+            if (LATENT && a.sink != nullptr) sink2 = a.sink[head] * FW_LOG2E;
+            if (a.unit) sink2 = 0.f;
+            const float top = fmaxf(m2, sink2), corr = fw_exp2(m2 - top);
+            l = l * corr + fw_exp2(sink2 - top);
+            const float inv = l > 0.f ? corr / l : 0.f;
+            const size_t row = (size_t)(row0 + q_lo + r);
+#pragma unroll 1
+            for (int c = h * (DV / 2); c < (h + 1) * (DV / 2); c += 32) {
+                uint32_t ov[32];
+                tmem_load32(lane_base + (uint32_t)(G::O_COL + c), ov);
+                if (q_lo + r >= nrows) continue;
+#pragma unroll
+                for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * inv);
+                if (LATENT) {
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
+#pragma unroll
+                    for (int k = 0; k < 32; k += 8)
+                        *reinterpret_cast<uint4*>(dst + k) = make_uint4(pack2(ov[k], ov[k + 1]), pack2(ov[k + 2], ov[k + 3]), pack2(ov[k + 4], ov[k + 5]),
+                                                                        pack2(ov[k + 6], ov[k + 7]));
+                } else {
+                    float* dst = reinterpret_cast<float*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
+#pragma unroll
+                    for (int k = 0; k < 32; k += 4)
+                        *reinterpret_cast<uint4*>(dst + k) = make_uint4(ov[k], ov[k + 1], ov[k + 2], ov[k + 3]);
+                }
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        if (lane == 0 && sh.abort_flag) {                       // copies that nobody consumed may still be in flight
+            auto drain = [&](uint64_t* bar, uint32_t parity) {
+                const long long t0 = clock64();
+                while (!mbar_try_wait(bar, parity) && clock64() - t0 < TC_WAIT_CYCLES) {}
+            };
+            if (sh.q_issued && !sh.q_consumed) drain(&sh.q_full, 0);
+            for (int it = sh.consumed[0]; it < sh.issued[0]; ++it) drain(&sh.k_full[it % G::K_STAGES], (it / G::K_STAGES) & 1);
+            for (int it = sh.consumed[1]; it < sh.issued[1]; ++it) drain(&sh.v_full[it % G::V_STAGES], (it / G::V_STAGES) & 1);
+        }
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------------------------------- host
+static int fw_map_q(CUtensorMap* map, const void* q, long long n, int H, int dim, const char* who) {
+    TcEncodeTiledFn fn = tc_encode_fn();
+    GB_REQUIRE(fn != nullptr, "%s: the driver does not offer cuTensorMapEncodeTiled", who);
+    cuuint64_t dims[3] = {(cuuint64_t)dim, (cuuint64_t)H, (cuuint64_t)n};
+    cuuint64_t strides[2] = {(cuuint64_t)dim * 2, (cuuint64_t)dim * H * 2};
+    cuuint32_t box[3] = {64, 1, FW_BM}, one[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    GB_REQUIRE(r == CUDA_SUCCESS, "%s: cuTensorMapEncodeTiled failed with code %d", who, (int)r);
+    return 0;
+}
+
+template <int KB, int DV, bool LATENT>
+static int fw_launch(const void* q, const void* kcache, const void* vcache, int n, int dim, int num_seqs, int max_rows, const FwArgs& a,
+                     cudaStream_t stream, const char* who) {
+    using G = FwGeometry<KB, DV, LATENT>;
+    CUtensorMap mq, mk, mv;
+    if (fw_map_q(&mq, q, n, a.H, dim, who)) return 1;
+    if (tc_make_map_2d(&mk, kcache, a.num_pages * a.kv_heads * a.page_size, dim, dim, a.page_size, 64, who)) return 1;
+    if (LATENT) mv = mk;
+    else if (tc_make_map_2d(&mv, vcache, a.num_pages * a.kv_heads * a.page_size, a.vdim, a.vdim, a.page_size, 64, who)) return 1;
+    auto kernel = flash_wide_kernel<KB, DV, LATENT>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+    GB_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory refused: %s", who, G::SMEM, cudaGetErrorString(e));
+    const int tiles = gb_ceil_div(max_rows, FW_BM);
+    GB_REQUIRE(tiles <= 65535 && (long long)num_seqs * a.col_blocks <= 65535, "%s: bad batch shape", who);
+    e = gb_launch(GB_PDL_ATTENTION, kernel, dim3(a.H, num_seqs * a.col_blocks, tiles), dim3(FW_WARPS * 32), G::SMEM, stream, mq, mk, mv, a);
+    GB_REQUIRE(e == cudaSuccess, "%s: launch failed: %s", who, cudaGetErrorString(e));
+    return gb_check_launch(who);
+}
+
+static int fw_page_shift(int page_size) {
+    int shift = 0;
+    while ((1 << shift) < page_size) ++shift;
+    return shift;
+}
+static bool fw_pages_ok(int page_size) { return page_size >= 8 && page_size <= FW_BN && (page_size & (page_size - 1)) == 0; }
+
+// Talking-heads attention of prompt portions: keys of 64 channels, value heads of 64 or 128, the values of all heads a whole
+// number of 128-channel blocks.
+GB_EXPORT int gb_talking_attention_flash_supported(int D, int V, int VG, int page_size) {
+    return D == 64 && (V == 64 || V == 128) && VG > 0 && (VG * V) % 128 == 0 && fw_pages_ok(page_size);
+}
+
+// As gb_talking_attention_tiles (talking_attention.cu), VG == G. q bfloat16 [n, H, 64], out float32 [n, H, G * V].
+// Measured, 2,048 tokens, 16/4 heads of 64, capped: 402 us in tiles of mma.sync, 52 us here.
+GB_EXPORT int gb_talking_attention_flash(const void* q, float* out, const void* kcache, const void* vcache, const int* block_tables, int max_pages,
+                                         const int* seq_first_row, const int* seq_start_pos, int n, int num_seqs, int max_rows_per_seq, int H, int G,
+                                         int V, int page_size, long long num_pages, float scale, float cap, int unit, int window, int* status,
+                                         cudaStream_t stream) {
+    GB_REQUIRE(gb_talking_attention_flash_supported(64, V, G, page_size) && H > 0 && H % G == 0,
+               "gb_talking_attention_flash: %d/%d heads, values of %d, pages of %d are not built", H, G, V, page_size);
+    GB_REQUIRE((((uintptr_t)q | (uintptr_t)out | (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0, "gb_talking_attention_flash: operands must be 16-byte aligned");
+    GB_REQUIRE(n >= 0 && num_seqs >= 0 && max_pages > 0 && num_pages * G * page_size < (1ll << 31), "gb_talking_attention_flash: bad batch shape");
+    if (n == 0 || num_seqs == 0 || max_rows_per_seq <= 0) return 0;
+    const int wide = G * V;
+    FwArgs a = {out, block_tables, max_pages, seq_first_row, seq_start_pos, nullptr, H, G, page_size, fw_page_shift(page_size), num_pages, scale, cap,
+                unit, window, wide, V, 4, 1, status};
+    if (wide % 256 == 0) {
+        a.col_blocks = wide / 256;
+        return fw_launch<1, 256, false>(q, kcache, vcache, n, 64, num_seqs, max_rows_per_seq, a, stream, "gb_talking_attention_flash");
+    }
+    a.col_blocks = wide / 128;
+    return fw_launch<1, 128, false>(q, kcache, vcache, n, 64, num_seqs, max_rows_per_seq, a, stream, "gb_talking_attention_flash");
+}
+
+GB_EXPORT int gb_latent_flash_supported(int c, int r, int page_size) {
+    return c == 128 && (r == 16 || r == 32 || r == 64) && fw_pages_ok(page_size);
+}
+
+// Attention of prompt portions over a latent cache [pages, page_size, 128 + r]: q bfloat16 [n, H, 128 + r], out bfloat16
+// [n, H, 128]; arguments as gb_latent_attention_mma. Measured, two portions of 1,500 tokens in all
+// behind up to 900, 32 heads, 128 + 64: 197 us in tiles of mma.sync, 70 us here.
+GB_EXPORT int gb_latent_flash(const void* q, void* out, const void* cache, const int* block_tables, int max_pages, const int* seq_first_row,
+                              const int* seq_start_pos, const float* sink, int n, int num_seqs, int max_rows_per_seq, int H, int c, int r,
+                              int page_size, long long num_pages, float scale, int window, int* status, cudaStream_t stream) {
+    GB_REQUIRE(gb_latent_flash_supported(c, r, page_size) && H > 0, "gb_latent_flash: latent %d, rotated part %d, pages of %d are not built", c, r, page_size);
+    GB_REQUIRE((((uintptr_t)q | (uintptr_t)out | (uintptr_t)cache) & 15) == 0, "gb_latent_flash: operands must be 16-byte aligned");
+    GB_REQUIRE(n >= 0 && num_seqs >= 0 && max_pages > 0 && num_pages * page_size < (1ll << 31), "gb_latent_flash: bad batch shape");
+    if (n == 0 || num_seqs == 0 || max_rows_per_seq <= 0) return 0;
+    FwArgs a = {out, block_tables, max_pages, seq_first_row, seq_start_pos, sink, H, 1, page_size, fw_page_shift(page_size), num_pages, scale, 0.f,
+                0, window, 128, 128, (c + r) / 16, 1, status};
+    return fw_launch<3, 128, true>(q, cache, cache, n, c + r, num_seqs, max_rows_per_seq, a, stream, "gb_latent_flash");
+}

@@ -119,6 +119,10 @@ _SIGNATURES = {
     "gb_talking_attention_decode_plan": [_I, _I, _I, _I],
     "gb_talking_attention_tiles": [_P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _F, _F, _I, _P, _P],
     "gb_talking_attention_tiles_columns": [_I, _I, _I],
+    "gb_talking_attention_flash_supported": [_I, _I, _I, _I],
+    "gb_talking_attention_flash": [_P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _F, _I, _I, _P, _P],
+    "gb_latent_flash_supported": [_I, _I, _I],
+    "gb_latent_flash": [_P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P],
     "gb_talk_combine": [_P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _P],
     "gb_short_conv": [_P, _LL, _P, _P, _LL, _P, _LL, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "gb_channel_delta": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P],
@@ -1248,6 +1252,25 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
         launch_count += 1
 
 
+def latent_flash_supported(q: torch.Tensor, num_seqs: int, c: int, r: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel takes a step of prompt portions with these sizes, and the portions are long enough for it."""
+    return (q.dtype == torch.bfloat16 and q.shape[0] >= FLASH_WIDE_MIN_ROWS * num_seqs
+            and bool(lib().gb_latent_flash_supported(c, r, page_size)))
+
+
+def latent_flash(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor, seq_first_row: torch.Tensor,
+                 seq_start_pos: torch.Tensor, sink: Optional[torch.Tensor], heads: int, c: int, r: int, page_size: int, scale: float,
+                 window: Optional[int], status: torch.Tensor, max_rows_per_seq: int) -> None:
+    """``latent_attention_mma`` for prompt portions on tcgen05: 128 rows of one request x one head per block."""
+    _cuda(q, out, cache, block_tables, seq_first_row, seq_start_pos, sink, status)
+    n = q.shape[0]
+    assert q.dtype == out.dtype == cache.dtype == torch.bfloat16 and q.is_contiguous() and out.is_contiguous() and cache.is_contiguous()
+    assert q.numel() == n * heads * (c + r) and out.numel() == n * heads * c and cache.shape[-1] == c + r and block_tables.is_contiguous()
+    _call("gb_latent_flash", _ptr(q), _ptr(out), _ptr(cache), _ptr(block_tables), block_tables.shape[1], _ptr(seq_first_row),
+          _ptr(seq_start_pos), _ptr(sink), n, seq_start_pos.shape[0], int(max_rows_per_seq), heads, c, r, page_size,
+          cache.numel() // ((c + r) * page_size), float(scale), int(window) if window else 0, _ptr(status), _stream())
+
+
 class NormedPair:
     """A branch output that exists only as its parts: a_scale * rms(a[r], gain_a) + b_scale * rms(b[r], gain_b), two branches that
     share an input and are each normed over the row before they join. ``post_norm`` takes it in the place of a stored y."""
@@ -2137,6 +2160,32 @@ def talking_attention_tiles(q: torch.Tensor, wide: torch.Tensor, kcache: torch.T
           _ptr(seq_first_row), _ptr(seq_start_pos), seq_start_pos.shape[0], int(max_rows_per_seq), heads, kv_heads, dim, vdim, value_heads,
           page_size, kcache.shape[0], float(scale), float(softcap or 0.0), 1.0 if unit_sink else 0.0, int(window or 0), _ptr(status),
           _stream())
+
+
+#: rows that the requests of a step bring on average from which the 128-row tiles of the wide flash kernels are worth their
+#: padding (single tokens in a mixed batch fill one row of a tile)
+FLASH_WIDE_MIN_ROWS = 32
+
+
+def talking_attention_flash_supported(q: torch.Tensor, num_seqs: int, dim: int, vdim: int, value_heads: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel takes a step of prompt portions with these sizes, and the portions are long enough for it."""
+    return (q.dtype == torch.bfloat16 and q.shape[0] >= FLASH_WIDE_MIN_ROWS * num_seqs
+            and bool(lib().gb_talking_attention_flash_supported(dim, vdim, value_heads, page_size)))
+
+
+def talking_attention_flash(q: torch.Tensor, wide: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, block_tables: torch.Tensor,
+                            seq_first_row: torch.Tensor, seq_start_pos: torch.Tensor, max_rows_per_seq: int, heads: int, kv_heads: int,
+                            dim: int, vdim: int, value_heads: int, page_size: int, scale: float, softcap: Optional[float],
+                            unit_sink: bool, window: Optional[int], status: torch.Tensor) -> None:
+    """``talking_attention_tiles`` on tcgen05: 128 rows of one request x one head x 256 columns of the wide value row per block."""
+    _cuda(q, wide, kcache, vcache, block_tables, seq_first_row, seq_start_pos, status)
+    n = q.shape[0]
+    assert q.dtype == kcache.dtype == vcache.dtype == torch.bfloat16 and q.shape == (n, heads * dim) and q.is_contiguous()
+    assert wide.dtype == torch.float32 and wide.shape == (n, heads * value_heads * vdim) and wide.is_contiguous()
+    assert block_tables.is_contiguous() and kcache.is_contiguous() and vcache.is_contiguous() and value_heads == kv_heads and dim == 64
+    _call("gb_talking_attention_flash", _ptr(q), _ptr(wide), _ptr(kcache), _ptr(vcache), _ptr(block_tables), block_tables.shape[1],
+          _ptr(seq_first_row), _ptr(seq_start_pos), n, seq_start_pos.shape[0], int(max_rows_per_seq), heads, kv_heads, vdim, page_size,
+          kcache.shape[0], float(scale), float(softcap or 0.0), 1 if unit_sink else 0, int(window or 0), _ptr(status), _stream())
 
 
 def talk_combine(wide: torch.Tensor, talk: Optional[torch.Tensor], att: torch.Tensor, positions: torch.Tensor, heads: int, kv_heads: int,

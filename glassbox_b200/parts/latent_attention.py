@@ -151,9 +151,13 @@ class LatentAttention(Mixer):
 
     def attend(self, ctx, qabs, lat, cache) -> None:
         """lat[row, head, :] = the softmax-weighted sum of the latents the row sees. bfloat16 at the sizes the
-        tensor-core kernel is built for: decode steps cut each row's keys into shares so that few requests still fill the
-        GPU; steps with prompt portions run tiles of tokens x heads. Anything else: one warp per (row, head)."""
+        tensor-core kernels are built for: decode steps cut each row's keys into shares so that few requests still fill the
+        GPU; steps with prompt portions run tiles of 128 tokens of a head (long portions) or of tokens x heads. Anything else: one warp per (row, head)."""
         n = qabs.shape[0]
+        if not ctx.decode_only and kernels.latent_flash_supported(qabs, ctx.seq_start_pos.shape[0], self.c, self.r, cache.page_size):
+            kernels.latent_flash(qabs, lat, cache.k, cache.block_tables, ctx.seq_first_row, ctx.seq_start_pos, self.params.get("sink"), self.H,
+                                 self.c, self.r, cache.page_size, self.spec.scale, self.spec.window, ctx.status, ctx.max_rows_per_seq)
+            return
         if kernels.latent_attention_mma_supported(qabs.dtype, self.c, self.r, cache.page_size):
             common = (qabs, lat, cache.k, cache.block_tables, ctx.seq_first_row, ctx.seq_start_pos, ctx.positions,
                       self.params.get("sink"), self.H, self.c, self.r, cache.page_size, self.spec.scale, self.spec.window,

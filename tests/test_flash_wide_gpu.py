@@ -1,0 +1,119 @@
+"""The tcgen05 flash kernel with wide values (talking heads, latent cache) against float64 attention over the same bfloat16 numbers, at
+the edges of its 128 x 128 tiles. Scores are spread so far that a few keys carry a row: a key, page or column read in another's
+place moves the result by the size of a value."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+BATCHES = [  # page size, window, [(cached tokens, new rows) or None for a padding sequence, ...]
+    (16, None, [(0, 200), (0, 128), None, (0, 1), (0, 129)]),
+    (8, None, [(100, 31), (640, 140), (127, 127)]),
+    (32, 100, [(0, 300), (250, 77)]),
+    (64, 37, [(500, 130)]),
+    (128, None, [(1000, 300)]),
+]
+
+
+def _layout(page, batch, seed):
+    """Scattered pages: (slots of every request's tokens, block tables, rows' first, start, number of pages)."""
+    g = torch.Generator().manual_seed(seed)
+    need = [-(-(c + n) // page) if b else 0 for b in batch for c, n in [b or (0, 0)]]
+    order = torch.randperm(sum(need) + 2, generator=g).tolist()
+    width = max(need) + 1
+    tables, first, start, at = torch.full((len(batch), width), -1, dtype=torch.int32), [0], [], 0
+    for i, b in enumerate(batch):
+        tables[i, :need[i]] = torch.tensor(order[at:at + need[i]], dtype=torch.int32)
+        at += need[i]
+        first.append(first[-1] + (b[1] if b else 2))
+        start.append(b[0] if b else -1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    return tables.to(DEV), i32(first), i32(start), sum(need) + 2, max(b[1] for b in batch if b)
+
+
+def _dense(pool, table, page, length):
+    """[length, heads, dim] of one request; pool [pages, heads, page, dim]."""
+    pages = table[:-(-length // page)].long()
+    return pool[pages].transpose(1, 2).flatten(0, 1)[:length].double()
+
+
+def _weights(scores, pos, window, sink):
+    key = torch.arange(scores.shape[-1], device=scores.device)
+    seen = (key <= pos[:, None]) & ((key > pos[:, None] - window) if window else True)
+    s = scores.masked_fill(~seen, -math.inf)
+    if sink is not None:
+        s = torch.cat([s, torch.full_like(s[:, :1], sink)], -1)
+    w = torch.softmax(s, -1)
+    return w[:, :-1] if sink is not None else w
+
+
+@pytest.mark.parametrize("page, window, batch", BATCHES)
+@pytest.mark.parametrize("H, G, V, cap, unit", [(4, 4, 64, 30.0, True), (6, 2, 64, None, False), (4, 2, 128, 5.0, True), (8, 8, 64, None, True)])
+def test_talking_heads(page, window, batch, H, G, V, cap, unit):
+    from glassbox_b200 import kernels
+    g = torch.Generator(device=DEV).manual_seed(page + H)
+    tables, first, start, pages, longest = _layout(page, batch, 3)
+    n = int(first[-1])
+    q = torch.randn(n, H * 64, generator=g, device=DEV).bfloat16()
+    k, v = (torch.randn(pages, G, page, d, generator=g, device=DEV).bfloat16() for d in (64, V))
+    out = torch.full((n, H * G * V), 7.0, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kernels.talking_attention_flash(q, out, k, v, tables, first, start, longest, H, G, 64, V, G, page, 0.5, cap, unit, window, status)
+    assert int(status) == 0
+    got = out.double().view(n, H, G, V)
+    for i, b in enumerate(batch):
+        a, z = int(first[i]), int(first[i + 1])
+        if b is None:
+            assert torch.all(got[a:z] == 7.0)
+            continue
+        pos = b[0] + torch.arange(b[1], device=DEV)
+        kk, vv = _dense(k, tables[i], page, b[0] + b[1]), _dense(v, tables[i], page, b[0] + b[1])
+        for h in range(H):
+            s = q.view(n, H, 64)[a:z, h].double() @ kk[:, h // (H // G)].T * 0.5
+            s = cap * torch.tanh(s / cap) if cap else s
+            want = torch.einsum("rk,kgv->rgv", _weights(s, pos, window, 0.0 if unit else None), vv)
+            # weights rounded to bfloat16, 2^-9 of each, in the sum and in its denominator: 2^-9 (sum w |v| + |result|)
+            assert (got[a:z, h] - want).abs().max() <= 2 ** -9 * 2 * vv.abs().max(), (i, h, float((got[a:z, h] - want).abs().max()))
+
+
+@pytest.mark.parametrize("page, window, batch", BATCHES)
+@pytest.mark.parametrize("H, r, sink", [(3, 64, True), (2, 32, False), (1, 16, True)])
+def test_latent_cache(page, window, batch, H, r, sink):
+    from glassbox_b200 import kernels
+    g = torch.Generator(device=DEV).manual_seed(page + r)
+    tables, first, start, pages, longest = _layout(page, batch, 4)
+    n = int(first[-1])
+    q = torch.randn(n, H * (128 + r), generator=g, device=DEV).bfloat16()
+    cache = torch.randn(pages, page, 128 + r, generator=g, device=DEV).bfloat16()
+    sinks = torch.randn(H, generator=g, device=DEV) * 5 if sink else None
+    out = torch.full((n, H * 128), 7.0, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kernels.latent_flash(q, out, cache, tables, first, start, sinks, H, 128, r, page, 0.4, window, status, longest)
+    assert int(status) == 0
+    got = out.double().view(n, H, 128)
+    for i, b in enumerate(batch):
+        a, z = int(first[i]), int(first[i + 1])
+        if b is None:
+            assert torch.all(got[a:z] == 7.0)
+            continue
+        pos = b[0] + torch.arange(b[1], device=DEV)
+        rows = _dense(cache[:, None], tables[i], page, b[0] + b[1])[:, 0]
+        for h in range(H):
+            s = q.view(n, H, 128 + r)[a:z, h].double() @ rows.T * 0.4
+            want = _weights(s, pos, window, float(sinks[h]) if sink else None) @ rows[:, :128]
+            # weights rounded to bfloat16 (as above), and the result
+            assert (got[a:z, h] - want).abs().max() <= 2 ** -9 * 3 * rows[:, :128].abs().max(), (i, h, float((got[a:z, h] - want).abs().max()))
+
+
+def test_positions_beyond_the_table_and_missing_pages_are_reported():
+    from glassbox_b200 import kernels
+    tables, first, start, pages, longest = _layout(16, [(0, 40)], 5)
+    q = torch.randn(40, 2 * 160, device=DEV).bfloat16()
+    cache = torch.randn(pages, 16, 160, device=DEV).bfloat16()
+    for bad, bit in ((tables[:, :2].contiguous(), 4), (tables.clone().index_fill_(1, torch.tensor([1], device=DEV), -1), 2)):
+        out, status = torch.zeros(40, 256, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        kernels.latent_flash(q, out, cache, bad, first, start, None, 2, 128, 32, 16, 0.1, None, status, longest)
+        assert int(status) == bit
