@@ -2,12 +2,11 @@
 //
 // This is the true 32-bit matrix product (no TF32, no tensor cores) and also the generic
 // fallback for any mix of float32 / bfloat16 operands at any size. Three kernels:
-//   * a register-tiled kernel with tiles of 128 x 128 or 128 x 64 and packed FMA where such tiles fill the chip (float32
-//     activations, rows aligned to 16 bytes),
+//   * register-tiled kernels with packed FMA for M > 8 (float32 activations, rows aligned to 16 bytes),
 //   * a 64x64x16 register-tiled kernel for every other M > 8,
 //   * a weight-streaming kernel for M <= 8 (one warp per output column), which is what a
 //     decode step needs: every weight is read once, coalesced along K.
-// Each output element is reduced over K in an order that depends only on K (and on whether M > 8: both tiled kernels
+// Each output element is reduced over K in an order that depends only on K (and on whether M > 8: all tiled kernels
 // add one product after the other from k = 0, so they give the same bits), never on M or on the element's place in the batch.
 // Row-major [out, in] weights as in crates/glassbox-core/src/kernels.rs:381, 586-655.
 #include "common.cuh"
@@ -105,44 +104,57 @@ __global__ void __launch_bounds__(256) gemm_tiled_kernel(const TA* __restrict__ 
     }
 }
 
-// -------------------------------------------------------------------------- wide tiled kernel
-// Tiles of 128 x WN outputs, 256 threads, 8 x (WN / 16) outputs each, k in slices of 16 double-buffered in shared memory (the
-// next slice's loads are in flight while one is worked on; one barrier per slice). Bound by the FMA pipe: a packed FMA does
-// two neighbouring rows, so a k costs 8 x (WN / 16) / 2 packed FMAs against 2 + WN / 64 16-byte loads and the copies of W's
-// numbers into both halves, where the 64 x 64 tile paid 8 loads for 16 scalar FMAs. Shared-memory bandwidth comes next: 8 x 4
-// outputs a thread read 3 x 16 bytes per 16 packed FMAs. Measured, 2,047 rows (64 x 64 tiles -> these): 960 x 576
-// 87 -> 66 us, 576 x 576 58 -> 41, 3072 x 576 228 -> 184 (39 TFLOP/s), 576 x 1536 139 -> 100.
+// ------------------------------------------------------------------------ packed tiled kernels
+// Tiles of BM x BN outputs, 128 threads of TM x TN outputs each, k in slices of KS double-buffered in shared memory (the next
+// slice's loads are in flight while one is worked on; one barrier per slice). A packed FMA does two neighbouring rows. Bound by
+// shared memory: a load costs its bytes to every lane whoever shares them, so the 64 x 64 tile of 256 threads (8 words for 16
+// products, no loads in flight) reached 26-32 TFLOP/s; 8 x 4 outputs a thread read 12 words for 32. Two shapes: 64 x 64, and
+// 32 x 64 where all tiles of that shape have an SM of their own (a lone block's time is its chain of slices, and a smaller slice
+// is a shorter one). Measured, us for 576 x 576 at 200 / 800 / 2,047 rows: 31 / 32 / 50 before, 27 / 28 / 38 in 64 x 64, 19 / 29 /
+// 54 in 32 x 64; 960 x 2560: 132 / 212 / 374, 109 / 155 / 281, 74 / 166 / 375; 3072 x 576: 49 / 106 / 227, 37 / 84 / 173, 40 / 111 /
+// 252. (128 x 64 and 128 x 128 tiles: no better but for the last, 163.)
 typedef unsigned long long simt_pair;
-constexpr int WIDE_M = 128, WIDE_K = 16;
 
-template <typename TA, typename TW, typename TC, int WN>
-__global__ void __launch_bounds__(256, 2) gemm_wide_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, int M,
-                                                           int N, int K, long long lda, long long ldw, long long ldc, int mode) {
-    constexpr int NQ = WN / 64;                          // groups of four columns of a thread, 64 apart
-    __shared__ __align__(16) float As[2][WIDE_K][WIDE_M + 4];
-    __shared__ __align__(16) float Ws[2][WIDE_K][WN + 4];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * WIDE_M, n0 = blockIdx.x * WN;
-    const int lr = tid >> 2, lk = (tid & 3) * 4;         // the row (and those 64 further on) and the k's that this thread fetches
-    simt_pair acc[4][NQ * 4];
+// WM x WN warps of LM x (32 / LM) lanes
+template <int WM, int WN, int LM, int TM, int TN, int KS> struct PackedTile {
+    static constexpr int LN = 32 / LM, THREADS = WM * WN * 32, BM = WM * LM * TM, BN = WN * LN * TN;
+    static constexpr int WARPS_M = WM, LANES_M = LM, ROWS = TM, COLS = TN, SLICE = KS;
+    static constexpr int FETCH_ROWS = THREADS / (KS / 4), FA = BM / FETCH_ROWS, FW = BN / FETCH_ROWS;
+    static_assert(BM % FETCH_ROWS == 0 && BN % FETCH_ROWS == 0 && TM % 4 == 0 && TN % 4 == 0, "whole rounds of 16-byte loads");
+};
+typedef PackedTile<2, 2, 4, 8, 4, 16> Packed64x64;
+typedef PackedTile<2, 2, 4, 4, 4, 32> Packed32x64;
+
+template <typename P, typename TA, typename TW, typename TC>
+__global__ void __launch_bounds__(P::THREADS, 4) gemm_packed_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, int M,
+                                                                    int N, int K, long long lda, long long ldw, long long ldc, int mode) {
+    constexpr int TM = P::ROWS, TN = P::COLS, KS = P::SLICE, LM = P::LANES_M, LN = P::LN;
+    __shared__ __align__(16) float As[2][KS][P::BM + 4];
+    __shared__ __align__(16) float Ws[2][KS][P::BN + 4];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // a thread's rows: four at m1, four 4 * LM further on, ...; its columns likewise
+    const int m1 = (warp % P::WARPS_M) * LM * TM + (lane / LN) * 4, n1 = (warp / P::WARPS_M) * LN * TN + (lane % LN) * 4;
+    const int m0 = blockIdx.y * P::BM, n0 = blockIdx.x * P::BN;
+    const int lr = tid / (KS / 4), lk = (tid % (KS / 4)) * 4;      // the row (and those FETCH_ROWS further on) and the k's this thread fetches
+    simt_pair acc[TM / 2][TN];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < NQ * 4; ++j) acc[i][j] = 0ull;
-    float fa[2][4], fw[NQ][4];
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+    float fa[P::FA][4], fw[P::FW][4];
     auto fetch = [&](int k0) {
         const int gk = k0 + lk;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int gm = m0 + lr + 64 * h;
+        for (int h = 0; h < P::FA; ++h) {
+            const int gm = m0 + lr + P::FETCH_ROWS * h;
             if (gm < M && gk < K) Vec4Load<TA>::load(A + (size_t)gm * lda + gk, fa[h]);
             else
 #pragma unroll
                 for (int e = 0; e < 4; ++e) fa[h][e] = 0.f;
         }
 #pragma unroll
-        for (int h = 0; h < NQ; ++h) {
-            const int gn = n0 + lr + 64 * h;
+        for (int h = 0; h < P::FW; ++h) {
+            const int gn = n0 + lr + P::FETCH_ROWS * h;
             if (gn < N && gk < K) Vec4Load<TW>::load(W + (size_t)gn * ldw + gk, fw[h]);
             else
 #pragma unroll
@@ -153,35 +165,36 @@ __global__ void __launch_bounds__(256, 2) gemm_wide_kernel(const TA* __restrict_
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) As[buf][lk + e][lr + 64 * h] = fa[h][e];
+            for (int h = 0; h < P::FA; ++h) As[buf][lk + e][lr + P::FETCH_ROWS * h] = fa[h][e];
 #pragma unroll
-            for (int h = 0; h < NQ; ++h) Ws[buf][lk + e][lr + 64 * h] = fw[h][e];
+            for (int h = 0; h < P::FW; ++h) Ws[buf][lk + e][lr + P::FETCH_ROWS * h] = fw[h][e];
         }
     };
     fetch(0);
     put(0);
     __syncthreads();
     int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += WIDE_K, buf ^= 1) {
-        const bool more = k0 + WIDE_K < K;
-        if (more) fetch(k0 + WIDE_K);
+    for (int k0 = 0; k0 < K; k0 += KS, buf ^= 1) {
+        const bool more = k0 + KS < K;
+        if (more) fetch(k0 + KS);
 #pragma unroll
-        for (int kk = 0; kk < WIDE_K; ++kk) {
-            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][ty * 8]);
-            const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][ty * 8 + 4]);
-            const simt_pair a[4] = {a0.x, a0.y, a1.x, a1.y};
+        for (int kk = 0; kk < KS; ++kk) {
+            simt_pair a[TM / 2];
+            float w[TN];
 #pragma unroll
-            for (int g = 0; g < NQ; ++g) {
-                const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][kk][g * 64 + tx * 4]);
-                const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+            for (int g = 0; g < TM / 4; ++g) {
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][m1 + g * LM * 4]);
+                a[2 * g] = t.x;
+                a[2 * g + 1] = t.y;
+            }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    simt_pair both;
-                    asm("mov.b64 %0, {%1, %1};" : "=l"(both) : "f"(w[j]));
+            for (int g = 0; g < TN / 4; ++g) *reinterpret_cast<float4*>(w + 4 * g) = *reinterpret_cast<const float4*>(&Ws[buf][kk][n1 + g * LN * 4]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][g * 4 + j]) : "l"(a[i]), "l"(both));
-                }
+            for (int j = 0; j < TN; ++j) {
+                simt_pair both;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(both) : "f"(w[j]));
+#pragma unroll
+                for (int i = 0; i < TM / 2; ++i) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(a[i]), "l"(both));
             }
         }
         if (more) put(buf ^ 1);
@@ -189,12 +202,12 @@ __global__ void __launch_bounds__(256, 2) gemm_wide_kernel(const TA* __restrict_
     }
     const bool whole = N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)C & 15) == 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int gm = m0 + ty * 8 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int gm = m0 + m1 + (i / 4) * LM * 4 + i % 4;
         if (gm >= M) continue;
 #pragma unroll
-        for (int g = 0; g < NQ; ++g) {
-            const int gn = n0 + g * 64 + tx * 4;
+        for (int g = 0; g < TN / 4; ++g) {
+            const int gn = n0 + n1 + g * LN * 4;
             float v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -219,6 +232,13 @@ __global__ void __launch_bounds__(256, 2) gemm_wide_kernel(const TA* __restrict_
             }
         }
     }
+}
+
+template <typename P, typename TA, typename TW, typename TC>
+static void packed_launch(const TA* A, const TW* W, TC* C, int M, int N, int K, long long lda, long long ldw, long long ldc, int mode,
+                          cudaStream_t stream) {
+    gemm_packed_kernel<P, TA, TW, TC><<<dim3(gb_ceil_div(N, P::BN), gb_ceil_div(M, P::BM)), P::THREADS, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc,
+                                                                                                                 mode);
 }
 
 // ------------------------------------------------------------------- weight-streaming kernel
@@ -278,17 +298,11 @@ static int launch_gemm(const void* a, const void* w, void* c, int M, int N, int 
         if (vec) gemm_skinny_kernel<TA, TW, TC, true><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
         else gemm_skinny_kernel<TA, TW, TC, false><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
     } else {
-        // The tile whose rounds over the SMs end soonest; a wide tile has a quarter more than an SM's share of the outputs at
-        // most before the 64 x 64 tiles, which run at half its rate, would be level.
         if constexpr (sizeof(TA) == 4 && sizeof(TC) == 4) {
-            const long long rows = gb_ceil_div(M, WIDE_M);
-            const long long t128 = rows * gb_ceil_div(N, 128), t64 = rows * gb_ceil_div(N, 64);
-            const long long small = (long long)gb_ceil_div(M, BM) * gb_ceil_div(N, BN);
-            const long long c128 = 4 * ((t128 + 147) / 148), c64 = 2 * ((t64 + 147) / 148);        // in 64 x 64 outputs an SM
-            const long long c_small = 2 * ((small + 147) / 148);
-            if (vec && M > 64 && (c64 <= c_small || c128 <= c_small)) {
-                if (c128 < c64) gemm_wide_kernel<TA, TW, TC, 128><<<dim3(gb_ceil_div(N, 128), rows), 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
-                else gemm_wide_kernel<TA, TW, TC, 64><<<dim3(gb_ceil_div(N, 64), rows), 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
+            if (vec) {
+                if ((long long)gb_ceil_div(M, Packed32x64::BM) * gb_ceil_div(N, Packed32x64::BN) <= 148)
+                    packed_launch<Packed32x64>(A, W, C, M, N, K, lda, ldw, ldc, mode, stream);
+                else packed_launch<Packed64x64>(A, W, C, M, N, K, lda, ldw, ldc, mode, stream);
                 return gb_check_launch("gb_gemm_simt");
             }
         }

@@ -1303,22 +1303,19 @@ def test_attention_prefill_float32_rows_beyond_the_table_and_padding_read_nothin
 
 
 @pytest.mark.parametrize("w_dt", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("M, N, K", [(2048, 576, 576), (1025, 960, 100), (2047, 2500, 36), (4000, 577, 20)])
-def test_gemm_simt_wide_tiles_give_the_bits_of_the_small_ones(M, N, K, w_dt):
-    """Both tiled kernels add one product after the other: the wide tiles' bits are those of a call small enough for the
-    64 x 64 tiles, at sizes with ragged edges in every direction, stored and added."""
+@pytest.mark.parametrize("M, N, K", [(2048, 576, 576), (1025, 960, 100), (2047, 2500, 36), (4000, 577, 20), (9, 65, 4), (33, 64, 132), (95, 1000, 68)])
+def test_gemm_simt_packed_tiles_give_the_bits_of_the_plain_ones(M, N, K, w_dt):
+    """All tiled kernels add one product after the other: the packed tiles' bits are those of the plain 64 x 64 tile (which rows
+    that are not aligned to 16 bytes still take), at sizes with ragged edges in every direction, stored and added."""
     from glassbox_b200 import kernels
     torch.manual_seed(M + N)
     a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV).to(w_dt)
     c = torch.randn(M, N, device=DEV)
-    got, added = torch.empty(M, N, device=DEV), c.clone()
+    got, added, plain = torch.empty(M, N, device=DEV), c.clone(), torch.empty(M, N, device=DEV)
     kernels.gemm_simt(a, w, got)
     kernels.gemm_simt(a, w, added, accumulate=True)
-    small = torch.empty(M, N, device=DEV)
-    for lo in range(0, M, 40):
-        hi = min(M, lo + 40) if M - lo >= 49 else M
-        kernels.gemm_simt(a[lo:hi], w, small[lo:hi])
-        if hi == M:
-            break
-    assert torch.equal(got, small) and torch.equal(added, c + small)
+    odd = torch.zeros(M, K + 1, device=DEV)
+    odd[:, 1:] = a
+    kernels.gemm_simt(odd[:, 1:], w, plain)
+    assert torch.equal(got, plain) and torch.equal(added, c + plain)
     assert (got.double() - a.double() @ w.double().T).abs().max() <= 1e-5 * K ** 0.5 * 4
