@@ -53,6 +53,9 @@ _SIGNATURES = {
     "gb_attention_decode_counters": [_I, _I, _I],
     "gb_gemm_stream_row_groups": [_I, _I, _I, _I],
     "gb_gemm_stream": [_P, _LL, _P, _LL, _P, _F, _P, _LL, _P, _LL, _I, _I, _I, _I, _P, _LL, _I, _P],
+    "gb_gemm_few_supported": [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL],
+    "gb_gemm_few": [_P, _LL, _P, _LL, _P, _LL, _I, _I, _I, _I, _P, _I, _P],
+    "gb_gemm_few_qkv": [_P, _LL, _P, _LL, _P, _LL, _I, _I, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _LL, _I, _P, _I, _P],
     "gb_gemm_stream_qkv": [_P, _LL, _P, _LL, _P, _F, _P, _LL, _P, _LL, _I, _I, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I,
                            _LL, _I, _P, _P, _LL, _I, _P],
     "gb_attention_decode_mma_pdl": [_P, _LL, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _LL, _F, _I, _I, _P, _P,
@@ -577,6 +580,44 @@ def gemm_stream_qkv(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cos_s
           _ptr(cos_sin), cos_sin.shape[0] if cos_sin is not None else 0, _ptr(positions), _ptr(slots), _ptr(kcache),
           _ptr(vcache), nh, nkv, hd, page_size, kcache.shape[0], 1 if write_kv else 0, _ptr(status),
           *_prefetch_args(prefetch), 1 if USE_PDL else 0, _stream())
+
+
+def gemm_few_supported(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, gated: bool = False) -> bool:
+    """Whether the tcgen05 kernel for few rows (W as the full-height operand, K split over a cluster) takes these operands."""
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or c.dtype not in (torch.bfloat16, torch.float32) or a.shape[0] > STREAM_MAX_ROWS:
+        return False
+    return bool(lib().gb_gemm_few_supported(_ptr(a), _ptr(w), _ptr(c), a.shape[0], w.shape[0] // (2 if gated else 1), a.shape[1], a.stride(0),
+                                            w.stride(0), c.stride(0)))
+
+
+def gemm_few(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, status: torch.Tensor, accumulate: bool = False, gated: bool = False,
+             relu2: bool = False, gelu: bool = False) -> None:
+    """``gemm_stream`` without a norm for up to 64 rows on tcgen05; ``status`` is the word in which a wait that gives up is recorded."""
+    _cuda(a, w, c, status)
+    M, K = a.shape
+    N = w.shape[0] // 2 if gated else w.shape[0]
+    assert w.shape[1] == K and c.shape == (M, N) and a.stride(1) == 1 and w.stride(1) == 1 and c.stride(1) == 1
+    assert c.dtype == (torch.float32 if accumulate else c.dtype) and not ((gated or relu2 or gelu) and c.dtype != torch.bfloat16)
+    mode = 3 if gated else 5 if relu2 else 7 if gelu else 2 if accumulate else 0 if c.dtype == torch.bfloat16 else 1
+    _call("gb_gemm_few", _ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(c), c.stride(0), mode, M, N, K, _ptr(status), 1 if USE_PDL else 0, _stream())
+
+
+def gemm_few_qkv_supported(a: torch.Tensor, w: torch.Tensor, hd: int, q_out: torch.Tensor, kcache: torch.Tensor) -> bool:
+    return (hd in (64, 128) and q_out.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16 and gemm_few_supported(a, w, q_out))
+
+
+def gemm_few_qkv(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cos_sin: Optional[torch.Tensor], positions: torch.Tensor,
+                 slots: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, nh: int, nkv: int, hd: int, page_size: int, write_kv: bool,
+                 status: torch.Tensor) -> None:
+    """``gemm_tc_qkv`` for up to 64 rows on the tcgen05 kernel for few rows."""
+    _cuda(a, w, q_out, cos_sin, positions, slots, kcache, vcache, status)
+    M, K = a.shape
+    assert w.shape == ((nh + 2 * nkv) * hd, K) and a.stride(1) == 1 and w.stride(1) == 1 and q_out.stride(1) == 1
+    assert q_out.shape[0] == M and q_out.shape[1] >= nh * hd and kcache.is_contiguous() and vcache.is_contiguous()
+    assert cos_sin is None or (cos_sin.dtype == torch.float32 and cos_sin.shape[1:] == (hd // 2, 2) and cos_sin.is_contiguous())
+    _call("gb_gemm_few_qkv", _ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(q_out), q_out.stride(0), M, K, _ptr(cos_sin),
+          cos_sin.shape[0] if cos_sin is not None else 0, _ptr(positions), _ptr(slots), _ptr(kcache), _ptr(vcache), nh, nkv, hd, page_size,
+          kcache.shape[0], 1 if write_kv else 0, _ptr(status), 1 if USE_PDL else 0, _stream())
 
 
 def gemm_tc_supported(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> bool:

@@ -14,7 +14,7 @@ import torch
 from .. import kernels
 from ..weights.binding import ParamSpec
 from .base import Mixer, PagedKvSpec, Position, build_part, register_part
-from .linear import _resolve, linear, weights_ahead
+from .linear import _few_rows, _resolve, linear, weights_ahead
 
 
 class GqaAttention(Mixer):
@@ -52,10 +52,15 @@ class GqaAttention(Mixer):
         n = h.shape[0]
         qkv = ctx.scratch("qkv", (n, self.qd + 2 * self.kvd))
         table = self.position.fused_table(qkv.device)
-        x, norm, _, scale = _resolve(h, self.params["wqkv"])
         plain_rotary = (table is not None and self.position.rotary_dim == self.hd) or \
             (table is None and type(self.position).apply_qk is Position.apply_qk)
-        if (plain_rotary and (norm is not None or x.dtype == torch.bfloat16)
+        few = _few_rows(h, self.params["wqkv"], qkv) if plain_rotary and qkv.dtype == torch.bfloat16 and self.hd in (64, 128) else None
+        x, norm, _, scale = _resolve(h, self.params["wqkv"]) if few is None else (few, None, None, None)
+        if few is not None and kernels.gemm_few_qkv_supported(few, self.params["wqkv"], self.hd, qkv, cache.k):
+            # a decode batch against a large matrix: one kernel projects, rotates and writes the cache
+            kernels.gemm_few_qkv(few, self.params["wqkv"], qkv, table, ctx.positions, cache.slots, cache.k, cache.v, self.nh, self.nkv,
+                                 self.hd, cache.page_size, writes_cache, ctx.status)
+        elif (plain_rotary and (norm is not None or x.dtype == torch.bfloat16)
                 and kernels.gemm_stream_qkv_supported(x, self.params["wqkv"], self.hd, qkv)):
             # few rows: one kernel normalises, projects, rotates and writes the cache
             kernels.gemm_stream_qkv(x, self.params["wqkv"], qkv, table, ctx.positions, cache.slots, cache.k, cache.v,

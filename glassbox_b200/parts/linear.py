@@ -62,9 +62,41 @@ def _tile_kernel_wins(rows: int, w: torch.Tensor) -> bool:
     return (rows > 16 and n >= 16384) or (rows > 32 and n >= 4096 and k >= 1024)
 
 
+#: weight bytes from which the tcgen05 kernel for few rows is the fast one (``_few_rows``)
+FEW_MIN_BYTES, FEW_BIG_BYTES = 4_800_000, 32 << 20
+
+
+def _few_rows(a, w: torch.Tensor, out: torch.Tensor, gated: bool = False):
+    """The input rows as the tcgen05 kernel for few rows takes them, if that kernel is the fast one here; else None.
+    Measured alone (csrc/gemm_few_tc.cu): with 17 to 64 rows it wins from about 5 MB of weights on, with 9 to 16 rows from
+    there where K is long (2,048 or more) or from 16 MB on; at 8 rows the streaming kernel is level or better. The streaming
+    kernel applies a norm on the way in, which costs a launch of its own here (2 to 3 us): that is worth it for the largest
+    matrices only (2 x 8192 x 2048 at 16 rows: 17 us against 24). More tiles than the chip has multiprocessors (a head) stay
+    with the other kernels."""
+    rows, (n, k) = a.shape[0], w.shape
+    size = 2 * n * k
+    if not 8 < rows <= kernels.STREAM_MAX_ROWS or size < FEW_MIN_BYTES or -(-n // 128) > 148:
+        return None
+    if rows <= 16 and k < 2048 and size < (16 << 20):
+        return None
+    if isinstance(a, DeferredNorm):
+        if a.prepared() is not None or (size < FEW_BIG_BYTES and a.norm.as_rms() is not None and a._tensor is None and kernels.stream_folds(rows, w)):
+            return None
+        if w.dtype != torch.bfloat16:
+            return None
+        a = a.tensor()
+    return a if kernels.gemm_few_supported(a, w, out, gated) else None
+
+
 def linear(ctx, a, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> None:
     """``a`` is a tensor or a ``DeferredNorm``; the latter is folded into the weight-streaming kernel
     when that kernel runs, and computed first otherwise."""
+    few = _few_rows(a, w, out)
+    if few is not None:
+        if accumulate:
+            ctx.prepared_norm = None
+        kernels.gemm_few(few, w, out, ctx.status, accumulate)
+        return
     x, norm, deferred, scale = _resolve(a, w)
     if accumulate:
         ctx.prepared_norm = None      # ``out`` changes: what was prepared from its old values is void
@@ -103,6 +135,10 @@ def gated_linear(ctx, a, w_gate_up: torch.Tensor, act: torch.Tensor, unit: str =
             a = a.tensor()
         return clamped_glu_linear(ctx, a, w_gate_up, None, *kernels.GELU_UNIT, act)
     inter = w_gate_up.shape[0] // 2
+    few = _few_rows(a, w_gate_up, act, gated=True) if act.dtype == torch.bfloat16 else None
+    if few is not None:
+        kernels.gemm_few(few, w_gate_up, act, ctx.status, gated=True)
+        return True
     x, norm, _, scale = _resolve(a, w_gate_up)
     if scale is not None:
         if (w_gate_up.dtype == torch.bfloat16 and act.dtype == torch.bfloat16
@@ -136,6 +172,10 @@ def activated_linear(ctx, a, w: torch.Tensor, act: torch.Tensor, unit: str) -> b
     which = {unit: True}
     if w.dtype != torch.bfloat16 or act.dtype != torch.bfloat16:
         return False
+    few = _few_rows(a, w, act)
+    if few is not None:
+        kernels.gemm_few(few, w, act, ctx.status, **which)
+        return True
     x, norm, deferred, scale = _resolve(a, w)
     if scale is not None:
         x, scale = deferred.tensor(), None
