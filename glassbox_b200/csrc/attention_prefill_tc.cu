@@ -257,31 +257,29 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
         if (bad && what == 0) atomicOr(status, GB_STATUS_BAD_SLOT);
     } else if (warp == 1) {
         // ------------------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_qk = umma_idesc(AT_BM, AT_BN);
             const uint32_t idesc_pv = umma_idesc(AT_BM, HD) | (1u << 16);   // B is MN-major
-            const uint32_t q_addr = smem_u32(Qs), k_addr = smem_u32(Ks), v_addr = smem_u32(Vs);
+            const uint64_t q_desc = umma_desc(smem_u32(Qs)), k_desc = umma_desc(smem_u32(Ks)), v_desc = umma_desc_mn(smem_u32(Vs), AT_BN * 128);
             bool ok = mbar_wait(&sh.q_full, 0, abort_flag, status);
             if (ok) sh.q_consumed = 1;
             // Whatever is ready is issued: S_j as soon as its keys have landed and its group has read S_{j-2} out of
             // the buffer (so S runs up to two tiles ahead and neither softmax group waits for the other), O += P_j V_j
             // as soon as P_j is written and its values have landed. The loop polls without blocking; the limit
-            // counts from the last instruction issued.
+            // counts from the first look that found nothing.
             int next_qk = 0, next_pv = 0;
-            long long t_last = clock64();
+            long long t_idle = 0;
             while (ok && next_pv < ntiles) {
                 bool progressed = false;
                 if (next_qk < ntiles) {
                     const int j = next_qk, st = j % AT_STAGES;
                     if (mbar_test(&sh.k_full[st], (j / AT_STAGES) & 1) &&
                         (j < 2 || mbar_test(&sh.s_free[j & 1], ((j >> 1) - 1) & 1))) {
-                        sh.consumed[0] = j + 1;
                         tc_fence_after();
-                        const uint32_t kb = k_addr + (uint32_t)(st * G::KV_BYTES);
+                        const uint64_t kd = k_desc + (uint64_t)((st * G::KV_BYTES) >> 4);
 #pragma unroll
                         for (int k = 0; k < HD / 16; ++k)
-                            umma_bf16(tmem + (uint32_t)((j & 1) * AT_BN), umma_desc(q_addr + k * 32), umma_desc(kb + k * 32),
-                                      idesc_qk, k ? 1u : 0u);
+                            umma_bf16(tmem + (uint32_t)((j & 1) * AT_BN), q_desc + k * 2, kd + k * 2, idesc_qk, k ? 1u : 0u);
                         umma_commit(&sh.s_full[j & 1]);
                         umma_commit(&sh.k_empty[st]);
                         ++next_qk;
@@ -291,14 +289,13 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
                 if (next_pv < next_qk) {
                     const int j = next_pv, st = j % AT_STAGES;
                     if (mbar_test(&sh.p_ready[j & 1], (j >> 1) & 1) && mbar_test(&sh.v_full[st], (j / AT_STAGES) & 1)) {
-                        sh.consumed[1] = j + 1;
                         tc_fence_after();
-                        const uint32_t vb = v_addr + (uint32_t)(st * G::KV_BYTES);
+                        const uint64_t vd = v_desc + (uint64_t)((st * G::KV_BYTES) >> 4);
                         const uint32_t pt = tmem + (uint32_t)(G::P_COL + (j & 1) * (AT_BN / 2));
 #pragma unroll
                         for (int kk = 0; kk < AT_BN / 16; ++kk)   // 16 keys per instruction: 8 columns of P
                             umma_bf16_ts(tmem + (uint32_t)(G::O_COL + (j & 1) * HD), pt + (uint32_t)(kk * 8),
-                                         umma_desc_mn(vb + kk * 16 * 128, AT_BN * 128), idesc_pv, (j >= 2 || kk) ? 1u : 0u);
+                                         vd + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, (j >= 2 || kk) ? 1u : 0u);
                         umma_commit(&sh.pv_done[j & 1]);
                         umma_commit(&sh.v_empty[st]);
                         ++next_pv;
@@ -306,15 +303,19 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
                     }
                 }
                 if (progressed) {
-                    t_last = clock64();
+                    t_idle = 0;
                 } else if (*abort_flag) {
                     ok = false;
-                } else if (clock64() - t_last > TC_WAIT_CYCLES) {
+                } else if (t_idle == 0) {
+                    t_idle = clock64();
+                } else if (clock64() - t_idle > TC_WAIT_CYCLES) {
                     *abort_flag = 1;
                     atomicOr(status, GB_STATUS_WAIT_TIMEOUT);
                     ok = false;
                 }
             }
+            sh.consumed[0] = next_qk;
+            sh.consumed[1] = next_pv;
         }
     } else {
         // ------------------------------------------------------------------------- softmax

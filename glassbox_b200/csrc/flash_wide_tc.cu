@@ -193,9 +193,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         if (bad && what == 0) atomicOr(a.status, GB_STATUS_BAD_SLOT);
     } else if (warp == 1) {
         // ------------------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_qk = umma_idesc(FW_BM, FW_BN), idesc_pv = umma_idesc(FW_BM, DV) | (1u << 16);     // (B is MN-major)
-            const uint32_t q_addr = smem_u32(Qs), k_addr = smem_u32(Ks), v_addr = smem_u32(Vs);
+            const uint64_t q_desc = umma_desc(smem_u32(Qs)), k_desc = umma_desc(smem_u32(Ks)), v_desc = fw_desc_mn(smem_u32(Vs));
             bool ok = mbar_wait(&sh.q_full, 0, abort_flag, a.status);
             if (ok) sh.q_consumed = 1;
             auto scores = [&](int j) {
@@ -203,10 +203,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 if (!mbar_wait(&sh.k_full[s], (j / G::K_STAGES) & 1, abort_flag, a.status)) return false;
                 sh.consumed[0] = j + 1;
                 tc_fence_after();
-                const uint32_t kb = k_addr + (uint32_t)(s * G::K_BYTES);
+                const uint64_t kd = k_desc + (uint64_t)((s * G::K_BYTES) >> 4);
                 for (int k = 0; k < a.key_steps; ++k) {
-                    const uint32_t at = (uint32_t)((k >> 2) * FW_BLOCK + (k & 3) * 32);
-                    umma_bf16(tmem + (uint32_t)((j & 1) * FW_BN), umma_desc(q_addr + at), umma_desc(kb + at), idesc_qk, k ? 1u : 0u);
+                    const uint64_t at = (uint64_t)(((k >> 2) * FW_BLOCK + (k & 3) * 32) >> 4);
+                    umma_bf16(tmem + (uint32_t)((j & 1) * FW_BN), q_desc + at, kd + at, idesc_qk, k ? 1u : 0u);
                 }
                 umma_commit(&sh.s_full[j & 1]);
                 if (!LATENT) umma_commit(&sh.k_empty[s]);
@@ -219,10 +219,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 if (!LATENT) sh.consumed[1] = j + 1;
                 if (!(ok = mbar_wait(&sh.p_ready[j & 1], (j >> 1) & 1, abort_flag, a.status))) break;
                 tc_fence_after();
-                const uint32_t vb = v_addr + (uint32_t)(s * (LATENT ? G::K_BYTES : G::V_BYTES));
+                const uint64_t vd = v_desc + (uint64_t)((s * (LATENT ? G::K_BYTES : G::V_BYTES)) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < FW_BN / 16; ++kk)         // 16 keys an instruction: 8 columns of P, 16 rows of the values
-                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + kk * 8), fw_desc_mn(vb + kk * 16 * 128), idesc_pv,
+                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + kk * 8), vd + (uint64_t)((kk * 16 * 128) >> 4), idesc_pv,
                                  (j | kk) ? 1u : 0u);
                 umma_commit(&sh.pv_done);
                 umma_commit(LATENT ? &sh.k_empty[s] : &sh.v_empty[s]);

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_few_kernel(const __grid_const
     gb_pdl_launch_dependents();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             auto weights = [&](int it) {
                 unsigned char* dst = stages + (it % GF_STAGES) * GF_STAGE;
                 uint64_t* bar = &sh.full[it % GF_STAGES];
@@ -134,22 +134,25 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_few_kernel(const __grid_const
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc(GF_BM, a.x_rows);
+            const uint64_t w_desc = umma_desc(smem_u32(stages)), x_desc = umma_desc(smem_u32(stages) + GF_W_BYTES);
+            int consumed = 0;
             bool ok = true;
             for (int it = 0; it < kblocks && ok; ++it) {
                 const int s = it % GF_STAGES;
                 if (!(ok = mbar_wait(&sh.full[s], (it / GF_STAGES) & 1, abort_flag, a.status))) break;
-                sh.consumed = it + 1;
+                consumed = it + 1;
                 tc_fence_after();
-                const uint32_t w_addr = smem_u32(stages + s * GF_STAGE), x_addr = w_addr + GF_W_BYTES;
+                const uint64_t step = (uint64_t)((s * GF_STAGE) >> 4);
 #pragma unroll
                 for (int k = 0; k < GF_BK / 16; ++k)
-                    umma_bf16(tmem, umma_desc(w_addr + (k >> 2) * (GF_W_BYTES / 2) + (k & 3) * 32),
-                              umma_desc(x_addr + (k >> 2) * (GF_X_BYTES / 2) + (k & 3) * 32), idesc, (it | k) ? 1u : 0u);
+                    umma_bf16(tmem, w_desc + step + (((k >> 2) * (GF_W_BYTES / 2) + (k & 3) * 32) >> 4),
+                              x_desc + step + (((k >> 2) * (GF_X_BYTES / 2) + (k & 3) * 32) >> 4), idesc, (it | k) ? 1u : 0u);
                 umma_commit(&sh.empty[s]);
             }
             if (ok) umma_commit(&sh.tfull);
+            sh.consumed = consumed;
         }
         __syncwarp();
         gb_pdl_wait();

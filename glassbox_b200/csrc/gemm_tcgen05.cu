@@ -146,53 +146,57 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     gb_pdl_wait();
 
     if (warp == 0) {
-        if (lane == 0 && kblocks > 0) {
+        if (kblocks > 0 && elect_one()) {
             // --------------------------------------------------------------------- producer
-            int it = 0;
+            int issued = 0, s = 0, phase = 1;
             bool ok = true;
             for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
                 const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BNO;
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (it >= STAGES && !mbar_wait(&sh.empty[s], ((it / STAGES) - 1) & 1, abort_flag, status)) { ok = false; break; }
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (issued >= STAGES && !mbar_wait(&sh.empty[s], phase, abort_flag, status)) { ok = false; break; }
                     unsigned char* a_dst = tiles + s * G::STAGE_BYTES;
                     mbar_expect_tx(&sh.full[s], G::STAGE_BYTES);
                     tma_load_2d(a_dst, &map_a, &sh.full[s], kb * TC_BK, m0);
-                    if (GATED) {
-                        tma_load_2d(a_dst + G::A_BYTES, &map_w, &sh.full[s], kb * TC_BK, n0);
-                        tma_load_2d(a_dst + G::A_BYTES + G::W_BYTES / 2, &map_w, &sh.full[s], kb * TC_BK, gate_rows + n0);
-                    } else {
-                        tma_load_2d(a_dst + G::A_BYTES, &map_w, &sh.full[s], kb * TC_BK, n0);
-                    }
-                    sh.issued = it + 1;
+                    tma_load_2d(a_dst + G::A_BYTES, &map_w, &sh.full[s], kb * TC_BK, n0);
+                    if (GATED) tma_load_2d(a_dst + G::A_BYTES + G::W_BYTES / 2, &map_w, &sh.full[s], kb * TC_BK, gate_rows + n0);
+                    ++issued;
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
             }
+            sh.issued = issued;
         }
     } else if (warp == 1) {
-        if (lane == 0 && kblocks > 0) {
+        if (kblocks > 0 && elect_one()) {
             // --------------------------------------------------------------------- MMA issuer
+            // The issue loop has to stay below the tensor core's time for a k-block (256 cycles at BN = 128): one elected thread,
+            // descriptors formed once and advanced by additions, the next stage's barrier looked at before this stage's
+            // products are waited for. Together with the epilogue's early residual loads, 2,048 rows: K 1536, N 576 add
+            // 13.7 -> 10.8 us, gated K 576, I 1536 14.1 -> 11.4 (back to back, weights from HBM).
             const uint32_t idesc = umma_idesc(TC_BM, BN);
-            int it = 0, tcount = 0;
-            bool ok = true;
+            const uint64_t a_desc = umma_desc(smem_u32(tiles)), w_desc = umma_desc(smem_u32(tiles) + G::A_BYTES);
+            int s = 0, phase = 0, tcount = 0, consumed = 0;
+            bool ok = true, ready = false;
             for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
                 const int acc = tcount & 1;
                 if (tcount >= 2 && !mbar_wait(&sh.tempty[acc], ((tcount >> 1) - 1) & 1, abort_flag, status)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem + (uint32_t)(acc * BN);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(&sh.full[s], (it / STAGES) & 1, abort_flag, status)) { ok = false; break; }
-                    sh.consumed = it + 1;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!ready && !mbar_wait(&sh.full[s], phase, abort_flag, status)) { ok = false; break; }
+                    ++consumed;
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(tiles + s * G::STAGE_BYTES);
-                    const uint32_t w_addr = a_addr + G::A_BYTES;
+                    const uint64_t step = (uint64_t)((s * G::STAGE_BYTES) >> 4);
+                    uint64_t* done = &sh.empty[s];
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
 #pragma unroll
                     for (int k = 0; k < TC_BK / 16; ++k)   // 16 bfloat16 = 32 bytes further along K inside the swizzled row
-                        umma_bf16(d_tmem, umma_desc(a_addr + k * 32), umma_desc(w_addr + k * 32), idesc, (kb | k) ? 1u : 0u);
-                    umma_commit(&sh.empty[s]);       // arrives when the MMAs above have read the stage
+                        umma_bf16(d_tmem, a_desc + step + k * 2, w_desc + step + k * 2, idesc, (kb | k) ? 1u : 0u);
+                    umma_commit(done);                   // arrives when the MMAs above have read the stage
+                    ready = mbar_test(&sh.full[s], phase);
                 }
                 if (ok) umma_commit(&sh.tfull[acc]);   // arrives when the tile's MMAs have finished
             }
+            sh.consumed = consumed;
         }
     } else {
         // ------------------------------------------------------------------------- epilogue
@@ -219,6 +223,16 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                 }
                 inv_rms = 1.0f / sqrtf(ss / (float)K + norm.eps);
             }
+            // mode TC_ADD_F32: the residual values of the next 32 columns to be written, requested while the tile's products (or
+            // the columns before) are still under way
+            float old[32];
+            const int rows_here = min(32, M - (m0 + q * 32));
+            auto load_old = [&](int col) {
+                const float* base = reinterpret_cast<const float*>(C) + (size_t)(m0 + q * 32) * ldc + col;
+#pragma unroll
+                for (int rr = 0; rr < 32; ++rr) old[rr] = (col < N && rr < rows_here) ? base[(size_t)rr * ldc] : 0.f;
+            };
+            if (!GATED && mode == TC_ADD_F32) load_old(n0 + lane);
             if (kblocks > 0) {
                 if (!mbar_wait_warp(&sh.tfull[acc], (tcount >> 1) & 1, abort_flag, status)) { ok = false; break; }
                 tc_fence_after();
@@ -401,31 +415,25 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                 for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(r[j]);
                 __syncwarp();
                 const int col = col0 + lane;
-                if (col < N) {
-                    float* base = reinterpret_cast<float*>(C) + (size_t)(m0 + q * 32) * ldc + col;
-                    const int rows = min(32, M - (m0 + q * 32));
-                    if (mode == TC_ADD_F32) {
-                        float old[32];   // read the 32 residual values first (independent loads), then add and write
+                float* base = reinterpret_cast<float*>(C) + (size_t)(m0 + q * 32) * ldc + col;
+                if (mode == TC_ADD_F32) {
 #pragma unroll
-                        for (int rr = 0; rr < 32; ++rr) old[rr] = rr < rows ? base[(size_t)rr * ldc] : 0.f;
-                        if (norm.gain != nullptr) {
-                            // producer half of a split RMSNorm: the new residual values go back into the tile as well
+                    for (int rr = 0; rr < 32; ++rr) old[rr] += stage[rr * 33 + lane];
+                    if (norm.gain != nullptr) {
+                        // producer half of a split RMSNorm: the new residual values go back into the tile as well
 #pragma unroll
-                            for (int rr = 0; rr < 32; ++rr) {
-                                const float v = old[rr] + stage[rr * 33 + lane];
-                                if (rr < rows) base[(size_t)rr * ldc] = v;
-                                stage[rr * 33 + lane] = v;
-                            }
-                        } else {
-#pragma unroll
-                            for (int rr = 0; rr < 32; ++rr)
-                                if (rr < rows) base[(size_t)rr * ldc] = old[rr] + stage[rr * 33 + lane];
-                        }
-                    } else {
+                        for (int rr = 0; rr < 32; ++rr) stage[rr * 33 + lane] = old[rr];
+                    }
+                    if (col < N) {
 #pragma unroll
                         for (int rr = 0; rr < 32; ++rr)
-                            if (rr < rows) base[(size_t)rr * ldc] = stage[rr * 33 + lane];
+                            if (rr < rows_here) base[(size_t)rr * ldc] = old[rr];
                     }
+                    if (c0 + 32 < BNO) load_old(col + 32);
+                } else if (col < N) {
+#pragma unroll
+                    for (int rr = 0; rr < 32; ++rr)
+                        if (rr < rows_here) base[(size_t)rr * ldc] = stage[rr * 33 + lane];
                 }
                 __syncwarp();
                 if (mode == TC_ADD_F32 && norm.gain != nullptr) {

@@ -159,28 +159,32 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc(ME_BM, BN);
-            int it = 0, tcount = 0;
-            bool ok = true;
+            const uint64_t a_desc = umma_desc(smem_u32(tiles)), w_desc = umma_desc(smem_u32(tiles) + G::A_BYTES);
+            int s = 0, phase = 0, tcount = 0, consumed = 0;
+            bool ok = true, ready = false;
             for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
                 const int acc = tcount & 1;
                 if (tcount >= 2 && !mbar_wait(&sh.tempty[acc], ((tcount >> 1) - 1) & 1, abort_flag, status)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem + (uint32_t)(acc * BN);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(&sh.full[s], (it / STAGES) & 1, abort_flag, status)) { ok = false; break; }
-                    sh.consumed = it + 1;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!ready && !mbar_wait(&sh.full[s], phase, abort_flag, status)) { ok = false; break; }
+                    ++consumed;
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(tiles + s * G::STAGE_BYTES), w_addr = a_addr + G::A_BYTES;
+                    const uint64_t step = (uint64_t)((s * G::STAGE_BYTES) >> 4);
+                    uint64_t* done = &sh.empty[s];
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
 #pragma unroll
                     for (int k = 0; k < ME_BK / 16; ++k)
-                        umma_bf16(d_tmem, umma_desc(a_addr + k * 32), umma_desc(w_addr + k * 32), idesc, (kb | k) ? 1u : 0u);
-                    umma_commit(&sh.empty[s]);
+                        umma_bf16(d_tmem, a_desc + step + k * 2, w_desc + step + k * 2, idesc, (kb | k) ? 1u : 0u);
+                    umma_commit(done);
+                    ready = mbar_test(&sh.full[s], phase);
                 }
                 if (ok) umma_commit(&sh.tfull[acc]);
             }
+            sh.consumed = consumed;
         }
     } else {
         const int q = warp & 3;                                   // the quarter of the tensor-memory lanes this warp may read

@@ -33,6 +33,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait. Returns false (and records it) if the limit passes or another thread gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+    if (mbar_try_wait(bar, parity)) return true;       // (the usual case in a running pipeline: no clock is read)
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity)) {
         if (*abort_flag) return false;
@@ -49,6 +50,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
     const bool ok = mbar_wait(bar, parity, abort_flag, status);
     return __all_sync(0xffffffffu, ok);
+}
+// True in one lane of a converged warp. The single-thread roles (TMA and tcgen05.mma issue) are entered through this and not
+// through a comparison of the lane number: the instructions take their descriptors from uniform registers, and only inside an
+// elect.sync branch does the compiler know that one thread is active. Behind `lane == 0` it guards each instruction for
+// threads that could differ: measured 63 instead of 48 cycles per 128 x 64 x 16 tcgen05.mma (the operand reads' 48 are the
+// bound) and 44 instead of 0 per commit.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile(
