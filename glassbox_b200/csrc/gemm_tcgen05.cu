@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float g = __uint_as_float(r[j]);
-                            r[j] = __float_as_uint(g / (1.0f + __expf(-g)) * (__uint_as_float(u[j]) * inv_rms));
+                            r[j] = __float_as_uint(gb_quotient(g, 1.0f + __expf(-g)) * (__uint_as_float(u[j]) * inv_rms));
                         }
                     }
                 }

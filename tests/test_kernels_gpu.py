@@ -1319,3 +1319,26 @@ def test_gemm_simt_packed_tiles_give_the_bits_of_the_plain_ones(M, N, K, w_dt):
     kernels.gemm_simt(odd[:, 1:], w, plain)
     assert torch.equal(got, plain) and torch.equal(added, c + plain)
     assert (got.double() - a.double() @ w.double().T).abs().max() <= 1e-5 * K ** 0.5 * 4
+
+
+def test_gemm_tcgen05_gated_at_the_ends_of_the_sigmoid():
+    """Gates where exp(-gate) is infinite, near its largest finite value, one, and nothing, against 64 bits: the quotient has one
+    path for all of them."""
+    from glassbox_b200 import kernels
+    gates = torch.tensor([-3.0e38, -1.0e4, -128.0, -90.0, -88.5, -88.0, -87.0, -86.5, -85.0, -60.0, -17.0, -1.0, -1e-30, 0.0, 1e-30, 0.5, 17.0, 88.0, 128.0, 3.0e4])
+    gates = gates.to(torch.bfloat16)
+    M, K, inter = 130, 64, 128
+    a = torch.zeros(M, K, dtype=torch.bfloat16, device=DEV)
+    a[:, 0] = 1.0
+    w = torch.zeros(2 * inter, K, dtype=torch.bfloat16, device=DEV)
+    w[:inter, 0] = gates.repeat(7)[:inter].to(DEV)
+    w[inter:, 0] = 1.5
+    act = torch.full((M, inter), 7.0, dtype=torch.bfloat16, device=DEV)
+    st = status()
+    kernels.gemm_tc_gated(a, w, act, status=st)
+    g = w[:inter, 0].double()
+    ref = torch.where(g < -700, torch.zeros_like(g), g / (1.0 + torch.exp(-g.clamp(min=-700)))) * 1.5
+    # one bfloat16 rounding (2^-8), the exponential's error (2^-21 of its argument's size, at most 90 here); what the smallest
+    # float32 of full precision cannot hold (below 1.2e-38, beyond gates of -83 with their factor) comes out as it or as zero
+    assert int(st) == 0
+    assert ((act.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 90 * 2.0 ** -21) + 1e-36).all()
