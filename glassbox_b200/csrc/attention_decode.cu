@@ -350,6 +350,205 @@ static int launch_decode(const void* q, long long q_stride, void* out, long long
 #undef GB_DK
 }
 
+// ----------------------------------------------------------------------------------------------
+// The float32 path at head sizes 64 and 128: the same splits, merge and scratch, with a warp as the unit and no tile in shared
+// memory. A warp takes 16 loads of 16 bytes a lane of keys and as many of values at once (HD 64: 32 keys, two a load; HD 128:
+// 16 keys), all requested before the first product, so a block's 256 (128) keys cost one latency; the partial dot products of a
+// key's lanes come together by a transposing reduction (15 shuffles for 16 keys and head), which leaves each lane the score of
+// one key. Scores, exponentials (expf), sums and the merge are float32 as above. What bounds it is that latency: page table, keys,
+// block merge, split merge. The tiles above take the keys 64 at a time through shared memory, four barriers a tile, and the
+// split rule's 592 blocks of 64 KB are two waves. Measured, 8 rows of 9 / 3 heads, contexts to 2,041: 34.4 -> 14.2 us.
+// ----------------------------------------------------------------------------------------------
+constexpr int DF_WARPS = 8;
+
+template <int HD, int GT>
+__global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
+    const float* __restrict__ q, long long q_stride, float* __restrict__ out, long long out_stride,
+    const float* __restrict__ kcache, const float* __restrict__ vcache, const int* __restrict__ block_tables, int max_pages,
+    const int* __restrict__ row_seq, const int* __restrict__ positions, int nh, int nkv, int page_size,
+    long long num_pages, float scale, int window, int splits, float* __restrict__ part_acc,
+    float* __restrict__ part_ml, int* __restrict__ counters, int* __restrict__ status) {
+    constexpr int LPK = HD / 4, KPS = 32 / LPK, STEPS = 16, CK = STEPS * KPS;   // lanes a key, keys a load, loads, keys a chunk
+    __shared__ float wacc[DF_WARPS][GT][HD], wm[DF_WARPS][GT], wl[DF_WARPS][GT];
+    __shared__ int is_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int split = blockIdx.x, row = blockIdx.z;
+    const int G = nh / nkv, subgroups = (G + GT - 1) / GT;
+    const int kvh = blockIdx.y / subgroups, sg = blockIdx.y % subgroups;
+    const int head0 = kvh * G + sg * GT, gcount = min(GT, G - sg * GT);
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    int pos = positions[row];
+    if (pos >= 0 && pos / page_size >= max_pages) {   // a position the block table does not reach: reported, and the
+        if (tid == 0) atomicOr(status, GB_STATUS_BAD_POSITION);   // row is treated as padding (nothing is read)
+        pos = -1;
+    }
+    float* orow = out + (size_t)row * out_stride;
+    if (pos < 0) {  // padding row
+        if (split == 0)
+            for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) orow[head0 * HD + i] = 0.f;
+        return;
+    }
+    const int* table = block_tables + (size_t)row_seq[row] * max_pages;
+    const int first = (window > 0 && pos + 1 > window) ? pos + 1 - window : 0;
+    const int total = pos + 1 - first;
+    // a split is whole rounds of the block's warps; the splits that get keys take part in the merge, the others leave
+    const int round = DF_WARPS * CK, chunk = ((total + splits - 1) / splits + round - 1) / round * round;
+    const int active = (total + chunk - 1) / chunk;
+    if (split >= active) return;
+    const int k_begin = first + split * chunk, k_end = min(pos + 1, k_begin + chunk);
+
+    float4 qv[GT];
+#pragma unroll
+    for (int g = 0; g < GT; ++g)
+        qv[g] = g < gcount ? *reinterpret_cast<const float4*>(q + (size_t)row * q_stride + (head0 + g) * HD + (lane % LPK) * 4)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+    float m_run[GT], l_run[GT];
+    float4 acc[GT];
+#pragma unroll
+    for (int g = 0; g < GT; ++g) {
+        m_run[g] = NEG_BIG;
+        l_run[g] = 0.f;
+        acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // after the reduction lane l has key KPS * (l % 16) + (l / 16 at HD 64) of the chunk; (HD 128: both halves the same key)
+    const int mine = KPS == 2 ? 2 * (lane & 15) + (lane >> 4) : (lane & 15);
+    const bool counted = KPS == 2 || lane < 16;
+    for (int base = k_begin + warp * CK; base < k_end; base += round) {
+        const int key = base + mine;
+        long long off = -1;
+        if (key < k_end) {
+            const long long page = table[key / page_size];
+            if (page < 0 || page >= num_pages) atomicOr(status, GB_STATUS_BAD_SLOT);
+            else off = ((page * nkv + kvh) * page_size + key % page_size) * HD;
+        }
+        float4 kr[STEPS], vr[STEPS];
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const long long o = __shfl_sync(0xffffffffu, off, i + (lane & 16));
+            kr[i] = o >= 0 ? *reinterpret_cast<const float4*>(kcache + o + (lane % LPK) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const long long o = __shfl_sync(0xffffffffu, off, i + (lane & 16));
+            vr[i] = o >= 0 ? *reinterpret_cast<const float4*>(vcache + o + (lane % LPK) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float p[GT];
+#pragma unroll
+        for (int g = 0; g < GT; ++g) {
+            float s[STEPS];
+#pragma unroll
+            for (int i = 0; i < STEPS; ++i)
+                s[i] = fmaf(qv[g].w, kr[i].w, fmaf(qv[g].z, kr[i].z, fmaf(qv[g].y, kr[i].y, qv[g].x * kr[i].x)));
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                const bool up = lane & o;
+#pragma unroll
+                for (int i = 0; i < o; ++i) {
+                    const float keep = up ? s[i + o] : s[i], send = up ? s[i] : s[i + o];
+                    s[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            if (KPS == 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], 16);
+            const float sc = off >= 0 ? s[0] * scale : NEG_BIG;
+            const float m_new = fmaxf(m_run[g], gb_warp_max(sc));
+            p[g] = off >= 0 ? expf(sc - m_new) : 0.f;
+            const float corr = expf(m_run[g] - m_new);
+            l_run[g] = l_run[g] * corr + gb_warp_sum(counted ? p[g] : 0.f);
+            m_run[g] = m_new;
+            acc[g] = make_float4(acc[g].x * corr, acc[g].y * corr, acc[g].z * corr, acc[g].w * corr);
+        }
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i)
+#pragma unroll
+            for (int g = 0; g < GT; ++g) {
+                const float w = __shfl_sync(0xffffffffu, p[g], i + (lane & 16));
+                acc[g].x = fmaf(w, vr[i].x, acc[g].x);
+                acc[g].y = fmaf(w, vr[i].y, acc[g].y);
+                acc[g].z = fmaf(w, vr[i].z, acc[g].z);
+                acc[g].w = fmaf(w, vr[i].w, acc[g].w);
+            }
+    }
+#pragma unroll
+    for (int g = 0; g < GT; ++g) {
+        if (KPS == 2) {      // the halves of the warp had every other key
+            acc[g].x += __shfl_xor_sync(0xffffffffu, acc[g].x, 16);
+            acc[g].y += __shfl_xor_sync(0xffffffffu, acc[g].y, 16);
+            acc[g].z += __shfl_xor_sync(0xffffffffu, acc[g].z, 16);
+            acc[g].w += __shfl_xor_sync(0xffffffffu, acc[g].w, 16);
+        }
+        if (lane < LPK) *reinterpret_cast<float4*>(&wacc[warp][g][lane * 4]) = acc[g];
+        if (lane == 0) {
+            wm[warp][g] = m_run[g];
+            wl[warp][g] = l_run[g];
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) {
+        const int g = i / HD, d = i % HD;
+        float m = wm[0][g], l = 0.f, v = 0.f;
+#pragma unroll
+        for (int w = 1; w < DF_WARPS; ++w) m = fmaxf(m, wm[w][g]);
+#pragma unroll
+        for (int w = 0; w < DF_WARPS; ++w) {
+            const float f = expf(wm[w][g] - m);
+            l = fmaf(wl[w][g], f, l);
+            v = fmaf(wacc[w][g][d], f, v);
+        }
+        if (active == 1) {
+            orow[(head0 + g) * HD + d] = l > 0.f ? v / l : 0.f;
+        } else {
+            part_acc[(((size_t)row * nh + head0 + g) * splits + split) * HD + d] = v;
+            if (d == 0) {
+                float* ml = part_ml + (((size_t)row * nh + head0 + g) * splits + split) * 2;
+                ml[0] = m;
+                ml[1] = l;
+            }
+        }
+    }
+    if (active == 1) return;
+    // the block that arrives last merges the splits
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        int* counter = counters + (size_t)row * gridDim.y + blockIdx.y;
+        const int prev = atomicAdd(counter, 1);
+        is_last = (prev == active - 1);
+        if (is_last) *counter = 0;  // ready for the next launch
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) {
+        const int g = i / HD, d = i % HD;
+        const float* ml = part_ml + ((size_t)row * nh + head0 + g) * splits * 2;
+        const float* pa = part_acc + ((size_t)row * nh + head0 + g) * splits * HD;
+        float m = NEG_BIG;
+#pragma unroll 8
+        for (int sidx = 0; sidx < active; ++sidx) m = fmaxf(m, __ldcg(ml + 2 * sidx));
+        float l = 0.f, v = 0.f;
+#pragma unroll 8
+        for (int sidx = 0; sidx < active; ++sidx) {
+            const float w = expf(__ldcg(ml + 2 * sidx) - m);
+            l = fmaf(__ldcg(ml + 2 * sidx + 1), w, l);
+            v = fmaf(__ldcg(pa + (size_t)sidx * HD + d), w, v);
+        }
+        orow[(head0 + g) * HD + d] = l > 0.f ? v / l : 0.f;
+    }
+}
+
+template <int HD, int GT>
+static int launch_decode_f32(const float* q, long long q_stride, float* out, long long out_stride, const float* kcache, const float* vcache,
+                             const int* block_tables, int max_pages, const int* row_seq, const int* positions, int n, int nh, int nkv,
+                             int page_size, long long num_pages, float scale, int window, int splits, float* part_acc,
+                             float* part_ml, int* counters, int* status, cudaStream_t stream) {
+    const int subgroups = (nh / nkv + GT - 1) / GT;
+    gb_launch(GB_PDL_ATTENTION, attention_decode_f32_kernel<HD, GT>, dim3(splits, nkv * subgroups, n), dim3(DF_WARPS * 32), 0, stream, q,
+              q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, row_seq, positions, nh, nkv, page_size, num_pages, scale,
+              window, splits, part_acc, part_ml, counters, status);
+    return gb_check_launch("gb_attention_decode");
+}
+
 // Number of int32 counters the kernel needs for `n` rows.
 GB_EXPORT int gb_attention_decode_counters(int n, int nh, int nkv) {
     const int G = nh / nkv;
@@ -372,6 +571,17 @@ GB_EXPORT int gb_attention_decode(const void* q, long long q_stride, void* out, 
     if (n == 0) return 0;
     const int G = nh / nkv;
     const int gt = G <= 4 ? G : 4;
+    if (dtype == GB_F32 && (hd == 64 || hd == 128) && q_stride % 4 == 0 &&
+        (((uintptr_t)q | (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0) {
+#define GB_DECODE32(HH, GG)                                                                                                            \
+    if (hd == HH && gt == GG)                                                                                                           \
+        return launch_decode_f32<HH, GG>((const float*)q, q_stride, (float*)out, out_stride, (const float*)kcache, (const float*)vcache, \
+                                         block_tables, max_pages, row_seq, positions, n, nh, nkv, page_size, num_pages, scale, window,   \
+                                         splits, part_acc, part_ml, counters, status, stream);
+        GB_DECODE32(64, 1) GB_DECODE32(64, 2) GB_DECODE32(64, 3) GB_DECODE32(64, 4)
+        GB_DECODE32(128, 1) GB_DECODE32(128, 2) GB_DECODE32(128, 3) GB_DECODE32(128, 4)
+#undef GB_DECODE32
+    }
 #define GB_DECODE(TT, GG)                                                                                       \
     return launch_decode<TT, GG>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, row_seq, \
                                  positions, n, nh, nkv, hd, page_size, num_pages, scale, window, splits,        \

@@ -1342,3 +1342,60 @@ def test_gemm_tcgen05_gated_at_the_ends_of_the_sigmoid():
     # float32 of full precision cannot hold (below 1.2e-38, beyond gates of -83 with their factor) comes out as it or as zero
     assert int(st) == 0
     assert ((act.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 90 * 2.0 ** -21) + 1e-36).all()
+
+
+@pytest.mark.parametrize("nh, nkv, hd, ps, window, splits", [(9, 3, 64, 16, None, 3), (2, 2, 64, 8, 40, 1), (5, 1, 128, 16, None, 2), (4, 2, 128, 32, 129, 9),
+                                                             (8, 2, 64, 64, None, 25), (6, 3, 128, 16, None, 1)])
+def test_attention_decode_float32_at_the_edges_of_a_warps_keys(nh, nkv, hd, ps, window, splits):
+    """Contexts around a warp's 16 or 32 keys, a block's 128 or 256 and several of them; splits that get no keys; what lies behind
+    a window or past the position is never read (infinities there)."""
+    from glassbox_b200 import kernels
+    lens = [1, 15, 16, 17, 31, 32, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 700, 1030]
+    k, v, tables, dense = make_cache(torch.float32, len(lens), lens, nkv, hd, ps, seed=hd + nh)
+    for s_i, L in enumerate(lens):
+        host = tables[s_i].tolist()
+        for key in list(range(0, max(0, L - window) if window else 0)) + list(range(L, -(-L // ps) * ps)):
+            k[host[key // ps], :, key % ps] = float("inf")
+            v[host[key // ps], :, key % ps] = float("nan")
+    n = len(lens) + 1
+    row_seq, positions = list(range(len(lens))) + [0], [L - 1 for L in lens] + [-1]
+    q = torch.randn(n, nh, hd)
+    out = torch.full((n, nh * hd), 7.0, device=DEV)
+    part_acc, part_ml = torch.empty(n * nh * splits * hd, device=DEV), torch.empty(n * nh * splits * 2, device=DEV)
+    counters = torch.zeros(n * nh, dtype=torch.int32, device=DEV)
+    st = status()
+    for _ in range(2):
+        kernels.attention_decode(q.to(DEV).reshape(n, -1), out, k, v, tables, torch.tensor(row_seq, dtype=torch.int32, device=DEV),
+                                 torch.tensor(positions, dtype=torch.int32, device=DEV), nh, nkv, hd, ps, hd ** -0.5, window, splits,
+                                 part_acc, part_ml, counters, st)
+        ref = ref_attention(q[:-1], dense, row_seq[:-1], positions[:-1], nh, nkv, hd ** -0.5, window)
+        got = out.cpu().double().reshape(n, nh, hd)
+        assert int(st) == 0 and int(counters.abs().max()) == 0
+        assert (got[:-1] - ref).abs().max() <= tol(torch.float32)
+        assert float(got[-1].abs().max()) == 0.0
+        out.fill_(7.0)
+
+
+@pytest.mark.parametrize("ta, tw, tc", [(torch.float32, torch.float32, torch.float32), (torch.float32, torch.bfloat16, torch.float32),
+                                        (torch.bfloat16, torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32, torch.float32)])
+@pytest.mark.parametrize("N, K", [(1, 4), (5, 100), (64, 128), (67, 1028), (33, 2052), (5003, 36), (8200, 260)])
+def test_gemm_simt_of_up_to_eight_rows_in_blocks_of_four_columns(N, K, ta, tw, tc):
+    """Ragged columns, K below, at and beyond a warp's 128 and a block's 1,024; a row's bits do not depend on how many there are."""
+    from glassbox_b200 import kernels
+    torch.manual_seed(N + K)
+    a, w = torch.randn(8, K, device=DEV).to(ta), torch.randn(N, K, device=DEV).to(tw)
+    ref = a.double() @ w.double().T
+    full = torch.empty(8, N, device=DEV, dtype=tc)
+    kernels.gemm_simt(a, w, full)
+    # sums of K products below 5 * 5 in float32, in any order (2^-24 a step at sqrt(K) of them), and one rounding of the output
+    bound = 25 * K ** 0.5 * 2.0 ** -22 + ref.abs() * (2.0 ** -8 if tc == torch.bfloat16 else 2.0 ** -23)
+    assert ((full.double() - ref).abs() <= bound).all()
+    for M in (1, 3, 7):
+        got = torch.empty(M, N, device=DEV, dtype=tc)
+        kernels.gemm_simt(a[:M], w, got)
+        assert torch.equal(got, full[:M])
+    if tc == torch.float32:
+        c = torch.randn(8, N, device=DEV)
+        added = c.clone()
+        kernels.gemm_simt(a, w, added, accumulate=True)
+        assert torch.equal(added, c + full)
