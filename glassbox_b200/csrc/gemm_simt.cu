@@ -1,12 +1,12 @@
 // C[M, N] (+)= A[M, K] * W[N, K]^T on the CUDA cores with float32 FMA only.
 //
 // This is the true 32-bit matrix product (no TF32, no tensor cores) and also the generic
-// fallback for any mix of float32 / bfloat16 operands at any size. Three kernels:
+// fallback for any mix of float32 / bfloat16 operands at any size. The kernels:
 //   * register-tiled kernels with packed FMA for M > 8 (float32 activations, rows aligned to 16 bytes),
 //   * a 64x64x16 register-tiled kernel for every other M > 8,
-//   * a weight-streaming kernel for M <= 8 (one warp per output column), which is what a
+//   * weight-streaming kernels for M <= 8 (a block or a warp per four output columns, or a warp per column), which is what a
 //     decode step needs: every weight is read once, coalesced along K.
-// Each output element is reduced over K in an order that depends only on K (and on whether M > 8: all tiled kernels
+// Each output element is reduced over K in an order that depends only on K and N (and on whether M > 8: all tiled kernels
 // add one product after the other from k = 0, so they give the same bits), never on M or on the element's place in the batch.
 // Row-major [out, in] weights as in crates/glassbox-core/src/kernels.rs:381, 586-655.
 #include "common.cuh"
@@ -284,6 +284,67 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const TA* __restrict__
     }
 }
 
+// The same four columns at a time, twelve 16-byte loads of a lane under way per 128 of K, the 32 sums of a lane brought together
+// by 31 shuffles. SPLIT: the block is the unit, K dealt out to its eight warps in slices of 128 (a lane holds four consecutive
+// k) whose sums meet in shared memory; else a warp takes its four columns alone, in the order, and so with the bits, of the
+// kernel above. That one walks K alone, nine loads and their latency after the other, and re-reads the activations for every
+// column: latency, a tenth of the copy rate at best. Measured, 8 rows float32: N 960, K 576 10.8 -> 2.3 us (split); N 576, K
+// 1536 22.5 -> 3.3 (split); N 3072, K 576 12.1 -> 6.9; N 49152, K 576 62.7 -> 38.1 (113 MB).
+template <typename TA, typename TW, typename TC, bool SPLIT>
+__global__ void __launch_bounds__(256) gemm_skinny4_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, int M, int N,
+                                                           int K, long long lda, long long ldw, long long ldc, int mode) {
+    __shared__ float part[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = (SPLIT ? blockIdx.x : blockIdx.x * 8 + warp) * 4;
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    float acc[32];                                      // [row][column]
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+    for (int k = (SPLIT ? warp * 128 : 0) + lane * 4; k < K; k += SPLIT ? 1024 : 128) {
+        float w[4][4], a[8][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (n0 + c < N) Vec4Load<TW>::load(W + (size_t)(n0 + c) * ldw + k, w[c]);
+            else w[c][0] = w[c][1] = w[c][2] = w[c][3] = 0.f;
+        }
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            if (m < M) Vec4Load<TA>::load(A + (size_t)m * lda + k, a[m]);
+            else a[m][0] = a[m][1] = a[m][2] = a[m][3] = 0.f;
+        }
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            if (m >= M) break;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m * 4 + c] = fmaf(a[m][e], w[c][e], acc[m * 4 + c]);
+        }
+    }
+    // lane l ends up with the warp's sum number l: in each round the half of the sums that the partner keeps is sent to it
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float keep = up ? acc[i + o] : acc[i], send = up ? acc[i] : acc[i + o];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    float v = acc[0];
+    if (SPLIT) {
+        part[warp][lane] = v;
+        __syncthreads();
+        if (warp > 0) return;
+#pragma unroll
+        for (int i = 1; i < 8; ++i) v += part[i][lane];
+    }
+    {
+        const int m = lane >> 2, n = n0 + (lane & 3);
+        if (m < M && n < N) store_out<TC>(C + (size_t)m * ldc + n, v, mode);
+    }
+}
+
 template <typename TA, typename TW, typename TC>
 static int launch_gemm(const void* a, const void* w, void* c, int M, int N, int K, long long lda, long long ldw,
                        long long ldc, int mode, cudaStream_t stream) {
@@ -295,7 +356,17 @@ static int launch_gemm(const void* a, const void* w, void* c, int M, int N, int 
     if (M <= 8) {
         int warps = 8;
         dim3 grid(gb_ceil_div(N, warps));
-        if (vec) gemm_skinny_kernel<TA, TW, TC, true><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
+        // Up to 2,048 columns (512 blocks of four: one round of the chip) the split form is the faster at every number of rows
+        // (N 2048, K 576, one row: 3.9 us against 5.1; K 8192: 18 against 40); beyond, its blocks are small change against their
+        // barriers (N 8192, K 576, one row: 12.3 against 6.2). There four columns a warp pay from three rows of 32-bit and five
+        // of 16-bit activations, whose conversions cost more (N 49152, K 576: one row 29.9 against 27.4, four 33.1 / 39.6, eight
+        // 38.1 / 62.7; bfloat16 four rows 46.8 / 42.3, eight 50.5 / 66.0). The line between these two is the only one that
+        // depends on M, and both sides give the same bits.
+        if (vec && N <= 2048)
+            gb_launch(GB_PDL_GEMM, gemm_skinny4_kernel<TA, TW, TC, true>, dim3(gb_ceil_div(N, 4)), dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, mode);
+        else if (vec && M > (sizeof(TA) == 4 ? 2 : 4))
+            gb_launch(GB_PDL_GEMM, gemm_skinny4_kernel<TA, TW, TC, false>, dim3(gb_ceil_div(N, 32)), dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, mode);
+        else if (vec) gemm_skinny_kernel<TA, TW, TC, true><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
         else gemm_skinny_kernel<TA, TW, TC, false><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
     } else {
         if constexpr (sizeof(TA) == 4 && sizeof(TC) == 4) {
