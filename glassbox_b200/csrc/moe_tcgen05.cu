@@ -136,6 +136,10 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
         bool ok = true;
         for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
             const Place p = place(tile);
+            // Groups of four rows that hold a pair; the rest of the tile keeps what was there, and its sums are not stored. A gather
+            // costs as much as a box of 128 rows' share of the load unit: with all 32 for every tile, 24 rows of four of 16 experts
+            // 2048 x 2048 took 150 us the feed-forward (mma.sync tiles before: 128), with the live ones 107.
+            const int gathers = (min(ME_BM, p.m_end - p.m0) + 3) >> 2;
             int r[4];
             if (UP) {
 #pragma unroll
@@ -149,13 +153,13 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
                 if (it >= STAGES && !mbar_wait_warp(&sh.empty[s], ((it / STAGES) - 1) & 1, abort_flag, status)) { ok = false; break; }
                 unsigned char* a_dst = tiles + s * G::STAGE_BYTES;
                 if (lane == 0) {
-                    mbar_expect_tx(&sh.full[s], G::STAGE_BYTES);
+                    mbar_expect_tx(&sh.full[s], UP ? G::W_BYTES + gathers * 512 : G::STAGE_BYTES);
                     tma_load_2d(a_dst + G::A_BYTES, &map_w, &sh.full[s], kb * ME_BK, p.e * N + p.n0);
                     if (!UP) tma_load_2d(a_dst, &map_a, &sh.full[s], kb * ME_BK, p.m0);
                     sh.issued = it + 1;
                 }
                 __syncwarp();
-                if (UP) me_gather4(a_dst + lane * 512, &map_a, &sh.full[s], kb * ME_BK, r[0], r[1], r[2], r[3]);
+                if (UP && lane < gathers) me_gather4(a_dst + lane * 512, &map_a, &sh.full[s], kb * ME_BK, r[0], r[1], r[2], r[3]);
             }
         }
     } else if (warp == 1) {
