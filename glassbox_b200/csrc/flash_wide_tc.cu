@@ -43,7 +43,7 @@ struct FwArgs {
 };
 
 struct __align__(8) FwShared {
-    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, x_bar[4];
+    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, o_done, x_bar[4];
     float stat[2][2][FW_BM];   // [parity of the tile][half][row]: a half's maximum, at the end its sum
     uint32_t tmem_base;
     int abort_flag, issued[2], consumed[2], q_issued, q_consumed;
@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             mbar_init(&sh.p_ready[i], 8);                       // one arrival per softmax warp
         }
         mbar_init(&sh.pv_done, 1);
+        mbar_init(&sh.o_done, 1);
         for (int i = 0; i < 4; ++i) mbar_init(&sh.x_bar[i], 2);   // the two warps of a quarter of the rows
         sh.abort_flag = sh.issued[0] = sh.issued[1] = sh.consumed[0] = sh.consumed[1] = sh.q_issued = sh.q_consumed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                                  (j | kk) ? 1u : 0u);
                 umma_commit(&sh.pv_done);
                 umma_commit(LATENT ? &sh.k_empty[s] : &sh.v_empty[s]);
+                if (j + 1 == ntiles) umma_commit(&sh.o_done);   // (a commit covers everything this thread issued before it)
                 // S_(j+2) goes where P_j is: only once the product that reads it is done
                 if (j + 2 < ntiles) ok = mbar_wait(&sh.pv_done, j & 1, abort_flag, a.status) && scores(j + 2);
             }
@@ -330,9 +332,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.x_bar[q]);
             ok = mbar_wait_warp(&sh.x_bar[q], ntiles & 1, abort_flag, a.status);
-            // the last two products may both be under way: their phases one after the other (a wait for a parity passes while the
-            // phase before it is still open)
-            for (int j = max(ntiles - 2, 0); j < ntiles && ok; ++j) ok = mbar_wait_warp(&sh.pv_done, j & 1, abort_flag, a.status);
+            // A barrier of its own, with one phase, says that all products are done: nothing orders this look against the last two
+            // phases of pv_done, and a parity tells an open phase from its neighbours only (with both complete, the wait for the
+            // last but one would take the next, open phase for it and never pass).
+            ok = ok && mbar_wait_warp(&sh.o_done, 0, abort_flag, a.status);
         }
         if (ok) {
             tc_fence_after();

@@ -118,3 +118,27 @@ def test_positions_beyond_the_table_and_missing_pages_are_reported():
         out, status = torch.zeros(40, 256, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
         kernels.latent_flash(q, out, cache, bad, first, start, None, 2, 128, 32, 16, 0.1, None, status, longest)
         assert int(status) == bit
+
+
+@pytest.mark.parametrize("rows", [72, 129, 256, 300])
+def test_every_launch_ends_by_itself(rows):
+    """Blocks of one to three key tiles, whose last products overlap their warps' last looks at the barriers in every order: launches
+    behind one another, beside work that takes multiprocessors away, must all finish (no wait that gives up) with the same result."""
+    from glassbox_b200 import kernels
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    tables, first, start, pages, longest = _layout(16, [(0, rows)] * 6, rows)
+    n, H = int(first[-1]), 8
+    q = torch.randn(n, H * 192, generator=g, device=DEV).bfloat16()
+    cache = torch.randn(pages, 16, 192, generator=g, device=DEV).bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    busy, side = torch.randn(4096, 4096, device=DEV), torch.cuda.Stream()
+    outs = [torch.full((n, H * 128), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(60)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            busy.mul_(1.0001)
+    for out in outs:
+        kernels.latent_flash(q, out, cache, tables, first, start, None, H, 128, 64, 16, 0.1, None, status, longest)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    assert all(torch.equal(outs[0], out) for out in outs[1:])
