@@ -351,21 +351,23 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             for (int c = h * (DV / 2); c < (h + 1) * (DV / 2); c += 32) {
                 uint32_t ov[32];
                 tmem_load32(lane_base + (uint32_t)(G::O_COL + c), ov);
-                if (q_lo + r >= nrows) continue;
+                if (q_lo + r < nrows) {
 #pragma unroll
-                for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * inv);
-                if (LATENT) {
-                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
+                    for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * inv);
+                    if (LATENT) {
+                        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
 #pragma unroll
-                    for (int k = 0; k < 32; k += 8)
-                        *reinterpret_cast<uint4*>(dst + k) = make_uint4(pack2(ov[k], ov[k + 1]), pack2(ov[k + 2], ov[k + 3]), pack2(ov[k + 4], ov[k + 5]),
-                                                                        pack2(ov[k + 6], ov[k + 7]));
-                } else {
-                    float* dst = reinterpret_cast<float*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
+                        for (int k = 0; k < 32; k += 8)
+                            *reinterpret_cast<uint4*>(dst + k) = make_uint4(pack2(ov[k], ov[k + 1]), pack2(ov[k + 2], ov[k + 3]),
+                                                                            pack2(ov[k + 4], ov[k + 5]), pack2(ov[k + 6], ov[k + 7]));
+                    } else {
+                        float* dst = reinterpret_cast<float*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
 #pragma unroll
-                    for (int k = 0; k < 32; k += 4)
-                        *reinterpret_cast<uint4*>(dst + k) = make_uint4(ov[k], ov[k + 1], ov[k + 2], ov[k + 3]);
+                        for (int k = 0; k < 32; k += 4)
+                            *reinterpret_cast<uint4*>(dst + k) = make_uint4(ov[k], ov[k + 1], ov[k + 2], ov[k + 3]);
+                    }
                 }
+                __syncwarp();      // the next load is the whole warp's; lanes past the last row have taken the other way here
             }
         }
     }
