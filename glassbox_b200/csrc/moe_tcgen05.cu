@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
                         const int row = __shfl_sync(0xffffffffu, out_row, rr);
                         if (rr < rows && col < N) reinterpret_cast<float*>(C)[(size_t)row * ldc + col] = stage[rr * 33 + lane];
                     }
-                    __syncwarp();
                 }
+                __syncwarp();      // the next load is the whole warp's; rows past the expert's last pair have taken another way here
             }
             tc_fence_before();
             __syncwarp();
