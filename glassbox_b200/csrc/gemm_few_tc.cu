@@ -134,6 +134,9 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_few_kernel(const __grid_const
         }
         __syncwarp();
     } else if (warp == 1) {
+        // (X, which the first barrier also waits for, is not requested before this: the limit of the bounded waits must not count
+        // the time that the kernel before takes)
+        gb_pdl_wait();
         if (elect_one()) {
             const uint32_t idesc = umma_idesc(GF_BM, a.x_rows);
             const uint64_t w_desc = umma_desc(smem_u32(stages)), x_desc = umma_desc(smem_u32(stages) + GF_W_BYTES);
@@ -154,8 +157,6 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_few_kernel(const __grid_const
             if (ok) umma_commit(&sh.tfull);
             sh.consumed = consumed;
         }
-        __syncwarp();
-        gb_pdl_wait();
     } else {
         gb_pdl_wait();
         const int q = warp & 3;                                   // the quarter of the tensor-memory lanes (outputs) of this warp

@@ -92,3 +92,28 @@ def test_qkv_with_rotation_and_cache_write(nh, nkv, hd, page, M, K):
     positions[0], slots[1] = 100, pages * page
     kernels.gemm_few_qkv(x, w, q, table, positions.to(DEV), slots.to(DEV), k, v, nh, nkv, hd, page, True, st)
     assert int(st) == 6                                                      # beyond the table; beyond the pool
+
+
+def test_a_long_kernel_before_it_is_no_timeout():
+    """The kernel may start while the one before it runs; the limits of its waits (0.2 s) must not count that one's time: a walk of
+    the delta rule over a million tokens."""
+    from glassbox_b200 import kernels
+    n, D, V = 1_000_000, 32, 8
+    f32 = lambda *s: torch.zeros(*s, device=DEV)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    qkv, beta, a, state, out = f32(n, 2 * D + V), f32(n, 1), f32(n, 1), f32(1, D * V), f32(n, V)
+    x, w, want = _operands(40, 6144, 2048)
+    c, st = torch.empty(40, 6144, device=DEV), i32(0)
+    args = (qkv, beta, a, f32(1), f32(1), state, out, i32(0, n), i32(0), i32(0), 1, 1, D, V, True, st)
+    kernels.gemm_few(x, w, c, st)
+    kernels.channel_delta(*args, decay_per_head=True)
+    torch.cuda.synchronize()
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    start.record()
+    kernels.channel_delta(*args, decay_per_head=True)
+    kernels.gemm_few(x, w, c, st)
+    end.record()
+    torch.cuda.synchronize()
+    assert start.elapsed_time(end) > 210, "the walk is shorter than the limit: this test would say nothing"
+    assert int(st) == 0
+    _close(c, want, 0)
