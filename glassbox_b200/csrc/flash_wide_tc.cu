@@ -67,10 +67,6 @@ __device__ __forceinline__ float fw_rcp(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// two non-negative floats to a bfloat16 pair, rounding half up (integer instructions: the conversion shares ex2's pipe)
-__device__ __forceinline__ uint32_t fw_pack(float lo, float hi) {
-    return __byte_perm(__float_as_uint(lo) + 0x8000u, __float_as_uint(hi) + 0x8000u, 0x7632);
-}
 // MN-major B operand (rows are keys, 64-channel column blocks FW_BLOCK apart), 128-byte-swizzled rows
 __device__ __forceinline__ uint64_t fw_desc_mn(uint32_t smem_addr) {
     return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)(FW_BLOCK >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
@@ -318,7 +314,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 const float2 y = __ffma2_rn(make_float2(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), scale2, off2);
                 const float2 pp = make_float2(fw_exp2(y.x), fw_exp2(y.y));
                 // the denominator sums what the product uses: the weights as rounded to bfloat16
-                const uint32_t both = pw[c >> 1] = fw_pack(pp.x, pp.y);
+                const uint32_t both = pw[c >> 1] = pack2(__float_as_uint(pp.x), __float_as_uint(pp.y));
                 l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
             }
             l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);

@@ -142,3 +142,38 @@ def test_every_launch_ends_by_itself(rows):
     torch.cuda.synchronize()
     assert int(status) == 0
     assert all(torch.equal(outs[0], out) for out in outs[1:])
+
+
+@pytest.mark.parametrize("cap", [None])
+def test_a_nan_query_gives_nan(cap):
+    """A NaN in one row's query of one head makes that row's results of that head NaN, and no other number changes."""
+    from glassbox_b200 import kernels
+    if cap is None:
+        tables, first, start, pages, longest = _layout(16, [(30, 200)], 6)
+        n, H = int(first[-1]), 3
+        q = torch.randn(n, H, 160, device=DEV).bfloat16()
+        cache = torch.randn(pages, 16, 160, device=DEV).bfloat16()
+        run = lambda q, out, st: kernels.latent_flash(q.view(n, -1), out, cache, tables, first, start, None, H, 128, 32, 16, 0.2, None, st, longest)
+        make = lambda: torch.zeros(n, H * 128, dtype=torch.bfloat16, device=DEV)
+        _nan_row(run, make, q, n, H)
+    tables, first, start, pages, longest = _layout(16, [(30, 200)], 7)
+    n, H, G = int(first[-1]), 4, 2
+    q = torch.randn(n, H, 64, device=DEV).bfloat16()
+    k, v = (torch.randn(pages, G, 16, 64, device=DEV).bfloat16() for _ in range(2))
+    run = lambda q, out, st: kernels.talking_attention_flash(q.view(n, -1), out, k, v, tables, first, start, longest, H, G, 64, 64, G, 16, 0.5,
+                                                             cap, True, None, st)
+    _nan_row(run, lambda: torch.zeros(n, H * G * 64, device=DEV), q, n, H)
+
+
+def _nan_row(run, make, q, n, H):
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    clean, spoiled = make(), make()
+    run(q, clean, status)
+    bad = q.clone()
+    bad[77, 1, 5] = float("nan")
+    run(bad, spoiled, status)
+    assert int(status) == 0
+    a, b = clean.view(n, H, -1), spoiled.view(n, H, -1)
+    assert torch.isnan(b[77, 1]).all() and torch.isfinite(a).all()
+    b[77, 1] = a[77, 1]
+    assert torch.equal(a, b)
