@@ -13,8 +13,8 @@
 //              maximum with its partner, and writes its half of P_j. The running maximum is raised (and O rescaled) only when
 //              exceeded by more than 2^8 in the exponent, as in attention_prefill_tc.cu.
 //   warp 10    producer of the values (not for the latent cache, whose key tile serves both products)
-// Bound by the softmax warps' exponentials (with a cap two and a quarter special-function operations a score: 2,300 cycles a
-// tile against 1,280 of the tensor pipe); the mma.sync kernels that this replaced formed the scores once per 128 value
+// Bound by the softmax warps (an exponential a score: 1,024 cycles a tile of the special-function unit, and with a cap nine fused
+// multiply-adds, against 1,280 of the tensor pipe); the mma.sync kernels that this replaced formed the scores once per 128 value
 // channels and fed both products through ldmatrix. Measured: see gb_talking_attention_flash, gb_latent_flash.
 //
 // Every wait is bounded: on a timeout the block records GB_STATUS_WAIT_TIMEOUT, waits (bounded) for its copies, frees its tensor
@@ -62,10 +62,42 @@ __device__ __forceinline__ float fw_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float fw_rcp(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
+// s <- cap * tanh(s * in) for a warp's scores, as exactly as a call of tanhf (measured over |s * in| < 20: at most 1.5 units in the
+// last place of the tanh; NaN stays NaN). Below 1 the tanh is y + y t c(t), t = y^2, with c the interpolation of (tanh(sqrt t) / sqrt t
+// - 1) / t at the Chebyshev nodes of [0, 1] (2e-8 off): fused multiply-adds of two scores at a time and no special function, which is
+// all that most warps need (their scores lie within the cap). Where one of a warp's scores does not, all of them also form
+// 1 - 2 / (1 + e^(2|y|)). Talking-heads mixer of 2,048 tokens: 100 us; with tanhf for every score 112.
+__device__ __forceinline__ void fw_cap(uint32_t (&s)[64], float in, float cap) {
+    float top[2] = {0.f, 0.f};
+    const float2 in2 = make_float2(in, in), cap2 = make_float2(cap, cap);
+#pragma unroll
+    for (int k = 0; k < 64; k += 2) {
+        const float2 y = __fmul2_rn(make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), in2);
+        s[k] = __float_as_uint(y.x);
+        s[k + 1] = __float_as_uint(y.y);
+        top[(k >> 1) & 1] = fmaxf(top[(k >> 1) & 1], fmaxf(fabsf(y.x), fabsf(y.y)));
+    }
+    const bool beyond = __any_sync(0xffffffffu, fmaxf(top[0], top[1]) >= 1.0f);
+    auto both = [](float c) { return make_float2(c, c); };
+#pragma unroll
+    for (int k = 0; k < 64; k += 2) {
+        const float2 y = make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), t = __fmul2_rn(y, y);
+        float2 w = __ffma2_rn(both(-0.00042069549f), t, both(0.0025104594f));
+        w = __ffma2_rn(w, t, both(-0.0082189217f));
+        w = __ffma2_rn(w, t, both(0.021660116f));
+        w = __ffma2_rn(w, t, both(-0.05393479f));
+        w = __ffma2_rn(w, t, both(0.13333128f));
+        w = __ffma2_rn(w, t, both(-0.3333333135f));
+        float2 r = __ffma2_rn(y, __fmul2_rn(w, t), y);
+        if (beyond) {
+            auto far = [](float v) { return copysignf(1.0f - __fdividef(2.0f, 1.0f + fw_exp2(fabsf(v) * (2.0f * FW_LOG2E))), v); };
+            if (!(fabsf(y.x) < 1.0f)) r.x = far(y.x);
+            if (!(fabsf(y.y) < 1.0f)) r.y = far(y.y);
+        }
+        r = __fmul2_rn(r, cap2);
+        s[k] = __float_as_uint(r.x);
+        s[k + 1] = __float_as_uint(r.y);
+    }
 }
 // MN-major B operand (rows are keys, 64-channel column blocks FW_BLOCK apart), 128-byte-swizzled rows
 __device__ __forceinline__ uint64_t fw_desc_mn(uint32_t smem_addr) {
@@ -234,7 +266,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         const int r = q * 32 + lane, pos = pos_lo + r;
         const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
         const float sl2 = a.scale * FW_LOG2E;                   // scores are brought into the base-2 domain
-        const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? 2.0f * sl2 / a.cap : 0.f;
+        const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? a.scale / a.cap : 0.f;
         const float slx = cap2 > 0.f ? 1.0f : sl2;              // what is left to scale once capped
         const int first = gb_first_key(pos, a.window), first_last = gb_first_key(pos_lo + FW_BM - 1, a.window);
         float m_run = FW_NEG_BIG, l_run = 0.f;
@@ -246,27 +278,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             uint32_t sv[64];
             tmem_load64(lane_base + (uint32_t)(b * FW_BN + h * 64), sv);
             tc_fence_before();
-            if (cap2 > 0.f) {
-                // cap tanh(s / cap) = cap - 2 cap / (1 + exp(2 s / cap)); four scores share a reciprocal, of the product of their
-                // denominators (each at most 1 + 2^30, where the tanh is 1 to the last bit)
-                const float2 in2 = make_float2(cap_in, cap_in), one2 = make_float2(1.f, 1.f);
-                const float2 top2 = make_float2(cap2, cap2), down2 = make_float2(-2.0f * cap2, -2.0f * cap2);
-#pragma unroll
-                for (int k = 0; k < 64; k += 4) {
-                    const float2 ya = __fmul2_rn(make_float2(__uint_as_float(sv[k]), __uint_as_float(sv[k + 1])), in2);
-                    const float2 yb = __fmul2_rn(make_float2(__uint_as_float(sv[k + 2]), __uint_as_float(sv[k + 3])), in2);
-                    const float2 ea = __fadd2_rn(make_float2(fw_exp2(fminf(ya.x, 30.f)), fw_exp2(fminf(ya.y, 30.f))), one2);
-                    const float2 eb = __fadd2_rn(make_float2(fw_exp2(fminf(yb.x, 30.f)), fw_exp2(fminf(yb.y, 30.f))), one2);
-                    const float2 both = __fmul2_rn(ea, eb);
-                    const float rc = fw_rcp(both.x * both.y);
-                    const float2 rb = __fmul2_rn(make_float2(both.y, both.x), make_float2(rc, rc));
-                    const float2 sa = __ffma2_rn(__fmul2_rn(eb, rb), down2, top2), sb = __ffma2_rn(__fmul2_rn(ea, rb), down2, top2);
-                    sv[k] = __float_as_uint(sa.x);
-                    sv[k + 1] = __float_as_uint(sa.y);
-                    sv[k + 2] = __float_as_uint(sb.x);
-                    sv[k + 3] = __float_as_uint(sb.y);
-                }
-            }
+            if (cap2 > 0.f) fw_cap(sv, cap_in, cap2);
             if (key0 + 63 > pos_lo || key0 < first_last) {      // the tile crosses the diagonal, the window's edge or the last key
 #pragma unroll
                 for (int k = 0; k < 64; ++k)

@@ -144,7 +144,7 @@ def test_every_launch_ends_by_itself(rows):
     assert all(torch.equal(outs[0], out) for out in outs[1:])
 
 
-@pytest.mark.parametrize("cap", [None])
+@pytest.mark.parametrize("cap", [None, 30.0])
 def test_a_nan_query_gives_nan(cap):
     """A NaN in one row's query of one head makes that row's results of that head NaN, and no other number changes."""
     from glassbox_b200 import kernels
@@ -177,3 +177,28 @@ def _nan_row(run, make, q, n, H):
     assert torch.isnan(b[77, 1]).all() and torch.isfinite(a).all()
     b[77, 1] = a[77, 1]
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("cap", [0.5, 5.0, 50.0])
+def test_the_cap_is_as_exact_as_float32_allows(cap):
+    """The first token of a request sees one key: beside the unit of score 0 in the denominator its result is value * sigmoid(capped
+    score), and a single product makes the score exact, so what is off is the cap (and the last exponential and division)."""
+    from glassbox_b200 import kernels
+    S = 400
+    q = torch.zeros(S, 64, device=DEV)
+    q[:, 3] = torch.cat([torch.linspace(-16, 16, S // 2), torch.linspace(-60, 60, S // 2)]).to(DEV)
+    q = q.bfloat16()
+    k = torch.zeros(S, 1, 8, 64, dtype=torch.bfloat16, device=DEV)
+    k[:, 0, 0, 3] = 1.0
+    v = torch.full((S, 1, 8, 128), 1.0, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(DEV)
+    out, status = torch.zeros(S, 128, device=DEV), i32([0])
+    kernels.talking_attention_flash(q, out, k, v, i32(range(S))[:, None].contiguous(), i32(range(S + 1)), i32([0] * S), 1, 1, 1, 64, 128, 1, 8,
+                                    0.25, cap, True, None, status)
+    s = cap * torch.tanh(q[:, 3].double() * 0.25 / cap)
+    want = torch.sigmoid(s)
+    # relative: the tanh's two units in the last place (2^-23), its input's and the cap's roundings (3 * 2^-24), all times |s| (1 - sigmoid);
+    # the hardware's exponential (2^-22, times 1 - sigmoid) of a rounded difference (|s| log2(e) 2^-24) and the division (2^-23)
+    bound = want * ((1 - want) * (s.abs() * (5 * 2 ** -24 + 2 ** -24) + 2 ** -22) + 2 ** -22)
+    assert int(status) == 0
+    assert ((out.double() - want[:, None]).abs() <= bound[:, None]).all(), float(((out.double() - want[:, None]).abs() / bound[:, None]).max())
