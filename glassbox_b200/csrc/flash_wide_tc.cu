@@ -179,16 +179,14 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         uint64_t* empty = what == 0 ? sh.k_empty : sh.v_empty;
         unsigned char* ring = what == 0 ? Ks : Vs;
         int bad = 0;
-        auto page_of = [&](int kt) -> long long {               // this lane's page of key tile kt
-            long long page = 0;
+        const int nowhere = (int)(a.num_pages * a.kv_heads * a.page_size);      // a row past the pool: the load fills in zeros
+        auto page_of = [&](int kt) -> long long {               // this lane's page of key tile kt, -1: no key of it is seen, or missing
+            long long page = -1;
             if (lane < ppt) {
-                const int pi = ((kt * FW_BN) >> a.page_shift) + lane;
-                page = pi < a.max_pages ? table[pi] : -1;
-                if (page < 0 || page >= a.num_pages) {
-                    // only a page that holds a key some row can see is missed; page 0, finite, is read in the place of others
-                    const int first = pi << a.page_shift;
-                    if (first <= pos_hi && first + a.page_size - 1 >= key_lo) bad = 1;
-                    page = 0;
+                const int pi = ((kt * FW_BN) >> a.page_shift) + lane, first = pi << a.page_shift;
+                if (first <= pos_hi && first + a.page_size - 1 >= key_lo) {
+                    page = pi < a.max_pages ? table[pi] : -1;
+                    if (page < 0 || page >= a.num_pages) { bad = 1; page = -1; }
                 }
             }
             return page;
@@ -196,7 +194,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         long long page = page_of(kt_begin);
         int s = 0, round = 0;
         for (int j = 0; j < ntiles; ++j) {
-            const long long next_page = j + 1 < ntiles ? page_of(kt_begin + j + 1) : 0;   // in flight during the wait
+            const long long next_page = j + 1 < ntiles ? page_of(kt_begin + j + 1) : -1;   // in flight during the wait
             int ok = 1;
             if (lane == 0 && round > 0) ok = mbar_wait(&empty[s], (round - 1) & 1, abort_flag, a.status) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -207,10 +205,11 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 unsigned char* dst = ring + s * bytes + lane * a.page_size * 128;
                 for (int b = 0; b < boxes; ++b) {
                     if (what == 0) {
-                        tma_load_2d(dst + b * FW_BLOCK, &map_k, &full[s], b * 64, (int)((page * a.kv_heads + kvh) * a.page_size));
+                        tma_load_2d(dst + b * FW_BLOCK, &map_k, &full[s], b * 64, page < 0 ? nowhere : (int)((page * a.kv_heads + kvh) * a.page_size));
                     } else {
                         const int col = col0 + b * 64;          // of the wide value row
-                        tma_load_2d(dst + b * FW_BLOCK, &map_v, &full[s], col % a.vdim, (int)((page * a.kv_heads + col / a.vdim) * a.page_size));
+                        tma_load_2d(dst + b * FW_BLOCK, &map_v, &full[s], col % a.vdim,
+                                    page < 0 ? nowhere : (int)((page * a.kv_heads + col / a.vdim) * a.page_size));
                     }
                 }
             }
@@ -330,6 +329,20 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
             }
             l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
+            // Keys that no row of the block sees have a weight of 0, but what lies in their place in the pages (an earlier
+            // request's values, or nothing yet) may be no finite number: zeros take its place before the product. Only the tiles
+            // at the ends of the walk hold such keys.
+            const int lo = key_lo - (kt_begin + j) * FW_BN, hi = pos_hi - (kt_begin + j) * FW_BN;
+            if (lo > 0 || hi < FW_BN - 1) {
+                const int s = LATENT ? j % G::K_STAGES : j % G::V_STAGES, phase = (LATENT ? j / G::K_STAGES : j / G::V_STAGES) & 1;
+                if (!mbar_wait_warp(LATENT ? &sh.k_full[s] : &sh.v_full[s], phase, abort_flag, a.status)) { ok = false; break; }
+                unsigned char* values = LATENT ? Ks + s * G::K_BYTES : Vs + s * G::V_BYTES;
+                for (int i = (warp - 2) * 32 + lane; i < DV / 64 * FW_BN * 8; i += 256) {
+                    const int key = (i >> 3) & (FW_BN - 1);
+                    if (key < lo || key > hi) *reinterpret_cast<uint4*>(values + (i >> 10) * FW_BLOCK + key * 128 + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
             tmem_store32(lane_base + (uint32_t)(b * FW_BN + h * 32), pw);
             tc_fence_before();
             __syncwarp();

@@ -202,3 +202,39 @@ def test_the_cap_is_as_exact_as_float32_allows(cap):
     bound = want * ((1 - want) * (s.abs() * (5 * 2 ** -24 + 2 ** -24) + 2 ** -22) + 2 ** -22)
     assert int(status) == 0
     assert ((out.double() - want[:, None]).abs() <= bound[:, None]).all(), float(((out.double() - want[:, None]).abs() / bound[:, None]).max())
+
+
+@pytest.mark.parametrize("window", [None, 50])
+def test_what_no_row_sees_reaches_no_result(window):
+    """Pages hold what earlier requests left: past the last row, in front of a window, and in every page the table does not name.
+    Infinities and NaN there change no result."""
+    from glassbox_b200 import kernels
+    batch = [(130, 75), (0, 200), (300, 140)]
+    tables, first, start, pages, longest = _layout(16, batch, 8)
+    n = int(first[-1])
+    seen = torch.zeros(pages, 16, dtype=torch.bool, device=DEV)
+    for i, (c, r) in enumerate(batch):
+        for t in range(max(c + 1 - window, 0) if window else 0, c + r):
+            seen[int(tables[i, t // 16]), t % 16] = True
+        if window:                                          # pages wholly in front of the window may be gone
+            tables[i, :max(c + 1 - window, 0) // 16] = -1
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    spoil = lambda t, dim: torch.where(seen.view(seen.shape + (1,) * (t.dim() - 2)), t, torch.tensor(dim, device=DEV, dtype=t.dtype))
+    H, G = 4, 2
+    q = torch.randn(n, H * 64, device=DEV).bfloat16()
+    k, v = (torch.randn(pages, 16, G, d, device=DEV).bfloat16() for d in (64, 64))
+    outs = []
+    for bad in (0.0, float("inf"), float("nan")):
+        out = torch.zeros(n, H * G * 64, device=DEV)
+        kk, vv = (spoil(t, bad).transpose(1, 2).contiguous() for t in (k, v))
+        kernels.talking_attention_flash(q, out, kk, vv, tables, first, start, longest, H, G, 64, 64, G, 16, 0.5, 30.0, True, window, status)
+        outs.append(out)
+    assert int(status) == 0 and torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    q = torch.randn(n, H * 192, device=DEV).bfloat16()
+    cache = torch.randn(pages, 16, 192, device=DEV).bfloat16()
+    outs = []
+    for bad in (0.0, float("inf"), float("nan")):
+        out = torch.zeros(n, H * 128, dtype=torch.bfloat16, device=DEV)
+        kernels.latent_flash(q, out, spoil(cache, bad), tables, first, start, None, H, 128, 64, 16, 0.2, window, status, longest)
+        outs.append(out)
+    assert int(status) == 0 and torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
