@@ -123,10 +123,19 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
     const int qt = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, seq = blockIdx.y / a.col_blocks, col0 = (blockIdx.y % a.col_blocks) * DV;
     const int row0 = a.seq_first_row[seq], nrows = a.seq_first_row[seq + 1] - row0, q_lo = qt * FW_BM;
     const int start_pos = a.seq_start_pos[seq];
-    if (q_lo >= nrows || start_pos < 0) return;                 // (uniform for the block, before anything is allocated)
+    if (q_lo >= nrows) return;                                  // (uniform for the block, before anything is allocated)
     const int pos_lo = start_pos + q_lo, pos_hi = start_pos + min(nrows, q_lo + FW_BM) - 1;
-    if ((pos_hi >> a.page_shift) >= a.max_pages) {
-        if (tid == 0) atomicOr(a.status, GB_STATUS_BAD_POSITION);
+    // the last position that decides whether the table reaches far enough: of the request (latent), of the tile
+    const bool beyond = start_pos >= 0 && ((LATENT ? start_pos + nrows - 1 : pos_hi) >> a.page_shift) >= a.max_pages;
+    if (beyond && tid == 0) atomicOr(a.status, GB_STATUS_BAD_POSITION);
+    if (start_pos < 0 || beyond) {
+        if (LATENT) {                                           // a padding sequence: its rows read as zeros downstream
+            gb_pdl_launch_dependents();
+            gb_pdl_wait();
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + ((size_t)(row0 + q_lo) * a.H + head) * DV);
+            for (int i = tid; i < min(FW_BM, nrows - q_lo) * (DV / 8); i += FW_WARPS * 32)
+                dst[(size_t)(i / (DV / 8)) * a.H * (DV / 8) + i % (DV / 8)] = make_uint4(0, 0, 0, 0);
+        }
         return;
     }
     const int kvh = head / (a.H / a.kv_heads);

@@ -98,7 +98,7 @@ def test_latent_cache(page, window, batch, H, r, sink):
     for i, b in enumerate(batch):
         a, z = int(first[i]), int(first[i + 1])
         if b is None:
-            assert torch.all(got[a:z] == 7.0)
+            assert torch.all(got[a:z] == 0.0)       # (as the other kernels over this cache leave them)
             continue
         pos = b[0] + torch.arange(b[1], device=DEV)
         rows = _dense(cache[:, None], tables[i], page, b[0] + b[1])[:, 0]
@@ -115,9 +115,10 @@ def test_positions_beyond_the_table_and_missing_pages_are_reported():
     q = torch.randn(40, 2 * 160, device=DEV).bfloat16()
     cache = torch.randn(pages, 16, 160, device=DEV).bfloat16()
     for bad, bit in ((tables[:, :2].contiguous(), 4), (tables.clone().index_fill_(1, torch.tensor([1], device=DEV), -1), 2)):
-        out, status = torch.zeros(40, 256, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        out, status = torch.full((40, 256), 7.0, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
         kernels.latent_flash(q, out, cache, bad, first, start, None, 2, 128, 32, 16, 0.1, None, status, longest)
-        assert int(status) == bit
+        assert int(status) == bit and not (out == 7.0).any()
+        assert bit == 2 or not out.any()           # a request beyond its table reads as zeros
 
 
 @pytest.mark.parametrize("rows", [72, 129, 256, 300])
