@@ -42,14 +42,13 @@ __device__ __forceinline__ void me_gather4(void* dst, const CUtensorMap* map, ui
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
 
-// One gated unit as gb_gated_unit forms it, with the hardware's division (two units in the last place of float32, in front of
-// a rounding to bfloat16).
+// One gated unit with the numbers of gb_gated_unit.
 __device__ __forceinline__ float me_unit(float gate, float up, float limit, float slope) {
     if (slope > 0.f) {
         const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-        return __fdividef(g, 1.0f + expf(-slope * g)) * (u + 1.0f);
+        return gb_quotient(g, 1.0f + expf(-slope * g)) * (u + 1.0f);
     }
-    return slope < 0.f ? gb_gelu_tanh(gate) * up : __fdividef(gate, 1.0f + expf(-gate)) * up;
+    return slope < 0.f ? gb_gelu_tanh(gate) * up : gb_quotient(gate, 1.0f + expf(-gate)) * up;
 }
 
 template <int BN, bool UP>

@@ -66,3 +66,23 @@ def test_grouped_products(E, top, d, ff, unit, counts):
             # the activations are rounded to bfloat16 (2^-9 each) in front of a sum of ff products with weights of size ff^-1/2
             # (four of its standard deviations, and a quarter for the largest of some thousand sums)
             assert (got[r, k] - want).abs().max() <= 2 ** -9 * 5 * float(x.norm()) / ff ** 0.5 + 1e-5, (r, k, e)
+
+
+def test_the_unit_divides_as_float32_does():
+    """Gates near -87.5, whose denominators lie above 2^126: the quotients, some -1e-36, come out as numbers (times an up sum of 2^100)."""
+    from glassbox_b200 import kernels
+    n, d, ff = 40, 64, 64
+    h = torch.zeros(n, d)
+    h[:, 0] = 1.0
+    gates = -torch.linspace(86, 88, ff).bfloat16().float()
+    w_up, w_down = torch.zeros(ff, 2, d), torch.eye(d, ff)
+    w_up[:, 0, 0], w_up[:, 1, 0] = gates, 2.0 ** 100
+    dev = lambda t: t.bfloat16().to(DEV).contiguous()
+    i32 = lambda *shape: torch.zeros(*shape, dtype=torch.int32, device=DEV)
+    pair, status = torch.zeros(n, d, device=DEV), i32(1)
+    kernels.moe_experts_grouped(dev(h), dev(w_up.view(2 * ff, d)), dev(w_down), 1, i32(n, 1), torch.arange(n, dtype=torch.int32, device=DEV),
+                                i32(2 * 2 + n), torch.zeros(n, ff, dtype=torch.bfloat16, device=DEV), pair, unit=kernels.SILU_UNIT, status=status)
+    want = gates.double() / (1 + torch.exp(-gates.double())) * 2.0 ** 100
+    # float32: the exponential's argument is exact, its value and the quotient a few 2^-23 off; then one rounding to bfloat16
+    assert int(status) == 0
+    assert ((pair.double().cpu() - want).abs() <= 2 ** -8 * want.abs()).all()
