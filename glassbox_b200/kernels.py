@@ -1505,18 +1505,20 @@ def channel_delta(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bia
           seq_start_pos.shape[0], heads, kv_heads, dk, dv, state.shape[0], 1 if write_state else 0, _ptr(status), dc, 0, _stream())
 
 
-#: from how many rows of the longest portion on the delta rule runs in chunks of tokens instead of token by token, and how
-#: many rows more for every further request of the step
-DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 80, 8
+#: the delta rule runs in chunks of tokens instead of token by token from this many rows of a step on, and so many more for
+#: every request of the step
+DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 72, 7
 
 
-def delta_chunks_chosen(longest: int, num_seqs: int, dk: int) -> bool:
-    """Whether the delta rule takes a step of ``num_seqs`` requests, of which the longest brings ``longest`` rows, in chunks of 32
-    tokens (key sizes up to 128). The walk's time is its longest portion's; the chunks cost a further request more (its state
-    goes through shared memory). Whole mixer at 8 heads x 128 x 128, chunks / walk: one request of 48 rows 64 / 59 us, 64 rows
-    68 / 68, 96 rows 78 / 84, 256 rows 101 / 144; 36 requests of which the longest brings 19 rows 154 / 133; at 16 heads 88 / 83,
-    94 / 92, 100 / 108, 123 / 167 and 306 / 234."""
-    return dk <= 128 and longest >= DELTA_CHUNKS_FROM + DELTA_CHUNKS_PER_REQUEST * (num_seqs - 1)
+def delta_chunks_chosen(rows: int, num_seqs: int, dk: int) -> bool:
+    """Whether the delta rule takes a step of ``rows`` rows in ``num_seqs`` requests in chunks of 32 tokens (key sizes up to 128).
+    Both numbers are part of a recorded step's shape, which the longest portion is not. A request costs the chunks its state's way
+    through shared memory, a row costs the walk its place in the chain. Measured, kernels alone, heads of 128 x 128, walk /
+    chunks in us at 8 heads and at 16: one request of 48 rows 23 / 25 and 23 / 26, 64 rows 28 / 25 and 28 / 29, 96 rows 37 / 28; 8
+    requests of 64 rows in all 33 / 39 and 55 / 55, 128 rows 48 / 40 and 80 / 58; 36 requests (prompts' ends of up to 15 rows) of
+    192 rows 93 / 98 and 177 / 203, of 320 rows 119 / 99 and 227 / 210; 35 single tokens beside a portion of 100 rows 106 / 121 and 179
+    / 227, of 300 rows 174 / 141 and 278 / 263; 64 requests of 320 rows 156 / 181 and 302 / 395, of 1,024 rows 282 / 203 and 564 / 411."""
+    return dk <= 128 and rows >= DELTA_CHUNKS_FROM + DELTA_CHUNKS_PER_REQUEST * num_seqs
 
 
 def delta_chunks_needed(n: int, num_seqs: int) -> int:

@@ -26,9 +26,9 @@ from .linear import linear
 
 def run_delta(ctx, qkv, beta, decay, params, state, out, heads: int, kv_heads: int, dk: int, dv: int, writes_cache: bool,
               decay_per_head: bool = False) -> None:
-    """The recurrence over the step's runs of rows: in chunks of tokens where a portion is long enough, else token by token."""
+    """The recurrence over the step's runs of rows: in chunks of tokens where there are rows enough, else token by token."""
     args = (qkv, beta, decay, params["dt_bias"], params["a_log"], state, out, ctx.seq_first_row, ctx.seq_start_pos, ctx.seq_slots)
-    if not kernels.delta_chunks_chosen(ctx.max_rows_per_seq, ctx.seq_start_pos.shape[0], dk):
+    if not kernels.delta_chunks_chosen(qkv.shape[0], ctx.seq_start_pos.shape[0], dk):
         kernels.channel_delta(*args, heads, kv_heads, dk, dv, writes_cache, ctx.status, decay_per_head=decay_per_head)
         return
     chunks = kernels.delta_chunks_needed(qkv.shape[0], ctx.seq_start_pos.shape[0])

@@ -39,3 +39,39 @@ def test_decode_attention_plan_examples():
     assert kernels.decode_mma_plan(13, 32, 64, 4096) == (1, 16, 4)      # 416 pairs fit one wave by themselves
     assert kernels.decode_mma_plan(64, 32, 64, 4096) == (1, 16, 4)
     assert kernels.decode_mma_plan(64, 5, 64, 4096) == (1, 16, 4)
+
+
+class _DeltaStep:
+    """As much of a step context as the delta rule's dispatch reads; the arithmetic is replaced by a record of the route."""
+
+    def __init__(self, scratch, rows, seqs, longest):
+        import torch
+        from glassbox_b200.engine.context import Scratch, StepContext
+        cpu = torch.device("cpu")
+        self.own = Scratch(scratch.max_rows, torch.float32, cpu)             # what a recorded context keeps for itself
+        self.ctx = StepContext(scratch=scratch, cache=None, status=torch.zeros(1, dtype=torch.int32), dtype=torch.float32, grow_scratch=self.own)
+        self.ctx.max_rows_per_seq, self.ctx.seq_start_pos = longest, torch.zeros(seqs, dtype=torch.int32)
+        self.qkv, self.state = torch.zeros(rows, 1), torch.zeros(4, 8)
+
+    def route(self, monkeypatch, heads=2, dk=128):
+        from glassbox_b200.parts import delta_rule
+        taken = []
+        monkeypatch.setattr(kernels, "channel_delta", lambda *a, **k: taken.append(("walk", None)))
+        monkeypatch.setattr(kernels, "channel_delta_chunks", lambda *a, **k: taken.append(("chunks", a[-1])))
+        monkeypatch.setattr(kernels, "delta_chunk_floats", lambda: 6)
+        monkeypatch.setattr(kernels, "delta_chunks_needed", lambda n, s: n // 32 + s)
+        delta_rule.run_delta(self.ctx, self.qkv, None, None, {"dt_bias": None, "a_log": None}, self.state, None, heads, heads, dk, 128, True)
+        return taken[0]
+
+
+@pytest.mark.parametrize("rows, seqs, longest, dk, want", [
+    (64, 1, 128, 128, "walk"),           # a portion of up to 64 rows as a recorded step sees it: 64 rows, a tile of 128
+    (128, 1, 128, 128, "chunks"), (2048, 1, 2048, 64, "chunks"), (2048, 1, 2048, 256, "walk"),
+    (448, 64, 448, 128, "walk"),         # 36 portions of up to 19 rows, recorded with 64 sequences
+    (1024, 64, 1024, 128, "chunks"), (168, 41, 128, 128, "walk"), (2088, 41, 2048, 128, "chunks"),
+])
+def test_the_delta_rule_is_chosen_by_what_a_recorded_step_knows(monkeypatch, rows, seqs, longest, dk, want):
+    import torch
+    from glassbox_b200.engine.context import Scratch
+    step = _DeltaStep(Scratch(4096, torch.float32, torch.device("cpu")), rows, seqs, longest)
+    assert step.route(monkeypatch, dk=dk)[0] == want
