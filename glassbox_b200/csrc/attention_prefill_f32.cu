@@ -259,7 +259,8 @@ __global__ void __launch_bounds__(PS_THREADS, HD <= 64 ? 3 : 1) attention_prefil
                 }
             }
         } else {
-            for (int kk = 0; kk < PS_BN; ++kk) {
+            const int kk_begin = max(key_lo - key0, 0), kk_end = min(pos_hi - key0 + 1, PS_BN);      // (no row sees the others)
+            for (int kk = kk_begin; kk < kk_end; ++kk) {
                 const float4 pa = *reinterpret_cast<const float4*>(K + kk * PP + ty * 8);
                 const float4 pb = *reinterpret_cast<const float4*>(K + kk * PP + ty * 8 + 4);
                 const float w[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
