@@ -65,6 +65,17 @@ class Scratch:
         return buf
 
 
+    def flat(self, name: str, count: int, dtype: torch.dtype) -> torch.Tensor:
+        """A flat buffer of ``count`` numbers, contents undefined. The same count every time hands out the same buffer: a
+        recorded step keeps the address, so whoever asks names the most that any step of the engine can need."""
+        key = (name, dtype)
+        buf = self._bufs.get(key)
+        if buf is None or buf.numel() < count:
+            buf = torch.empty(count, dtype=dtype, device=self.device)
+            self._bufs[key] = buf
+        return buf
+
+
 class WeightOrder:
     """Learns the order in which weight matrices are used in a step (it is the same in every step of
     one model) from the calls themselves, so that a product can ask the memory system for the weights
@@ -149,6 +160,9 @@ class StepContext:
 
     def zeros_once(self, name: str, count: int, dtype: torch.dtype) -> torch.Tensor:
         return self._scratch.zeros_once(self.scratch_prefix + name, count, dtype)
+
+    def flat(self, name: str, count: int, dtype: torch.dtype) -> torch.Tensor:
+        return self._scratch.flat(self.scratch_prefix + name, count, dtype)
 
     @property
     def max_rows(self) -> int:

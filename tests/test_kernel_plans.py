@@ -75,3 +75,19 @@ def test_the_delta_rule_is_chosen_by_what_a_recorded_step_knows(monkeypatch, row
     from glassbox_b200.engine.context import Scratch
     step = _DeltaStep(Scratch(4096, torch.float32, torch.device("cpu")), rows, seqs, longest)
     assert step.route(monkeypatch, dk=dk)[0] == want
+
+
+def test_recorded_steps_share_the_delta_rules_workspace(monkeypatch):
+    """Steps of ten shapes, each with buffers of its own for what depends on the shape, work in one buffer, large enough for the
+    largest step of the engine."""
+    import torch
+    from glassbox_b200.engine.context import Scratch
+    shared = Scratch(2048, torch.float32, torch.device("cpu"))
+    seen = set()
+    for rows, seqs in [(128, 1), (256, 2), (512, 4), (1024, 8), (1536, 8), (2048, 12), (2048, 1), (640, 4), (320, 2), (192, 1)]:
+        step = _DeltaStep(shared, rows, seqs, rows)
+        how, work = step.route(monkeypatch)
+        assert how == "chunks" and work.numel() >= (rows // 32 + seqs) * 2 * 6
+        assert not step.own._bufs
+        seen.add((work.data_ptr(), work.numel()))
+    assert len(seen) == 1 and seen.pop()[1] == (2048 // 32 + 2 * 4 + 8) * 2 * 6
