@@ -1293,10 +1293,20 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
         launch_count += 1
 
 
-def latent_flash_supported(q: torch.Tensor, num_seqs: int, c: int, r: int, page_size: int) -> bool:
-    """Whether the tcgen05 kernel takes a step of prompt portions with these sizes, and the portions are long enough for it."""
-    return (q.dtype == torch.bfloat16 and q.shape[0] >= FLASH_WIDE_MIN_ROWS * num_seqs
-            and bool(lib().gb_latent_flash_supported(c, r, page_size)))
+def latent_flash_chosen(rows: int, num_seqs: int, heads: int, max_context: int) -> bool:
+    """Whether portions of ``rows`` rows in ``num_seqs`` requests go to ``latent_flash`` rather than to ``latent_attention_mma``, which packs
+    tokens x heads into its tiles and so loses nothing to short portions. A block of the flash kernel has a multiprocessor to
+    itself: as long as one block a request and head fits the chip's 148 at once it is the faster or level (one request of 32 heads,
+    tiles / flash in us: 8 and 32 fresh rows 6 / 7 and 7 / 7, behind 500 tokens 24 / 11 and 26 / 12, behind 4,000 159 / 47 and 160 / 47).
+    Beyond, its blocks come in rounds, and the rows must be worth it: 16 requests of 32 heads, fresh portions of 48, 64 and 96 rows
+    14 / 27, 16 / 28, 27 / 29; behind 500 tokens 32, 48 and 64 rows 35 / 50, 65 / 50, 68 / 51; behind 2,000 tokens 16, 48 and 64 rows
+    103 / 104, 190 / 106, 218 / 114. (``max_context`` is what the block tables of a recorded step cover.)"""
+    return heads * num_seqs <= 148 or rows >= (96 if max_context < 512 else 48) * num_seqs
+
+
+def latent_flash_supported(dtype: torch.dtype, c: int, r: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel takes prompt portions with these sizes."""
+    return dtype == torch.bfloat16 and bool(lib().gb_latent_flash_supported(c, r, page_size))
 
 
 def latent_flash(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor, seq_first_row: torch.Tensor,

@@ -152,30 +152,43 @@ class LatentAttention(Mixer):
     def attend(self, ctx, qabs, lat, cache) -> None:
         """lat[row, head, :] = the softmax-weighted sum of the latents the row sees. bfloat16 at the sizes the
         tensor-core kernels are built for: decode steps cut each row's keys into shares so that few requests still fill the
-        GPU; steps with prompt portions run tiles of 128 tokens of a head (long portions) or of tokens x heads. Anything else: one warp per (row, head)."""
-        n = qabs.shape[0]
-        if not ctx.decode_only and kernels.latent_flash_supported(qabs, ctx.seq_start_pos.shape[0], self.c, self.r, cache.page_size):
-            kernels.latent_flash(qabs, lat, cache.k, cache.block_tables, ctx.seq_first_row, ctx.seq_start_pos, self.params.get("sink"), self.H,
-                                 self.c, self.r, cache.page_size, self.spec.scale, self.spec.window, ctx.status, ctx.max_rows_per_seq)
+        GPU; steps with prompt portions run tiles of 128 tokens of a head (long portions) or of tokens x heads. The single tokens that
+        lead a step with long portions take the decode kernel: a tile of 128 tokens for each of them and head costs more than
+        the portions (32 tokens behind 2,000 keys beside 1,100 rows, 32 heads: 250 us in one kernel, 114 in tiles of tokens x heads,
+        26 + 27 us in two). Anything else: one warp per (row, head)."""
+        n, S = qabs.shape[0], ctx.seq_start_pos.shape[0]
+        mma = kernels.latent_attention_mma_supported(qabs.dtype, self.c, self.r, cache.page_size)
+        if ctx.decode_only and mma:
+            self._attend_decode(ctx, qabs, lat, cache, n)
             return
-        if kernels.latent_attention_mma_supported(qabs.dtype, self.c, self.r, cache.page_size):
-            common = (qabs, lat, cache.k, cache.block_tables, ctx.seq_first_row, ctx.seq_start_pos, ctx.positions,
-                      self.params.get("sink"), self.H, self.c, self.r, cache.page_size, self.spec.scale, self.spec.window,
-                      ctx.status)
-            if ctx.decode_only:
-                window = self.spec.window or ctx.max_context
-                splits = kernels.latent_decode_splits(n, self.H, min(ctx.max_context, window))
-                part_o = part_ml = None
-                if splits > 1:
-                    part_o = ctx.scratch("latent_part_o", (n, self.H * splits * self.c), torch.float32, grow=True)
-                    part_ml = ctx.scratch("latent_part_ml", (n, self.H * splits * 2), torch.float32, grow=True)
-                kernels.latent_attention_mma(*common, decode=True, splits=splits, part_o=part_o, part_ml=part_ml)
-            else:
-                kernels.latent_attention_mma(*common, max_rows_per_seq=ctx.max_rows_per_seq)
+        if not ctx.decode_only and kernels.latent_flash_supported(qabs.dtype, self.c, self.r, cache.page_size):
+            lead = ctx.leading_single if mma else 0
+            if kernels.latent_flash_chosen(n - lead, S - lead, self.H, ctx.max_context):
+                if lead:
+                    self._attend_decode(ctx, qabs, lat, cache, lead)
+                kernels.latent_flash(qabs, lat, cache.k, cache.block_tables[lead:], ctx.seq_first_row[lead:], ctx.seq_start_pos[lead:],
+                                     self.params.get("sink"), self.H, self.c, self.r, cache.page_size, self.spec.scale, self.spec.window,
+                                     ctx.status, ctx.max_rows_per_seq)
+                return
+        if mma:
+            kernels.latent_attention_mma(qabs, lat, cache.k, cache.block_tables, ctx.seq_first_row, ctx.seq_start_pos, ctx.positions,
+                                         self.params.get("sink"), self.H, self.c, self.r, cache.page_size, self.spec.scale, self.spec.window,
+                                         ctx.status, max_rows_per_seq=ctx.max_rows_per_seq)
             return
         kernels.latent_attention_rows(qabs, lat, cache.k, cache.block_tables, ctx.row_seq, ctx.positions,
                                       self.params.get("sink"), self.H, self.c, self.r, cache.page_size, self.spec.scale,
                                       self.spec.window, ctx.status)
+
+    def _attend_decode(self, ctx, qabs, lat, cache, n: int) -> None:
+        """Rows 0 .. n - 1, one per request (request i is row i), their keys cut into shares."""
+        splits = kernels.latent_decode_splits(n, self.H, min(ctx.max_context, self.spec.window or ctx.max_context))
+        part_o = part_ml = None
+        if splits > 1:
+            part_o = ctx.scratch("latent_part_o", (n, self.H * splits * self.c), torch.float32, grow=True)
+            part_ml = ctx.scratch("latent_part_ml", (n, self.H * splits * 2), torch.float32, grow=True)
+        kernels.latent_attention_mma(qabs[:n], lat[:n], cache.k, cache.block_tables[:n], ctx.seq_first_row[:n + 1], ctx.seq_start_pos[:n],
+                                     ctx.positions[:n], self.params.get("sink"), self.H, self.c, self.r, cache.page_size, self.spec.scale,
+                                     self.spec.window, ctx.status, decode=True, splits=splits, part_o=part_o, part_ml=part_ml)
 
 
 register_part("mixer", "latent_attention", LatentAttention, replace=True)

@@ -91,3 +91,44 @@ def test_recorded_steps_share_the_delta_rules_workspace(monkeypatch):
         assert not step.own._bufs
         seen.add((work.data_ptr(), work.numel()))
     assert len(seen) == 1 and seen.pop()[1] == (2048 // 32 + 2 * 4 + 8) * 2 * 6
+
+
+@pytest.mark.parametrize("rows, seqs, heads, context, want", [
+    (8, 1, 32, 64, True), (1500, 2, 32, 4096, True), (64, 16, 4, 128, True),      # one round of blocks
+    (16 * 64, 16, 32, 128, False), (16 * 96, 16, 32, 128, True),                   # fresh portions in several rounds
+    (16 * 32, 16, 32, 2048, False), (16 * 48, 16, 32, 2048, True),                 # behind cached tokens
+])
+def test_latent_portions_take_the_flash_kernel_where_it_is_the_faster(rows, seqs, heads, context, want):
+    assert kernels.latent_flash_chosen(rows, seqs, heads, context) is want
+
+
+def test_single_tokens_of_a_latent_step_take_the_decode_kernel(monkeypatch):
+    """A step of 40 leading single tokens and two portions: rows 0 to 39 to the decode kernel, the portions to the flash kernel, with
+    the tables and positions that belong to them."""
+    import torch
+    from types import SimpleNamespace
+    from glassbox_b200.parts.latent_attention import LatentAttention
+    taken = []
+    monkeypatch.setattr(kernels, "latent_attention_mma_supported", lambda *a: True)
+    monkeypatch.setattr(kernels, "latent_flash_supported", lambda *a: True)
+    monkeypatch.setattr(kernels, "latent_decode_splits", lambda *a: 1)
+    monkeypatch.setattr(kernels, "latent_attention_mma", lambda q, out, cache, tables, first, start, *a, **k: taken.append(
+        ("decode" if k.get("decode") else "tiles", q.shape[0], tables.shape[0], first.tolist(), start.tolist())))
+    monkeypatch.setattr(kernels, "latent_flash", lambda q, out, cache, tables, first, start, *a, **k: taken.append(
+        ("flash", q.shape[0], tables.shape[0], first.tolist(), start.tolist())))
+    lead, portions = 40, [300, 500]
+    first = list(range(lead + 1)) + [lead + 300, lead + 800]
+    start = list(range(100, 100 + lead)) + [7, 9]
+    ctx = SimpleNamespace(decode_only=False, leading_single=lead, max_context=2048, max_rows_per_seq=500, status=None,
+                          seq_first_row=torch.tensor(first), seq_start_pos=torch.tensor(start), positions=torch.zeros(840))
+    part = SimpleNamespace(H=32, c=128, r=64, params={}, spec=SimpleNamespace(scale=1.0, window=None))
+    part._attend_decode = lambda *a: LatentAttention._attend_decode(part, *a)
+    cache = SimpleNamespace(k=None, page_size=16, block_tables=torch.zeros(42, 8))
+    q = torch.zeros(840, 1, dtype=torch.bfloat16)
+    LatentAttention.attend(part, ctx, q, q, cache)
+    assert taken == [("decode", 40, 40, first[:41], start[:40]), ("flash", 840, 2, first[40:], start[40:])]
+    taken.clear()
+    ctx.max_context, ctx.seq_first_row = 128, torch.tensor(list(range(lead + 1)) + [lead + 20, lead + 40])      # short portions, many heads
+    part.H = 128
+    LatentAttention.attend(part, ctx, q[:80], q[:80], cache)
+    assert [t[:3] for t in taken] == [("tiles", 80, 42)]
