@@ -101,9 +101,8 @@ class TalkingAttention(Mixer):
         else:
             wide = ctx.scratch("tk_wide", (n, cols), torch.float32)
             if how == "tiles":
-                # (long portions at the sizes it is built for: the tcgen05 kernel)
-                flash = value_heads == self.G and kernels.talking_attention_flash_supported(q, ctx.seq_start_pos.shape[0], self.D, self.V, value_heads,
-                                                                                            cache.page_size)
+                # (the sizes it is built for: the tcgen05 kernel)
+                flash = value_heads == self.G and kernels.talking_attention_flash_supported(q.dtype, self.D, self.V, value_heads, cache.page_size)
                 attend = kernels.talking_attention_flash if flash else kernels.talking_attention_tiles
                 attend(q, wide, cache.k, cache.v, cache.block_tables, ctx.seq_first_row, ctx.seq_start_pos, ctx.max_rows_per_seq, **common)
             else:
