@@ -125,12 +125,15 @@ GB_EXPORT int gb_short_conv(const float* x, long long ldx, const float* w, float
                             int num_slots, int update_state, int* status, cudaStream_t stream) {
     GB_REQUIRE(n >= 0 && S >= 0 && C > 0 && taps >= 1 && taps <= 64, "gb_short_conv: bad sizes (taps %d)", taps);
     if (n == 0 || S == 0) return 0;
-    // strips only where they fill the chip (half a block of 256 channels an SM or more) and for the taps they are built for
+    // Strips for the taps they are built for, where there are three blocks of them an SM: with fewer, a thread's sixteen rows one after
+    // the other take longer than a thread a row. Four taps, rows apiece / strips in us (with the state's update): 3,072 channels, 384
+    // rows (288 blocks) of one request 12.9 / 13.1, of as many requests 19.9 / 22.9; 512 rows (384 blocks) 15.7 / 15.4 and 24.9 / 25.9;
+    // 768 rows (576 blocks) 21.2 / 15.2 and 34.9 / 30.7; 128 rows (96 blocks) 7.1 / 10.2 and 9.9 / 17.2.
     const dim3 strips(gb_ceil_div(n, SC_STRIP), gb_ceil_div(C, 256)), grid(n, gb_ceil_div(C, 256));
 #define SC_STRIPS(TAPS)                                                                                                            \
     gb_launch(GB_PDL_ELEMENTWISE, short_conv_strip_kernel<TAPS>, strips, dim3(256), 0, stream, x, ldx, w, y, ldy, (const float*)state, \
               state_stride, state_off, row_seq, positions, seq_first_row, seq_slots, n, C, num_slots, status)
-    const bool many = (long long)strips.x * strips.y >= 74;
+    const bool many = (long long)strips.x * strips.y >= 444;
     if (many && taps == 4) SC_STRIPS(4);
     else if (many && taps == 3) SC_STRIPS(3);
     else if (many && taps == 2) SC_STRIPS(2);
