@@ -119,7 +119,7 @@ class GqaAttention(Mixer):
                 return
         else:
             k = ctx.leading_single if ctx.leading_single * self.nh > SPLIT_MIXED_ABOVE else 0
-            if k and self._has_flash(q, att, cache) and self._attend_decode(ctx, q[:k], att[:k], cache, k):
+            if k and self._has_flash(ctx, q, att, cache) and self._attend_decode(ctx, q[:k], att[:k], cache, k):
                 self._attend_flash(ctx, q, att, cache, k)
                 return
             if self._attend_flash(ctx, q, att, cache, 0):
@@ -151,10 +151,13 @@ class GqaAttention(Mixer):
             return True
         return False
 
-    def _has_flash(self, q, att, cache) -> bool:
+    def _takes_flash_f32(self, ctx, q, att) -> bool:
+        return ctx.max_context > FLASH_F32_MIN_CONTEXT and kernels.attention_prefill_f32_supported(q, att, self.nh, self.nkv, self.hd)
+
+    def _has_flash(self, ctx, q, att, cache) -> bool:
         return (kernels.attention_prefill_tc_supported(q, att, self.nh, self.nkv, self.hd, cache.page_size)
                 or kernels.attention_prefill_supported(q.dtype, self.nh, self.nkv, self.hd, cache.page_size)
-                or kernels.attention_prefill_f32_supported(q, att, self.nh, self.nkv, self.hd))
+                or self._takes_flash_f32(ctx, q, att))
 
     def _attend_flash(self, ctx, q, att, cache, first_seq: int) -> bool:
         """The requests from ``first_seq`` on (runs of consecutive rows); False if no flash kernel takes the shape."""
@@ -170,7 +173,7 @@ class GqaAttention(Mixer):
                                       self.nh, self.nkv, self.hd, cache.page_size, self.spec.scale, self.spec.window,
                                       ctx.status)
             return True
-        if kernels.attention_prefill_f32_supported(q, att, self.nh, self.nkv, self.hd):
+        if self._takes_flash_f32(ctx, q, att):
             kernels.attention_prefill_f32(q, att, cache.k, cache.v, tables, first_row, start_pos, ctx.max_rows_per_seq,
                                           self.nh, self.nkv, self.hd, cache.page_size, self.spec.scale, self.spec.window,
                                           ctx.status)
@@ -181,5 +184,9 @@ class GqaAttention(Mixer):
 #: a mixed batch is split between the decode and the flash kernel when its leading single-token requests would
 #: otherwise add more 128-row tiles (one per request and head) than the GPU has SMs
 SPLIT_MIXED_ABOVE = 148
+
+#: up to this many tokens a request (cached and new) the one-warp kernel walks its few keys in less time than a 64 x 64 tile takes in
+#: float32: 32 prompts of 8 tokens at 32 heads 20 us against 30, at 9 heads 9 against 11; of 16 tokens 52 against 32 and 19 against 12
+FLASH_F32_MIN_CONTEXT = 8
 
 register_part("mixer", "gqa_attention", GqaAttention, replace=True)
