@@ -927,9 +927,11 @@ static int tkm_launch(const float* o, const float* talk, void* att, const int* p
     return gb_check_launch("gb_talk_combine");
 }
 
-// From this many (row, value head) pairs the mix goes to a thread per four channels: 64 of them fill the chip's 148 blocks of 256
-// threads twice over at 64 channels; below, the few blocks would leave SMs idle that the block per pair (32 rows: 6.4 us) reaches.
-constexpr long long TKM_MIN_PAIRS = 1024;
+// From this many (row, value head) pairs the mix goes to a thread per four channels; with fewer, its handful of blocks (16 pairs of 64
+// channels each) takes as long as the block per pair. Block per pair / thread per four channels in us: 16 heads, 4 value heads of 64, 8
+// rows (32 pairs) 2.7 / 2.9, 24 rows (96) 3.1 / 3.1, 32 rows (128) 3.4 / 3.1, 256 rows 6.1 / 3.3; 8 and 8 heads of 64, 16 rows (128) 2.9 /
+// 2.5; 16 and 8 heads of 128, 16 rows 3.9 / 2.9.
+constexpr long long TKM_MIN_PAIRS = 128;
 
 template <typename T>
 static int tkc_launch(const float* o, const float* ml, const float* talk, void* att, const int* positions, int n, int H, int G, int V,
