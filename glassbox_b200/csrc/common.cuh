@@ -9,6 +9,7 @@
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 #define GB_EXPORT extern "C" __attribute__((visibility("default")))
@@ -49,17 +50,16 @@ __device__ __forceinline__ float gb_clamped_unit(float gate, float up, float lim
     return g / (1.0f + expf(-slope * g)) * (u + 1.0f);
 }
 
-// v / d for d >= 1 (infinity included), the denominators of the sigmoid, rounded as v / d is: an estimate of 1 / d, one step of
-// Newton's method, and the correction of the quotient by its own remainder, exact in a fused multiply-add (Markstein, Computation of
-// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990). Where infinities make that a NaN,
-// the product with the estimate is the quotient. In an epilogue of 64 quotients a thread and tile the difference shows: gated product
-// of 2,048 rows (K 576, I 1536) 19.5 us with v / d, with this 12.7.
+// v / d for d >= 1 (infinity included), the denominators of the sigmoid, rounded as v / d is: the product with an estimate of 1 / d and its
+// correction by the remainder, exact in a fused multiply-add (Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor, IBM J. Res. Dev. 34, 1990). Where an infinity makes the remainder a NaN, the maximum puts a number in its
+// place that the infinite or zero quotient outweighs. In an epilogue of 64 quotients a thread and tile the way counts: gated product of 2,048
+// rows (K 576, I 1536) 19.5 us with v / d, 12.7 with this; with a comparison and a choice at the end instead of the maximum 17.
 __device__ __forceinline__ float gb_quotient(float v, float d) {
     float r0;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r0) : "f"(d));
-    const float r = fmaf(fmaf(-d, r0, 1.0f), r0, r0), q = v * r;
-    const float c = fmaf(fmaf(-q, d, v), r, q);
-    return c == c ? c : v * r0;
+    const float q = v * r0;
+    return fmaf(fmaxf(fmaf(-q, d, v), -FLT_MAX), r0, q);
 }
 
 // The tanh form of GELU: 0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))).
