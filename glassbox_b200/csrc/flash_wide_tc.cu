@@ -62,23 +62,36 @@ __device__ __forceinline__ float fw_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// s <- cap * tanh(s * in) for a warp's scores, as exactly as a call of tanhf (measured over |s * in| < 20: at most 1.5 units in the
-// last place of the tanh; NaN stays NaN). Below 1 the tanh is y + y t c(t), t = y^2, with c the interpolation of (tanh(sqrt t) / sqrt t
-// - 1) / t at the Chebyshev nodes of [0, 1] (2e-8 off): fused multiply-adds of two scores at a time and no special function, which is
-// all that most warps need (their scores lie within the cap). Where one of a warp's scores does not, all of them also form
-// 1 - 2 / (1 + e^(2|y|)). Talking-heads mixer of 2,048 tokens: 100 us; with tanhf for every score 112.
-__device__ __forceinline__ void fw_cap(uint32_t (&s)[64], float in, float cap) {
-    float top[2] = {0.f, 0.f};
-    const float2 in2 = make_float2(in, in), cap2 = make_float2(cap, cap);
+// s <- tanh(s * in) for a warp's scores, as exactly as a call of tanhf (at most 1.1 units in the last place below 1, two beyond; NaN
+// stays NaN). The tanh of y is y + y t c(t), t = y^2, with c the interpolation of (tanh(sqrt t) / sqrt t - 1) / t at Chebyshev nodes: of
+// [0, 0.36] for a warp whose scores all lie within 0.6 of the cap (most do), of [0, 1] otherwise, fused multiply-adds of two
+// scores at a time and no special function. Where a score lies beyond the cap, 1 - 2 / (1 + e^(2|y|)).
+__device__ __forceinline__ void fw_tanh(uint32_t (&s)[64], float in) {
+    float top = 0.f;
+    const float2 in2 = make_float2(in, in);
 #pragma unroll
     for (int k = 0; k < 64; k += 2) {
         const float2 y = __fmul2_rn(make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), in2);
         s[k] = __float_as_uint(y.x);
         s[k + 1] = __float_as_uint(y.y);
-        top[(k >> 1) & 1] = fmaxf(top[(k >> 1) & 1], fmaxf(fabsf(y.x), fabsf(y.y)));
+        top = fmaxf(fmaxf(top, fabsf(y.x)), fabsf(y.y));
     }
-    const bool beyond = __any_sync(0xffffffffu, fmaxf(top[0], top[1]) >= 1.0f);
     auto both = [](float c) { return make_float2(c, c); };
+    if (!__any_sync(0xffffffffu, top >= 0.6f)) {
+#pragma unroll
+        for (int k = 0; k < 64; k += 2) {
+            const float2 y = make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), t = __fmul2_rn(y, y);
+            float2 w = __ffma2_rn(both(-0.0062691197f), t, both(0.021110959f));
+            w = __ffma2_rn(w, t, both(-0.05387395f));
+            w = __ffma2_rn(w, t, both(0.13332915f));
+            w = __ffma2_rn(w, t, both(-0.3333333135f));
+            w = __ffma2_rn(y, __fmul2_rn(w, t), y);
+            s[k] = __float_as_uint(w.x);
+            s[k + 1] = __float_as_uint(w.y);
+        }
+        return;
+    }
+    const bool beyond = __any_sync(0xffffffffu, top >= 1.0f);
 #pragma unroll
     for (int k = 0; k < 64; k += 2) {
         const float2 y = make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), t = __fmul2_rn(y, y);
@@ -88,15 +101,14 @@ __device__ __forceinline__ void fw_cap(uint32_t (&s)[64], float in, float cap) {
         w = __ffma2_rn(w, t, both(-0.05393479f));
         w = __ffma2_rn(w, t, both(0.13333128f));
         w = __ffma2_rn(w, t, both(-0.3333333135f));
-        float2 r = __ffma2_rn(y, __fmul2_rn(w, t), y);
+        w = __ffma2_rn(y, __fmul2_rn(w, t), y);
         if (beyond) {
             auto far = [](float v) { return copysignf(1.0f - __fdividef(2.0f, 1.0f + fw_exp2(fabsf(v) * (2.0f * FW_LOG2E))), v); };
-            if (!(fabsf(y.x) < 1.0f)) r.x = far(y.x);
-            if (!(fabsf(y.y) < 1.0f)) r.y = far(y.y);
+            if (!(fabsf(y.x) < 1.0f)) w.x = far(y.x);
+            if (!(fabsf(y.y) < 1.0f)) w.y = far(y.y);
         }
-        r = __fmul2_rn(r, cap2);
-        s[k] = __float_as_uint(r.x);
-        s[k + 1] = __float_as_uint(r.y);
+        s[k] = __float_as_uint(w.x);
+        s[k + 1] = __float_as_uint(w.y);
     }
 }
 // MN-major B operand (rows are keys, 64-channel column blocks FW_BLOCK apart), 128-byte-swizzled rows
@@ -275,7 +287,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
         const float sl2 = a.scale * FW_LOG2E;                   // scores are brought into the base-2 domain
         const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? a.scale / a.cap : 0.f;
-        const float slx = cap2 > 0.f ? 1.0f : sl2;              // what is left to scale once capped
+        const float slx = cap2 > 0.f ? cap2 : sl2;              // what is left to scale
         const int first = gb_first_key(pos, a.window), first_last = gb_first_key(pos_lo + FW_BM - 1, a.window);
         float m_run = FW_NEG_BIG, l_run = 0.f;
         bool ok = true;
@@ -286,7 +298,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             uint32_t sv[64];
             tmem_load64(lane_base + (uint32_t)(b * FW_BN + h * 64), sv);
             tc_fence_before();
-            if (cap2 > 0.f) fw_cap(sv, cap_in, cap2);
+            if (cap2 > 0.f) fw_tanh(sv, cap_in);                // (the cap itself is left to the scale)
             if (key0 + 63 > pos_lo || key0 < first_last) {      // the tile crosses the diagonal, the window's edge or the last key
 #pragma unroll
                 for (int k = 0; k < 64; ++k)
@@ -304,6 +316,22 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             if (lane == 0) mbar_arrive(&sh.x_bar[q]);
             if (!mbar_wait_warp(&sh.x_bar[q], j & 1, abort_flag, a.status)) { ok = false; break; }
             mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
+            // Keys that no row of the block sees have a weight of 0, but what lies in their place in the pages (an earlier
+            // request's values, or nothing yet) may be no finite number: zeros take its place before the product. Only the tiles
+            // at the ends of the walk hold such keys.
+            const int lo = key_lo - (kt_begin + j) * FW_BN, hi = pos_hi - (kt_begin + j) * FW_BN;
+            const bool edge = lo > 0 || hi < FW_BN - 1;
+            if (edge) {
+                const int s = LATENT ? j % G::K_STAGES : j % G::V_STAGES, phase = (LATENT ? j / G::K_STAGES : j / G::V_STAGES) & 1;
+                if (!mbar_wait_warp(LATENT ? &sh.k_full[s] : &sh.v_full[s], phase, abort_flag, a.status)) { ok = false; break; }
+                unsigned char* values = LATENT ? Ks + s * G::K_BYTES : Vs + s * G::V_BYTES;
+                const int front = max(lo, 0), cleared = front + max(FW_BN - 1 - hi, 0);
+                constexpr int PIECES = DV / 8;                  // 16-byte pieces of a key's values, eight a column block
+                for (int i = (warp - 2) * 32 + lane; i < cleared * PIECES; i += 256) {
+                    const int k = i / PIECES, piece = i % PIECES, key = k < front ? k : hi + 1 + k - front;
+                    *reinterpret_cast<uint4*>(values + (piece >> 3) * FW_BLOCK + key * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
+                }
+            }
             const bool raise = (mx - m_run) * slx > 8.0f;
             if (j == 0) {
                 if (raise) m_run = mx;                          // nothing is accumulated yet
@@ -338,20 +366,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
             }
             l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
-            // Keys that no row of the block sees have a weight of 0, but what lies in their place in the pages (an earlier
-            // request's values, or nothing yet) may be no finite number: zeros take its place before the product. Only the tiles
-            // at the ends of the walk hold such keys.
-            const int lo = key_lo - (kt_begin + j) * FW_BN, hi = pos_hi - (kt_begin + j) * FW_BN;
-            if (lo > 0 || hi < FW_BN - 1) {
-                const int s = LATENT ? j % G::K_STAGES : j % G::V_STAGES, phase = (LATENT ? j / G::K_STAGES : j / G::V_STAGES) & 1;
-                if (!mbar_wait_warp(LATENT ? &sh.k_full[s] : &sh.v_full[s], phase, abort_flag, a.status)) { ok = false; break; }
-                unsigned char* values = LATENT ? Ks + s * G::K_BYTES : Vs + s * G::V_BYTES;
-                for (int i = (warp - 2) * 32 + lane; i < DV / 64 * FW_BN * 8; i += 256) {
-                    const int key = (i >> 3) & (FW_BN - 1);
-                    if (key < lo || key > hi) *reinterpret_cast<uint4*>(values + (i >> 10) * FW_BLOCK + key * 128 + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            }
+            if (edge) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tmem_store32(lane_base + (uint32_t)(b * FW_BN + h * 32), pw);
             tc_fence_before();
             __syncwarp();
