@@ -12,7 +12,8 @@
 //   warps 2-9  softmax, two threads per row: a thread reads 64 of its row's 128 scores, caps and masks them, exchanges its
 //              maximum with its partner, and writes its half of P_j. The running maximum is raised (and O rescaled) only when
 //              exceeded by more than 2^8 in the exponent, as in attention_prefill_tc.cu.
-//   warp 10    producer of the values (not for the latent cache, whose key tile serves both products)
+//   warp 10    producer of the values (not for the latent cache, whose key tile serves both products); puts zeros in the place of
+//              keys that no row of the block sees
 // Bound by the softmax warps (an exponential a score: 1,024 cycles a tile of the special-function unit, and with a cap nine fused
 // multiply-adds, against 1,280 of the tensor pipe); the mma.sync kernels that this replaced formed the scores once per 128 value
 // channels and fed both products through ldmatrix. Measured: see gb_talking_attention_flash, gb_latent_flash.
@@ -43,7 +44,7 @@ struct FwArgs {
 };
 
 struct __align__(8) FwShared {
-    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, o_done, x_bar[4];
+    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, o_done, x_bar[4], scored[2], cleared[2];
     float stat[2][2][FW_BM];   // [parity of the tile][half][row]: a half's maximum, at the end its sum
     uint32_t tmem_base;
     int abort_flag, issued[2], consumed[2], q_issued, q_consumed;
@@ -67,15 +68,16 @@ __device__ __forceinline__ float fw_exp2(float x) {
 // [0, 0.36] for a warp whose scores all lie within 0.6 of the cap (most do), of [0, 1] otherwise, fused multiply-adds of two
 // scores at a time and no special function. Where a score lies beyond the cap, 1 - 2 / (1 + e^(2|y|)).
 __device__ __forceinline__ void fw_tanh(uint32_t (&s)[64], float in) {
-    float top = 0.f;
+    float tops[4] = {0.f, 0.f, 0.f, 0.f};
     const float2 in2 = make_float2(in, in);
 #pragma unroll
     for (int k = 0; k < 64; k += 2) {
         const float2 y = __fmul2_rn(make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), in2);
         s[k] = __float_as_uint(y.x);
         s[k + 1] = __float_as_uint(y.y);
-        top = fmaxf(fmaxf(top, fabsf(y.x)), fabsf(y.y));
+        tops[(k >> 1) & 3] = fmaxf(fmaxf(tops[(k >> 1) & 3], fabsf(y.x)), fabsf(y.y));
     }
+    const float top = fmaxf(fmaxf(tops[0], tops[1]), fmaxf(tops[2], tops[3]));
     auto both = [](float c) { return make_float2(c, c); };
     if (!__any_sync(0xffffffffu, top >= 0.6f)) {
 #pragma unroll
@@ -166,6 +168,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         }
         mbar_init(&sh.pv_done, 1);
         mbar_init(&sh.o_done, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(&sh.scored[i], 1); mbar_init(&sh.cleared[i], 1); }
         for (int i = 0; i < 4; ++i) mbar_init(&sh.x_bar[i], 2);   // the two warps of a quarter of the rows
         sh.abort_flag = sh.issued[0] = sh.issued[1] = sh.consumed[0] = sh.consumed[1] = sh.q_issued = sh.q_consumed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -185,6 +188,22 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
     gb_pdl_launch_dependents();
     gb_pdl_wait();
 
+    // Keys that no row of the block sees have a weight of 0, but what lies in their place in the pages (an earlier request's values,
+    // or nothing yet) may be no finite number: zeros take its place before the product. Only the first and the last tile can hold
+    // such keys. (The barriers of this exchange have one phase each.)
+    const bool edge_first = key_lo % FW_BN != 0 || (ntiles == 1 && pos_hi % FW_BN != FW_BN - 1), edge_last = ntiles > 1 && pos_hi % FW_BN != FW_BN - 1;
+    auto clear = [&](unsigned char* values, int j) {            // a warp's work: tile j, whose values have landed
+        const int front = max(key_lo - (kt_begin + j) * FW_BN, 0), hi = pos_hi - (kt_begin + j) * FW_BN;
+        const int keys = front + max(FW_BN - 1 - hi, 0);
+        for (int i = lane; i < keys * (DV / 8); i += 32) {      // 16-byte pieces of a key's values, eight a column block
+            const int k = i / (DV / 8), piece = i % (DV / 8), key = k < front ? k : hi + 1 + k - front;
+            *reinterpret_cast<uint4*>(values + (piece >> 3) * FW_BLOCK + key * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.cleared[j == 0 ? 0 : 1]);
+    };
+
     if (warp == 0 || (!LATENT && warp == FW_WARPS - 1)) {
         // ------------------------------------------------------------------------- producers
         const int what = warp == 0 ? 0 : 1;                     // keys, values
@@ -201,21 +220,19 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         unsigned char* ring = what == 0 ? Ks : Vs;
         int bad = 0;
         const int nowhere = (int)(a.num_pages * a.kv_heads * a.page_size);      // a row past the pool: the load fills in zeros
-        auto page_of = [&](int kt) -> long long {               // this lane's page of key tile kt, -1: no key of it is seen, or missing
-            long long page = -1;
+        constexpr int UNSEEN = (int)0x80000000;
+        auto entry_of = [&](int kt) {                           // the table's entry of this lane's page of key tile kt
+            int entry = UNSEEN;                                 // (no key of it is seen by any row)
             if (lane < ppt) {
                 const int pi = ((kt * FW_BN) >> a.page_shift) + lane, first = pi << a.page_shift;
-                if (first <= pos_hi && first + a.page_size - 1 >= key_lo) {
-                    page = pi < a.max_pages ? table[pi] : -1;
-                    if (page < 0 || page >= a.num_pages) { bad = 1; page = -1; }
-                }
+                if (first <= pos_hi && first + a.page_size > key_lo) entry = pi < a.max_pages ? table[pi] : -1;
             }
-            return page;
+            return entry;
         };
-        long long page = page_of(kt_begin);
+        int entry = entry_of(kt_begin);
         int s = 0, round = 0;
         for (int j = 0; j < ntiles; ++j) {
-            const long long next_page = j + 1 < ntiles ? page_of(kt_begin + j + 1) : -1;   // in flight during the wait
+            const int next_entry = j + 1 < ntiles ? entry_of(kt_begin + j + 1) : UNSEEN;   // in flight until the next tile
             int ok = 1;
             if (lane == 0 && round > 0) ok = mbar_wait(&empty[s], (round - 1) & 1, abort_flag, a.status) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -223,20 +240,26 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             if (lane == 0) mbar_expect_tx(&full[s], bytes);
             __syncwarp();
             if (lane < ppt) {
+                const bool there = entry >= 0 && entry < a.num_pages;
+                if (!there && entry != UNSEEN) bad = 1;
                 unsigned char* dst = ring + s * bytes + lane * a.page_size * 128;
                 for (int b = 0; b < boxes; ++b) {
                     if (what == 0) {
-                        tma_load_2d(dst + b * FW_BLOCK, &map_k, &full[s], b * 64, page < 0 ? nowhere : (int)((page * a.kv_heads + kvh) * a.page_size));
+                        tma_load_2d(dst + b * FW_BLOCK, &map_k, &full[s], b * 64, there ? (entry * a.kv_heads + kvh) * a.page_size : nowhere);
                     } else {
                         const int col = col0 + b * 64;          // of the wide value row
                         tma_load_2d(dst + b * FW_BLOCK, &map_v, &full[s], col % a.vdim,
-                                    page < 0 ? nowhere : (int)((page * a.kv_heads + col / a.vdim) * a.page_size));
+                                    there ? (entry * a.kv_heads + col / a.vdim) * a.page_size : nowhere);
                     }
                 }
             }
             __syncwarp();
             if (lane == 0) sh.issued[what] = j + 1;
-            page = next_page;
+            if (!LATENT && what == 1 && ((j == 0 && edge_first) || (j + 1 == ntiles && edge_last))) {
+                if (!mbar_wait_warp(&full[s], round & 1, abort_flag, a.status)) break;
+                clear(ring + s * bytes, j);
+            }
+            entry = next_entry;
             if (++s == stages) { s = 0; ++round; }
         }
         if (bad && what == 0) atomicOr(a.status, GB_STATUS_BAD_SLOT);
@@ -259,6 +282,8 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 }
                 umma_commit(&sh.s_full[j & 1]);
                 if (!LATENT) umma_commit(&sh.k_empty[s]);
+                if (LATENT && j == 0 && edge_first) umma_commit(&sh.scored[0]);
+                if (LATENT && j + 1 == ntiles && edge_last) umma_commit(&sh.scored[1]);
                 return true;
             };
             for (int j = 0; j < 2 && j < ntiles && ok; ++j) ok = scores(j);
@@ -266,6 +291,8 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 const int s = LATENT ? j % G::K_STAGES : j % G::V_STAGES;
                 if (!LATENT && !(ok = mbar_wait(&sh.v_full[s], (j / G::V_STAGES) & 1, abort_flag, a.status))) break;
                 if (!LATENT) sh.consumed[1] = j + 1;
+                if (j == 0 && edge_first && !(ok = mbar_wait(&sh.cleared[0], 0, abort_flag, a.status))) break;
+                if (j + 1 == ntiles && edge_last && !(ok = mbar_wait(&sh.cleared[1], 0, abort_flag, a.status))) break;
                 if (!(ok = mbar_wait(&sh.p_ready[j & 1], (j >> 1) & 1, abort_flag, a.status))) break;
                 tc_fence_after();
                 const uint64_t vd = v_desc + (uint64_t)((s * (LATENT ? G::K_BYTES : G::V_BYTES)) >> 4);
@@ -316,22 +343,6 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             if (lane == 0) mbar_arrive(&sh.x_bar[q]);
             if (!mbar_wait_warp(&sh.x_bar[q], j & 1, abort_flag, a.status)) { ok = false; break; }
             mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
-            // Keys that no row of the block sees have a weight of 0, but what lies in their place in the pages (an earlier
-            // request's values, or nothing yet) may be no finite number: zeros take its place before the product. Only the tiles
-            // at the ends of the walk hold such keys.
-            const int lo = key_lo - (kt_begin + j) * FW_BN, hi = pos_hi - (kt_begin + j) * FW_BN;
-            const bool edge = lo > 0 || hi < FW_BN - 1;
-            if (edge) {
-                const int s = LATENT ? j % G::K_STAGES : j % G::V_STAGES, phase = (LATENT ? j / G::K_STAGES : j / G::V_STAGES) & 1;
-                if (!mbar_wait_warp(LATENT ? &sh.k_full[s] : &sh.v_full[s], phase, abort_flag, a.status)) { ok = false; break; }
-                unsigned char* values = LATENT ? Ks + s * G::K_BYTES : Vs + s * G::V_BYTES;
-                const int front = max(lo, 0), cleared = front + max(FW_BN - 1 - hi, 0);
-                constexpr int PIECES = DV / 8;                  // 16-byte pieces of a key's values, eight a column block
-                for (int i = (warp - 2) * 32 + lane; i < cleared * PIECES; i += 256) {
-                    const int k = i / PIECES, piece = i % PIECES, key = k < front ? k : hi + 1 + k - front;
-                    *reinterpret_cast<uint4*>(values + (piece >> 3) * FW_BLOCK + key * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
-                }
-            }
             const bool raise = (mx - m_run) * slx > 8.0f;
             if (j == 0) {
                 if (raise) m_run = mx;                          // nothing is accumulated yet
@@ -366,7 +377,6 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
             }
             l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
-            if (edge) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tmem_store32(lane_base + (uint32_t)(b * FW_BN + h * 32), pw);
             tc_fence_before();
             __syncwarp();
@@ -415,6 +425,11 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 __syncwarp();      // the next load is the whole warp's; lanes past the last row have taken the other way here
             }
         }
+    } else if (LATENT) {
+        // ------------------------------------------------------------------------- clears the ends of the walk
+        // (the keys are the values: a tile is cleared once its scores have been formed)
+        if (edge_first && mbar_wait_warp(&sh.scored[0], 0, abort_flag, a.status)) clear(Ks, 0);
+        if (edge_last && mbar_wait_warp(&sh.scored[1], 0, abort_flag, a.status)) clear(Ks + (ntiles - 1) % G::K_STAGES * G::K_BYTES, ntiles - 1);
     }
 
     tc_fence_before();
