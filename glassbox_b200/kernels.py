@@ -2086,7 +2086,7 @@ def moe_experts_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tenso
                         positions: torch.Tensor, tables: torch.Tensor, act: torch.Tensor, pair: torch.Tensor, unit=None,
                         status: Optional[torch.Tensor] = None) -> None:
     """The chosen experts of many rows as grouped products on the tensor cores (bfloat16): the (row, choice) pairs are
-    sorted by expert (``tables`` int32 [2 * (experts + 1) + n * top] is the sort's scratch), then one launch computes
+    sorted by expert (``tables`` int32 [experts + 1 + n * top] is the sort's scratch), then one launch computes
     act = relu(W_up[e] h)^2 for all pairs (bfloat16 [n, top * ff], in sorted order) and one pair = W_down[e] act
     (float32 [n, top * d], in pair order). ``unit`` as in ``moe_expert_halves``: the up product then has 2 ff outputs per
     expert, and its epilogue forms one unit from every two neighbours. ``status``: the word in which a wait that gives up is
@@ -2103,8 +2103,8 @@ def moe_experts_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tenso
     assert h.is_contiguous() and w_up.is_contiguous() and w_down.is_contiguous() and act.is_contiguous() and pair.is_contiguous()
     assert w_up.shape == (experts * up_rows, d) and w_down.shape == (experts * d, ff) and choice.is_contiguous()
     assert act.shape == (n, top * ff) and pair.shape == (n, top * d)
-    assert tables.dtype == torch.int32 and tables.is_contiguous() and tables.numel() >= 2 * (experts + 1) + P
-    offsets, order = tables[:experts + 1], tables[2 * (experts + 1):]
+    assert tables.dtype == torch.int32 and tables.is_contiguous() and tables.numel() >= experts + 1 + P
+    offsets, order = tables[:experts + 1], tables[experts + 1:]
     _call("gb_moe_sort", _ptr(choice), _ptr(positions), n, experts, top, _ptr(offsets), _ptr(order), _stream())
     _call("gb_moe_grouped_gemm", _ptr(h), d, n, _ptr(w_up), up_rows, d, _ptr(order), _ptr(offsets), experts, top, P,
           _ptr(act), ff, 1, 1 if unit else 0, float(unit[0]) if unit else 0.0, float(unit[1]) if unit else 0.0, _ptr(status), _stream())

@@ -111,7 +111,7 @@ class RoutedExperts(FeedForward):
         pair = ctx.scratch("moe_pair", (n, self.top * d), torch.float32)
         if n > GROUPED_ABOVE_ROWS and kernels.moe_grouped_supported(h.dtype, d, self.ff):
             # many rows: the pairs sorted by expert, one grouped product per half on the tensor cores
-            tables = ctx.zeros_once(f"moe_tables_{self.E}_{self.top}", 2 * (self.E + 1) + ctx.max_rows * self.top, torch.int32)
+            tables = ctx.zeros_once(f"moe_tables_{self.E}_{self.top}", self.E + 1 + ctx.max_rows * self.top, torch.int32)
             act = ctx.scratch("moe_act", (n, self.top * self.ff))
             kernels.moe_experts_grouped(h, p["w_up"], p["w_down"], self.E, choice, ctx.positions, tables, act, pair, unit=unit,
                                         status=ctx.status)

@@ -39,7 +39,7 @@ def test_grouped_products(E, top, d, ff, unit, counts):
     h, w_up, w_down, choice, positions = _case(E, top, d, ff, unit, counts, d + ff)
     n = h.shape[0]
     pair_unit = {None: None, "silu": kernels.SILU_UNIT, "clamped": (7.0, 1.702)}[unit]
-    tables = torch.zeros(2 * (E + 1) + n * top, dtype=torch.int32, device=DEV)
+    tables = torch.zeros(E + 1 + n * top, dtype=torch.int32, device=DEV)
     act = torch.full((n, top * ff), float("nan"), dtype=torch.bfloat16, device=DEV)
     pair = torch.full((n, top * d), 7.0, device=DEV)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
@@ -81,7 +81,7 @@ def test_the_unit_divides_as_float32_does():
     i32 = lambda *shape: torch.zeros(*shape, dtype=torch.int32, device=DEV)
     pair, status = torch.zeros(n, d, device=DEV), i32(1)
     kernels.moe_experts_grouped(dev(h), dev(w_up.view(2 * ff, d)), dev(w_down), 1, i32(n, 1), torch.arange(n, dtype=torch.int32, device=DEV),
-                                i32(2 * 2 + n), torch.zeros(n, ff, dtype=torch.bfloat16, device=DEV), pair, unit=kernels.SILU_UNIT, status=status)
+                                i32(2 + n), torch.zeros(n, ff, dtype=torch.bfloat16, device=DEV), pair, unit=kernels.SILU_UNIT, status=status)
     want = gates.double() / (1 + torch.exp(-gates.double())) * 2.0 ** 100
     # float32: the exponential's argument is exact, its value and the quotient a few 2^-23 off; then one rounding to bfloat16
     assert int(status) == 0
