@@ -602,8 +602,11 @@ def gemm_few(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, status: torch.Te
     _call("gb_gemm_few", _ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(c), c.stride(0), mode, M, N, K, _ptr(status), 1 if USE_PDL else 0, _stream())
 
 
-def gemm_few_qkv_supported(a: torch.Tensor, w: torch.Tensor, hd: int, q_out: torch.Tensor, kcache: torch.Tensor) -> bool:
-    return (hd in (64, 128) and q_out.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16 and gemm_few_supported(a, w, q_out))
+def gemm_few_qkv_supported(a: torch.Tensor, w: torch.Tensor, hd: int, q_out: torch.Tensor, kcache: torch.Tensor, vcache: Optional[torch.Tensor] = None,
+                           cos_sin: Optional[torch.Tensor] = None) -> bool:
+    """Whether ``gemm_few_qkv`` takes these operands (it stores 8 and reads 16 bytes at a time, so the cache and the table are aligned)."""
+    return (hd in (64, 128) and q_out.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16
+            and all(t is None or t.data_ptr() % 16 == 0 for t in (kcache, vcache, cos_sin)) and gemm_few_supported(a, w, q_out))
 
 
 def gemm_few_qkv(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cos_sin: Optional[torch.Tensor], positions: torch.Tensor,

@@ -56,7 +56,7 @@ class GqaAttention(Mixer):
             (table is None and type(self.position).apply_qk is Position.apply_qk)
         few = _few_rows(h, self.params["wqkv"], qkv) if plain_rotary and qkv.dtype == torch.bfloat16 and self.hd in (64, 128) else None
         x, norm, _, scale = _resolve(h, self.params["wqkv"]) if few is None else (few, None, None, None)
-        if few is not None and kernels.gemm_few_qkv_supported(few, self.params["wqkv"], self.hd, qkv, cache.k):
+        if few is not None and kernels.gemm_few_qkv_supported(few, self.params["wqkv"], self.hd, qkv, cache.k, cache.v, table):
             # a decode batch against a large matrix: one kernel projects, rotates and writes the cache
             kernels.gemm_few_qkv(few, self.params["wqkv"], qkv, table, ctx.positions, cache.slots, cache.k, cache.v, self.nh, self.nkv,
                                  self.hd, cache.page_size, writes_cache, ctx.status)

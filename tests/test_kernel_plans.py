@@ -132,3 +132,17 @@ def test_single_tokens_of_a_latent_step_take_the_decode_kernel(monkeypatch):
     part.H = 128
     LatentAttention.attend(part, ctx, q[:80], q[:80], cache)
     assert [t[:3] for t in taken] == [("tiles", 80, 42)]
+
+
+def test_the_few_rows_projection_leaves_unaligned_tables_and_caches_to_the_others(monkeypatch):
+    """A rotary table or a cache that does not start on 16 bytes is no error: another kernel takes the step, as ever."""
+    import torch
+    monkeypatch.setattr(kernels, "gemm_few_supported", lambda *a, **k: True)
+    q = torch.zeros(16, 64, dtype=torch.bfloat16)
+    cache, table = torch.zeros(1 + 8 * 64, dtype=torch.bfloat16), torch.zeros(1 + 4 * 32 * 2)
+    even, odd = cache[:512], cache[1:]
+    assert kernels.gemm_few_qkv_supported(q, q, 64, q, even, even, table[:256])
+    assert kernels.gemm_few_qkv_supported(q, q, 64, q, even, even, None)
+    assert not kernels.gemm_few_qkv_supported(q, q, 64, q, odd, even, None)
+    assert not kernels.gemm_few_qkv_supported(q, q, 64, q, even, odd, None)
+    assert not kernels.gemm_few_qkv_supported(q, q, 64, q, even, even, table[1:])
