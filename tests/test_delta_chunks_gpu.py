@@ -98,3 +98,34 @@ def test_a_token_does_not_reach_the_ones_before_it():
     data[1][45] = np.nan
     spoiled, _ = _run(True, lens, H, KH, D, V, False, *data)
     assert np.array_equal(clean[:45], spoiled[:45]) and not np.isfinite(spoiled[45:]).any()
+
+
+def test_recorded_prompt_shapes_share_one_workspace(tmp_path_factory):
+    """Ten prompt shapes through the engine, each unrecorded, while it is recorded and replayed: the same logits three times, again in
+    another order once all are recorded, and one workspace for all of them, none in what a recorded shape keeps for itself."""
+    import zurerax_util as zu
+    from glassbox_b200.engine.engine import Engine, StepEntry
+    cfg = zu.CONFIGS["even"]()
+    folder = zu.write_model(str(tmp_path_factory.mktemp("shapes")), cfg, zu.random_weights(cfg, 3))
+    eng = Engine(folder, "float32", cache_tokens=1200, page_size=16, max_batch_tokens=1024, max_requests=4)
+    tokens = [int(t) for t in np.random.default_rng(4).integers(0, cfg["vocab"], 1024)]
+    eng.add_request("r", [])
+    step = lambda n: eng.step([StepEntry("r", tokens[:n], [0, n - 1])], commit=False).clone()
+    lengths, first = [100 * k for k in range(1, 11)], {}
+    for n in lengths:
+        # (uncommitted: the request's state slot keeps what the step wrote, so it starts from zero each time)
+        for _ in range(3):
+            for t in eng.device_cache.state.values():
+                t.zero_()
+            out = step(n)
+            assert torch.equal(first.setdefault(n, out), out), n
+    eng.check()
+    assert eng.graph_replays >= len(lengths)
+    for n in reversed(lengths):
+        for t in eng.device_cache.state.values():
+            t.zero_()
+        assert torch.equal(first[n], step(n)), n
+    shared = [b for (name, _), b in eng.scratch._bufs.items() if "delta_chunks" in name]
+    own = [name for g in eng._graphs.values() for (name, _) in g["ctx"]._grow._bufs if "delta_chunks" in name]
+    heads = {L["mixer"]["heads"] for L in cfg["layers"] if L["type"] == "channel_delta"}
+    assert len(shared) == len(heads) and not own
