@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256) short_conv_kernel(const float* __restrict
 
 // The same for steps of many rows: a thread takes a channel of STRIP rows one after the other, every input once (the form above
 // reads each of them `taps` times and the channel's taps per row: bound by its loads' latency, a seventh of the copy rate).
-// Measured, 2,048 rows x 3,072 channels, four taps: 52 -> 23 us.
+// Measured, 2,048 rows x 3,072 channels, four taps, with the state's update: 48.8 -> 33.3 us.
 constexpr int SC_STRIP = 16;
 
 template <int TAPS>

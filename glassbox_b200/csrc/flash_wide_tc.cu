@@ -14,8 +14,9 @@
 //              exceeded by more than 2^8 in the exponent, as in attention_prefill_tc.cu.
 //   warp 10    producer of the values (not for the latent cache, whose key tile serves both products); puts zeros in the place of
 //              keys that no row of the block sees
-// Bound by the softmax warps (an exponential a score: 1,024 cycles a tile of the special-function unit, and with a cap nine fused
-// multiply-adds, against 1,280 of the tensor pipe); the mma.sync kernels that this replaced formed the scores once per 128 value
+// Bound by the chain of a tile (scores, the halves' maxima, weights, product, the next scores in the weights' place) in the one block
+// that a multiprocessor holds, and by the longest row tiles: over a prompt of 2,048 tokens no unit is above a quarter of its peak
+// (tensor pipe 19 %, special functions 16 %, FMA 22 %, issue 28 %; over a latent cache 35, 29, 11, 32). The mma.sync kernels that this replaced formed the scores once per 128 value
 // channels and fed both products through ldmatrix. Measured: see gb_talking_attention_flash, gb_latent_flash.
 //
 // Every wait is bounded: on a timeout the block records GB_STATUS_WAIT_TIMEOUT, waits (bounded) for its copies, frees its tensor
@@ -495,7 +496,7 @@ GB_EXPORT int gb_talking_attention_flash_supported(int D, int V, int VG, int pag
 }
 
 // As gb_talking_attention_tiles (talking_attention.cu), VG == G. q bfloat16 [n, H, 64], out float32 [n, H, G * V].
-// Measured, 2,048 tokens, 16/4 heads of 64, capped: 402 us in tiles of mma.sync, 52 us here.
+// Measured, 2,048 tokens, 16/4 heads of 64, capped: 402 us in tiles of mma.sync, 58 us here.
 GB_EXPORT int gb_talking_attention_flash(const void* q, float* out, const void* kcache, const void* vcache, const int* block_tables, int max_pages,
                                          const int* seq_first_row, const int* seq_start_pos, int n, int num_seqs, int max_rows_per_seq, int H, int G,
                                          int V, int page_size, long long num_pages, float scale, float cap, int unit, int window, int* status,
@@ -522,7 +523,7 @@ GB_EXPORT int gb_latent_flash_supported(int c, int r, int page_size) {
 
 // Attention of prompt portions over a latent cache [pages, page_size, 128 + r]: q bfloat16 [n, H, 128 + r], out bfloat16
 // [n, H, 128]; arguments as gb_latent_attention_mma. Measured, two portions of 1,500 tokens in all
-// behind up to 900, 32 heads, 128 + 64: 197 us in tiles of mma.sync, 70 us here.
+// behind up to 900, 32 heads, 128 + 64: 197 us in tiles of mma.sync, 65 us here.
 GB_EXPORT int gb_latent_flash(const void* q, void* out, const void* cache, const int* block_tables, int max_pages, const int* seq_first_row,
                               const int* seq_start_pos, const float* sink, int n, int num_seqs, int max_rows_per_seq, int H, int c, int r,
                               int page_size, long long num_pages, float scale, int window, int* status, cudaStream_t stream) {

@@ -11,7 +11,8 @@
 //              sums through distributed shared memory (in rank order: a fixed order) and runs the epilogue on whole rows: store,
 //              add to the residual, squared ReLU, GELU, silu(gate) * up, or rotation and cache write of a stacked QKV product.
 //
-// Bound by the memory's latency at these sizes (3.5 to 5 TB/s). Measured alone, weights from memory, us at 16 / 40 / 64 rows, this
+// Bound by the memory's latency at these sizes (3.5 to 5 TB/s; 67 MB gated, 40 rows, by ncu from a cold start: DRAM 36 % of its peak, tensor
+// pipe 9 %, issue 10 %). Measured alone, weights from memory, us at 16 / 40 / 64 rows, this
 // and in brackets the better of the weight-streaming and the tile kernel: 6144 x 2048 8.8 / 9.7 / 10.6 (8.8 / 13 / 13);
 // 2048 x 2048 5.3 / 6.3 / 6.6 (5.7 / 9.0 / 14); 2 x 8192 x 2048 gated 17 / 21 / 25 (24 / 26 / 26); 2048 x 8192 10 / 12 / 12
 // (16 / 33 / 35); 960 x 2560 5.0 / 5.5 / 6.2 (5.2 / 7.5 / 7.8). Below about 5 MB of weights it is no better: what is left is the

@@ -52,10 +52,8 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     return __all_sync(0xffffffffu, ok);
 }
 // True in one lane of a converged warp. The single-thread roles (TMA and tcgen05.mma issue) are entered through this and not
-// through a comparison of the lane number: the instructions take their descriptors from uniform registers, and only inside an
-// elect.sync branch does the compiler know that one thread is active. Behind `lane == 0` it guards each instruction for
-// threads that could differ: measured 63 instead of 48 cycles per 128 x 64 x 16 tcgen05.mma (the operand reads' 48 are the
-// bound) and 44 instead of 0 per commit.
+// through a comparison of the lane number: behind `lane == 0` a 128 x 64 x 16 tcgen05.mma takes 63 cycles instead of the 48 of its
+// operand reads, and a commit 44 instead of none (measured).
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));

@@ -2173,9 +2173,9 @@ def talking_attention_decode_supported(dtype: torch.dtype, heads: int, kv_heads:
 def talking_decode_shares(n: int, heads: int, kv_heads: int, vdim: int, value_heads: int, reach: int) -> int:
     """Into how many shares the decoding kernel cuts a row's keys: the count whose rounds of blocks (two per multiprocessor, 296
     at once) take the least time, a round costing a block's keys and about 400 more for its start and merge; no share shorter
-    than 256 keys, at most 16. Measured (16 heads, 4 value heads of 64, contexts to 2,048), mixer with this rule / with the
-    smallest count that fills 296 blocks: 16 rows 45.3 us (4 shares) / 50.5 (5), 24 rows 53.8 (3) / 63.7 (4), 32 rows 67.6 (2) /
-    75.0 (3), 48 rows 87.6 (3) / 98.9 (2), 96 rows 159 (2) / 183 (1)."""
+    than 256 keys, at most 16. Measured (16 heads, 4 value heads of 64, contexts to 2,047), mixer with this rule / with the
+    smallest count that fills 296 blocks: 16 rows 46.2 us (4 shares) / 51.6 (5), 24 rows 55.9 (3) / 67.0 (4), 32 rows 70.3 (2) /
+    80.3 (3), 48 rows 92.0 (3) / 102.5 (2), 96 rows 160 (2) / 184 (1)."""
     plan = lib().gb_talking_attention_decode_plan(heads, kv_heads, vdim, value_heads)
     blocks = max(1, n * (heads // max(plan % 10000 // 100, 1)) * max(plan // 10000, 1))
     most = max(1, min(16, reach // 256, 4096 // heads))

@@ -108,8 +108,8 @@ class GqaAttention(Mixer):
         """att[row, head, :] = softmax over the row's visible keys; the kernel is picked by the shape
         of the batch: rows that are single decoded tokens share the keys of a request between
         several blocks (on the tensor cores in bfloat16 where the head size is one the kernel is built
-        for, else with float32 FMA); prompt portions take a flash kernel in bfloat16 at head sizes one
-        is built for; anything else takes the one-warp-per-(row, head) kernel. A mixed batch that starts
+        for, else with float32 FMA); prompt portions take a flash kernel (bfloat16 or float32) at head sizes
+        one is built for; anything else takes the one-warp-per-(row, head) kernel. A mixed batch that starts
         with many single-token requests (the scheduler puts them first) is split: those rows go to the
         decode kernel, the portions to the flash kernel, which would otherwise spend a 128-row tile per
         head on each of them."""

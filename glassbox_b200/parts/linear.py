@@ -3,7 +3,8 @@
 
 The kernel is chosen by operand types only: all-float32 operands run the FMA kernel (the true
 32-bit path); bfloat16 operands run the tensor-core kernel when the shape allows and the FMA
-kernel otherwise; with at most 64 rows (decoding) they run the weight-streaming kernel.
+kernel otherwise; with at most 64 rows (decoding) they run the weight-streaming kernel, or from 9 rows on
+against large matrices the tcgen05 kernel for few rows (``_few_rows``).
 ``accumulate`` adds into a float32 ``out`` (the residual stream).
 """
 from __future__ import annotations
