@@ -239,3 +239,40 @@ def test_what_no_row_sees_reaches_no_result(window):
         kernels.latent_flash(q, out, spoil(cache, bad), tables, first, start, None, H, 128, 64, 16, 0.2, window, status, longest)
         outs.append(out)
     assert int(status) == 0 and torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+def test_a_mixed_step_of_the_latent_mixer_equals_one_kernel_over_all_rows():
+    """Leading single tokens (two padding sequences among them) to the decode kernel and the portions behind them to the flash kernel,
+    against the tiles of tokens x heads over the whole step."""
+    from types import SimpleNamespace
+    from glassbox_b200 import kernels
+    from glassbox_b200.parts.latent_attention import LatentAttention
+    H, c, r, page = 32, 128, 64, 16
+    singles = [(60 + 97 * i % 900, 1) for i in range(22)] + [None, None]
+    portions = [(40, 300), (0, 200)]
+    tables, _, start, pages, longest = _layout(page, [s or (0, 1) for s in singles] + portions, 9)
+    lead = len(singles)
+    start = torch.tensor([s[0] if s else -1 for s in singles] + [p for p, _ in portions], dtype=torch.int32, device=DEV)
+    first = torch.tensor([*range(lead + 1), lead + 300, lead + 500], dtype=torch.int32, device=DEV)
+    positions = torch.tensor([s[0] if s else -1 for s in singles] + [p + i for p, n in portions for i in range(n)], dtype=torch.int32, device=DEV)
+    n = lead + 500
+    g = torch.Generator(device=DEV).manual_seed(5)
+    q = torch.randn(n, H * (c + r), generator=g, device=DEV).bfloat16()
+    pool = torch.randn(pages, 1, page, c + r, generator=g, device=DEV).bfloat16()
+    sink = torch.randn(H, generator=g, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    taken = []
+    ctx = SimpleNamespace(decode_only=False, leading_single=lead, max_context=1024, max_rows_per_seq=longest, status=status, seq_first_row=first,
+                          seq_start_pos=start, positions=positions,
+                          scratch=lambda name, shape, dtype, grow: taken.append(name) or torch.empty(shape, dtype=dtype, device=DEV))
+    part = SimpleNamespace(H=H, c=c, r=r, params={"sink": sink}, spec=SimpleNamespace(scale=0.1, window=None))
+    part._attend_decode = lambda *a: LatentAttention._attend_decode(part, *a)
+    assert kernels.latent_flash_chosen(500, 2, H, 1024)
+    got, want = (torch.full((n, H * c), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    LatentAttention.attend(part, ctx, q, got, SimpleNamespace(k=pool, page_size=page, block_tables=tables))
+    kernels.latent_attention_mma(q, want, pool, tables, first, start, positions, sink, H, c, r, page, 0.1, None, status, max_rows_per_seq=longest)
+    assert int(status) == 0
+    # both round their weights and results to bfloat16, 2^-8 of the largest value at most each (see test_latent_cache)
+    live = positions >= 0
+    assert (got[live].float() - want[live].float()).abs().max() <= 2 ** -9 * 3 * 2 * pool[..., :c].float().abs().max()
+    assert torch.isfinite(got.float()).all()
