@@ -205,12 +205,12 @@ def test_the_cap_is_as_exact_as_float32_allows(cap):
     assert ((out.double() - want[:, None]).abs() <= bound[:, None]).all(), float(((out.double() - want[:, None]).abs() / bound[:, None]).max())
 
 
-@pytest.mark.parametrize("window", [None, 50])
-def test_what_no_row_sees_reaches_no_result(window):
+@pytest.mark.parametrize("window, G", [(None, 2), (50, 2), (None, 4), (50, 4)])
+def test_what_no_row_sees_reaches_no_result(window, G):
     """Pages hold what earlier requests left: past the last row, in front of a window, and in every page the table does not name.
     Infinities and NaN there change no result."""
     from glassbox_b200 import kernels
-    batch = [(130, 75), (0, 200), (300, 140)]
+    batch = [(130, 75), (0, 200), (300, 140), (100, 20), (0, 3)]        # of one to four key tiles
     tables, first, start, pages, longest = _layout(16, batch, 8)
     n = int(first[-1])
     seen = torch.zeros(pages, 16, dtype=torch.bool, device=DEV)
@@ -221,7 +221,7 @@ def test_what_no_row_sees_reaches_no_result(window):
             tables[i, :max(c + 1 - window, 0) // 16] = -1
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
     spoil = lambda t, dim: torch.where(seen.view(seen.shape + (1,) * (t.dim() - 2)), t, torch.tensor(dim, device=DEV, dtype=t.dtype))
-    H, G = 4, 2
+    H = 4
     q = torch.randn(n, H * 64, device=DEV).bfloat16()
     k, v = (torch.randn(pages, 16, G, d, device=DEV).bfloat16() for d in (64, 64))
     outs = []
