@@ -10,10 +10,13 @@
 //   warp 1, one lane: issues 4 tcgen05.mma (M 128, N BN, K 16) per k-block from shared-memory matrix
 //       descriptors, then tcgen05.commit to the stage's "empty" mbarrier (the stage is free once the
 //       tensor core has read it) and, after the last k-block, to the "accumulator ready" mbarrier.
-//   warps 2-5: epilogue. Each reads its quarter of the TMEM lanes (rows of the tile), 32 columns at a
-//       time, and stores bfloat16 / float32, adds into float32 (the residual stream) or applies the
+//   warps 2-9: epilogue. Each reads its quarter of the TMEM lanes (rows of the tile) and its half of the columns, 32
+//       columns at a time, and stores bfloat16 / float32, adds into float32 (the residual stream) or applies the
 //       gated activation. Two accumulators alternate, so the epilogue of a tile overlaps the main loop
-//       of the next.
+//       of the next. Rows turn over in shared memory on the way out (tc_turn_put_*), so that an instruction writes whole rows.
+//       A launch of few rounds ends with an epilogue that nothing covers, and a wide float32 tile's took longer than its main
+//       loop: with four warps and 4-byte stores (bfloat16: 16 bytes in each of 32 rows) 8192 x 2048, K 1024 stored float32 in
+//       53.2 us, bfloat16 31.6; 2048 x 576, K 576 6.3 and 5.1; now 36.4, 29.7, 4.9 and 4.7.
 // Both operands are K-major ([rows, K] with K contiguous), exactly as activations and [out, in]
 // weights are stored (crates/glassbox-core/src/kernels.rs:381), so nothing is transposed.
 //
@@ -67,6 +70,7 @@ struct TcUnit {
 };
 
 constexpr int TC_MAX_STAGES = 8;
+constexpr int TC_EPI_WARPS = 8, TC_THREADS = 64 + 32 * TC_EPI_WARPS;
 
 struct __align__(8) TcShared {
     uint64_t full[TC_MAX_STAGES];    // TMA -> MMA: a stage's operands have landed
@@ -83,23 +87,23 @@ template <int BN, bool GATED> struct TcGeometry {
     static constexpr int BNO = GATED ? BN / 2 : BN;                 // output columns per tile
     static constexpr int A_BYTES = TC_BM * TC_BK * 2, W_BYTES = BN * TC_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     static constexpr int STAGES = (192 * 1024 / STAGE_BYTES) < TC_MAX_STAGES ? (192 * 1024 / STAGE_BYTES) : TC_MAX_STAGES;
-    static constexpr int EPI_BYTES = 4 * 32 * 33 * 4;               // per-warp transposition tiles
+    static constexpr int EPI_BYTES = TC_EPI_WARPS * 32 * 128;       // a tile of 32 rows x 128 bytes per epilogue warp
     static constexpr int SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 1024;
 };
 
-// A persistent block walks over output tiles (tile = blockIdx.x, + gridDim.x, ...). Six warps:
+// A persistent block walks over output tiles (tile = blockIdx.x, + gridDim.x, ...). Ten warps:
 //   warp 0 (one lane)  producer: TMA loads of A and W k-blocks into the stage ring, across tiles;
 //   warp 1 (one lane)  MMA issuer: per tile, tcgen05.mma over the k-blocks into one of two TMEM
 //                      accumulators, so that the next tile's main loop runs while the epilogue
 //                      warps read the previous accumulator out;
-//   warps 2-5          epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile), 32 columns at
+//   warps 2-9          epilogue: warp w reads TMEM lanes 32*(w%4).. (rows of the tile), half of the columns, 32 at
 //                      a time, and stores bfloat16 / float32, adds into float32 (the residual
 //                      stream), or, GATED, stores silu(gate)*up: the tile's accumulator then holds the
 //                      gate columns in its first half and the matching up columns (weight rows
 //                      gate_rows further down, loaded by a second TMA box) in its second half
 //                      (crates/glassbox-core/src/model.rs:335-340).
 template <int BN, bool GATED>
-__global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
+__global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                                            const __grid_constant__ CUtensorMap map_w, void* __restrict__ C,
                                                            int mode, int M, int N, int K, long long ldc, int gate_rows,
                                                            int* __restrict__ status, const TcQkv qkv, const TcNorm norm,
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     extern __shared__ unsigned char smem_dyn[];
     // 128-byte-swizzled tiles want 1024-byte alignment
     unsigned char* tiles = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
-    float* epi = reinterpret_cast<float*>(tiles + STAGES * G::STAGE_BYTES);
+    uint4* epi = reinterpret_cast<uint4*>(tiles + STAGES * G::STAGE_BYTES);
     __shared__ TcShared sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kblocks = (K + TC_BK - 1) / TC_BK;
@@ -123,7 +127,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sh.tfull[b], 1);
-            mbar_init(&sh.tempty[b], 4);   // one arrival per epilogue warp
+            mbar_init(&sh.tempty[b], TC_EPI_WARPS);   // one arrival per epilogue warp
         }
         sh.abort_flag = 0;
         sh.issued = 0;
@@ -201,7 +205,10 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     } else {
         // ------------------------------------------------------------------------- epilogue
         const int q = warp & 3;                       // the quarter of TMEM lanes this warp may read
-        float* stage = epi + q * (32 * 33);
+        const int part = (warp - 2) >> 2;             // ... and its half of the tile's columns
+        uint4* stage = epi + (warp - 2) * (32 * 8);
+        // whole 16-byte pieces may be stored where the output's rows are aligned (pieces start at multiples of their size)
+        const bool vec_f32 = ((uintptr_t)C & 15) == 0 && (ldc & 3) == 0, vec_bf16 = ((uintptr_t)C & 15) == 0 && (ldc & 7) == 0;
         int tcount = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
@@ -223,27 +230,60 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                 }
                 inv_rms = 1.0f / sqrtf(ss / (float)K + norm.eps);
             }
-            // mode TC_ADD_F32: the residual values of the next 32 columns to be written, requested while the tile's products (or
-            // the columns before) are still under way
-            float old[32];
+            // mode TC_ADD_F32: the residual values of the next 32 columns to be written (as the turned tile deals them out), requested
+            // while the tile's products (or the columns before) are still under way
+            float4 old[8];
             const int rows_here = min(32, M - (m0 + q * 32));
-            auto load_old = [&](int col) {
+            const int first_col = n0 + part * (BNO / 2);
+            auto load_old = [&](int col0) {
+                const int col = col0 + (lane & 7) * 4;
                 const float* base = reinterpret_cast<const float*>(C) + (size_t)(m0 + q * 32) * ldc + col;
 #pragma unroll
-                for (int rr = 0; rr < 32; ++rr) old[rr] = (col < N && rr < rows_here) ? base[(size_t)rr * ldc] : 0.f;
+                for (int i = 0; i < 8; ++i) {
+                    const int rr = 4 * i + (lane >> 3);
+                    const float* src = base + (size_t)rr * ldc;
+                    old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (rr >= rows_here) continue;
+                    if (vec_f32 && col + 4 <= N) {
+                        old[i] = *reinterpret_cast<const float4*>(src);
+                    } else {
+                        if (col < N) old[i].x = src[0];
+                        if (col + 1 < N) old[i].y = src[1];
+                        if (col + 2 < N) old[i].z = src[2];
+                        if (col + 3 < N) old[i].w = src[3];
+                    }
+                }
             };
-            if (!GATED && mode == TC_ADD_F32) load_old(n0 + lane);
+            if (!GATED && mode == TC_ADD_F32) load_old(first_col);
+            // mode TC_ROPE_QKV: this lane's row's position and slot, and the rotations of the channels that it will turn for the rows
+            // 8 i + lane / 4, requested while the products run
+            const bool is_qkv = !GATED && mode == TC_ROPE_QKV;
+            const int hd = is_qkv ? qkv.hd : 64, half = hd >> 1;
+            // (the two warps of a quarter share the tile's heads or, where it holds one, the head's channels)
+            const int h_first = BN > hd ? part * hd : 0, h_step = BN > hd ? 2 * hd : hd;
+            const int c_first = BN > hd ? 0 : part * 16, c_step = BN > hd ? 16 : 32;
+            const int pos = is_qkv && row < M ? qkv.positions[row] : -1;
+            float4 (&cs)[8] = old;      // (a launch is one or the other)
+            auto load_cs = [&](int c) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int p = __shfl_sync(0xffffffffu, pos, 8 * i + (lane >> 2));
+                    const bool have = qkv.rope != nullptr && p >= 0 && p < qkv.max_pos;
+                    const float4* src = reinterpret_cast<const float4*>(qkv.rope + (size_t)p * half + c + 4 * (lane & 3));
+                    cs[2 * i] = have ? src[0] : make_float4(1.f, 0.f, 1.f, 0.f);
+                    cs[2 * i + 1] = have ? src[1] : make_float4(1.f, 0.f, 1.f, 0.f);
+                }
+            };
+            if (is_qkv) load_cs(c_first);
             if (kblocks > 0) {
                 if (!mbar_wait_warp(&sh.tfull[acc], (tcount >> 1) & 1, abort_flag, status)) { ok = false; break; }
                 tc_fence_after();
             }
             const uint32_t t_base = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-            if (!GATED && mode == TC_ROPE_QKV) {
+            if (is_qkv) {
                 // Stacked QKV (crates/glassbox-core/src/model.rs:266-276): a tile holds whole heads (BN is a multiple
                 // of the head size). Query and key heads are rotated, channel i with channel i + hd/2, from the
                 // float32 sums; queries go to C, rotated keys and the values to the row's cache slot.
-                const int hd = qkv.hd, half = hd >> 1;
-                const int pos = row < M ? qkv.positions[row] : -1;
                 const long long slot = (row < M && pos >= 0) ? qkv.slots[row] : -1;
                 const bool bad_pos = qkv.rope != nullptr && pos >= qkv.max_pos;
                 const bool bad_slot = qkv.write_kv && pos >= 0 && (slot < 0 || slot >= qkv.num_slots);
@@ -251,17 +291,10 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                 if (bad_slot) atomicOr(status, GB_STATUS_BAD_SLOT);
                 const int heads_total = qkv.nh + 2 * qkv.nkv;
 #pragma unroll 1
-                for (int c = 0; c < half; c += 32) {
-                    // (cos, sin) of channels c .. c+31 at this row's position: read once, used by every head of the tile
-                    float4 cs[16];
-                    const bool have_cs = qkv.rope != nullptr && !bad_pos && pos >= 0;
-                    if (have_cs) {
-                        const float4* src = reinterpret_cast<const float4*>(qkv.rope + (size_t)pos * half + c);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) cs[j] = src[j];
-                    }
+                for (int c = c_first; c < half; c += c_step) {
+                    if (c != c_first) load_cs(c);
 #pragma unroll 1
-                    for (int h0 = 0; h0 < BN; h0 += hd) {
+                    for (int h0 = h_first; h0 < BN; h0 += h_step) {
                         const int head = (n0 + h0) / hd;
                         if (head >= heads_total) break;               // columns beyond the matrix (uniform for the block)
                         const bool is_q = head < qkv.nh, is_k = !is_q && head < qkv.nh + qkv.nkv;
@@ -275,40 +308,40 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                                       (((slot / qkv.page_size) * qkv.nkv + kvh) * qkv.page_size + slot % qkv.page_size) * hd;
                             }
                         }
-                        uint32_t x0[32], x1[32];   // the warp-collective loads run for every row; the stores only for live ones
-                        tmem_load32(t_base + (uint32_t)(h0 + c), x0);
-                        tmem_load32(t_base + (uint32_t)(h0 + half + c), x1);
+                        // sixteen channels and their partners of every row turn in one tile; the warp-collective load runs for every row
+                        uint32_t x[32];
+                        tmem_load16x2(t_base + (uint32_t)(h0 + c), t_base + (uint32_t)(h0 + half + c), x);
                         if (norm.ss_in != nullptr) {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                x0[j] = __float_as_uint(__uint_as_float(x0[j]) * inv_rms);
-                                x1[j] = __float_as_uint(__uint_as_float(x1[j]) * inv_rms);
-                            }
+                            for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(__uint_as_float(x[j]) * inv_rms);
                         }
-                        if ((is_q || is_k) && have_cs) {
+                        tc_turn_put_f32(stage, lane, x);
+                        __syncwarp();
 #pragma unroll
-                            for (int j = 0; j < 32; j += 2) {
-                                const float4 t = cs[j >> 1];   // (cos, sin) of channels c+j and c+j+1
-                                const float a0 = __uint_as_float(x0[j]), b0 = __uint_as_float(x1[j]);
-                                const float a1 = __uint_as_float(x0[j + 1]), b1 = __uint_as_float(x1[j + 1]);
-                                x0[j] = __float_as_uint(a0 * t.x - b0 * t.y);
-                                x1[j] = __float_as_uint(b0 * t.x + a0 * t.y);
-                                x0[j + 1] = __float_as_uint(a1 * t.z - b1 * t.w);
-                                x1[j + 1] = __float_as_uint(b1 * t.z + a1 * t.w);
-                            }
-                        }
-                        if (dst != nullptr) {
+                        for (int i = 0; i < 4; ++i) {
+                            const int rr = 8 * i + (lane >> 2), piece = lane & 3;
+                            __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(
+                                __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), rr));
+                            const uint4 av = stage[rr * 8 + (piece ^ (rr & 7))], bv = stage[rr * 8 + ((piece + 4) ^ (rr & 7))];
+                            float a[4] = {__uint_as_float(av.x), __uint_as_float(av.y), __uint_as_float(av.z), __uint_as_float(av.w)};
+                            float b[4] = {__uint_as_float(bv.x), __uint_as_float(bv.y), __uint_as_float(bv.z), __uint_as_float(bv.w)};
+                            if ((is_q || is_k) && qkv.rope != nullptr) {
+                                const float t[8] = {cs[2 * i].x, cs[2 * i].y, cs[2 * i].z, cs[2 * i].w, cs[2 * i + 1].x, cs[2 * i + 1].y, cs[2 * i + 1].z, cs[2 * i + 1].w};
 #pragma unroll
-                            for (int j = 0; j < 32; j += 8) {
-                                uint4 v0, v1;
-                                v0.x = pack2(x0[j], x0[j + 1]); v0.y = pack2(x0[j + 2], x0[j + 3]);
-                                v0.z = pack2(x0[j + 4], x0[j + 5]); v0.w = pack2(x0[j + 6], x0[j + 7]);
-                                v1.x = pack2(x1[j], x1[j + 1]); v1.y = pack2(x1[j + 2], x1[j + 3]);
-                                v1.z = pack2(x1[j + 4], x1[j + 5]); v1.w = pack2(x1[j + 6], x1[j + 7]);
-                                *reinterpret_cast<uint4*>(dst + c + j) = v0;
-                                *reinterpret_cast<uint4*>(dst + half + c + j) = v1;
+                                for (int e = 0; e < 4; ++e) {
+                                    const float p = a[e] * t[2 * e] - b[e] * t[2 * e + 1];
+                                    b[e] = b[e] * t[2 * e] + a[e] * t[2 * e + 1];
+                                    a[e] = p;
+                                }
                             }
+                            if (to == nullptr) continue;
+                            to += c + 4 * piece;
+                            *reinterpret_cast<uint2*>(to) = make_uint2(pack2(__float_as_uint(a[0]), __float_as_uint(a[1])),
+                                                                       pack2(__float_as_uint(a[2]), __float_as_uint(a[3])));
+                            *reinterpret_cast<uint2*>(to + half) = make_uint2(pack2(__float_as_uint(b[0]), __float_as_uint(b[1])),
+                                                                              pack2(__float_as_uint(b[2]), __float_as_uint(b[3])));
                         }
+                        __syncwarp();
                     }
                 }
                 tc_fence_before();
@@ -316,9 +349,10 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                 if (lane == 0) mbar_arrive(&sh.tempty[acc]);
                 continue;
             }
-            float ssq = 0.f;   // producer half of a split RMSNorm: this thread's row's sum of squares over the tile's columns
+            float ssq[8] = {};   // producer half of a split RMSNorm: sums of squares over this lane's columns of rows 4 i + lane / 8
 #pragma unroll 1
-            for (int c0 = 0; c0 < BNO; c0 += 32) {
+            for (int c0 = part * (BNO / 2); c0 < (part + 1) * (BNO / 2); c0 += 32) {
+                if (n0 + c0 >= N) break;               // (uniform for the warp)
                 uint32_t r[32];
                 if (kblocks > 0) {
                     tmem_load32(t_base + (uint32_t)c0, r);
@@ -391,99 +425,91 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                     for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gb_gelu_fast(__uint_as_float(r[j])));
                 }
                 if (GATED || mode == TC_STORE_BF16 || mode == TC_RELU2_BF16 || mode == TC_GELU_BF16) {
-                    // a thread's 32 columns are 64 contiguous bytes: store them directly, 16 bytes at a time
-                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)row * ldc + col0;
-                    if (row < M) {
-                        if (col0 + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
+                    tc_turn_put_bf16(stage, lane, r);
+                    __syncwarp();
+                    const int col = col0 + 8 * (lane & 3);
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)(m0 + q * 32) * ldc + col;
 #pragma unroll
-                            for (int j = 0; j < 32; j += 8) {
-                                uint4 v;
-                                v.x = pack2(r[j], r[j + 1]); v.y = pack2(r[j + 2], r[j + 3]);
-                                v.z = pack2(r[j + 4], r[j + 5]); v.w = pack2(r[j + 6], r[j + 7]);
-                                *reinterpret_cast<uint4*>(dst + j) = v;
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < N) dst[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
-                        }
-                    }
-                    continue;
-                }
-                // float32: through shared memory, so that one instruction writes one row (128 contiguous bytes)
-#pragma unroll
-                for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(r[j]);
-                __syncwarp();
-                const int col = col0 + lane;
-                float* base = reinterpret_cast<float*>(C) + (size_t)(m0 + q * 32) * ldc + col;
-                if (mode == TC_ADD_F32) {
-#pragma unroll
-                    for (int rr = 0; rr < 32; ++rr) old[rr] += stage[rr * 33 + lane];
-                    if (norm.gain != nullptr) {
-                        // producer half of a split RMSNorm: the new residual values go back into the tile as well
-#pragma unroll
-                        for (int rr = 0; rr < 32; ++rr) stage[rr * 33 + lane] = old[rr];
-                    }
-                    if (col < N) {
-#pragma unroll
-                        for (int rr = 0; rr < 32; ++rr)
-                            if (rr < rows_here) base[(size_t)rr * ldc] = old[rr];
-                    }
-                    if (c0 + 32 < BNO) load_old(col + 32);
-                } else if (col < N) {
-#pragma unroll
-                    for (int rr = 0; rr < 32; ++rr)
-                        if (rr < rows_here) base[(size_t)rr * ldc] = stage[rr * 33 + lane];
-                }
-                __syncwarp();
-                if (mode == TC_ADD_F32 && norm.gain != nullptr) {
-                    // ... and come back row by row: this thread's row leaves as bfloat16(x * gain), 64 contiguous
-                    // bytes, and adds its squares to the row's sum (columns beyond N hold what the zero-filled
-                    // weight rows gave: nothing is stored or summed for them)
-                    __nv_bfloat16* dst = norm.pre + (size_t)row * norm.ldp + col0;
-                    uint32_t packed[16];
-                    if (col0 + 32 <= N) {
-                        const float4* g4 = reinterpret_cast<const float4*>(norm.gain + col0);   // 16-byte aligned (checked by the host)
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            const float4 g = g4[j >> 2];
-                            const float v0 = stage[lane * 33 + j], v1 = stage[lane * 33 + j + 1];
-                            const float v2 = stage[lane * 33 + j + 2], v3 = stage[lane * 33 + j + 3];
-                            ssq = fmaf(v0, v0, ssq); ssq = fmaf(v1, v1, ssq); ssq = fmaf(v2, v2, ssq); ssq = fmaf(v3, v3, ssq);
-                            packed[j >> 1] = pack2(__float_as_uint(v0 * g.x), __float_as_uint(v1 * g.y));
-                            packed[(j >> 1) + 1] = pack2(__float_as_uint(v2 * g.z), __float_as_uint(v3 * g.w));
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 2) {
-                            const bool in0 = col0 + j < N, in1 = col0 + j + 1 < N;
-                            const float v0 = in0 ? stage[lane * 33 + j] : 0.f, v1 = in1 ? stage[lane * 33 + j + 1] : 0.f;
-                            const float g0 = in0 ? norm.gain[col0 + j] : 0.f, g1 = in1 ? norm.gain[col0 + j + 1] : 0.f;
-                            ssq = fmaf(v0, v0, ssq);
-                            ssq = fmaf(v1, v1, ssq);
-                            packed[j >> 1] = pack2(__float_as_uint(v0 * g0), __float_as_uint(v1 * g1));
-                        }
-                    }
-                    if (row < M) {
-                        if (col0 + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
-#pragma unroll
-                            for (int j = 0; j < 16; j += 4)
-                                *reinterpret_cast<uint4*>(dst + 2 * j) = make_uint4(packed[j], packed[j + 1], packed[j + 2], packed[j + 3]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < N) dst[j] = __ushort_as_bfloat16((unsigned short)(packed[j >> 1] >> ((j & 1) * 16)));
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        const int rr = 8 * i + (lane >> 2);
+                        if (rr < rows_here) tc_store8_bf16(dst + (size_t)rr * ldc, tc_turn_get_bf16(stage, lane, i), col, N, vec_bf16);
                     }
                     __syncwarp();
+                    continue;
                 }
+                tc_turn_put_f32(stage, lane, r);
+                __syncwarp();
+                const int col = col0 + 4 * (lane & 7);
+                float* dst = reinterpret_cast<float*>(C) + (size_t)(m0 + q * 32) * ldc + col;
+                if (mode == TC_ADD_F32) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int rr = 4 * i + (lane >> 3);
+                        const float4 v = tc_turn_get_f32(stage, lane, i);
+                        old[i].x += v.x; old[i].y += v.y; old[i].z += v.z; old[i].w += v.w;
+                        if (rr < rows_here) tc_store4_f32(dst + (size_t)rr * ldc, old[i], col, N, vec_f32);
+                    }
+                    if (norm.gain != nullptr) {
+                        // producer half of a split RMSNorm: the new residual values also leave as bfloat16(x * gain) and add their
+                        // squares to their rows' sums (columns beyond N hold what the zero-filled weight rows gave: nothing is
+                        // stored or summed for them)
+                        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (col + 4 <= N) {
+                            g = *reinterpret_cast<const float4*>(norm.gain + col);      // 16-byte aligned (checked by the host)
+                        } else {
+                            if (col < N) g.x = norm.gain[col];
+                            if (col + 1 < N) g.y = norm.gain[col + 1];
+                            if (col + 2 < N) g.z = norm.gain[col + 2];
+                        }
+                        const bool vec_pre = ((uintptr_t)norm.pre & 7) == 0 && (norm.ldp & 3) == 0 && col + 4 <= N;
+                        __nv_bfloat16* pre = norm.pre + (size_t)(m0 + q * 32) * norm.ldp + col;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int rr = 4 * i + (lane >> 3);
+                            const float4 x = old[i];
+                            ssq[i] = fmaf(x.x, col < N ? x.x : 0.f, ssq[i]);
+                            ssq[i] = fmaf(x.y, col + 1 < N ? x.y : 0.f, ssq[i]);
+                            ssq[i] = fmaf(x.z, col + 2 < N ? x.z : 0.f, ssq[i]);
+                            ssq[i] = fmaf(x.w, col + 3 < N ? x.w : 0.f, ssq[i]);
+                            if (rr >= rows_here) continue;
+                            const uint2 w = make_uint2(pack2(__float_as_uint(x.x * g.x), __float_as_uint(x.y * g.y)),
+                                                       pack2(__float_as_uint(x.z * g.z), __float_as_uint(x.w * g.w)));
+                            __nv_bfloat16* to = pre + (size_t)rr * norm.ldp;
+                            if (vec_pre) {
+                                *reinterpret_cast<uint2*>(to) = w;
+                            } else {
+                                if (col < N) to[0] = __ushort_as_bfloat16((unsigned short)w.x);
+                                if (col + 1 < N) to[1] = __ushort_as_bfloat16((unsigned short)(w.x >> 16));
+                                if (col + 2 < N) to[2] = __ushort_as_bfloat16((unsigned short)w.y);
+                                if (col + 3 < N) to[3] = __ushort_as_bfloat16((unsigned short)(w.y >> 16));
+                            }
+                        }
+                    }
+                    if (c0 + 32 < (part + 1) * (BNO / 2)) load_old(col0 + 32);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int rr = 4 * i + (lane >> 3);
+                        if (rr < rows_here) tc_store4_f32(dst + (size_t)rr * ldc, tc_turn_get_f32(stage, lane, i), col, N, vec_f32);
+                    }
+                }
+                __syncwarp();
             }
             // this warp is done with the accumulator: hand it back to the MMA issuer
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.tempty[acc]);
-            if (!GATED && mode == TC_ADD_F32 && norm.gain != nullptr && row < M)
-                norm.ss_out[(size_t)row * tiles_n + (tile / tiles_m)] = ssq;
+            if (!GATED && mode == TC_ADD_F32 && norm.gain != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int rr = 4 * i + (lane >> 3);
+                    float v = ssq[i];
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    if ((lane & 7) == 0 && rr < rows_here)
+                        norm.ss_out[(size_t)(m0 + q * 32 + rr) * (2 * tiles_n) + 2 * (tile / tiles_m) + part] = v;
+                }
+            }
         }
     }
 
@@ -530,7 +556,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* c, int 
     }
     const int ntiles = gb_ceil_div(M, TC_BM) * gb_ceil_div(N, G::BNO);
     const int grid = ntiles < sms ? ntiles : sms;   // persistent: one block per SM walks the tiles
-    cudaError_t e = gb_launch(GB_PDL_GEMM, kernel, dim3(grid), dim3(192), G::SMEM, stream, ma, mw, c, mode, M, N, K, ldc, gate_rows, status, qkv, norm, unit);
+    cudaError_t e = gb_launch(GB_PDL_GEMM, kernel, dim3(grid), dim3(TC_THREADS), G::SMEM, stream, ma, mw, c, mode, M, N, K, ldc, gate_rows, status, qkv, norm, unit);
     GB_REQUIRE(e == cudaSuccess, "gb_gemm_tcgen05: launch failed: %s", cudaGetErrorString(e));
     return gb_check_launch("gb_gemm_tcgen05");
 }
@@ -553,33 +579,29 @@ static int tc_sm_count() {
     return sms;
 }
 
-// Output tile width. A block's time for one tile is about 0.33 us per 64-wide k-block, whatever the width (at these
-// sizes the operands come from L2 at a rate that the tile count, not the tile size, sets), plus an epilogue that
-// grows with the width and with what it does; a launch takes as many rounds of tiles as its busiest block has.
-// The width with the smallest estimate wins; ties go to the wider tile, which reads the A operand less often.
-// Measured at 2048 rows on a B200, microseconds for widths 64 / 128 / 256: N 960, K 576 store 9.5 / 7.3 / 8.7;
-// N 576, K 1536 add 13.1 / 15.6 / 19.9; N 1600, K 960 store 18.9 / 15.1 / 11.4; N 960, K 2560 add 30.3 / 21.4 / 25.1;
-// gated, I 1536, K 576: 20.0 (128) / 22.3 (256); I 8192, K 2048: 153 / 107.
-enum { TC_EPI_STORE = 0, TC_EPI_ADD = 1, TC_EPI_GATED = 2 };
+// Output tile width: the one whose rounds of tiles end soonest (tc_rounds_us); ties go to the wider tile, which reads the A
+// operand less often. Epilogue times by kind and width from launches of one round (measured time less 2 us of launch and the
+// main loop). Measured on a B200, microseconds for widths 64 / 128 / 256: 2048 x 576, K 1536 add 7.7 / 10.4 / 16.2; 2048 x 960,
+// K 576 store 6.5 / 5.7 / 8.0; 2048 x 3208, K 1024 store float32 21.8 / 16.5 / 18.6; 1500 x 4288, K 2048 store 33.3 / 23.5 / 25.3;
+// 2048 x 2048, K 2048 store 23.4 / 16.5 / 15.4; gated, 2048 x 1536, K 576: 10.3 (128) / 11.8 (256).
+enum { TC_EPI_STORE = 0, TC_EPI_F32 = 1, TC_EPI_ADD = 2, TC_EPI_GATED = 3 };
 static int pick_bn(int M, int N, int K, int epilogue, int narrowest = 64) {
-    static const float epi_us[3][3] = {{1.5f, 2.5f, 4.5f}, {2.8f, 5.5f, 11.0f}, {0.f, 3.0f, 7.0f}};
+    static const float epi_us[4][3] = {{1.2f, 1.9f, 3.2f}, {1.5f, 2.4f, 4.2f}, {1.9f, 3.8f, 7.3f}, {0.f, 1.6f, 3.2f}};
     const long long tm = gb_ceil_div(M, TC_BM);
-    const float main_us = 0.33f * (float)gb_ceil_div(K, TC_BK);
     int best = 0;
     float best_us = 0.f;
     for (int i = 0, bn = 64; bn <= 256; ++i, bn *= 2) {
         if (bn < narrowest) continue;
         const int out_cols = epilogue == TC_EPI_GATED ? bn / 2 : bn;
-        const long long rounds = gb_ceil_div(tm * gb_ceil_div(N, out_cols), (long long)tc_sm_count());
-        const float us = (float)rounds * (main_us + epi_us[epilogue][i]);
+        const float us = tc_rounds_us(tm * gb_ceil_div(N, out_cols), tc_sm_count(), gb_ceil_div(K, TC_BK), bn, epi_us[epilogue][i]);
         if (best == 0 || us <= best_us) { best = bn; best_us = us; }
     }
     return best;
 }
 
-// Column tiles of gb_gemm_tcgen05's output for this shape: the second extent of the partial sums of squares
-// that a producer of a split RMSNorm writes.
-GB_EXPORT int gb_gemm_tcgen05_column_tiles(int M, int N, int K) { return gb_ceil_div(N, pick_bn(M, N, K, TC_EPI_ADD)); }
+// Pieces of columns (half a tile: one epilogue warp's share) of gb_gemm_tcgen05's output for this shape: the second extent of the
+// partial sums of squares that a producer of a split RMSNorm writes.
+GB_EXPORT int gb_gemm_tcgen05_column_tiles(int M, int N, int K) { return 2 * gb_ceil_div(N, pick_bn(M, N, K, TC_EPI_ADD)); }
 
 // mode: 0 store bfloat16, 1 store float32, 2 add into float32, 4 store bfloat16(max(c, 0)^2), 5 store bfloat16(gelu(c)).
 // Split RMSNorm (see TcNorm): with mode 2 and norm_gain != nullptr the launch also writes pre[M, N] =
@@ -597,7 +619,7 @@ GB_EXPORT int gb_gemm_tcgen05(const void* a, const void* w, void* c, int mode, i
                                         (uintptr_t)norm_gain % 16 == 0),
                "gb_gemm_tcgen05: a norm is prepared only by a product that adds into float32, into pre and ss_out");
     GB_REQUIRE(ss_in == nullptr || ss_parts > 0, "gb_gemm_tcgen05: ss_parts must be positive");
-    const int bn = pick_bn(M, N, K, mode == TC_ADD_F32 ? TC_EPI_ADD : TC_EPI_STORE);
+    const int bn = pick_bn(M, N, K, mode == TC_ADD_F32 ? TC_EPI_ADD : mode == TC_STORE_F32 ? TC_EPI_F32 : TC_EPI_STORE);
     CUtensorMap ma, mw;
     if (make_map(&ma, a, M, K, lda, TC_BM)) return 1;
     if (make_map(&mw, w, N, K, ldw, bn)) return 1;

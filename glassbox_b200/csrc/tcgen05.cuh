@@ -103,6 +103,20 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Sixteen columns from each of two places of this thread's TMEM lane, waited for in the same statement.
+__device__ __forceinline__ void tmem_load16x2(uint32_t taddr0, uint32_t taddr1, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]),
+          "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(r[16]),
+          "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23]), "=&r"(r[24]),
+          "=&r"(r[25]), "=&r"(r[26]), "=&r"(r[27]), "=&r"(r[28]), "=&r"(r[29]), "=&r"(r[30]), "=&r"(r[31])
+        : "r"(taddr0), "r"(taddr1)
+        : "memory");
+}
+
 // 64 consecutive columns of this thread's TMEM lane in one instruction, waited for in the same statement
 // (so that no use of the registers can be scheduled before the data has arrived).
 __device__ __forceinline__ void tmem_load64(uint32_t taddr, uint32_t (&r)[64]) {
@@ -205,6 +219,53 @@ __device__ __forceinline__ uint32_t pack2(uint32_t lo_bits, uint32_t hi_bits) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// A warp's 32 x 32 sums change hands on their way out: a lane leaves tensor memory with a row (32 columns) and goes to global
+// memory with 16-byte pieces of several rows, so that an instruction writes whole rows and not 16 bytes in each of 32 lines.
+// The pieces of a row lie in an order that its number turns, so that neither side meets a bank twice.
+// float32: 8 pieces a row (`tile`: 32 * 8 uint4); lane l reads piece l & 7 of rows 4 i + l / 8.
+__device__ __forceinline__ void tc_turn_put_f32(uint4* tile, int lane, const uint32_t (&r)[32]) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) tile[lane * 8 + (c ^ (lane & 7))] = make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+}
+__device__ __forceinline__ float4 tc_turn_get_f32(const uint4* tile, int lane, int i) {
+    const int row = 4 * i + (lane >> 3);
+    const uint4 v = tile[row * 8 + ((lane & 7) ^ (row & 7))];
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+// bfloat16 (rounded to nearest here): 4 pieces a row (`tile`: 32 * 4 uint4); lane l reads piece l & 3 of rows 8 i + l / 4.
+__device__ __forceinline__ void tc_turn_put_bf16(uint4* tile, int lane, const uint32_t (&r)[32]) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        tile[lane * 4 + (c ^ ((lane >> 1) & 3))] = make_uint4(pack2(r[8 * c], r[8 * c + 1]), pack2(r[8 * c + 2], r[8 * c + 3]),
+                                                              pack2(r[8 * c + 4], r[8 * c + 5]), pack2(r[8 * c + 6], r[8 * c + 7]));
+}
+__device__ __forceinline__ uint4 tc_turn_get_bf16(const uint4* tile, int lane, int i) {
+    const int row = 8 * i + (lane >> 2);
+    return tile[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
+}
+// Eight bfloat16 of a row whose first column is `col` of N: one store where the row is aligned and the piece whole.
+__device__ __forceinline__ void tc_store8_bf16(__nv_bfloat16* dst, uint4 v, int col, int N, bool vec) {
+    if (vec && col + 8 <= N) {
+        *reinterpret_cast<uint4*>(dst) = v;
+        return;
+    }
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (col + j < N) dst[j] = __ushort_as_bfloat16((unsigned short)(w[j >> 1] >> ((j & 1) * 16)));
+}
+// Four float32, likewise.
+__device__ __forceinline__ void tc_store4_f32(float* dst, float4 v, int col, int N, bool vec) {
+    if (vec && col + 4 <= N) {
+        *reinterpret_cast<float4*>(dst) = v;
+        return;
+    }
+    if (col < N) dst[0] = v.x;
+    if (col + 1 < N) dst[1] = v.y;
+    if (col + 2 < N) dst[2] = v.z;
+    if (col + 3 < N) dst[3] = v.w;
+}
+
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -242,4 +303,13 @@ static inline int tc_make_map_2d(CUtensorMap* map, const void* base, long long r
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     GB_REQUIRE(r == CUDA_SUCCESS, "%s: cuTensorMapEncodeTiled failed with code %d", who, (int)r);
     return 0;
+}
+
+// Time of a persistent launch over `tiles` tiles of 128 x bn, in microseconds, less the launch itself: a block's rounds of main loop
+// (per 64-wide k-block 0.165, 0.19 and 0.285 us at widths 64, 128 and 256, from launches of one round with K 576 to 3,072) and of
+// epilogue, which runs beside the next tile's main loop; the last epilogue stands alone.
+static inline float tc_rounds_us(long long tiles, int sms, int kblocks, int bn, float epi_us) {
+    const float main_us = (bn == 64 ? 0.165f : bn == 128 ? 0.19f : 0.285f) * (float)kblocks;
+    const float longer = main_us > epi_us ? main_us : epi_us, shorter = main_us > epi_us ? epi_us : main_us;
+    return (float)((tiles + sms - 1) / sms) * longer + shorter;
 }

@@ -47,7 +47,7 @@ def _prepare_next_norm(ctx, out: torch.Tensor, k: int):
     if rms is None or rms[0].numel() != n or rms[0].dtype != torch.float32 or n % 8:
         return None
     pre = ctx.scratch("h_pre", (rows, n), torch.bfloat16)
-    widest = -(-n // 64)     # the narrowest tile gives the most partial sums; the buffer never has to grow
+    widest = 2 * -(-n // 64)     # the narrowest tile gives the most partial sums, two a tile; the buffer never has to grow
     parts = kernels.gemm_tc_column_tiles(rows, n, k)
     ss = ctx.scratch("h_ss", (rows, widest), torch.float32).view(-1)[:rows * parts].view(rows, parts)
     return norm, rms, pre, ss

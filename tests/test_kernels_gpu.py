@@ -489,6 +489,22 @@ def test_gemm_tcgen05(M, N, K):
     assert float(wide_c[:, N:].abs().max()) == 0.0 and int(st) == 0
 
 
+@pytest.mark.parametrize("M, N, pad", [(130, 37, 1), (33, 66, 0), (257, 131, 5), (64, 3, 0), (160, 320, 2)])
+def test_gemm_tcgen05_rows_that_end_inside_a_piece(M, N, pad):
+    """Output rows that are no whole 16-byte pieces, or do not start on one: stored, added, as bfloat16; nothing beside them."""
+    from glassbox_b200 import kernels
+    K, st = 72, status()
+    a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
+    ref = a.double() @ w.double().T
+    for dtype, add in ((torch.float32, False), (torch.float32, True), (torch.bfloat16, False)):
+        buf = torch.full((M, N + pad), 3.0, device=DEV, dtype=dtype)
+        kernels.gemm_tc(a, w, buf[:, :N], accumulate=add, status=st)
+        assert (buf[:, :N].double() - ref - (3.0 if add else 0.0)).abs().max() <= (tol(dtype, 2) if dtype == torch.bfloat16 else 2e-5 * math.sqrt(K) + 1e-6)
+        assert torch.all(buf[:, N:] == 3.0)
+    assert int(st) == 0
+
+
 def test_gemm_tcgen05_refuses_misaligned_operands():
     from glassbox_b200 import kernels
     a = torch.zeros(128, 68, device=DEV, dtype=torch.bfloat16)
