@@ -4,23 +4,23 @@
 // A tile is 128 of an expert's pairs x BN of its outputs; a block (one per SM) walks the tiles of all experts in turn, an
 // expert's tiles next to each other and its rows innermost, so that a piece of its matrix is read from memory once and from L2
 // by the expert's other row tiles. Six warps, as in the dense product (gemm_tcgen05.cu):
-//   warp 0     producer: per 64-wide k-block a TMA box of the expert's matrix and the 128 input rows. UP: the rows of h lie
-//              anywhere (sorted[slot] / top); every lane fetches four of them by TMA gather, straight into the swizzled tile.
-//              DOWN: the rows are the slots themselves, one box.
+//   warp 0     producer: per 64-wide k-block a TMA box of the expert's matrix and the 128 input rows. DOWN, and UP where the rows
+//              were gathered before (moe_gather_rows_kernel): the rows are the slots themselves, one box. UP otherwise: the rows of h
+//              lie anywhere (sorted[slot] / top); every lane fetches four of them by TMA gather, straight into the swizzled tile.
 //   warp 1     issues tcgen05.mma (M 128, N BN, K 16) into one of two accumulators in tensor memory
-//   warps 2-5  epilogue: UP stores bfloat16 relu(c)^2, or one gated unit of every two neighbouring outputs; DOWN scatters
-//              float32 rows to pair[pair, :].
-// Rows past an expert's last pair are loaded (another row's numbers) and never stored. Bound by the loads' latency: 1.0 us a
-// k-block with a box of rows and 1.4 with gathers, where the products take 0.26 (up half, 2,048 rows: tensor pipe 19 % of its peak, L2
-// 14 %, DRAM 9 %); with few pairs per expert by reading every expert's matrices once. The mma.sync kernel that this replaced was
-// bound by that instruction's rate and by its operands' way through registers. Measured, 2,048 rows, 16 experts, four per token
-// (1024 -> 2 x 1024 -> 1024): up half 167 -> 102 us, down half 86 -> 40 us.
+//   warps 2-9  epilogue, as in the dense product: UP stores bfloat16 relu(c)^2, or one gated unit of every two neighbouring
+//              outputs; DOWN scatters float32 rows to pair[pair, :].
+// Rows past an expert's last pair are loaded (another row's numbers) and never stored. A k-block takes 1.4 us with 32 gathers, 0.3 with
+// a box of rows (the products 0.26), so a pass that brings the rows into slot order (16.8 MB: 4 us) pays from 64 pairs per expert
+// on; with fewer a tile needs only a gather or two and the pass would cost its launch. Measured, 2,048 rows, 16 experts, four per
+// token (1024 -> 2 x 1024 -> 1024): up half 101 us with gathers, 47 + 4 with the pass; down half 38 -> 23 with the epilogue of eight warps
+// and 16-byte stores. With few pairs per expert it is bound by reading every expert's matrices once.
 //
 // Every wait is bounded, as in the dense product: on a timeout the block records GB_STATUS_WAIT_TIMEOUT, waits (bounded) for its
 // copies, frees its tensor memory and returns. No multicast.
 #include "tcgen05.cuh"
 
-constexpr int ME_BM = 128, ME_BK = 64, ME_THREADS = 192, ME_MAX_EXPERTS = 512, ME_MAX_STAGES = 8;
+constexpr int ME_BM = 128, ME_BK = 64, ME_EPI_WARPS = 8, ME_THREADS = 64 + 32 * ME_EPI_WARPS, ME_MAX_EXPERTS = 512, ME_MAX_STAGES = 8;
 
 struct __align__(8) MeShared {
     uint64_t full[ME_MAX_STAGES], empty[ME_MAX_STAGES], tfull[2], tempty[2];
@@ -33,7 +33,7 @@ struct __align__(8) MeShared {
 template <int BN> struct MeGeometry {
     static constexpr int A_BYTES = ME_BM * ME_BK * 2, W_BYTES = BN * ME_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     static constexpr int STAGES = (192 * 1024 / STAGE_BYTES) < ME_MAX_STAGES ? (192 * 1024 / STAGE_BYTES) : ME_MAX_STAGES;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 4 * 32 * 33 * 4 + 1024;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + ME_EPI_WARPS * 32 * 64 + 1024;      // (32 rows x 64 bytes per epilogue warp)
 };
 
 // four rows of the tensor map's matrix (box: one row of 64), 128 bytes each, one behind the other
@@ -55,13 +55,13 @@ __device__ __forceinline__ float me_unit(float gate, float up, float limit, floa
 template <int BN, bool UP>
 __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                                                                  const int* __restrict__ sorted, const int* __restrict__ offsets, int E,
-                                                                 int top, int N, int K, void* __restrict__ C, long long ldc, int unit,
+                                                                 int top, int N, int K, void* __restrict__ C, long long ldc, int unit, int gather,
                                                                  float limit, float slope, int* __restrict__ status) {
     using G = MeGeometry<BN>;
     constexpr int STAGES = G::STAGES;
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* tiles = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);      // swizzled tiles: 1024-byte aligned
-    float* epi = reinterpret_cast<float*>(tiles + STAGES * G::STAGE_BYTES);
+    uint4* epi = reinterpret_cast<uint4*>(tiles + STAGES * G::STAGE_BYTES);
     __shared__ MeShared sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kblocks = (K + ME_BK - 1) / ME_BK;
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sh.tfull[b], 1);
-            mbar_init(&sh.tempty[b], 4);
+            mbar_init(&sh.tempty[b], ME_EPI_WARPS);
         }
         sh.abort_flag = sh.issued = sh.consumed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
             // 2048 x 2048 took 150 us the feed-forward (mma.sync tiles before: 128), with the live ones 107.
             const int gathers = (min(ME_BM, p.m_end - p.m0) + 3) >> 2;
             int r[4];
-            if (UP) {
+            if (UP && gather) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int slot = p.m0 + 4 * lane + i;
@@ -153,13 +153,13 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
                 if (it >= STAGES && !mbar_wait_warp(&sh.empty[s], ((it / STAGES) - 1) & 1, abort_flag, status)) { ok = false; break; }
                 unsigned char* a_dst = tiles + s * G::STAGE_BYTES;
                 if (lane == 0) {
-                    mbar_expect_tx(&sh.full[s], UP ? G::W_BYTES + gathers * 512 : G::STAGE_BYTES);
+                    mbar_expect_tx(&sh.full[s], UP && gather ? G::W_BYTES + gathers * 512 : G::STAGE_BYTES);
                     tma_load_2d(a_dst + G::A_BYTES, &map_w, &sh.full[s], kb * ME_BK, p.e * N + p.n0);
-                    if (!UP) tma_load_2d(a_dst, &map_a, &sh.full[s], kb * ME_BK, p.m0);
+                    if (!UP || !gather) tma_load_2d(a_dst, &map_a, &sh.full[s], kb * ME_BK, p.m0);
                     sh.issued = it + 1;
                 }
                 __syncwarp();
-                if (UP && lane < gathers) me_gather4(a_dst + lane * 512, &map_a, &sh.full[s], kb * ME_BK, r[0], r[1], r[2], r[3]);
+                if (UP && gather && lane < gathers) me_gather4(a_dst + lane * 512, &map_a, &sh.full[s], kb * ME_BK, r[0], r[1], r[2], r[3]);
             }
         }
     } else if (warp == 1) {
@@ -192,80 +192,80 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
         }
     } else {
         const int q = warp & 3;                                   // the quarter of the tensor-memory lanes this warp may read
-        float* stage = epi + q * (32 * 33);
+        const int part = (warp - 2) >> 2;                         // ... and its half of the tile's columns
+        uint4* stage = epi + (warp - 2) * (32 * 4);
+        const bool vec_f32 = ((uintptr_t)C & 15) == 0 && (ldc & 3) == 0, vec_bf16 = ((uintptr_t)C & 15) == 0 && (ldc & 7) == 0;
         int tcount = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
             const Place p = place(tile);
-            const int acc = tcount & 1, slot = p.m0 + q * 32 + lane;
-            const bool live = slot < p.m_end;
-            const int out_row = UP ? slot : (live ? sorted[slot] : -1);
-            const int rows = min(32, p.m_end - (p.m0 + q * 32));              // (may be negative: no row of this warp is live)
+            const int acc = tcount & 1, slot0 = p.m0 + q * 32;
+            const int out_row = UP || slot0 + lane >= p.m_end ? -1 : sorted[slot0 + lane];
+            const int rows = min(32, p.m_end - slot0);                        // (may be negative: no row of this warp is live)
             if (!mbar_wait_warp(&sh.tfull[acc], (tcount >> 1) & 1, abort_flag, status)) { ok = false; break; }
             tc_fence_after();
             const uint32_t t_base = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
+            // 32 outputs a turn: of a gated unit, 64 sums
+            const int step = UP && unit ? 64 : 32;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                const int col0 = p.n0 + c0;
-                if (col0 >= N) break;                                         // (uniform for the block)
+            for (int c0 = part * (BN / 2); c0 < (part + 1) * (BN / 2); c0 += step) {
+                if (p.n0 + c0 >= N || rows <= 0) break;                       // (uniform for the warp)
                 uint32_t v[32];
                 tmem_load32(t_base + (uint32_t)c0, v);
-                if (UP && unit) {
-                    // neighbouring outputs are the gate sum and the up sum of one unit
-                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)out_row * ldc + (col0 >> 1);
-                    if (live) {
-                        float u[16];
+                if (UP) {
+                    int col0 = p.n0 + c0, cols = N;
+                    if (unit) {
+                        // neighbouring outputs are the gate sum and the up sum of one unit
+                        col0 >>= 1;
+                        cols >>= 1;
+                        uint32_t u[32];
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) u[j] = me_unit(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), limit, slope);
-                        if (col0 + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
+                        for (int j = 0; j < 16; ++j)
+                            u[j] = __float_as_uint(me_unit(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), limit, slope));
+                        tmem_load32(t_base + (uint32_t)(c0 + 32), v);
 #pragma unroll
-                            for (int j = 0; j < 16; j += 8) {
-                                uint4 w;
-                                w.x = pack2(__float_as_uint(u[j]), __float_as_uint(u[j + 1])); w.y = pack2(__float_as_uint(u[j + 2]), __float_as_uint(u[j + 3]));
-                                w.z = pack2(__float_as_uint(u[j + 4]), __float_as_uint(u[j + 5])); w.w = pack2(__float_as_uint(u[j + 6]), __float_as_uint(u[j + 7]));
-                                *reinterpret_cast<uint4*>(dst + j) = w;
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (col0 + 2 * j + 1 < N) dst[j] = __float2bfloat16_rn(u[j]);
-                        }
-                    }
-                } else if (UP) {
-                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)out_row * ldc + col0;
-                    if (live) {
+                        for (int j = 0; j < 16; ++j)
+                            u[16 + j] = __float_as_uint(me_unit(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), limit, slope));
+                        tc_turn_put_bf16(stage, lane, u);
+                    } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float g = fmaxf(__uint_as_float(v[j]), 0.f);
                             v[j] = __float_as_uint(g * g);
                         }
-                        if (col0 + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
+                        tc_turn_put_bf16(stage, lane, v);
+                    }
+                    __syncwarp();
+                    const int col = col0 + 8 * (lane & 3);
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + (size_t)slot0 * ldc + col;
 #pragma unroll
-                            for (int j = 0; j < 32; j += 8) {
-                                uint4 w;
-                                w.x = pack2(v[j], v[j + 1]); w.y = pack2(v[j + 2], v[j + 3]);
-                                w.z = pack2(v[j + 4], v[j + 5]); w.w = pack2(v[j + 6], v[j + 7]);
-                                *reinterpret_cast<uint4*>(dst + j) = w;
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < N) dst[j] = __float2bfloat16_rn(__uint_as_float(v[j]));
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        const int rr = 8 * i + (lane >> 2);
+                        if (rr < rows) tc_store8_bf16(dst + (size_t)rr * ldc, tc_turn_get_bf16(stage, lane, i), col, cols, vec_bf16);
                     }
                 } else {
-                    // float32 through shared memory, so that one instruction writes 128 contiguous bytes of one pair's row
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(v[j]);
-                    __syncwarp();
-                    const int col = col0 + lane;
-#pragma unroll 8
-                    for (int rr = 0; rr < 32; ++rr) {
-                        const int row = __shfl_sync(0xffffffffu, out_row, rr);
-                        if (rr < rows && col < N) reinterpret_cast<float*>(C)[(size_t)row * ldc + col] = stage[rr * 33 + lane];
+                    for (int h = 0; h < 2; ++h) {                             // 16 columns, 64 bytes a row, at a time
+                        if (h) __syncwarp();
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const int j = 16 * h + 4 * c;
+                            stage[lane * 4 + (c ^ ((lane >> 1) & 3))] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                        }
+                        __syncwarp();
+                        const int col = p.n0 + c0 + 16 * h + 4 * (lane & 3);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int rr = 8 * i + (lane >> 2), row = __shfl_sync(0xffffffffu, out_row, rr);
+                            const uint4 w = tc_turn_get_bf16(stage, lane, i);
+                            if (rr < rows)
+                                tc_store4_f32(reinterpret_cast<float*>(C) + (size_t)row * ldc + col,
+                                              make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)),
+                                              col, N, vec_f32);
+                        }
                     }
                 }
-                __syncwarp();      // the next load is the whole warp's; rows past the expert's last pair have taken another way here
+                __syncwarp();      // the next load is the whole warp's; lanes of rows past the expert's last pair have taken another way here
             }
             tc_fence_before();
             __syncwarp();
@@ -289,13 +289,13 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
 
 template <int BN, bool UP>
 static int me_launch(const CUtensorMap& ma, const CUtensorMap& mw, const int* sorted, const int* offsets, int E, int top, int N, int K, void* c,
-                     long long ldc, int unit, float limit, float slope, int* status, long long most_tiles, cudaStream_t stream) {
+                     long long ldc, int unit, int gather, float limit, float slope, int* status, long long most_tiles, cudaStream_t stream) {
     auto kernel = moe_tcgen05_kernel<BN, UP>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MeGeometry<BN>::SMEM);
     GB_REQUIRE(e == cudaSuccess, "gb_moe_grouped_gemm: %d bytes of shared memory refused: %s", MeGeometry<BN>::SMEM, cudaGetErrorString(e));
     const int grid = most_tiles < 148 ? (int)most_tiles : 148;                // one block per SM walks the tiles
     e = gb_launch(GB_PDL_GEMM, kernel, dim3(grid), dim3(ME_THREADS), MeGeometry<BN>::SMEM, stream, ma, mw, sorted, offsets, E, top, N, K, c, ldc,
-                  unit, limit, slope, status);
+                  unit, gather, limit, slope, status);
     GB_REQUIRE(e == cudaSuccess, "gb_moe_grouped_gemm: launch failed: %s", cudaGetErrorString(e));
     return gb_check_launch("gb_moe_grouped_gemm");
 }
@@ -305,29 +305,62 @@ GB_EXPORT int gb_moe_grouped_supported(int d, int ff) { return d % 8 == 0 && ff 
 
 // up: a = h [rows, K] (row stride lda), c bfloat16 [pairs, ldc] in slot order; otherwise a = the up half's output [pairs, K] and c
 // float32 [pairs, ldc] in pair order. w: the experts' matrices [E * N, K]. sorted, offsets: as moe_sort leaves them.
+// gather (up only): the rows of a slot are found through sorted; otherwise a [pairs, K] holds them in slot order.
 GB_EXPORT int gb_moe_grouped_gemm(const void* a, long long lda, int rows, const void* w, int N, int K, const int* sorted, const int* offsets,
-                                  int E, int top, int pairs, void* c, long long ldc, int up, int unit, float limit, float slope, int* status,
-                                  cudaStream_t stream) {
+                                  int E, int top, int pairs, void* c, long long ldc, int up, int unit, float limit, float slope, int gather,
+                                  int* status, cudaStream_t stream) {
     GB_REQUIRE(!unit || (up && N % 2 == 0), "gb_moe_grouped_gemm: the gated unit belongs to the up half and needs pairs of rows");
     GB_REQUIRE(N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && pairs >= 0 && E > 0 && E <= ME_MAX_EXPERTS && status != nullptr,
                "gb_moe_grouped_gemm: rows must be whole 16-byte pieces (K=%d), at most %d experts (%d)", K, ME_MAX_EXPERTS, E);
     GB_REQUIRE(((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0, "gb_moe_grouped_gemm: operands must be 16-byte aligned");
     GB_REQUIRE((long long)E * N <= 0x7fffffff, "gb_moe_grouped_gemm: too many rows of weights");
     if (pairs == 0) return 0;
-    // The width whose rounds of tiles end soonest, as in the dense product: a k-block takes about as long whatever the width.
-    // How many row tiles there are is known on the device alone: every expert's last one is taken to be half full.
+    // The width whose rounds of tiles end soonest, as in the dense product (gemm_tcgen05.cu), with its epilogues' times. How many
+    // row tiles there are is known on the device alone: every expert's last one is taken to be half full. Measured, microseconds
+    // for widths 128 / 256: four of 16 experts 1024 -> 2 x 1024 -> 1024, 2,048 rows up 53.5 / 47.3, down 25.7 / 23.3; 512 rows up
+    // 24.1 / 26.2; two of 16 experts 2048 -> 2 x 2048 -> 2048, 1,024 rows down 36.2 / 40.9, 2,048 rows up 105 / 86.
     const long long used = pairs < E ? pairs : E;
     const long long likely = pairs / ME_BM + used / 2, row_tiles = likely > used ? likely : used;
-    const float main_us = 0.33f * (float)gb_ceil_div(K, ME_BK);
-    const float epi[2] = {up ? 2.5f : 5.5f, up ? 4.5f : 11.0f};
-    const long long t128 = row_tiles * gb_ceil_div(N, 128), t256 = row_tiles * gb_ceil_div(N, 256);
-    const bool wide = (float)((t256 + 147) / 148) * (main_us + epi[1]) <= (float)((t128 + 147) / 148) * (main_us + epi[0]);
+    const int kblocks = gb_ceil_div(K, ME_BK);
+    const bool wide = tc_rounds_us(row_tiles * gb_ceil_div(N, 256), 148, kblocks, 256, up ? 3.2f : 4.2f) <=
+                      tc_rounds_us(row_tiles * gb_ceil_div(N, 128), 148, kblocks, 128, up ? 1.6f : 2.4f);
     CUtensorMap ma, mw;
-    if (tc_make_map_2d(&ma, a, rows, K, lda, up ? 1 : ME_BM, ME_BK, "gb_moe_grouped_gemm")) return 1;
+    if (tc_make_map_2d(&ma, a, rows, K, lda, up && gather ? 1 : ME_BM, ME_BK, "gb_moe_grouped_gemm")) return 1;
     if (tc_make_map_2d(&mw, w, (long long)E * N, K, K, wide ? 256 : 128, ME_BK, "gb_moe_grouped_gemm")) return 1;
-#define ME_CASE(BN_, UP_) me_launch<BN_, UP_>(ma, mw, sorted, offsets, E, top, N, K, c, ldc, unit, limit, slope, status, \
+#define ME_CASE(BN_, UP_) me_launch<BN_, UP_>(ma, mw, sorted, offsets, E, top, N, K, c, ldc, unit, gather, limit, slope, status, \
                                               (pairs / ME_BM + used) * gb_ceil_div(N, BN_), stream)
     if (up) return wide ? ME_CASE(256, true) : ME_CASE(128, true);
     return wide ? ME_CASE(256, false) : ME_CASE(128, false);
 #undef ME_CASE
+}
+
+// Rows of h in the order of the slots: out[slot, :] = h[sorted[slot] / top, :], a warp per row, four rows' pieces under way.
+__global__ void __launch_bounds__(256) moe_gather_rows_kernel(const uint4* __restrict__ h, int pieces, const int* __restrict__ sorted,
+                                                              const int* __restrict__ offsets, int E, int top, uint4* __restrict__ out) {
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    const int slot = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (slot >= offsets[E]) return;
+    const uint4* src = h + (size_t)(sorted[slot] / top) * pieces;
+    uint4* dst = out + (size_t)slot * pieces;
+    for (int i0 = lane; i0 < pieces; i0 += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i0 + 32 * u < pieces) v[u] = src[i0 + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i0 + 32 * u < pieces) dst[i0 + 32 * u] = v[u];
+    }
+}
+
+// h bfloat16 [rows, K] and out bfloat16 [pairs, K], both contiguous and 16-byte aligned; sorted, offsets: as moe_sort leaves them.
+GB_EXPORT int gb_moe_gather_rows(const void* h, int K, const int* sorted, const int* offsets, int E, int top, int pairs, void* out,
+                                 cudaStream_t stream) {
+    GB_REQUIRE(K > 0 && K % 8 == 0 && (((uintptr_t)h | (uintptr_t)out) & 15) == 0 && E > 0 && top > 0 && pairs >= 0,
+               "gb_moe_gather_rows: rows must be whole 16-byte pieces (K=%d)", K);
+    if (pairs == 0) return 0;
+    gb_launch(GB_PDL_ELEMENTWISE, moe_gather_rows_kernel, dim3(gb_ceil_div(pairs, 8)), dim3(256), 0, stream, (const uint4*)h, K / 8, sorted,
+              offsets, E, top, (uint4*)out);
+    return gb_check_launch("gb_moe_gather_rows");
 }

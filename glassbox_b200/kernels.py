@@ -157,7 +157,8 @@ _SIGNATURES = {
     "gb_moe_expert_halves": [_P, _I, _I, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _F, _F, _P],
     "gb_moe_sort": [_P, _P, _I, _I, _I, _P, _P, _P],
     "gb_moe_grouped_supported": [_I, _I],
-    "gb_moe_grouped_gemm": [_P, _LL, _I, _P, _I, _I, _P, _P, _I, _I, _I, _P, _LL, _I, _I, _F, _F, _P, _P],
+    "gb_moe_grouped_gemm": [_P, _LL, _I, _P, _I, _I, _P, _P, _I, _I, _I, _P, _LL, _I, _I, _F, _F, _I, _P, _P],
+    "gb_moe_gather_rows": [_P, _I, _P, _P, _I, _I, _I, _P, _P],
     "gb_moe_combine": [_P, _P, _I, _P, _LL, _P, _P, _P, _LL, _I, _I, _I, _P],
     "gb_post_norm": [_P, _LL, _P, _F, _F, _I, _P, _P, _P, _P, _F, _F, _F, _P, _P, _I, _P, _P, _P, _I, _P, _I, _I, _P],
     "gb_gate_group_norm": [_P, _P, _LL, _P, _P, _I, _P, _I, _I, _I, _F, _P],
@@ -2085,18 +2086,29 @@ def moe_grouped_supported(dtype: torch.dtype, d: int, ff: int) -> bool:
     return dtype == torch.bfloat16 and bool(lib().gb_moe_grouped_supported(d, ff))
 
 
+#: pairs per expert from which the up half's input rows are gathered by a pass of their own before the product (feed-forward in us,
+#: gathered before / in the product: 16 experts of 1,024, four a row: 128 rows 38.6 / 36.5, 256 41.4 / 41.3, 512 54.6 / 75.4, 2,048
+#: 87.8 / 133.7; 2,048, two a row: 256 rows 88.8 / 85.0, 512 92.0 / 102.5; 64 experts of 512, eight a row: 512 rows 70.2 / 69.5)
+MOE_GATHER_FIRST_PAIRS = 64
+
+
+def moe_gather_first(pairs: int, experts: int) -> bool:
+    return pairs >= MOE_GATHER_FIRST_PAIRS * experts
+
+
 def moe_experts_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, choice: torch.Tensor,
                         positions: torch.Tensor, tables: torch.Tensor, act: torch.Tensor, pair: torch.Tensor, unit=None,
-                        status: Optional[torch.Tensor] = None) -> None:
+                        status: Optional[torch.Tensor] = None, gathered: Optional[torch.Tensor] = None) -> None:
     """The chosen experts of many rows as grouped products on the tensor cores (bfloat16): the (row, choice) pairs are
     sorted by expert (``tables`` int32 [experts + 1 + n * top] is the sort's scratch), then one launch computes
     act = relu(W_up[e] h)^2 for all pairs (bfloat16 [n, top * ff], in sorted order) and one pair = W_down[e] act
     (float32 [n, top * d], in pair order). ``unit`` as in ``moe_expert_halves``: the up product then has 2 ff outputs per
     expert, and its epilogue forms one unit from every two neighbours. ``status``: the word in which a wait that gives up is
-    recorded (``check_status``)."""
+    recorded (``check_status``). ``gathered`` (bfloat16 [n, top * d]): scratch into which a pass of its own brings the input rows in the
+    order of the pairs (``moe_gather_first``); without it the up product fetches them row by row."""
     if status is None:
         status = torch.zeros(1, dtype=torch.int32, device=h.device)
-    _cuda(h, w_up, w_down, choice, positions, tables, act, pair, status)
+    _cuda(h, w_up, w_down, choice, positions, tables, act, pair, status, gathered)
     n, d = h.shape
     top = choice.shape[1]
     up_rows = w_up.shape[0] // experts
@@ -2109,10 +2121,16 @@ def moe_experts_grouped(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tenso
     assert tables.dtype == torch.int32 and tables.is_contiguous() and tables.numel() >= experts + 1 + P
     offsets, order = tables[:experts + 1], tables[experts + 1:]
     _call("gb_moe_sort", _ptr(choice), _ptr(positions), n, experts, top, _ptr(offsets), _ptr(order), _stream())
-    _call("gb_moe_grouped_gemm", _ptr(h), d, n, _ptr(w_up), up_rows, d, _ptr(order), _ptr(offsets), experts, top, P,
-          _ptr(act), ff, 1, 1 if unit else 0, float(unit[0]) if unit else 0.0, float(unit[1]) if unit else 0.0, _ptr(status), _stream())
+    rows, gather = h, True
+    if gathered is not None:
+        assert gathered.dtype == torch.bfloat16 and gathered.is_contiguous() and gathered.numel() == P * d
+        rows, gather = gathered.view(P, d), False
+        _call("gb_moe_gather_rows", _ptr(h), d, _ptr(order), _ptr(offsets), experts, top, P, _ptr(rows), _stream())
+    _call("gb_moe_grouped_gemm", _ptr(rows), d, rows.shape[0], _ptr(w_up), up_rows, d, _ptr(order), _ptr(offsets), experts, top, P,
+          _ptr(act), ff, 1, 1 if unit else 0, float(unit[0]) if unit else 0.0, float(unit[1]) if unit else 0.0, 1 if gather else 0,
+          _ptr(status), _stream())
     _call("gb_moe_grouped_gemm", _ptr(act), ff, P, _ptr(w_down), d, ff, _ptr(order), _ptr(offsets), experts, top, P,
-          _ptr(pair), d, 0, 0, 0.0, 0.0, _ptr(status), _stream())
+          _ptr(pair), d, 0, 0, 0.0, 0.0, 0, _ptr(status), _stream())
 
 
 def moe_combine(pair: torch.Tensor, weight: torch.Tensor, shared: Optional[torch.Tensor], gate: Optional[torch.Tensor],

@@ -113,8 +113,9 @@ class RoutedExperts(FeedForward):
             # many rows: the pairs sorted by expert, one grouped product per half on the tensor cores
             tables = ctx.zeros_once(f"moe_tables_{self.E}_{self.top}", self.E + 1 + ctx.max_rows * self.top, torch.int32)
             act = ctx.scratch("moe_act", (n, self.top * self.ff))
+            gathered = ctx.scratch("moe_rows", (n, self.top * d)) if kernels.moe_gather_first(n * self.top, self.E) else None
             kernels.moe_experts_grouped(h, p["w_up"], p["w_down"], self.E, choice, ctx.positions, tables, act, pair, unit=unit,
-                                        status=ctx.status)
+                                        status=ctx.status, gathered=gathered)
         else:
             # few rows (or float32): the chosen experts' matrices streamed once per (row, choice), many blocks each
             act = ctx.scratch("moe_act32", (n, self.top * self.ff), torch.float32)

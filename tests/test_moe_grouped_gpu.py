@@ -86,3 +86,23 @@ def test_the_unit_divides_as_float32_does():
     # float32: the exponential's argument is exact, its value and the quotient a few 2^-23 off; then one rounding to bfloat16
     assert int(status) == 0
     assert ((pair.double().cpu() - want).abs() <= 2 ** -8 * want.abs()).all()
+
+
+@pytest.mark.parametrize("E, top, d, ff, unit, counts", [
+    (3, 2, 72, 40, "silu", [129, 0, 64]),
+    (2, 1, 264, 136, None, [1, 255]),
+    (4, 3, 1032, 64, None, [128, 127, 65, 3]),
+])
+def test_rows_gathered_before_the_product(E, top, d, ff, unit, counts):
+    """The input rows brought into the pairs' order by a pass of their own: the bits of the product that fetches them row by row."""
+    from glassbox_b200 import kernels
+    h, w_up, w_down, choice, positions = (t.to(DEV) for t in _case(E, top, d, ff, unit, counts, d))
+    n, out = h.shape[0], []
+    for gathered in (None, torch.full((n, top * d), float("nan"), dtype=torch.bfloat16, device=DEV)):
+        tables, status = torch.zeros(E + 1 + n * top, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        act, pair = torch.zeros((n, top * ff), dtype=torch.bfloat16, device=DEV), torch.full((n, top * d), 7.0, device=DEV)
+        kernels.moe_experts_grouped(h, w_up, w_down, E, choice, positions, tables, act, pair, unit=kernels.SILU_UNIT if unit else None,
+                                    status=status, gathered=gathered)
+        assert int(status) == 0
+        out.append(pair)
+    assert torch.equal(*out)
