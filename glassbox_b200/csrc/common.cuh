@@ -126,6 +126,17 @@ __device__ __forceinline__ float gb_gated_unit(float gate, float up, float limit
     return slope < 0.f ? gb_gelu_tanh(gate) * up : gate / (1.0f + expf(-gate)) * up;
 }
 
+// x and y as three bfloat16 each, by truncation (8 + 8 + 8 bits: the terms' sum is the number), packed with x in the low halves.
+__device__ __forceinline__ void gb_split_bf16(float x, float y, uint32_t (&term)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
+        term[i] = __byte_perm(xb, yb, 0x7632);
+        x -= __uint_as_float(xb & 0xffff0000u);
+        y -= __uint_as_float(yb & 0xffff0000u);
+    }
+}
+
 __device__ __forceinline__ float gb_warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

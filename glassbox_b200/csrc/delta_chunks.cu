@@ -7,29 +7,45 @@
 //     o_i = (q_i P_i)^T S_0 + sum_{j<=i} B_ij u_j,                            B_ij = sum_c q_i[c] D_ij[c] k_j[c]
 //     S_32 = diag(P_32) S_0 + sum_j (k_j D_(32)j) u_j^T
 // (the WY form of a product of Householder-like factors; Bischof and Van Loan 1987, with decays as in gated linear
-// attention). With T = (1 + diag(beta) A)^(-1) diag(beta) (A strictly lower triangular: forward substitution) and M = B T a
-// chunk is W = V - (K P) S_0, U = T W, O = (Q P) S_0 + M W, S_32 = P_32 S_0 + (K D)^T U: products, and nothing but S passes
-// from chunk to chunk. Decays only ever appear as products of themselves, never as quotients, so nothing overflows
-// however fast a channel forgets. Everything is float32, sums and operands, as in the walk.
+// attention). With T = (1 + diag(beta) A)^(-1) diag(beta) (A strictly lower triangular: forward substitution) a chunk is
+// U = T V - (T K P) S_0, O = (Q P) S_0 + B U, S_32 = P_32 S_0 + (K D)^T U: products, and nothing but S passes from chunk to
+// chunk. Decays only ever appear as products of themselves, never as quotients, so nothing overflows however fast a channel
+// forgets.
 //
-//   delta_prepare_kernel  every (chunk, head) side by side: unit vectors, decays, A, B, T, M into a workspace
-//   delta_scan_kernel     a block per (request, head, 8 columns of S): chunk after chunk, S in shared memory
+//   delta_prepare_kernel  every (chunk, head) side by side: unit vectors, decays, A, B, T K P and T V into a workspace
+//   delta_scan_kernel     a block per (request, head, 8 or 16 columns of S): U and S chunk after chunk, S in registers
+//   delta_out_kernel      every (chunk, head) side by side: O from the chunk's S_0 and U
 //
-// What bounds it: the walk was a chain of 0.3 us per token whatever the chip could do (one warp's dependent instructions);
-// here a block pays a chunk's shared-memory traffic (a 16-byte load takes the pipe four cycles whoever shares it: 1,280 of 4,000
-// cycles a chunk in the first product alone) and six barriers, 0.07 us per token.
-// Measured, 8 heads x 128 x 128, 2,048 tokens of one request: walk 724 us; prepare 44 + scan 139 us (16 heads 85 + 215 us).
+// Everything is float32. The products run on the tensor cores with every float32 operand as three bfloat16 numbers whose sum it is
+// exactly (8 + 8 + 8 bits, by truncation) and six products of them, the largest in an accumulator of its own: what is left out is below
+// 2^-24 of a product. Measured against 64 bits, random inputs with decays from next to none to a channel forgotten at once (2-norm of
+// the error over that of the result, read-out / state): one request of 700 tokens 8.0e-7 / 9.1e-7, 2,048 tokens 1.7e-7 / 1.3e-7; with
+// sums by FMA and the hardware's exponentials for the decays 1.25e-6 / 1.33e-6 and 1.65e-6 / 1.52e-6.
+// What bounds the scan: a chain of 1,350 cycles a chunk (two products, two barriers and a sum over the warps) and a chunk's two operands
+// for a block, 48 KB from L2 (with all operands in L1 45 us of the 68). A warp owns 16 channels of S: S never leaves its registers
+// (movmatrix turns the accumulators into the next product's operand); the sums over the channels meet in shared memory. Operands come
+// in the order of the fragments, two chunks ahead, straight into registers. 16 columns a block where 8 would make more blocks than
+// multiprocessors: the operands' way counts once for both.
+// Measured, 2,048 tokens of one request, prepare + scan + read-out: 8 heads x 128 x 128 44 + 68 + 21 us (the chunk's products by FMA from
+// shared memory, read-out in the scan: 44 + 139), 16 heads 83 + 106 + 42 (85 + 215).
 #include "common.cuh"
 
 constexpr int DC_C = 32;                            // tokens of a chunk
 constexpr int DC_K = 128;                           // key channels (smaller key sizes are padded: k = q = 0, decay 1)
-constexpr int DC_COLS = 8;                          // columns of S of a scanning block
-constexpr int DC_RP = DC_K + 4;                     // floats from row to row of K P and Q P: 8 lanes on 8 rows hit 32 banks
-constexpr int DC_TP = DC_C + 4;                     // ... of T and M
+constexpr int DC_V = 128;                           // columns of S that one pass takes
+constexpr int DC_RP = DC_K + 8;                     // floats from row to row in shared memory: a fragment's 8-byte loads hit 32 banks
+constexpr int DC_TP = DC_C + 4;                     // ... of A and B
 constexpr int DC_THREADS = 256;
-// the workspace of a (chunk, head): K P [32][132], Q P [32][132] | T [32][36], M [32][36] | K D [32][128], P_32 [128]
-constexpr int DC_WS_KQ = 2 * DC_C * DC_RP, DC_WS_TM = 2 * DC_C * DC_TP, DC_WS_KD = DC_C * DC_K + DC_K;
-constexpr int DC_WS = DC_WS_KQ + DC_WS_TM + DC_WS_KD;
+// The workspace of a (chunk, head), in 32-bit words. Fragments of mma.m16n8k16, [tile][3 terms][32 lanes][4 words]:
+//   T K P   [8 groups of 16 channels][2 groups of 16 tokens]       rows tokens, k channels
+//   K D     [8 groups of 16 channels][2 halves of each 8 tokens]   rows channels, k tokens (lane t of four: 8 t + 4 half ..)
+//   Q P     as T K P
+//   B       [2 groups of 16 tokens][2 groups of 16 tokens]         zero above the diagonal
+// float32: P_32 [128], T V and later U [32 tokens][128 columns], S_0 [16 groups of 8 columns][8 groups of 16 channels][32 lanes][4]
+constexpr int DC_FRAG = 3 * 32 * 4;
+constexpr int DC_AT_KT = 0, DC_AT_KD = DC_AT_KT + 16 * DC_FRAG, DC_AT_QP = DC_AT_KD + 16 * DC_FRAG, DC_AT_B = DC_AT_QP + 16 * DC_FRAG;
+constexpr int DC_AT_P = DC_AT_B + 4 * DC_FRAG, DC_AT_U = DC_AT_P + DC_K, DC_AT_S = DC_AT_U + DC_C * DC_V;
+constexpr int DC_WS = DC_AT_S + DC_K * DC_V;
 constexpr float DC_UNIT_EPS = 1e-6f;
 
 struct DeltaChunkArgs {
@@ -49,6 +65,7 @@ struct DeltaChunkArgs {
     const int* seq_slots;
     float* ws;
     int heads, kv_heads, dk, dv, num_slots, write_state, decay_channels;
+    int col0, cols;         // the columns of S of this pass: at most DC_V
     int* status;
 };
 
@@ -73,8 +90,29 @@ __device__ __forceinline__ void dc_cp16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
 }
-__device__ __forceinline__ void dc_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N> __device__ __forceinline__ void dc_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
+__device__ __forceinline__ uint32_t dc_turn(uint32_t v) {       // an 8 x 8 matrix of 16-bit numbers, a row per four lanes, transposed
+    uint32_t r;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ void dc_mma(float (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+// The largest of an operand pair's products: 8 and 8 of the 16 channels or tokens apart, their sums added as float32 adds. The tensor
+// core cuts what lies below its window: over 16 numbers near one an error of 2.5e-8 of the result, so 2.3e-8, in a chain of FMA 2.2e-8.
+__device__ __forceinline__ void dc_mma_add(float (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+    float d[4], f[4];
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a.x), "r"(a.y), "r"(b0), "f"(0.f));
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+        : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(a.z), "r"(a.w), "r"(b1), "f"(0.f));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] += d[e] + f[e];
+}
+// The six products of two operands of three terms, the smallest first: (a's term, b's term); the last has its own accumulator.
+constexpr int DC_PRODUCTS = 6;
+__device__ constexpr int DC_A_TERM[DC_PRODUCTS] = {2, 0, 1, 1, 0, 0}, DC_B_TERM[DC_PRODUCTS] = {0, 2, 1, 0, 1, 0};
 
 // where a request's chunks lie in the workspace: requests own rows one after the other, so r0 / 32 + seq leaves room for
 // each one's last, ragged chunk
@@ -98,8 +136,8 @@ __device__ __forceinline__ float dc_transpose_sum(float (&v)[32], int lane) {
 
 __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunkArgs p) {
     extern __shared__ __align__(16) float dc_mem[];
-    float* Q = dc_mem, *K = Q + DC_C * DC_RP, *G = K + DC_C * DC_RP;       // [32][132] each
-    __shared__ __align__(16) float A[DC_C][DC_TP], B[DC_C][DC_TP], Tm[DC_C][DC_TP];
+    float* Q = dc_mem, *K = Q + DC_C * DC_RP, *G = K + DC_C * DC_RP;       // [32][136] each
+    __shared__ __align__(16) float A[DC_C][DC_TP], B[DC_C][DC_TP];
     __shared__ float beta_s[DC_C];
     gb_pdl_launch_dependents();
     gb_pdl_wait();
@@ -132,13 +170,13 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int t = t0 + 2 * u;
-                const float sp = zv[u] > 15.f ? zv[u] : __logf(1.0f + __expf(zv[u]));     // (as in the walk)
+                const float sp = zv[u] > 15.f ? zv[u] : log1pf(expf(zv[u]));
                 Q[t * DC_RP + c] = qv[u];
                 K[t * DC_RP + c] = kv[u];
-                G[t * DC_RP + c] = t < nt && c < dk ? __expf(-rate * sp) : 1.f;
+                G[t * DC_RP + c] = t < nt && c < dk ? expf(-rate * sp) : 1.f;
             }
         }
-        if (tid < DC_C) beta_s[tid] = tid < nt ? 1.0f / (1.0f + __expf(-p.beta[(size_t)(c0 + tid) * p.ldb + head])) : 0.f;
+        if (tid < DC_C) beta_s[tid] = tid < nt ? 1.0f / (1.0f + expf(-p.beta[(size_t)(c0 + tid) * p.ldb + head])) : 0.f;
     }
     __syncthreads();
     const float q_scale = 1.0f / sqrtf((float)dk);
@@ -155,25 +193,6 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
         *k4 = make_float4(k.x * ik, k.y * ik, k.z * ik, k.w * ik);
     }
     __syncthreads();
-    // products of decays: from the front for K P and Q P (half of the block), from the back for K D (the other half)
-    if (tid < DC_K) {
-        float d = 1.f;
-#pragma unroll 8
-        for (int t = 0; t < DC_C; ++t) {
-            d *= G[t * DC_RP + tid];
-            ws[t * DC_RP + tid] = K[t * DC_RP + tid] * d;
-            ws[(DC_C + t) * DC_RP + tid] = Q[t * DC_RP + tid] * d;
-        }
-        ws[DC_WS_KQ + DC_WS_TM + DC_C * DC_K + tid] = d;
-    } else {
-        const int c = tid - DC_K;
-        float d = 1.f;
-#pragma unroll 8
-        for (int t = DC_C - 1; t >= 0; --t) {
-            ws[DC_WS_KQ + DC_WS_TM + t * DC_K + c] = K[t * DC_RP + c] * d;
-            d *= G[t * DC_RP + c];
-        }
-    }
     // A and B: a warp takes four rows, a lane four channels; walking j downwards, the decays between the tokens grow factor
     // by factor. The sums over the lanes go 32 at a time (four j of four rows and two matrices).
     {
@@ -216,42 +235,109 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
         }
     }
     __syncthreads();
-    // T by forward substitution, a lane per column
-    if (warp == 0) {
-        float t[DC_C];
+    // A thread per column of [K P | V]: forward substitution gives T K P and T V without T (row i needs rows in front of it alone, so
+    // a token never meets a later one's numbers, not even times zero). Half of the block also leaves Q P and K D where Q and K were.
+    {
+        float x[DC_C];
+        const int c = tid & (DC_K - 1);
+        const bool keys = tid < DC_K;
+        if (keys) {
+            float d = 1.f;
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) {
+                d *= G[t * DC_RP + c];
+                x[t] = K[t * DC_RP + c] * d;
+                Q[t * DC_RP + c] *= d;
+            }
+            ws[DC_AT_P + c] = d;
+            d = 1.f;
+#pragma unroll
+            for (int t = DC_C - 1; t >= 0; --t) {
+                K[t * DC_RP + c] *= d;
+                d *= G[t * DC_RP + c];
+            }
+        } else {
+            const float* v = p.qkv + (size_t)2 * p.kv_heads * dk + (size_t)head * p.dv + p.col0 + c;
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) x[t] = t < nt && c < p.cols ? v[(size_t)(c0 + t) * p.ldq] : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < DC_C; ++i) {
-            const float bi = beta_s[i];
             float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int j = 0; j < i; ++j) s[j & 3] = fmaf(A[i][j], t[j], s[j & 3]);
-            t[i] = bi * ((lane == i ? 1.f : 0.f) - ((s[0] + s[1]) + (s[2] + s[3])));
-            Tm[i][lane] = t[i];
-            ws[DC_WS_KQ + i * DC_TP + lane] = t[i];
+            for (int j = 0; j < i; j += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(&A[i][j]);
+                s[0] = fmaf(a.x, x[j], s[0]);
+                if (j + 1 < i) s[1] = fmaf(a.y, x[j + 1], s[1]);
+                if (j + 2 < i) s[2] = fmaf(a.z, x[j + 2], s[2]);
+                if (j + 3 < i) s[3] = fmaf(a.w, x[j + 3], s[3]);
+            }
+            x[i] = beta_s[i] * (x[i] - ((s[0] + s[1]) + (s[2] + s[3])));
+        }
+#pragma unroll
+        for (int t = 0; t < DC_C; ++t) {
+            if (keys) G[t * DC_RP + c] = x[t];
+            else ws[DC_AT_U + t * DC_V + c] = x[t];
         }
     }
     __syncthreads();
+    // the operands in the order of the fragments
+    const int g = lane >> 2, t4 = lane & 3;
+    for (int it = warp; it < 52; it += DC_THREADS / 32) {
+        float2 v[4];
+        int at;
+        if (it < 32) {                                                     // T K P, then Q P
+            const int tile = it & 15;
+            const float* src = (it < 16 ? G : Q) + ((tile & 1) * 16 + g) * DC_RP + (tile >> 1) * 16 + 2 * t4;
+            at = (it < 16 ? DC_AT_KT : DC_AT_QP) + tile * DC_FRAG;
+            v[0] = *reinterpret_cast<const float2*>(src);
+            v[1] = *reinterpret_cast<const float2*>(src + 8 * DC_RP);
+            v[2] = *reinterpret_cast<const float2*>(src + 8);
+            v[3] = *reinterpret_cast<const float2*>(src + 8 * DC_RP + 8);
+        } else if (it < 48) {                                              // K D
+            const int tile = it - 32;
+            const float* src = K + (8 * t4 + 4 * (tile & 1)) * DC_RP + (tile >> 1) * 16 + g;
+            at = DC_AT_KD + tile * DC_FRAG;
+            v[0] = make_float2(src[0], src[DC_RP]);
+            v[1] = make_float2(src[8], src[DC_RP + 8]);
+            v[2] = make_float2(src[2 * DC_RP], src[3 * DC_RP]);
+            v[3] = make_float2(src[2 * DC_RP + 8], src[3 * DC_RP + 8]);
+        } else {                                                           // B (above its diagonal nothing was written)
+            const int tile = it - 48, i = (tile >> 1) * 16 + g, j = (tile & 1) * 16 + 2 * t4;
+            at = DC_AT_B + tile * DC_FRAG;
+            auto b = [&](int r, int c) { return make_float2(c <= r ? B[r][c] : 0.f, c + 1 <= r ? B[r][c + 1] : 0.f); };
+            v[0] = b(i, j); v[1] = b(i + 8, j); v[2] = b(i, j + 8); v[3] = b(i + 8, j + 8);
+        }
+        uint32_t w[4][3];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {                                          // M = B T, sums over j .. i
-        const int i = warp + 8 * u, j = lane;
-        float s = 0.f;
-        for (int l = 0; l <= i; ++l)
-            if (l >= j) s = fmaf(B[i][l], Tm[l][j], s);
-        ws[DC_WS_KQ + (DC_C + i) * DC_TP + j] = s;
+        for (int r = 0; r < 4; ++r) gb_split_bf16(v[r].x, v[r].y, w[r]);
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+            *reinterpret_cast<uint4*>(ws + at + e * 128 + lane * 4) = make_uint4(w[0][e], w[1][e], w[2][e], w[3][e]);
     }
 }
 
-// (two blocks share an SM where there are that many)
-constexpr int DC_SCAN_SMEM = (2 * DC_WS_KQ + 2 * DC_WS_TM + DC_WS_KD + DC_COLS * DC_RP + 2 * DC_COLS * DC_TP) * 4;
+// S of a warp's 16 channels and 8 columns as the right operand of a product over the channels
+__device__ __forceinline__ void dc_right(const float (&s)[4], uint32_t (&b)[3][2]) {
+    uint32_t lo[3], hi[3];
+    gb_split_bf16(s[0], s[1], lo);
+    gb_split_bf16(s[2], s[3], hi);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        b[e][0] = dc_turn(lo[e]);
+        b[e][1] = dc_turn(hi[e]);
+    }
+}
 
-__global__ void __launch_bounds__(DC_THREADS, 2) delta_scan_kernel(DeltaChunkArgs p) {
-    extern __shared__ __align__(16) float dc_mem[];
-    float* KQ = dc_mem;                                     // two of [64][132]: K P, then Q P
-    float* TM = KQ + 2 * DC_WS_KQ;                          // two of [64][36]: T, then M
-    float* KD = TM + 2 * DC_WS_TM;                          // [32][128], then P_32 [128]
-    float* Ss = KD + DC_WS_KD;                              // S by columns: [8][132]
-    float* Wt = Ss + DC_COLS * DC_RP;                       // W and U by columns: [8][36] each
-    float* Ut = Wt + DC_COLS * DC_TP;
+template <int NT> struct DeltaOperands {                     // what a chunk brings to a thread
+    uint4 kt[2][3], kd[2][3];
+    float decay[2], tv[NT];
+};
+
+template <int NT>
+__global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArgs p) {
+    __shared__ float red[NT][8][DC_C][8];                    // T K P S by warp (16 channels each): [column group][warp][token][column]
+    __shared__ __align__(16) unsigned short Ub[NT][3][8][DC_C];     // U's terms by column
     gb_pdl_launch_dependents();
     gb_pdl_wait();
     const int head = blockIdx.y, seq = blockIdx.z;
@@ -264,166 +350,240 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_scan_kernel(DeltaChunkArg
     const int r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];
     const int chunks = (r1 - r0 + DC_C - 1) / DC_C;
     if (chunks <= 0) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int dk = p.dk, dv = p.dv, col0 = blockIdx.x * DC_COLS;
-    float* sbase = p.state + (size_t)slot * p.state_stride + (size_t)head * dk * dv;
-    const float* ws0 = p.ws + dc_slot(r0, seq, 0, p.heads, head);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int dk = p.dk, dv = p.dv, col0 = blockIdx.x * 8 * NT;              // (of this pass)
+    float* sbase = p.state + (size_t)slot * p.state_stride + (size_t)head * dk * dv + p.col0;
+    float* ws0 = p.ws + dc_slot(r0, seq, 0, p.heads, head);
     const size_t ws_step = (size_t)p.heads * DC_WS;
+    const int ti = tid >> 3, tc = tid & 7;                   // a thread's token and column between the two products
+    const int ch = warp * 16 + g;
 
-    auto load_first = [&](int chunk) {                      // what the first two phases of a chunk read
-        const float* src = ws0 + chunk * ws_step;
-        float* kq = KQ + (chunk & 1) * DC_WS_KQ, *tm = TM + (chunk & 1) * DC_WS_TM;
-        for (int i = tid; i < DC_WS_KQ / 4; i += DC_THREADS) dc_cp16(kq + 4 * i, src + 4 * i);
-        for (int i = tid; i < DC_WS_TM / 4; i += DC_THREADS) dc_cp16(tm + 4 * i, src + DC_WS_KQ + 4 * i);
-        dc_commit();
+    float S[NT][4];                                          // channels ch and ch + 8, columns 2 t4 and 2 t4 + 1 of each group
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int d = ch + 8 * (e >> 1), c = col0 + 8 * n + 2 * t4 + (e & 1);
+            S[n][e] = d < dk && c < p.cols ? sbase[(size_t)d * dv + c] : 0.f;
+        }
+    auto load = [&](int chunk, DeltaOperands<NT>& o) {
+        const float* ws = ws0 + chunk * ws_step;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                o.kt[m][e] = *reinterpret_cast<const uint4*>(ws + DC_AT_KT + (warp * 2 + m) * DC_FRAG + e * 128 + lane * 4);
+                o.kd[m][e] = *reinterpret_cast<const uint4*>(ws + DC_AT_KD + (warp * 2 + m) * DC_FRAG + e * 128 + lane * 4);
+            }
+        o.decay[0] = ws[DC_AT_P + ch];
+        o.decay[1] = ws[DC_AT_P + ch + 8];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) o.tv[n] = ws[DC_AT_U + ti * DC_V + col0 + 8 * n + tc];
     };
-    auto load_last = [&](int chunk) {                       // ... and its third
-        const float* src = ws0 + chunk * ws_step + DC_WS_KQ + DC_WS_TM;
-        for (int i = tid; i < DC_WS_KD / 4; i += DC_THREADS) dc_cp16(KD + 4 * i, src + 4 * i);
-        dc_commit();
-    };
-    load_first(0);
-    load_last(0);
-    for (int i = tid; i < DC_K * DC_COLS; i += DC_THREADS) {
-        const int d = i / DC_COLS, c = i % DC_COLS;
-        Ss[c * DC_RP + d] = d < dk && col0 + c < dv ? sbase[(size_t)d * dv + col0 + c] : 0.f;
-    }
-    // a thread's token and column in the second phase; its value is asked for a chunk ahead
-    const int ti = tid >> 3, tc = tid & 7;
-    const bool col_in = col0 + tc < dv;
-    const float* vcol = p.qkv + (size_t)2 * p.kv_heads * dk + (size_t)head * dv + col0 + tc;
-    auto value_of = [&](int chunk) {
-        const int row = r0 + chunk * DC_C + ti;
-        return col_in && row < r1 ? vcol[(size_t)row * p.ldq] : 0.f;
-    };
-    float v_next = value_of(0);
-
-    for (int chunk = 0; chunk < chunks; ++chunk) {
-        const float* kq = KQ + (chunk & 1) * DC_WS_KQ, *tm = TM + (chunk & 1) * DC_WS_TM;
-        // [8 warps][64 rows][8 columns], later the second half of the update: where the chunk's K P and Q P were
-        float* red = KQ + (chunk & 1) * DC_WS_KQ;
-        dc_wait<1>();                                       // this chunk's first half (its last part may still be under way)
-        __syncthreads();                                    // ... for everyone; S is complete; the other buffers are free
-        if (chunk + 1 < chunks) load_first(chunk + 1);
-        else dc_commit();
-        const float v = v_next;
-        if (chunk + 1 < chunks) v_next = value_of(chunk + 1);
-
-        // (K P) S and (Q P) S: a warp takes 16 channels, a lane rows `lane` and `lane + 32` against all columns
+    auto step = [&](int chunk, const DeltaOperands<NT>& o) {
+        float* ws = ws0 + chunk * ws_step;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+            *reinterpret_cast<float4*>(ws + DC_AT_S + ((blockIdx.x * NT + n) * 8 + warp) * 128 + lane * 4) = make_float4(S[n][0], S[n][1], S[n][2], S[n][3]);
         {
-            dc_pair acc[2][DC_COLS];
+            uint32_t b[NT][3][2];
+            float hi[2][NT][4] = {}, lo[2][NT][2][4] = {};
 #pragma unroll
-            for (int c = 0; c < DC_COLS; ++c) acc[0][c] = acc[1][c] = 0ull;
+            for (int n = 0; n < NT; ++n) dc_right(S[n], b[n]);
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const int d = warp * 16 + 4 * s;
-                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(kq + lane * DC_RP + d);
-                const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(kq + (lane + 32) * DC_RP + d);
+            for (int k = 0; k < DC_PRODUCTS; ++k)
 #pragma unroll
-                for (int c = 0; c < DC_COLS; ++c) {
-                    const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(Ss + c * DC_RP + d);
-                    dc_fma(acc[0][c], x.x, sv.x);
-                    dc_fma(acc[1][c], y.x, sv.x);
-                    dc_fma(acc[0][c], x.y, sv.y);
-                    dc_fma(acc[1][c], y.y, sv.y);
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        if (k < DC_PRODUCTS - 1) dc_mma(lo[m][n][k & 1], o.kt[m][DC_A_TERM[k]], b[n][DC_B_TERM[k]][0], b[n][DC_B_TERM[k]][1]);
+                        else dc_mma_add(hi[m][n], o.kt[m][DC_A_TERM[k]], b[n][DC_B_TERM[k]][0], b[n][DC_B_TERM[k]][1]);
+                    }
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    float v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[e] = hi[m][n][e] + (lo[m][n][0][e] + lo[m][n][1][e]);
+                    *reinterpret_cast<float2*>(&red[n][warp][m * 16 + g][2 * t4]) = make_float2(v[0], v[1]);
+                    *reinterpret_cast<float2*>(&red[n][warp][m * 16 + g + 8][2 * t4]) = make_float2(v[2], v[3]);
                 }
-            }
-            __syncthreads();                                // everyone has read K P and Q P
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                // (the two 16-byte halves of a row change places by row, so that eight lanes hit 32 banks)
-                float* dst = red + (warp * 64 + lane + 32 * h) * DC_COLS;
-                const float4 lo = make_float4(dc_sum(acc[h][0]), dc_sum(acc[h][1]), dc_sum(acc[h][2]), dc_sum(acc[h][3]));
-                const float4 hi = make_float4(dc_sum(acc[h][4]), dc_sum(acc[h][5]), dc_sum(acc[h][6]), dc_sum(acc[h][7]));
-                const int flip = (lane >> 2) & 1;
-                reinterpret_cast<float4*>(dst)[flip] = lo;
-                reinterpret_cast<float4*>(dst)[flip ^ 1] = hi;
-            }
         }
         __syncthreads();
-        float qs = 0.f;
-        {
-            const int at = tc ^ (((ti >> 2) & 1) << 2);
-            float ks = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                ks += red[(w * 64 + ti) * DC_COLS + at];
-                qs += red[(w * 64 + 32 + ti) * DC_COLS + at];
-            }
-            Wt[tc * DC_TP + ti] = v - ks;
+        for (int n = 0; n < NT; ++n) {
+            float r[8];
+#pragma unroll
+            for (int w = 0; w < 8; ++w) r[w] = red[n][w][ti][tc];
+            const float u = o.tv[n] - (((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7])));
+            ws[DC_AT_U + ti * DC_V + col0 + 8 * n + tc] = u;
+            uint32_t term[3];
+            gb_split_bf16(u, 0.f, term);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) Ub[n][e][tc][ti] = (unsigned short)term[e];
         }
         __syncthreads();
-        // U = T W and O = (Q P) S + M W; a token never meets a later one's numbers, not even times zero
-        {
-            float u = 0.f, o = qs;
-            const float* trow = tm + ti * DC_TP, *mrow = tm + (DC_C + ti) * DC_TP, *wcol = Wt + tc * DC_TP;
-            const int last = (ti | 3);                      // the largest token of this warp
-            for (int j = 0; j <= last; j += 4) {
-                const float4 t4 = *reinterpret_cast<const float4*>(trow + j);
-                const float4 m4 = *reinterpret_cast<const float4*>(mrow + j);
-                const float4 w4 = *reinterpret_cast<const float4*>(wcol + j);
-                if (j <= ti) { u = fmaf(t4.x, w4.x, u); o = fmaf(m4.x, w4.x, o); }
-                if (j + 1 <= ti) { u = fmaf(t4.y, w4.y, u); o = fmaf(m4.y, w4.y, o); }
-                if (j + 2 <= ti) { u = fmaf(t4.z, w4.z, u); o = fmaf(m4.z, w4.z, o); }
-                if (j + 3 <= ti) { u = fmaf(t4.w, w4.w, u); o = fmaf(m4.w, w4.w, o); }
-            }
-            Ut[tc * DC_TP + ti] = u;
-            const int row = r0 + chunk * DC_C + ti;
-            if (row < r1 && col_in) p.out[(size_t)row * p.heads * dv + (size_t)head * dv + col0 + tc] = o;
-        }
-        dc_wait<1>();                                       // K D (the next chunk's first half may still be under way)
-        __syncthreads();
-        // S <- P S + (K D)^T U: warps 0 to 3 take tokens 0 to 15, the others 16 to 31; a warp 64 channels of four columns
-        {
-            const int half = warp >> 2, cg = (warp >> 1) & 1, d = (warp & 1) * 64 + 2 * lane;
-            dc_pair acc[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-                float u4[4][4];
+        for (int n = 0; n < NT; ++n) {
+            uint4 u[3];
+            float hi[2][4] = {}, lo[2][2][4] = {};
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<float4*>(u4[c]) = *reinterpret_cast<const float4*>(Ut + (cg * 4 + c) * DC_TP + half * 16 + j);
+            for (int e = 0; e < 3; ++e) u[e] = *reinterpret_cast<const uint4*>(&Ub[n][e][g][8 * t4]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const dc_pair k = *reinterpret_cast<const dc_pair*>(KD + (half * 16 + j + e) * DC_K + d);
+            for (int k = 0; k < DC_PRODUCTS; ++k)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) dc_fma(acc[c], k, dc_pack(u4[c][e], u4[c][e]));
+                for (int s = 0; s < 2; ++s) {
+                    const uint4& r = u[DC_B_TERM[k]];
+                    if (k < DC_PRODUCTS - 1) dc_mma(lo[s][k & 1], o.kd[s][DC_A_TERM[k]], s ? r.z : r.x, s ? r.w : r.y);
+                    else dc_mma_add(hi[s], o.kd[s][DC_A_TERM[k]], s ? r.z : r.x, s ? r.w : r.y);
                 }
-            }
-            dc_pair* other = reinterpret_cast<dc_pair*>(red);                  // [4 warps][4 columns][32 lanes]
-            if (half) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) other[((warp & 3) * 4 + c) * 32 + lane] = acc[c];
-            }
-            __syncthreads();
-            if (!half) {
-                const dc_pair decay = *reinterpret_cast<const dc_pair*>(KD + DC_C * DC_K + d);
-                const dc_pair one = dc_pack(1.f, 1.f);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    dc_pair* s = reinterpret_cast<dc_pair*>(Ss + (cg * 4 + c) * DC_RP + d);
-                    dc_fma(acc[c], decay, *s);
-                    dc_fma(acc[c], one, other[((warp & 3) * 4 + c) * 32 + lane]);
-                    *s = acc[c];
-                }
-            }
+            for (int e = 0; e < 4; ++e)
+                S[n][e] = fmaf(o.decay[e >> 1], S[n][e], (hi[0][e] + hi[1][e]) + ((lo[0][0][e] + lo[0][1][e]) + (lo[1][0][e] + lo[1][1][e])));
         }
-        __syncthreads();                                    // K D has been read: the next chunk's may come
-        if (chunk + 1 < chunks) load_last(chunk + 1);
-        else dc_commit();
+    };
+    DeltaOperands<NT> o[3];
+    load(0, o[0]);
+    if (chunks > 1) load(1, o[1]);
+    for (int chunk = 0; chunk < chunks; chunk += 3) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (chunk + i >= chunks) break;
+            if (chunk + i + 2 < chunks) load(chunk + i + 2, o[(i + 2) % 3]);
+            step(chunk + i, o[i]);
+        }
     }
     if (p.write_state) {
-        for (int i = tid; i < DC_K * DC_COLS; i += DC_THREADS) {
-            const int d = i / DC_COLS, c = i % DC_COLS;
-            if (d < dk && col0 + c < dv) sbase[(size_t)d * dv + col0 + c] = Ss[c * DC_RP + d];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int d = ch + 8 * (e >> 1), c = col0 + 8 * n + 2 * t4 + (e & 1);
+                if (d < dk && c < p.cols) sbase[(size_t)d * dv + c] = S[n][e];
+            }
+    }
+}
+
+// O = (Q P) S_0 + B U: a warp takes two groups of 8 columns.
+__global__ void __launch_bounds__(DC_THREADS, 2) delta_out_kernel(DeltaChunkArgs p) {
+    __shared__ uint4 left[20 * DC_FRAG / 4];                 // the left operands: Q P, then B
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    const int chunk = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
+    if (p.seq_start_pos[seq] < 0) return;
+    const int slot = p.seq_slots[seq];
+    if (slot < 0 || slot >= p.num_slots) return;
+    const int r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1], c0 = r0 + chunk * DC_C;
+    if (c0 >= r1) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const float* ws = p.ws + dc_slot(r0, seq, chunk, p.heads, head);
+    for (int i = threadIdx.x; i < 20 * DC_FRAG / 4; i += DC_THREADS) dc_cp16(left + i, ws + DC_AT_QP + 4 * i);      // Q P and B
+    asm volatile("cp.async.commit_group;");
+    // (a group of columns past this pass's last has a slot, which nothing wrote: its sums are not stored)
+    auto state = [&](int k16, float4 (&s)[2]) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) s[n] = *reinterpret_cast<const float4*>(ws + DC_AT_S + ((warp * 2 + n) * 8 + k16) * 128 + lane * 4);
+    };
+    float4 next[2][2];                                       // S_0, two groups of channels ahead
+    state(0, next[0]);
+    state(1, next[1]);
+    asm volatile("cp.async.wait_group 0;");
+    __syncthreads();
+    if (warp * 16 >= p.cols) return;
+    float hi[2][2][4] = {}, lo[2][2][4] = {};                // [16 tokens][8 columns]
+#pragma unroll
+    for (int k16 = 0; k16 < DC_K / 16; ++k16) {
+        uint4 a[2][3];
+        uint32_t b[2][3][2];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const float4 s4 = next[k16 & 1][n];
+            const float s[4] = {s4.x, s4.y, s4.z, s4.w};
+            dc_right(s, b[n]);
+        }
+        if (k16 + 2 < DC_K / 16) state(k16 + 2, next[k16 & 1]);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) a[m][e] = left[((k16 * 2 + m) * DC_FRAG + e * 128) / 4 + lane];
+#pragma unroll
+        for (int k = 0; k < DC_PRODUCTS; ++k)
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    if (k < DC_PRODUCTS - 1) dc_mma(lo[m][n], a[m][DC_A_TERM[k]], b[n][DC_B_TERM[k]][0], b[n][DC_B_TERM[k]][1]);
+                    else dc_mma_add(hi[m][n], a[m][DC_A_TERM[k]], b[n][DC_B_TERM[k]][0], b[n][DC_B_TERM[k]][1]);
+                }
+    }
+    // U's rows as the right operand. A token must not meet a later one's numbers, not even times zero: what is not finite is left out
+    // here and added below for the tokens that see it.
+    const float* U = ws + DC_AT_U + warp * 16 + g;
+    float u[2][2][4];
+    bool odd = false;
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int k16 = 0; k16 < 2; ++k16)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float v = U[(k16 * 16 + 2 * t4 + (e & 1) + 8 * (e >> 1)) * DC_V + 8 * n];
+                const bool finite = fabsf(v) <= FLT_MAX;
+                odd |= !finite;
+                u[n][k16][e] = finite ? v : 0.f;
+            }
+    const bool plain = __any_sync(0xffffffffu, odd);
+#pragma unroll
+    for (int k16 = 0; k16 < 2; ++k16) {
+        uint32_t b[2][2][3];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            gb_split_bf16(u[n][k16][0], u[n][k16][1], b[n][0]);
+            gb_split_bf16(u[n][k16][2], u[n][k16][3], b[n][1]);
+        }
+#pragma unroll
+        for (int m = k16; m < 2; ++m) {
+            uint4 a[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) a[e] = left[((16 + m * 2 + k16) * DC_FRAG + e * 128) / 4 + lane];
+#pragma unroll
+            for (int k = 0; k < DC_PRODUCTS; ++k)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    if (k < DC_PRODUCTS - 1) dc_mma(lo[m][n], a[DC_A_TERM[k]], b[n][0][DC_B_TERM[k]], b[n][1][DC_B_TERM[k]]);
+                    else dc_mma_add(hi[m][n], a[DC_A_TERM[k]], b[n][0][DC_B_TERM[k]], b[n][1][DC_B_TERM[k]]);
+                }
         }
     }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = m * 16 + g + 8 * (e >> 1), c = (warp * 2 + n) * 8 + 2 * t4 + (e & 1);
+                float o = hi[m][n][e] + lo[m][n][e];
+                if (plain) {
+                    const unsigned short* words = reinterpret_cast<const unsigned short*>(ws + DC_AT_B);
+                    for (int j = 0; j <= i; ++j) {
+                        const float v = ws[DC_AT_U + j * DC_V + c];
+                        if (fabsf(v) <= FLT_MAX) continue;
+                        const int lane_of = (i & 7) * 4 + ((j & 7) >> 1), word = ((i >> 3) & 1) + 2 * ((j >> 3) & 1);
+                        const int at = (((i >> 4) * 2 + (j >> 4)) * DC_FRAG + lane_of * 4 + word) * 2 + (j & 1);
+                        float bij = 0.f;
+                        for (int e3 = 2; e3 >= 0; --e3) bij += __uint_as_float((uint32_t)words[at + e3 * 256] << 16);
+                        o = fmaf(bij, v, o);
+                    }
+                }
+                if (c0 + i < r1 && c < p.cols) p.out[(size_t)(c0 + i) * p.heads * p.dv + (size_t)head * p.dv + p.col0 + c] = o;
+            }
 }
 
 GB_EXPORT int gb_delta_chunk_rows() { return DC_C; }
 GB_EXPORT int gb_delta_chunk_floats() { return DC_WS; }            // workspace of a (chunk, head)
 
-// As gb_channel_delta (delta_rule.cu) for key sizes up to 128, with a workspace of n / 32 + S chunks of heads *
+// As gb_channel_delta (delta_rule.cu) for key sizes up to 128 (value columns in passes of 128), with a workspace of n / 32 + S chunks of heads *
 // gb_delta_chunk_floats() numbers, 16-byte aligned. max_rows: the most rows that a request brings.
 GB_EXPORT int gb_channel_delta_chunks(const float* qkv, long long ldq, const float* beta, long long ldb, const float* a, long long lda,
                                       const float* dt_bias, const float* a_log, float* state, long long state_stride, float* out,
@@ -438,14 +598,26 @@ GB_EXPORT int gb_channel_delta_chunks(const float* qkv, long long ldq, const flo
     GB_REQUIRE((uintptr_t)ws % 16 == 0, "gb_channel_delta_chunks: the workspace must be 16-byte aligned");
     if (S == 0 || max_rows <= 0) return 0;
     DeltaChunkArgs p = {qkv, ldq, beta, ldb, a, lda, dt_bias, a_log, state, state_stride, out, seq_first_row, seq_start_pos, seq_slots,
-                        ws, heads, kv_heads, dk, dv, num_slots, write_state, decay_channels, status};
+                        ws, heads, kv_heads, dk, dv, num_slots, write_state, decay_channels, 0, 0, status};
     const int prepare_smem = 3 * DC_C * DC_RP * 4;
     cudaError_t e = cudaFuncSetAttribute(delta_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SCAN_SMEM);
-    GB_REQUIRE(e == cudaSuccess, "gb_channel_delta_chunks: %d bytes of shared memory refused: %s", DC_SCAN_SMEM, cudaGetErrorString(e));
-    gb_launch(GB_PDL_ATTENTION, delta_prepare_kernel, dim3(gb_ceil_div(max_rows, DC_C), heads, S), dim3(DC_THREADS), prepare_smem, stream, p);
-    int rc = gb_check_launch("gb_channel_delta_chunks (prepare)");
-    if (rc) return rc;
-    gb_launch(GB_PDL_ATTENTION, delta_scan_kernel, dim3(gb_ceil_div(dv, DC_COLS), heads, S), dim3(DC_THREADS), DC_SCAN_SMEM, stream, p);
-    return gb_check_launch("gb_channel_delta_chunks");
+    GB_REQUIRE(e == cudaSuccess, "gb_channel_delta_chunks: %d bytes of shared memory refused: %s", prepare_smem, cudaGetErrorString(e));
+    const dim3 every(gb_ceil_div(max_rows, DC_C), heads, S);
+    for (p.col0 = 0; p.col0 < dv; p.col0 += DC_V) {
+        p.cols = dv - p.col0 < DC_V ? dv - p.col0 : DC_V;
+        gb_launch(GB_PDL_ATTENTION, delta_prepare_kernel, every, dim3(DC_THREADS), prepare_smem, stream, p);
+        int rc = gb_check_launch("gb_channel_delta_chunks (prepare)");
+        if (rc) return rc;
+        const long long narrow = (long long)gb_ceil_div(p.cols, 8) * heads * S;
+        if (narrow <= 148)
+            gb_launch(GB_PDL_ATTENTION, delta_scan_kernel<1>, dim3(gb_ceil_div(p.cols, 8), heads, S), dim3(DC_THREADS), 0, stream, p);
+        else
+            gb_launch(GB_PDL_ATTENTION, delta_scan_kernel<2>, dim3(gb_ceil_div(p.cols, 16), heads, S), dim3(DC_THREADS), 0, stream, p);
+        rc = gb_check_launch("gb_channel_delta_chunks (scan)");
+        if (rc) return rc;
+        gb_launch(GB_PDL_ATTENTION, delta_out_kernel, every, dim3(DC_THREADS), 0, stream, p);
+        rc = gb_check_launch("gb_channel_delta_chunks (read-out)");
+        if (rc) return rc;
+    }
+    return 0;
 }

@@ -1521,17 +1521,17 @@ def channel_delta(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bia
 
 #: the delta rule runs in chunks of tokens instead of token by token from this many rows of a step on, and so many more for
 #: every request of the step
-DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 72, 7
+DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 88, 7
 
 
 def delta_chunks_chosen(rows: int, num_seqs: int, dk: int) -> bool:
     """Whether the delta rule takes a step of ``rows`` rows in ``num_seqs`` requests in chunks of 32 tokens (key sizes up to 128).
-    Both numbers are part of a recorded step's shape, which the longest portion is not. A request costs the chunks its state's way
-    through shared memory, a row costs the walk its place in the chain. Measured, kernels alone, heads of 128 x 128, walk /
-    chunks in us at 8 heads and at 16: one request of 48 rows 23 / 25 and 23 / 26, 64 rows 28 / 25 and 28 / 29, 96 rows 37 / 28; 8
-    requests of 64 rows in all 33 / 39 and 55 / 55, 128 rows 48 / 40 and 80 / 58; 36 requests (prompts' ends of up to 15 rows) of
-    192 rows 93 / 98 and 177 / 203, of 320 rows 119 / 99 and 227 / 210; 35 single tokens beside a portion of 100 rows 106 / 121 and 179
-    / 227, of 300 rows 174 / 141 and 278 / 263; 64 requests of 320 rows 156 / 181 and 302 / 395, of 1,024 rows 282 / 203 and 564 / 411."""
+    Both numbers are part of a recorded step's shape, which the longest portion is not. A request costs the chunks its state's way in and
+    out, a row costs the walk its place in the chain. Measured, kernels alone, heads of 128 x 128, walk / chunks in us at 8 heads and at
+    16: one request of 64 rows 27 / 35 and 27 / 37, 96 rows 36 / 37 and 37 / 34, 200 rows 68 / 36 and 69 / 44; 8 requests of 64 rows in
+    all 27 / 38 and 48 / 52, 128 rows 42 / 38 and 74 / 52; 36 requests (prompts' ends) of 180 rows 85 / 79 and 166 / 159, of 324 rows 118
+    / 79 and 231 / 160; 35 single tokens beside a portion of 30 rows 76 / 78 and 138 / 160, of 100 rows 105 / 102 and 177 / 183, of 300
+    rows 173 / 118 and 276 / 206; 64 requests of 320 rows 149 / 149 and 294 / 290, of 1,024 rows 290 / 151 and 585 / 293."""
     return dk <= 128 and rows >= DELTA_CHUNKS_FROM + DELTA_CHUNKS_PER_REQUEST * num_seqs
 
 

@@ -129,3 +129,12 @@ def test_recorded_prompt_shapes_share_one_workspace(tmp_path_factory):
     own = [name for g in eng._graphs.values() for (name, _) in g["ctx"]._grow._bufs if "delta_chunks" in name]
     heads = {L["mixer"]["heads"] for L in cfg["layers"] if L["type"] == "channel_delta"}
     assert len(shared) == len(heads) and not own
+
+
+@pytest.mark.parametrize("H, KH, D, V, lens", [(20, 4, 36, 128, [33, 64]), (19, 19, 128, 70, [40]), (2, 1, 64, 128 + 9, [65, 3])])
+def test_chunks_of_sixteen_columns_and_of_more_than_a_pass(H, KH, D, V, lens):
+    """More blocks of eight columns than multiprocessors (a block then takes sixteen), the last of them past the values' end, and value
+    sizes of more than one pass."""
+    data = _inputs(lens, H, KH, D, V, False, H)
+    for g, w in zip(_run(True, lens, H, KH, D, V, False, *data), _truth(lens, H, KH, D, V, False, *data)):
+        np.testing.assert_allclose(g, w, atol=1e-5 * max(1.0, np.abs(w).max()), rtol=1e-5)       # (the bound of the test above)
