@@ -44,6 +44,8 @@ _SIGNATURES = {
     "gb_rope_kv_write": [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _LL, _I, _P, _P],
     "gb_swiglu": [_P, _P, _I, _I, _I, _P],
     "gb_copy_pages": [_P, _P, _P, _I, _LL, _LL, _LL, _LL, _I, _P],
+    "gb_gemm_f32_tc_supported": [_P, _P, _I, _I, _LL, _LL],
+    "gb_gemm_f32_tc": [_P, _P, _I, _P, _I, _I, _I, _I, _LL, _LL, _LL, _P, _P],
     "gb_gemm_simt": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _LL, _LL, _LL, _P],
     "gb_attention_rows": [_P, _LL, _P, _LL, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P],
     "gb_sample": [_P, _LL, _P, _P, _P, _P, _I, _P, _P, _I, _I, _P],
@@ -467,6 +469,37 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, accumulate: boo
     assert a.stride(1) == 1 and w.stride(1) == 1 and c.stride(1) == 1
     _call("gb_gemm_simt", _ptr(a), _dt(a), _ptr(w), _dt(w), _ptr(c), _dt(c), 1 if accumulate else 0, M, N, K,
           a.stride(0), w.stride(0), c.stride(0), _stream())
+
+
+#: the product of float32 rows runs on the tensor cores above so many rows (a handful streams the weights) and from this K on (a shorter
+#: sum is more exact by FMA)
+F32_TC_ABOVE_ROWS, F32_TC_MIN_K = 8, 64
+
+
+def gemm_f32_tc_chosen(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> bool:
+    """Whether the product of float32 rows on the tensor cores takes these operands: float32 activations and output, float32 or bfloat16
+    weights, rows of whole 16-byte pieces, by the rule above. (Not by more: what a row becomes must not depend on the rows beside it.)"""
+    if a.dtype != torch.float32 or c.dtype != torch.float32 or w.dtype not in (torch.float32, torch.bfloat16):
+        return False
+    if a.shape[0] <= F32_TC_ABOVE_ROWS or a.shape[1] < F32_TC_MIN_K:
+        return False
+    return bool(lib().gb_gemm_f32_tc_supported(_ptr(a), _ptr(w), w.shape[0], a.shape[1], a.stride(0), w.stride(0)))
+
+
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, accumulate: bool = False, status: Optional[torch.Tensor] = None) -> None:
+    """c[M, N] (+)= a[M, K] @ w[N, K]^T of float32 rows with the exactness of float32 sums, on the tensor cores (csrc/gemm_f32_tc.cu).
+    ``status`` receives the wait-timeout bit if a bounded wait inside the kernel ever gives up."""
+    _cuda(a, w, c, status)
+    M, K = a.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and c.shape == (M, N) and a.dtype == c.dtype == torch.float32
+    assert a.stride(1) == 1 and w.stride(1) == 1 and c.stride(1) == 1
+    if status is None:
+        status = _tc_status.get(a.device)
+        if status is None:
+            status = _tc_status[a.device] = torch.zeros(1, dtype=torch.int32, device=a.device)
+    _call("gb_gemm_f32_tc", _ptr(a), _ptr(w), _dt(w), _ptr(c), 1 if accumulate else 0, M, N, K, a.stride(0), w.stride(0), c.stride(0),
+          _ptr(status), _stream())
 
 
 STREAM_MAX_ROWS = 64

@@ -120,6 +120,8 @@ def linear(ctx, a, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False)
             ctx.prepared_norm = PreparedNorm(next_norm, out, pre, kernels.RowScale(ss, eps))
         else:
             kernels.gemm_tc(x, w, out, accumulate, ctx.status)
+    elif kernels.gemm_f32_tc_chosen(x, w, out):
+        kernels.gemm_f32_tc(x, w, out, accumulate, ctx.status)
     else:
         kernels.gemm_simt(x, w, out, accumulate)
 
