@@ -1,20 +1,19 @@
-// Causal grouped-query flash attention for prompt portions in the true 32-bit path, over the paged cache: float32 operands,
-// FMA only, online softmax in float32.
+// Causal grouped-query flash attention for prompt portions in the true 32-bit path at head sizes 96 and 128, over the paged cache: float32
+// operands, FMA only, online softmax in float32. (Smaller heads: attention_prefill_f32_mma.cu.)
 //
 // Bound by the FMA pipe: 4 * head_dim operations per visible (query, key) pair against 8 * head_dim bytes per key that 64
 // rows share. A block is 64 consecutive query rows of one request for one query head, four warps; a thread holds an 8 x 4
 // piece of the 64 x 64 scores and an 8 x (head_dim / 16) piece of the output. Scores pair neighbouring channels in one packed
 // FMA (query and key rows lie as they come, so a 16-byte load is two operands); the product with the values pairs two
 // query rows (the weights are kept with the rows of a key side by side). Keys arrive a tile ahead through cp.async, the values
-// of a tile while its scores are formed; the weights take the place of the tile's keys, so that three blocks (head size 64:
-// 69 KB, 168 registers) share an SM. One warp per (row, head), which this replaces for prompt portions, walked its keys alone
+// of a tile while its scores are formed; the weights take the place of the tile's keys. One warp per (row, head), which this replaces for prompt portions, walked its keys alone
 // and read every key and value row once per query row.
-// Measured, three prompts of 2,047 rows in all, 9/3 heads of 64: 2,543 -> 176 us (a third of the FMA rate: the longest prompt's
-// last blocks walk their tiles alone).
+// Measured, one prompt of 1,000 rows, 8/2 heads of 128: 172 us.
 //
 // Key tiles start at multiples of 64 and a row's masked keys add nothing, so the order of a row's sums depends on its
 // position and window alone, not on the batch, on how its prompt was cut, or on which pages hold the keys.
 #include "common.cuh"
+#include "attention_prefill_f32.h"
 
 #include <float.h>
 
@@ -61,7 +60,7 @@ template <int HD> struct PsCols {
 template <int HD> constexpr int ps_smem() { return (PS_BM * (HD + 4) + 2 * PS_BN * (HD + 4 > PS_BM + 4 ? HD + 4 : PS_BM + 4) + PS_BN * HD) * 4; }
 
 template <int HD>
-__global__ void __launch_bounds__(PS_THREADS, HD <= 64 ? 3 : 1) attention_prefill_f32_kernel(
+__global__ void __launch_bounds__(PS_THREADS, 1) attention_prefill_f32_kernel(
     const float* __restrict__ q, long long q_stride, float* __restrict__ out, long long out_stride, const float* __restrict__ kcache,
     const float* __restrict__ vcache, const int* __restrict__ block_tables, int max_pages, const int* __restrict__ seq_first_row,
     const int* __restrict__ seq_start_pos, int nh, int nkv, int page_size, long long num_pages, float scale, int window,
@@ -338,7 +337,14 @@ GB_EXPORT int gb_attention_prefill_f32(const void* q, long long q_stride, void* 
         return launch_prefill_f32<HD_>((const float*)q, q_stride, (float*)out, out_stride, (const float*)kcache, (const float*)vcache, \
                                        block_tables, max_pages, seq_first_row, seq_start_pos, num_seqs, max_rows_per_seq, nh, nkv, page_size, \
                                        num_pages, scale, window, status, stream);
-    GB_CASE(16) GB_CASE(32) GB_CASE(64) GB_CASE(96) GB_CASE(128)
+    GB_CASE(96) GB_CASE(128)
+#undef GB_CASE
+#define GB_CASE(HD_)                                                                                                               \
+    if (hd == HD_)                                                                                                                 \
+        return gb_launch_prefill_f32_mma<HD_>((const float*)q, q_stride, (float*)out, out_stride, (const float*)kcache, (const float*)vcache, \
+                                              block_tables, max_pages, seq_first_row, seq_start_pos, num_seqs, max_rows_per_seq, nh, nkv, \
+                                              page_size, num_pages, scale, window, status, stream);
+    GB_CASE(16) GB_CASE(32) GB_CASE(64)
 #undef GB_CASE
     return 1;
 }

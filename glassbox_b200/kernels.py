@@ -1023,7 +1023,7 @@ def attention_prefill_f32(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tens
                           block_tables: torch.Tensor, seq_first_row: torch.Tensor, seq_start_pos: torch.Tensor,
                           max_rows_per_seq: int, nh: int, nkv: int, hd: int, page_size: int, scale: float,
                           window: Optional[int], status: torch.Tensor) -> None:
-    """float32 flash attention (FMA only) for batches whose requests bring runs of consecutive rows; arguments as
+    """float32 flash attention for batches whose requests bring runs of consecutive rows; arguments as
     ``attention_prefill``."""
     _cuda(q, out, kcache, vcache, block_tables, seq_first_row, seq_start_pos, status)
     assert q.dtype == out.dtype == kcache.dtype == vcache.dtype == torch.float32 and q.stride(1) == 1 and out.stride(1) == 1

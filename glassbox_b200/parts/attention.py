@@ -186,7 +186,7 @@ class GqaAttention(Mixer):
 SPLIT_MIXED_ABOVE = 148
 
 #: up to this many tokens a request (cached and new) the one-warp kernel walks its few keys in less time than a 64 x 64 tile takes in
-#: float32: 32 prompts of 8 tokens at 32 heads 20 us against 30, at 9 heads 9 against 11; of 16 tokens 52 against 32 and 19 against 12
+#: float32: 32 prompts of 8 tokens at 32 heads 20 us against 30, at 9 heads 9 against 11; of 16 tokens 52 against 24 and 19 against 12
 FLASH_F32_MIN_CONTEXT = 8
 
 register_part("mixer", "gqa_attention", GqaAttention, replace=True)

@@ -1,0 +1,78 @@
+"""float32 prompt attention on the tensor cores: what a row does not see stays away from it whatever it holds, what it sees counts as in
+float32, and both forms of the kernel give the same bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _run(q, k, v, tables, first, start, rows, window=None):
+    from glassbox_b200 import kernels
+    nkv, ps, hd = k.shape[1:]
+    out, status = torch.full_like(q, 7.0), torch.zeros(1, dtype=torch.int32, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    kernels.attention_prefill_f32(q, out, k, v, i32(tables), i32(first), i32(start), rows, q.shape[1] // hd, nkv, hd, ps, hd ** -0.5, window, status)
+    assert int(status) == 0
+    return out
+
+
+def _truth(q, keys, values, start, window=None):
+    """One head: q [rows, hd], keys and values [context, hd]; what a row does not see is left out of its sums."""
+    rows = []
+    for r in range(q.shape[0]):
+        lo, hi = max(0, start + r + 1 - window) if window else 0, start + r + 1
+        s = (q[r].double() * q.shape[1] ** -0.5) @ keys[lo:hi].double().T
+        rows.append(torch.softmax(s, 0) @ values[lo:hi].double())
+    return torch.stack(rows)
+
+
+def _pool(n, hd, seed):
+    g = torch.Generator().manual_seed(seed)
+    pages = -(-n // 16)
+    return tuple(torch.randn(pages, 1, 16, hd, generator=g).to(DEV) for _ in range(2)) + (torch.randn(n, hd, generator=g).to(DEV),)
+
+
+@pytest.mark.parametrize("hd", [16, 32, 64])
+@pytest.mark.parametrize("n, start, window", [(1, 0, None), (64, 0, None), (65, 0, 33), (130, 63, None), (257, 127, 100)])
+def test_against_float64(hd, n, start, window):
+    k, v, _ = _pool(start + n, hd, n)
+    q = torch.randn(n, hd, generator=torch.Generator().manual_seed(hd)).to(DEV)
+    got = _run(q, k, v, [list(range(k.shape[0]))], [0, n], [start], n, window)
+    want = _truth(q, k.reshape(-1, hd), v.reshape(-1, hd), start, window)
+    # scores to some 1e-6 and sums of weights and values to 2^-24 times a few: 1e-5 is several of each
+    assert (got.double() - want).abs().max() <= 1e-5
+
+
+def test_numbers_that_are_none_reach_the_rows_that_see_them():
+    n, hd = 150, 64
+    k, v, q = _pool(n, hd, 2)
+    clean = _run(q, k, v, [list(range(k.shape[0]))], [0, n], [0], n)
+    k2, v2 = k.clone(), v.clone()
+    flat_k, flat_v = k2.view(-1, hd), v2.view(-1, hd)
+    flat_v[70, 3], flat_v[101, 9] = float("inf"), float("nan")
+    flat_k[40], q2 = 0.0, q.clone()
+    flat_k[40, 0] = float("-inf")
+    q2[:, 0] = q[:, 0].abs() + 0.1                          # key 40 scores minus infinity with every row: it weighs nothing
+    got = _run(q2, k2, v2, [list(range(k.shape[0]))], [0, n], [0], n)
+    assert torch.isinf(got[70:, 3]).all() and torch.isnan(got[101:, 9]).all()
+    others = [c for c in range(hd) if c not in (3, 9)]
+    for r in (39, 41, 69, 70, 149):
+        rows = [i for i in range(r + 1) if i != 40]
+        s = (q2[r].double() * hd ** -0.5) @ flat_k[rows].double().T
+        want = torch.softmax(s, 0) @ flat_v[rows].double()
+        assert (got[r, others].double() - want[others]).abs().max() <= 1e-5, r
+    assert torch.equal(_run(q, k2, v, [list(range(k.shape[0]))], [0, n], [0], n)[:40], clean[:40])
+    assert torch.equal(_run(q, k, v2, [list(range(k.shape[0]))], [0, n], [0], n)[:70], clean[:70])
+
+
+@pytest.mark.parametrize("start, n, window", [(0, 20, None), (10, 30, None), (300, 64, None), (301, 50, 90)])
+def test_a_request_among_many_gives_the_same_bits(start, n, window):
+    """Many short portions take a form of one group of warps per block, which walks what four groups share: the bits of a lone request."""
+    hd, seqs = 64, 150
+    k, v, _ = _pool(start + n, hd, 3)
+    q = torch.randn(n, hd, generator=torch.Generator().manual_seed(n)).to(DEV)
+    table = list(range(k.shape[0]))
+    one = _run(q, k, v, [table], [0, n], [start], n, window)
+    many = _run(q.repeat(seqs, 1), k, v, [table] * seqs, [n * i for i in range(seqs + 1)], [start] * seqs, n, window)
+    assert torch.equal(many.view(seqs, n, hd), one.expand(seqs, n, hd))
