@@ -293,6 +293,112 @@ __global__ void __launch_bounds__(RB > 1 ? MOE_ROUTE_THREADS / 2 : MOE_ROUTE_THR
     }
 }
 
+// The logits of many bfloat16 rows on the tensor cores (mma.sync): 16 rows a block, the K of their products dealt out to 16 warps in pieces
+// of 32, sums over the warps in shared memory, then a warp per row chooses. A router weight is the exact sum of three bfloat16 numbers; the
+// largest product of 16 channels has an accumulator of its own and is added in float32 (the tensor core cuts what it adds to).
+// Operands come straight from memory in 16-byte loads: a lane's eight neighbouring channels stand for the fragment's pairs, the same way
+// on both sides. The FMA form brings every row through shared memory as float32 for every two experts: bound by those reads.
+// Measured, 16 experts, width 1,024, FMA / this, us: 300 rows 14.0 / 7.7, 2,048 rows 15.4 / 7.9;
+// width 2,048 17.4 / 9.2 and 19.5 / 9.5; 128 experts 36 / 27 and 72 / 27.
+constexpr int MR_ROWS = 16, MR_WARPS = 16, MR_COLS = 32, MR_EMAX = 128;
+struct MrShared {
+    float part[MR_WARPS][MR_ROWS][MR_COLS + 1];
+    float score[MR_ROWS][MR_EMAX], choice[MR_ROWS][MR_EMAX], run_score[MR_ROWS][MR_EMAX];
+    unsigned char kept[MR_ROWS][MR_EMAX];
+};
+
+__device__ __forceinline__ void mr_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__global__ void __launch_bounds__(MR_WARPS * 32) moe_route_mma_kernel(
+    const __nv_bfloat16* __restrict__ h, int d, const float* __restrict__ w_router, const float* __restrict__ correction,
+    const float* __restrict__ w_gate, const int* __restrict__ positions, int n, int E, int top, int groups, int keep, float route_scale,
+    int* __restrict__ choice_out, float* __restrict__ weight_out, float* __restrict__ gate_out, const float* __restrict__ router_bias,
+    int scoring, int run_best, float renorm_eps) {
+    extern __shared__ __align__(16) unsigned char mr_mem[];
+    MrShared& sh = *reinterpret_cast<MrShared*>(mr_mem);
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    const int row0 = blockIdx.x * MR_ROWS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int cols = E + (w_gate ? 1 : 0);
+    auto column = [&](int e) { return e < E ? w_router + (size_t)e * d : e < cols ? w_gate : nullptr; };
+    for (int e0 = 0; e0 < cols; e0 += MR_COLS) {
+        float hi[MR_COLS / 8][4] = {}, lo[MR_COLS / 8][4] = {};
+        for (int k = warp * 32 + 8 * t4; k - 8 * t4 < d; k += MR_WARPS * 32) {
+            const uint4 none = make_uint4(0, 0, 0, 0);
+            const bool in = k < d;
+            const uint4 x0 = in && row0 + g < n ? *reinterpret_cast<const uint4*>(h + (size_t)(row0 + g) * d + k) : none;
+            const uint4 x1 = in && row0 + g + 8 < n ? *reinterpret_cast<const uint4*>(h + (size_t)(row0 + g + 8) * d + k) : none;
+            float4 w[MR_COLS / 8][2];
+#pragma unroll
+            for (int c = 0; c < MR_COLS / 8; ++c) {
+                const float* src = column(e0 + 8 * c + g);
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+                    w[c][s] = in && src ? *reinterpret_cast<const float4*>(src + k + 4 * s) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int c = 0; c < MR_COLS / 8; ++c) {
+                if (e0 + 8 * c >= cols) break;                          // (uniform for the block)
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    uint32_t b0[3], b1[3];
+                    gb_split_bf16(w[c][s].x, w[c][s].y, b0);
+                    gb_split_bf16(w[c][s].z, w[c][s].w, b1);
+                    const uint32_t a0 = s ? x0.z : x0.x, a1 = s ? x1.z : x1.x, a2 = s ? x0.w : x0.y, a3 = s ? x1.w : x1.y;
+                    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+                    mr_mma(lo[c], a0, a1, a2, a3, b0[2], b1[2]);
+                    mr_mma(lo[c], a0, a1, a2, a3, b0[1], b1[1]);
+                    mr_mma(sum, a0, a1, a2, a3, b0[0], b1[0]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) hi[c][i] += sum[i];
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < MR_COLS / 8; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sh.part[warp][g + 8 * (i >> 1)][8 * c + 2 * t4 + (i & 1)] = hi[c][i] + lo[c][i];
+        __syncthreads();
+        {
+            const int r = threadIdx.x / MR_COLS, e = e0 + threadIdx.x % MR_COLS, row = row0 + r;
+            if (e < cols && row < n && positions[row] >= 0) {
+                float z = 0.f;
+#pragma unroll
+                for (int i = 0; i < MR_WARPS; ++i) z += sh.part[i][r][e - e0];
+                if (!(fabsf(z) <= FLT_MAX)) {                           // (an infinite operand's lesser terms are no numbers)
+                    const float* src = column(e);
+                    z = 0.f;
+                    for (int k = 0; k < d; ++k) z = fmaf(__bfloat162float(h[(size_t)row * d + k]), src[k], z);
+                }
+                const float sg = moe_sigmoid(z);
+                if (e == E) gate_out[row] = sg;
+                else if (scoring != MOE_SIGMOID) sh.score[r][e] = sh.choice[r][e] = z + (router_bias ? router_bias[e] : 0.f);
+                else {
+                    sh.score[r][e] = sg;
+                    sh.choice[r][e] = sg + (correction ? correction[e] : 0.f);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    const int r = warp, row = row0 + r;
+    if (row >= n || positions[row] < 0) return;
+    if (scoring == MOE_SOFTMAX) {                                       // the row's logits become its softmax over all experts
+        float m = -INFINITY, sum = 0.f;
+        for (int e = lane; e < E; e += 32) m = fmaxf(m, sh.score[r][e]);
+        m = gb_warp_max(m);
+        for (int e = lane; e < E; e += 32) sum += expf(sh.score[r][e] - m);
+        sum = gb_warp_sum(sum);
+        for (int e = lane; e < E; e += 32) sh.score[r][e] = sh.choice[r][e] = expf(sh.score[r][e] - m) / sum;
+        __syncwarp();
+    }
+    moe_choose(sh.score[r], sh.choice[r], sh.run_score[r], sh.kept[r], E, top, groups, keep, scoring == MOE_SOFTMAX_CHOSEN ? 1.0f : route_scale,
+               choice_out + (size_t)row * top, weight_out + (size_t)row * top, lane, scoring, run_best, renorm_eps);
+}
+
 template <typename T, int RB, int EMAX>
 static void moe_route_launch(const void* h, int d, const float* w_router, const float* correction, const float* w_gate,
                              const int* positions, int n, int E, int top, int groups, int keep, float route_scale, int* choice_out,
@@ -323,6 +429,16 @@ GB_EXPORT int gb_moe_route(const void* h, int h_dtype, int d, const float* w_rou
     GB_REQUIRE(w_gate == nullptr || gate_out != nullptr, "gb_moe_route: a gate needs its output");
     GB_REQUIRE(h_dtype == GB_F32 || h_dtype == GB_BF16, "gb_moe_route: unsupported dtype %d", h_dtype);
     if (n == 0) return 0;
+    // From the rows on for which the FMA form takes eight rows a block: 256 rows, a row a block, 16 experts 5.7 us against 7.7, 128 experts
+    // 24 against 27.
+    if (h_dtype == GB_BF16 && n > 256 && E <= MR_EMAX && d % 8 == 0 && (((uintptr_t)h | (uintptr_t)w_router | (uintptr_t)w_gate) & 15) == 0) {
+        cudaError_t e = cudaFuncSetAttribute(moe_route_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MrShared));
+        GB_REQUIRE(e == cudaSuccess, "gb_moe_route: %d bytes of shared memory refused: %s", (int)sizeof(MrShared), cudaGetErrorString(e));
+        gb_launch(GB_PDL_ELEMENTWISE, moe_route_mma_kernel, dim3(gb_ceil_div(n, MR_ROWS)), dim3(MR_WARPS * 32), sizeof(MrShared), stream,
+                  (const __nv_bfloat16*)h, d, w_router, correction, w_gate, positions, n, E, top, groups, keep, route_scale, choice_out, weight_out,
+                  gate_out, router_bias, scoring, run_best, renorm_eps);
+        return gb_check_launch("gb_moe_route");
+    }
     // eight rows per block when there are many rows, the experts are few enough for the block's arrays and eight rows fit
     const bool many = n > 256 && E <= 128 && (size_t)8 * ((d + 3) & ~3) * 4 <= 160 * 1024;      // (below: too few blocks to fill the GPU)
 #define MOE_ROUTE_GO(T)                                                                                                              \
