@@ -1,11 +1,12 @@
 // Causal grouped-query flash attention for prompt portions in the true 32-bit path at head sizes up to 64, over the paged cache: both
 // products on the tensor cores (mma.sync) with the exactness of float32 sums, online softmax in float32.
 //
-// Every float32 operand (queries, keys, weights, values) is the exact sum of three bfloat16 numbers, of whose nine products six stay
-// (what is left out lies below 2^-24 of a product). The largest product of 16 channels or keys gets an accumulator of its own and is
-// added in float32, since the tensor core cuts what it adds to; the five small ones share one per 32 keys.
-// Measured against 64 bits, normal operands (2-norm of the error over that of the result), this / sums by FMA: three prompts of 2,047 rows
-// in all 1.5e-7 / 2.5e-7, 1,200 rows behind 500 2.0e-7 / 6.0e-7, prompts of 20 tokens 9.0e-8 / 1.1e-7.
+// Every float32 operand (queries, keys, weights, values) is the exact sum of three bfloat16 numbers, each what is left rounded to the
+// nearest (Henry, Tang and Heinecke 2019), of whose nine products six stay: what is left out lies below 2^-24 of a product and has either
+// sign. The largest product of 16 channels or keys gets an accumulator of its own and is added in float32, since the tensor core cuts what
+// it adds to; the five small ones share one per 32 keys.
+// Measured against 64 bits (2-norm of the error over that of the result), this / sums by FMA: normal operands, prompts of 2 tokens 3.6e-8 /
+// 4.3e-8, of 8 5.9e-8 / 8.3e-8, of 64 8.9e-8 / 1.4e-7, with queries eight times as long 2.1e-7 / 3.5e-7, 500 tokens of these 3.4e-7 / 5.5e-7.
 //
 // A block is 64 consecutive query rows of one request for one query head: four groups of four warps, each with every fourth tile of 32
 // keys (a way), which merge at the end; a warp has 16 rows. A group's tile arrives a turn ahead through cp.async as float32, each piece
@@ -46,6 +47,7 @@ __device__ __forceinline__ void pm_cp16(void* smem, const void* gmem, bool valid
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ bool pm_finite(float v) { return fabsf(v) <= FLT_MAX; }
+__device__ __forceinline__ bool pm_splits(float v) { return fabsf(v) < __uint_as_float(0x7f7f8000u); }    // (gb_split_bf16: all terms are numbers)
 
 // c (tiles of 8 columns) = left (16 rows, K16 groups of 16) x right: the sums over the groups. left(group, term), right(group, pair of
 // tiles, term): fragments.
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(PM_GROUP * GROUPS, GROUPS == 1 ? 3 : 1) attent
     extern __shared__ __align__(128) unsigned char pm_mem[];
     __shared__ long long off_s[GROUPS][4][PM_BN];           // where a tile's keys lie in the pool (elements), -1: nowhere
     __shared__ unsigned there_s[GROUPS][4];                 // ... which are there, as bits
-    __shared__ int odd_s[GROUPS][4];                        // ... and whether a value of theirs is no finite number
+    __shared__ int odd_s[GROUPS][4];                        // ... and whether the split does not take a value of theirs
 
     const int tid = threadIdx.x % PM_GROUP, group = threadIdx.x / PM_GROUP, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int qt = gridDim.z - 1 - blockIdx.z;              // later rows see more keys: the longest blocks start first
@@ -264,9 +266,9 @@ __global__ void __launch_bounds__(PM_GROUP * GROUPS, GROUPS == 1 ? 3 : 1) attent
 #pragma unroll 2
         for (int i = 0; i < LOADS; ++i) {
             store(Ks, TERM, lkey + i * KSTEP, *reinterpret_cast<const float4*>(raw_k + raw_of(i)));
-            // (values without what is no finite number)
+            // (values without what the split does not take)
             float4 v = *reinterpret_cast<const float4*>(raw_v + raw_of(i));
-            const bool fx = pm_finite(v.x), fy = pm_finite(v.y), fz = pm_finite(v.z), fw = pm_finite(v.w);
+            const bool fx = pm_splits(v.x), fy = pm_splits(v.y), fz = pm_splits(v.z), fw = pm_splits(v.w);
             odd_v |= !(fx && fy && fz && fw);
             store(Vs, TERM, lkey + i * KSTEP, make_float4(fx ? v.x : 0.f, fy ? v.y : 0.f, fz ? v.z : 0.f, fw ? v.w : 0.f));
         }
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(PM_GROUP * GROUPS, GROUPS == 1 ? 3 : 1) attent
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
                                 const float v = vrow[8 * n + 2 * t4 + (e & 1)];
-                                if (!pm_finite(v) && key0 + kk <= last[e >> 1] && key0 + kk >= first[e >> 1]) o[n][e] = fmaf(w[e >> 1], v, o[n][e]);
+                                if (!pm_splits(v) && key0 + kk <= last[e >> 1] && key0 + kk >= first[e >> 1]) o[n][e] = fmaf(w[e >> 1], v, o[n][e]);
                             }
                     }
                 __syncwarp();

@@ -126,14 +126,19 @@ __device__ __forceinline__ float gb_gated_unit(float gate, float up, float limit
     return slope < 0.f ? gb_gelu_tanh(gate) * up : gate / (1.0f + expf(-gate)) * up;
 }
 
-// x and y as three bfloat16 each, by truncation (8 + 8 + 8 bits: the terms' sum is the number), packed with x in the low halves.
+// x and y as three bfloat16 each, every term what is left rounded to the nearest (8 + 8 + at most 8 bits: the terms' sum is the number, and
+// a term is below 2^-8 of the one before), packed with x in the low halves. A number that rounds to an infinity (from 2^128 - 2^119 on)
+// leaves a term that is no number, unless CLAMPED: its first term is then the largest bfloat16, and only infinities do.
+template <bool CLAMPED = false>
 __device__ __forceinline__ void gb_split_bf16(float x, float y, uint32_t (&term)[3]) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
-        term[i] = __byte_perm(xb, yb, 0x7632);
-        x -= __uint_as_float(xb & 0xffff0000u);
-        y -= __uint_as_float(yb & 0xffff0000u);
+        const float most = __uint_as_float(0x7f7f7fffu);                 // (the largest float32 that rounds to a finite bfloat16)
+        const bool clamp = CLAMPED && i == 0;
+        const __nv_bfloat162 t = __floats2bfloat162_rn(clamp ? fminf(fmaxf(x, -most), most) : x, clamp ? fminf(fmaxf(y, -most), most) : y);
+        term[i] = *reinterpret_cast<const uint32_t*>(&t);
+        x -= __uint_as_float(term[i] << 16);
+        y -= __uint_as_float(term[i] & 0xffff0000u);
     }
 }
 

@@ -17,10 +17,11 @@
 //   delta_out_kernel      every (chunk, head) side by side: O from the chunk's S_0 and U
 //
 // Everything is float32. The products run on the tensor cores with every float32 operand as three bfloat16 numbers whose sum it is
-// exactly (8 + 8 + 8 bits, by truncation) and six products of them, the largest in an accumulator of its own: what is left out is below
-// 2^-24 of a product. Measured against 64 bits, random inputs with decays from next to none to a channel forgotten at once (2-norm of
-// the error over that of the result, read-out / state): one request of 700 tokens 8.0e-7 / 9.1e-7, 2,048 tokens 1.7e-7 / 1.3e-7; with
-// sums by FMA and the hardware's exponentials for the decays 1.25e-6 / 1.33e-6 and 1.65e-6 / 1.52e-6.
+// exactly, each what is left rounded to the nearest (Henry, Tang and Heinecke 2019), and six products of them, the largest in an
+// accumulator of its own: what is left out is below 2^-24 of a product and has either sign. Measured against 64 bits, random inputs
+// (2-norm of the error over that of the result, read-out / state), 160 and 700 tokens of one request: 1.3e-7 / 1.2e-7 and 1.4e-7 /
+// 1.2e-7; by the walk 2.4e-7 / 2.0e-7 and 2.6e-7 / 2.3e-7; nothing written and a state of one number a head 7.0e-7 / 1.2e-6 and 2.8e-6 /
+// 4.8e-6, by the walk 1.1e-6 / 1.8e-6 and 4.2e-6 / 7.2e-6 (the decays' product).
 // What bounds the scan: a chain of 1,350 cycles a chunk (two products, two barriers and a sum over the warps) and a chunk's two operands
 // for a block, 48 KB from L2 (with all operands in L1 45 us of the 68). A warp owns 16 channels of S: S never leaves its registers
 // (movmatrix turns the accumulators into the next product's operand); the sums over the channels meet in shared memory. Operands come
@@ -320,8 +321,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
 // S of a warp's 16 channels and 8 columns as the right operand of a product over the channels
 __device__ __forceinline__ void dc_right(const float (&s)[4], uint32_t (&b)[3][2]) {
     uint32_t lo[3], hi[3];
-    gb_split_bf16(s[0], s[1], lo);
-    gb_split_bf16(s[2], s[3], hi);
+    gb_split_bf16<true>(s[0], s[1], lo);
+    gb_split_bf16<true>(s[2], s[3], hi);
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
         b[e][0] = dc_turn(lo[e]);
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArg
             const float u = o.tv[n] - (((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7])));
             ws[DC_AT_U + ti * DC_V + col0 + 8 * n + tc] = u;
             uint32_t term[3];
-            gb_split_bf16(u, 0.f, term);
+            gb_split_bf16<true>(u, 0.f, term);
 #pragma unroll
             for (int e = 0; e < 3; ++e) Ub[n][e][tc][ti] = (unsigned short)term[e];
         }
@@ -539,8 +540,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_out_kernel(DeltaChunkArgs
         uint32_t b[2][2][3];
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-            gb_split_bf16(u[n][k16][0], u[n][k16][1], b[n][0]);
-            gb_split_bf16(u[n][k16][2], u[n][k16][3], b[n][1]);
+            gb_split_bf16<true>(u[n][k16][0], u[n][k16][1], b[n][0]);
+            gb_split_bf16<true>(u[n][k16][2], u[n][k16][3], b[n][1]);
         }
 #pragma unroll
         for (int m = k16; m < 2; ++m) {

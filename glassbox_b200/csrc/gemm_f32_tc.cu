@@ -1,22 +1,26 @@
 // C[M, N] (+)= A[M, K] * W[N, K]^T of float32 activations (and float32 or bfloat16 weights) on the 5th-generation tensor cores,
 // with the exactness of float32 FMA.
 //
-// Every float32 operand is the exact sum of three bfloat16 numbers (8 + 8 + 8 bits, by truncation; a bfloat16 weight is one). Six of
-// the nine products of two operands' terms (three of three) stay: what is left out lies below 2^-24 of a product. The tensor core's
-// accumulator cuts instead of rounding, 1.1e-8 of the sum per 16 of K, always downwards: a product over K 576 in one accumulator is off by
-// 5.4e-7 where FMA is by 1.7e-7. So an accumulator takes 32 of K, the smallest products first, and the sums of 32 are added in
-// registers, rounded to nearest.
-// Measured against 64 bits, normal operands, float32 weights (2-norm of the error over that of the result), this / FMA: K 64 1.1e-7 / 1.4e-7,
-// K 576 1.3e-7 / 4.3e-7, K 1536 1.7e-7 / 7.0e-7, K 4096 2.3e-7 / 1.2e-6; at K 32 1.05e-7 / 1.02e-7: shorter products stay with FMA.
+// Every float32 operand is the exact sum of three bfloat16 numbers, each what is left rounded to the nearest (a bfloat16 weight is one;
+// Henry, Tang and Heinecke 2019). Eight of the nine products of two operands' terms stay: what is left out lies below 2^-34 of a
+// product (with six, and terms cut off instead of rounded, it was up to 2^-21, always towards zero). Operands below some 2^-110 lose their
+// last terms to bfloat16's smallest number: 2^-134 each. The tensor core's accumulator cuts instead of rounding, 1.1e-8 of the sum per 16
+// of K, always downwards: a product over K 576 in one accumulator is off by 5.4e-7 where FMA is by 1.7e-7. So the products of the first terms
+// get an accumulator for every 32 of K, and these sums are added in registers, rounded to nearest; all other products, at most
+// 2^-8 of those, keep theirs to the end.
+// Measured against 64 bits, float32 weights (2-norm of the error over that of the result), this / FMA: normal operands, K 64 5.3e-8 / 1.4e-7,
+// K 576 9.4e-8 / 4.3e-7, K 1536 1.4e-7 / 7.0e-7, K 4096 2.2e-7 / 1.2e-6; rows of one number 2.5e-8 / 2.5e-8 (largest 6.0e-8 of a
+// product for both), of two 2.6e-8 / 3.1e-8, of eight 2.9e-8 / 5.4e-8.
 //
 // A block computes one 128 x BN tile, 32 of K at a time. Sixteen warps do the same: bring float32 values into registers (two steps ahead),
 // split them and store the terms as 64-byte-swizzled K-major tiles (two stages), then add the accumulator of the step before (of two) to
 // their sums. A thread of a seventeenth issues the products, M 128, N BN, K 16.
-// Bound by the workers' chain of a step (values, split, stores, the fence in front of the tensor core, the sums): 0.65 us at BN 64 and 0.86 at
-// 128, where the products take 0.3 and 0.4 and their operands' reads and the stores fill shared memory to three quarters.
+// Bound by the workers' chain of a step (values, split, stores, the fence in front of the tensor core, the sums): 0.67 us at BN 64 and 0.89 at
+// 128, where the products' operands alone keep shared memory busy for 0.3 and 0.4. One product takes two of W's terms side by side
+// where it can and reads A's once for both (eight products apart: 22.1 us in the place of 20.6 for the first of the following).
 // Measured, us, the FMA tiles (bound by the operands' way through shared memory at half of the FMA rate) and this: 2,047 rows N 960, K 576
-// 67 -> 19; N 576, K 576 37 -> 15; N 3072, K 576 175 -> 55; N 576, K 1536 95 -> 34; 1,200 rows N 960, K 2560 150 -> 71; 9 rows N 576, K
-// 576 17 -> 13; bfloat16 weights, 2,048 rows N 1024, K 64 10.2 -> 4.9. A step's products issued by a worker instead: 1.2 us a step.
+// 67 -> 21; N 576, K 576 37 -> 15; N 3072, K 576 175 -> 58; N 576, K 1536 95 -> 35; 1,200 rows N 960, K 2560 150 -> 75; 9 rows N 576, K
+// 576 17 -> 13; bfloat16 weights, 2,048 rows N 1024, K 64 10.2 -> 5.3. A step's products issued by a worker instead: 1.2 us a step.
 //
 // A result that is no finite number is formed again by FMA, one product after the other (an infinite operand's lesser terms are not
 // numbers). Each output element's order of sums depends on K alone. Every wait is bounded (GB_STATUS_WAIT_TIMEOUT); there are no TMA
@@ -49,7 +53,8 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const float*
     constexpr int WT = sizeof(TW) == 4 ? 3 : 1;                       // terms of a weight
     constexpr int A_TERM = F3_BM * F3_ROW, W_TERM = BN * F3_ROW, STAGE = 3 * A_TERM + WT * W_TERM;
     constexpr int LR = F3_WORKERS / 8, AL = F3_BM / LR, WL = BN / LR; // 16-byte loads of a thread and step
-    constexpr int PRODUCTS = WT == 3 ? 6 : 3;
+    // accumulators side by side, BN columns each: two that take turns for the products of the first terms, then LESSER for all others
+    constexpr int LESSER = WT == 1 ? 1 : 2, TMEM = 4 * BN;
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* tiles = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     __shared__ F3Shared sh;
@@ -64,7 +69,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const float*
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(2 * BN) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -78,20 +83,29 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const float*
     if (warp == F3_WORKERS / 32) {
         // (a warp of its own: the issuing thread is held up about as long as the products take)
         if (elect_one()) {
-            constexpr int a_term[6] = {2, WT == 3 ? 0 : 1, WT == 3 ? 1 : 0, 1, 0, 0}, w_term[6] = {0, WT == 3 ? 2 : 0, WT == 3 ? 1 : 0, 0, 1, 0};
-            const uint32_t idesc = umma_idesc(F3_BM, BN);
             const uint64_t a_desc = f3_desc(smem_u32(tiles)), w_desc = f3_desc(smem_u32(tiles) + 3 * A_TERM);
             for (int step = 0; step < steps; ++step) {
                 const int s = step & 1;
                 if (!mbar_wait(&sh.full[s], (step >> 1) & 1, abort_flag, status)) break;
                 tc_fence_after();
                 const uint64_t da = a_desc + ((s * STAGE) >> 4), dw = w_desc + ((s * STAGE) >> 4);
-#pragma unroll
-                for (int p = 0; p < PRODUCTS; ++p)
+                // A's term `a` by `n` of W's terms from `w` on, which lie one behind the other: one product of n * BN columns reads A once
+                auto product = [&](int a, int w, int n, int column, bool first) {
 #pragma unroll
                     for (int k = 0; k < F3_BK / 16; ++k)
-                        umma_bf16(tmem + (uint32_t)(s * BN), da + ((a_term[p] * A_TERM) >> 4) + k * 2, dw + ((w_term[p] * W_TERM) >> 4) + k * 2, idesc,
-                                  (p | k) ? 1u : 0u);
+                        umma_bf16(tmem + (uint32_t)column, da + ((a * A_TERM) >> 4) + k * 2, dw + ((w * W_TERM) >> 4) + k * 2, umma_idesc(F3_BM, n * BN),
+                                  first && k == 0 ? 0u : 1u);
+                };
+                if (WT == 1) {
+                    product(2, 0, 1, 2 * BN, step == 0);
+                    product(1, 0, 1, 2 * BN, false);
+                } else {
+                    product(2, 0, 2, 2 * BN, step == 0);
+                    product(1, 2, 1, 2 * BN, false);
+                    product(1, 0, 2, 2 * BN, false);
+                    product(0, 1, 2, 2 * BN, false);
+                }
+                product(0, 0, 1, s * BN, true);
                 umma_commit(&sh.done[s]);
             }
         }
@@ -162,6 +176,19 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const float*
         }
         if (ok) collect(steps - 1);
         if (ok) {
+#pragma unroll
+            for (int c = 0; c < CW; c += 16) {                            // the sums of the lesser terms' products
+                float sum[16] = {};
+#pragma unroll
+                for (int e = 0; e < LESSER; ++e) {
+                    uint32_t r[16];
+                    tmem_load16(t_base + (uint32_t)((2 + e) * BN + c), r);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[j] += __uint_as_float(r[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c + j] += sum[j];
+            }
             const int row = m0 + q * 32 + lane;
             bool odd = false;
 #pragma unroll
@@ -219,7 +246,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const float*
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM) : "memory");
 }
 
 template <int BN, typename TW>
@@ -248,11 +275,11 @@ GB_EXPORT int gb_gemm_f32_tc(const void* a, const void* w, int w_dtype, void* c,
                "gb_gemm_f32_tc: rows must be whole aligned 16-byte pieces (M=%d N=%d K=%d)", M, N, K);
     GB_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gb_gemm_f32_tc: a leading dimension is smaller than its row");
     if (M == 0) return 0;
-    // The width whose rounds of tiles end soonest: a tile takes 0.65 us a step and 2.9 beside it at BN 64, 0.86 and 3.4 at 128 (from launches
-    // of one round). 2,047 rows, us at 64 / 128: N 576, K 1536 34 / 45; N 960, K 576 29 / 19; N 3072, K 576 84 / 55.
+    // The width whose rounds of tiles end soonest: a tile takes 0.67 us a step and 2.9 beside it at BN 64, 0.89 and 3.4 at 128 (from launches
+    // of one round). Both add in the same order.
     const int steps = gb_ceil_div(K, F3_BK);
     const long long tiles_m = gb_ceil_div(M, F3_BM), r64 = (tiles_m * gb_ceil_div(N, 64) + 147) / 148, r128 = (tiles_m * gb_ceil_div(N, 128) + 147) / 148;
-    const bool wide = (float)r128 * (0.86f * (float)steps + 3.4f) < (float)r64 * (0.65f * (float)steps + 2.9f);
+    const bool wide = (float)r128 * (0.89f * (float)steps + 3.4f) < (float)r64 * (0.67f * (float)steps + 2.9f);
 #define F3_CASE(BN_, TW_) f3_launch<BN_, TW_>((const float*)a, (const TW_*)w, (float*)c, M, N, K, lda, ldw, ldc, accumulate, status, stream)
     if (w_dtype == GB_F32) return wide ? F3_CASE(128, float) : F3_CASE(64, float);
     GB_REQUIRE(w_dtype == GB_BF16, "gb_gemm_f32_tc: unsupported weights' dtype %d", w_dtype);

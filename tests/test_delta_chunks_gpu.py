@@ -138,3 +138,28 @@ def test_chunks_of_sixteen_columns_and_of_more_than_a_pass(H, KH, D, V, lens):
     data = _inputs(lens, H, KH, D, V, False, H)
     for g, w in zip(_run(True, lens, H, KH, D, V, False, *data), _truth(lens, H, KH, D, V, False, *data)):
         np.testing.assert_allclose(g, w, atol=1e-5 * max(1.0, np.abs(w).max()), rtol=1e-5)       # (the bound of the test above)
+
+
+def test_a_state_of_one_number_per_column():
+    """What is left of a sum is one product: it is rounded, and the products of its factors' terms that are left out stay below its rounding.
+    A number next to the largest float32 is taken as well."""
+    from glassbox_b200 import kernels
+    D = V = 64
+    rng = np.random.default_rng(1)
+    q = np.zeros((2, D), np.float32)
+    q[:, 5], q[:, 9] = 3000.0, 4000.0               # (a length of 5,000, next to which 1e-6 is nothing; channel 9 of the state is empty)
+    f = np.float32
+    unit = f(3000) * (f(1) / np.sqrt(f(25e6)))
+    read = float(f(3000) * (f(0.125) / np.sqrt(f(25e6))))
+    states = np.zeros((1, 1, D, V), np.float32)
+    states[0, 0, 5] = rng.standard_normal(V)
+    states[0, 0, 5, :2] = np.array([0x3F80FFFF, 0x7F7F9000], np.uint32).view(np.float32)
+    qkv = np.concatenate([q, q, np.zeros((2, V), np.float32)], 1)
+    # the first token leaves the state alone (beta 0, no decay) and reads it, the second writes with beta 1
+    out, after = _run(True, [2], 1, 1, D, V, True, qkv, np.float32([[-1e4], [1e4]]), np.zeros((2, 1), np.float32), np.zeros(1, np.float32),
+                      np.float32([-200.0]), states)
+    S, k = states[0, 0, 5].astype(np.float64), float(unit)
+    # a product: its rounding and what is left out (2^-24 each), sums of three terms
+    assert (np.abs(out[0] - read * S) <= 2.25 * 2 ** -24 * np.abs(read * S)).all()
+    # u = -k S, then S + k u: 2.25 of 2^-24 of k S times k, as much of k u, the sum's rounding
+    assert (np.abs(after[0, 0, 5] - S * (1 - k * k)) <= 2 ** -24 * (4.5 * k * k + 1) * np.abs(S)).all()

@@ -50,6 +50,26 @@ def test_as_exact_as_fma(K, kind):
     assert out[0] <= out[1], out
 
 
+@pytest.mark.parametrize("numbers", [1, 2, 8])
+@pytest.mark.parametrize("N", [64, 4000])                   # (both tile widths)
+def test_rows_of_few_numbers_are_as_exact_as_by_fma(numbers, N):
+    from glassbox_b200 import kernels
+    a, w, _ = _operands(512, N, 576, torch.float32, numbers)
+    g = torch.Generator().manual_seed(numbers)
+    keep = torch.zeros(512, 576).scatter_(1, torch.rand(512, 576, generator=g).argsort(1)[:, :numbers], 1.0).to(DEV)
+    a *= keep
+    a[:64] = torch.where(keep[:64] > 0, torch.tensor(0x3F80FFFF, dtype=torch.int32).view(torch.float32).item(), 0.0)
+    w[:32] = a.max() if numbers == 1 else w[:32]
+    ref, error = a.double() @ w.double().T, []
+    for product in (kernels.gemm_f32_tc, kernels.gemm_simt):
+        c = torch.empty(512, N, device=DEV)
+        product(a, w, c)
+        error.append((c.double() - ref).abs())
+    if numbers == 1:                                        # one product: 2^-24 for its rounding, a few 2^-32 for terms left out and cut
+        assert (error[0] <= 2 ** -24 * (1 + 2 ** -6) * ref.abs()).all()
+    assert float(error[0].norm()) <= float(error[1].norm()) * (1 + 2 ** -6)
+
+
 def test_what_is_not_finite_is_as_by_fma():
     """Infinities, NaN and sums that overflow, in their own rows and columns alone."""
     from glassbox_b200 import kernels

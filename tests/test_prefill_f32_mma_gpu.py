@@ -44,6 +44,23 @@ def test_against_float64(hd, n, start, window):
     assert (got.double() - want).abs().max() <= 1e-5
 
 
+@pytest.mark.parametrize("hd", [16, 64])
+def test_a_score_of_one_product(hd):
+    """Two keys weigh about the same; the first one's score is one product of two numbers with as many bits as they have."""
+    k, v, q = (torch.zeros_like(x) for x in _pool(2, hd, 1))
+    x = torch.tensor(0x3F80FFFF, dtype=torch.int32).view(torch.float32).item()
+    root = hd ** 0.5
+    q[:, 0], k[0, 0, 0, 0], k[0, 0, 1, 0] = x * 16, x * root, root * (x * x * 16).__round__() / 16
+    v[0, 0, 0], v[0, 0, 1, 0] = 1.0, 3.395e38               # (a value that bfloat16 rounds to infinity)
+    got = _run(q, k, v, [[0]], [0, 2], [0], 2)
+    want = _truth(q, k.reshape(-1, hd), v.reshape(-1, hd), 0)
+    # scores of 16.25, each off by at most 2.25 * 2^-24 of that and the scale's rounding: a weight near a half moves by a quarter of their
+    # difference; the exponential, sum and quotient add some 2^-22
+    bound = 0.25 * 2 * 16.25 * 3.25 * 2 ** -24 + 2 ** -22
+    assert (got[:, 1:].double() - want[:, 1:]).abs().max() <= bound
+    assert ((got[:, 0].double() - want[:, 0]).abs() <= 4 * bound * want[:, 0].abs()).all()
+
+
 def test_numbers_that_are_none_reach_the_rows_that_see_them():
     n, hd = 150, 64
     k, v, q = _pool(n, hd, 2)
