@@ -324,7 +324,7 @@ GB_EXPORT int gb_attention_prefill_f32_supported(int nh, int nkv, int hd) {
 // seq_start_pos[s] + local index. q, out, caches: float32, rows aligned to 16 bytes.
 GB_EXPORT int gb_attention_prefill_f32(const void* q, long long q_stride, void* out, long long out_stride, const void* kcache,
                                        const void* vcache, const int* block_tables, int max_pages, const int* seq_first_row,
-                                       const int* seq_start_pos, int num_seqs, int max_rows_per_seq, int nh, int nkv, int hd, int page_size,
+                                       const int* seq_start_pos, int rows, int num_seqs, int max_rows_per_seq, int nh, int nkv, int hd, int page_size,
                                        long long num_pages, float scale, int window, int* status, cudaStream_t stream) {
     GB_REQUIRE(gb_attention_prefill_f32_supported(nh, nkv, hd), "gb_attention_prefill_f32: %d/%d heads of %d are not built", nh, nkv, hd);
     GB_REQUIRE(q_stride % 4 == 0 && out_stride % 4 == 0 && ((uintptr_t)q | (uintptr_t)out | (uintptr_t)kcache | (uintptr_t)vcache) % 16 == 0,
@@ -342,7 +342,7 @@ GB_EXPORT int gb_attention_prefill_f32(const void* q, long long q_stride, void* 
 #define GB_CASE(HD_)                                                                                                               \
     if (hd == HD_)                                                                                                                 \
         return gb_launch_prefill_f32_mma<HD_>((const float*)q, q_stride, (float*)out, out_stride, (const float*)kcache, (const float*)vcache, \
-                                              block_tables, max_pages, seq_first_row, seq_start_pos, num_seqs, max_rows_per_seq, nh, nkv, \
+                                              block_tables, max_pages, seq_first_row, seq_start_pos, rows, num_seqs, max_rows_per_seq, nh, nkv, \
                                               page_size, num_pages, scale, window, status, stream);
     GB_CASE(16) GB_CASE(32) GB_CASE(64)
 #undef GB_CASE

@@ -11,12 +11,12 @@
 // A block is 64 consecutive query rows of one request for one query head: four groups of four warps, each with every fourth tile of 32
 // keys (a way), which merge at the end; a warp has 16 rows. A group's tile arrives a turn ahead through cp.async as float32, each piece
 // for the thread that splits it and stores the terms as bfloat16 rows (16-byte pieces turned by the row), from which ldmatrix reads the
-// fragments; the queries lie so in shared memory for all groups. The longest tiles of all heads and requests start first. Many short
-// portions take blocks of one group that walks the four ways one after the other: three such blocks share a multiprocessor.
+// fragments; the queries lie so in shared memory for all groups. The longest tiles of all heads and requests start first. The first tiles
+// of many requests take blocks of one group that walks the four ways one after the other: three such blocks share a multiprocessor.
 // Bound by instructions and their latency (a third of the issue slots with two groups of 64-key tiles, 8 warps an SM) and by shared
 // memory's bandwidth (a third of the time). Measured, us, FMA from shared memory / this: 9/3 heads of 64, three prompts of 2,047 rows
 // 173 / 60, one of 2,047 rows 294 / 120, with a window of 256 62 / 44; 15/5 heads, 1,200 rows behind 500 267 / 131; 32 prompts of 20 tokens
-// 16 / 12, of 16 tokens at 32 heads 34 / 24; heads of 32, 1,500 rows 154 / 53, of 16 134 / 38. Two groups of 64-key tiles: 66 and 135 for
+// 12 / 9.6, of 16 tokens at 32 heads 32 / 24; heads of 32, 1,500 rows 154 / 53, of 16 134 / 38. Two groups of 64-key tiles: 66 and 135 for
 // the first two, prompts of 16 tokens at 32 heads 60.
 //
 // Key tiles start at multiples of 32, a way's are every fourth from a multiple on, and a row's masked keys add nothing, so the order of a
@@ -125,12 +125,49 @@ template <int HD> struct PmRows {
     }
 };
 
-template <int HD, int GROUPS>
+// Two launches may share a call's row tiles: the second then does not wait for the first.
+enum { PM_ALONE = 0, PM_FIRST = 1, PM_SECOND = 2 };
+
+// The requests' row tiles behind their first ones, a higher one, whose rows see more keys, before all lower ones: which request has the i-th,
+// and which of its tiles is it? Every warp looks for the tile number that i falls on, by how many tiles have a number or a higher one
+// (-1: no tile is left). A call of its own, so that its registers are not the kernel's.
+__device__ __noinline__ int2 pm_later_tile(int i, const int* __restrict__ first_row, int num_seqs) {
+    const int lane = threadIdx.x & 31;
+    auto tiles_of = [&](int s) { return s < num_seqs ? (first_row[s + 1] - first_row[s] + PM_BM - 1) / PM_BM : 0; };
+    const int own = tiles_of(lane);                         // (of the first 32 requests)
+    auto from = [&](int t) {
+        int sum = max(own - t, 0);
+        for (int s = 32 + lane; s < num_seqs; s += 32) sum += max(tiles_of(s) - t, 0);
+        return __reduce_add_sync(0xffffffffu, sum);
+    };
+    if (from(1) <= i) return make_int2(-1, 0);
+    int most = own;
+    for (int s = 32 + lane; s < num_seqs; s += 32) most = max(most, tiles_of(s));
+    int qt = 1, hi = __reduce_max_sync(0xffffffffu, most);  // from(qt) > i >= from(hi)
+    while (hi - qt > 1) {
+        const int t = (qt + hi) / 2;
+        if (from(t) > i) qt = t;
+        else hi = t;
+    }
+    int nth = i - from(qt + 1);                             // among the requests that have a tile of this number
+    for (int s0 = 0; s0 < num_seqs; s0 += 32) {
+        const unsigned have = __ballot_sync(0xffffffffu, (s0 ? tiles_of(s0 + lane) : own) > qt);
+        if (nth < __popc(have)) {
+            const unsigned it = __ballot_sync(0xffffffffu, (have >> lane & 1) && __popc(have & ((1u << lane) - 1)) == nth);
+            return make_int2(s0 + __ffs(it) - 1, qt);
+        }
+        nth -= __popc(have);
+    }
+    return make_int2(-1, 0);
+}
+
+// SEARCH: blocks y are the requests' later tiles (`later` of them at most), then their first ones; else y is the request and z its tile.
+template <int HD, int GROUPS, bool SEARCH>
 __global__ void __launch_bounds__(PM_GROUP * GROUPS, GROUPS == 1 ? 3 : 1) attention_prefill_f32_mma_kernel(
     const float* __restrict__ q, long long q_stride, float* __restrict__ out, long long out_stride, const float* __restrict__ kcache,
     const float* __restrict__ vcache, const int* __restrict__ block_tables, int max_pages, const int* __restrict__ seq_first_row,
-    const int* __restrict__ seq_start_pos, int nh, int nkv, int page_size, long long num_pages, float scale, int window,
-    int* __restrict__ status) {
+    const int* __restrict__ seq_start_pos, int num_seqs, int nh, int nkv, int page_size, long long num_pages, float scale, int window,
+    int* __restrict__ status, int later, int part) {
     constexpr int CPR = HD / 8, K16 = HD / 16;              // 16-byte pieces of a row of one term; groups of 16 channels
     constexpr int TERM = PM_BN * HD * 2, TILE = 3 * TERM;   // bytes of a tile's term; of its terms
     constexpr int LOADS = PM_BN * HD / 4 / PM_GROUP;        // 16-byte loads of a thread and tile
@@ -140,10 +177,28 @@ __global__ void __launch_bounds__(PM_GROUP * GROUPS, GROUPS == 1 ? 3 : 1) attent
     __shared__ int odd_s[GROUPS][4];                        // ... and whether the split does not take a value of theirs
 
     const int tid = threadIdx.x % PM_GROUP, group = threadIdx.x / PM_GROUP, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const int qt = gridDim.z - 1 - blockIdx.z;              // later rows see more keys: the longest blocks start first
-    const int head = blockIdx.x, seq = blockIdx.y;
-    gb_pdl_launch_dependents();
-    gb_pdl_wait();
+    const int head = blockIdx.x;
+    // The second of two launches may start when all blocks of the first have passed their wait for what came before both; it waits for
+    // the first at its end, so that whoever waits for the second has waited for both.
+    if (part != PM_FIRST) gb_pdl_launch_dependents();
+    if (part != PM_SECOND) gb_pdl_wait();
+    if (part == PM_FIRST) gb_pdl_launch_dependents();
+    struct AtEnd {
+        bool wait;
+        __device__ ~AtEnd() {
+            if (wait) gb_pdl_wait();
+        }
+    } at_end{part == PM_SECOND};
+    int seq = blockIdx.y, qt = gridDim.z - 1 - blockIdx.z;  // later rows see more keys: the longest blocks start first
+    if (SEARCH) {
+        seq -= later;
+        if (seq < 0) {
+            const int2 at = pm_later_tile(blockIdx.y, seq_first_row, num_seqs);
+            if (at.x < 0) return;
+            seq = at.x;
+            qt = at.y;
+        }
+    }
     const int row0 = seq_first_row[seq];
     const int nrows = seq_first_row[seq + 1] - row0;
     const int q_lo = qt * PM_BM;
@@ -438,36 +493,50 @@ __global__ void __launch_bounds__(PM_GROUP * GROUPS, GROUPS == 1 ? 3 : 1) attent
     }
 }
 
-template <int HD, int GROUPS>
+template <int HD, int GROUPS, bool SEARCH>
 static int pm_launch(const float* q, long long q_stride, float* out, long long out_stride, const float* kcache, const float* vcache,
-                     const int* block_tables, int max_pages, const int* seq_first_row, const int* seq_start_pos, int num_seqs,
-                     int max_rows_per_seq, int nh, int nkv, int page_size, long long num_pages, float scale, int window, int* status,
-                     cudaStream_t stream) {
+                     const int* block_tables, int max_pages, const int* seq_first_row, const int* seq_start_pos, int num_seqs, int nh, int nkv, int page_size, long long num_pages, float scale, int window, int* status,
+                     cudaStream_t stream, long long y, long long z, int later, int part) {
     constexpr int tiles_bytes = 3 * PM_BM * HD * 2 + GROUPS * 2 * PM_BN * HD * (3 * 2 + 4), merge_bytes = (GROUPS - 1) * 4 * 32 * (HD / 2 + 4) * 4;
     constexpr int smem = tiles_bytes > merge_bytes ? tiles_bytes : merge_bytes;
-    auto kernel = attention_prefill_f32_mma_kernel<HD, GROUPS>;
+    auto kernel = attention_prefill_f32_mma_kernel<HD, GROUPS, SEARCH>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     GB_REQUIRE(e == cudaSuccess, "gb_attention_prefill_f32: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-    const int tiles = gb_ceil_div(max_rows_per_seq, PM_BM);
-    GB_REQUIRE(tiles <= 65535, "gb_attention_prefill_f32: too many rows per request (%d)", max_rows_per_seq);
-    gb_launch(GB_PDL_ATTENTION, kernel, dim3(nh, num_seqs, tiles), dim3(PM_GROUP * GROUPS), smem, stream, q, q_stride, out, out_stride, kcache,
-              vcache, block_tables, max_pages, seq_first_row, seq_start_pos, nh, nkv, page_size, num_pages, scale, window, status);
+    GB_REQUIRE(y <= 65535 && z <= 65535, "gb_attention_prefill_f32: too many row tiles (%lld x %lld)", y, z);
+    gb_launch(GB_PDL_ATTENTION, kernel, dim3(nh, (unsigned)y, (unsigned)z), dim3(PM_GROUP * GROUPS), smem, stream, q, q_stride, out, out_stride, kcache,
+              vcache, block_tables, max_pages, seq_first_row, seq_start_pos, num_seqs, nh, nkv, page_size, num_pages, scale, window, status, later, part);
     return gb_check_launch("gb_attention_prefill_f32");
 }
 
 template <int HD>
 int gb_launch_prefill_f32_mma(const float* q, long long q_stride, float* out, long long out_stride, const float* kcache, const float* vcache,
-                              const int* block_tables, int max_pages, const int* seq_first_row, const int* seq_start_pos, int num_seqs,
+                              const int* block_tables, int max_pages, const int* seq_first_row, const int* seq_start_pos, int rows, int num_seqs,
                               int max_rows_per_seq, int nh, int nkv, int page_size, long long num_pages, float scale, int window,
                               int* status, cudaStream_t stream) {
-    // One row tile a request and more blocks than multiprocessors: short portions, where a block's start and end count (32 prompts of 16 tokens
-    // at 32 heads 24 us with one group, some 60 with all). Both forms give the same bits.
-    const bool many = max_rows_per_seq <= PM_BM && (long long)nh * num_seqs > 148;
-    auto launch = many ? pm_launch<HD, 1> : pm_launch<HD, PM_WAYS>;
-    return launch(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, seq_first_row, seq_start_pos, num_seqs, max_rows_per_seq,
-                  nh, nkv, page_size, num_pages, scale, window, status, stream);
+#define PM_LAUNCH(GROUPS_, SEARCH_, Y_, Z_, LATER_, PART_)                                                                                 \
+    pm_launch<HD, GROUPS_, SEARCH_>(q, q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, seq_first_row, seq_start_pos, num_seqs, \
+                                    nh, nkv, page_size, num_pages, scale, window, status, stream, Y_, Z_, LATER_, PART_)
+    // A recorded step gives its shape's longest possible portion, of which a grid of requests by tiles is mostly empty: where that has twice
+    // as many tiles as the requests can have between them (a whole one for every 64 rows, one for each request), these are looked for.
+    // The first tiles of many requests (more blocks than multiprocessors) then take one group a block, where a block's start and end
+    // count, and the others four, side by side; where a first tile may see many keys, from 512 blocks on (fewer leave a walk of one
+    // group alone at the end). All forms give the same bits. Measured, us, recorded shapes, grid of requests by tiles with four groups /
+    // by this rule: 32 prompts of 16 tokens at 9, 15, 32 and 64 heads 18 / 11, 33 / 16, 60 / 26 and 118 / 45 (FMA 16, 23, 38 and
+    // 67); a prompt of 1,000 beside 31 of 16 tokens 64 / 60, 101 / 79, 209 / 145 and 411 / 282; 16 x 64 tokens behind 500 at 15 heads 79 / 73
+    // (first tiles by one group 97); eight of 100 tokens at 9 heads 12.9 / 11.9. Longest portion known: 8 x 100 11.1 without a search
+    // (12.0 with), 32 x 16 tokens at 32 heads 23.1 with one group (49 with four).
+    const long long tiles = gb_ceil_div(max_rows_per_seq, PM_BM), most = num_seqs * (tiles - 1);
+    const long long later = rows / PM_BM < most ? rows / PM_BM : most, blocks = (long long)nh * num_seqs;
+    const bool known = num_seqs * tiles <= 2 * (later + num_seqs);
+    const bool one = blocks > 148 && (later == 0 || (!known && (blocks >= 512 || (long long)max_pages * page_size <= 256)));
+    if (one && later == 0) return PM_LAUNCH(1, false, num_seqs, 1, 0, PM_ALONE);
+    if (known) return PM_LAUNCH(PM_WAYS, false, num_seqs, tiles, 0, PM_ALONE);
+    if (!one) return PM_LAUNCH(PM_WAYS, true, later + num_seqs, 1, (int)later, PM_ALONE);
+    const int rc = PM_LAUNCH(PM_WAYS, true, later, 1, (int)later, PM_FIRST);
+    return rc ? rc : PM_LAUNCH(1, false, num_seqs, 1, 0, PM_SECOND);
+#undef PM_LAUNCH
 }
 #define PM_BUILD(HD_)                                                                                                                      \
     template int gb_launch_prefill_f32_mma<HD_>(const float*, long long, float*, long long, const float*, const float*, const int*, int, \
-                                                const int*, const int*, int, int, int, int, int, long long, float, int, int*, cudaStream_t);
+                                                const int*, const int*, int, int, int, int, int, int, long long, float, int, int*, cudaStream_t);
 PM_BUILD(16) PM_BUILD(32) PM_BUILD(64)

@@ -93,3 +93,52 @@ def test_a_request_among_many_gives_the_same_bits(start, n, window):
     one = _run(q, k, v, [table], [0, n], [start], n, window)
     many = _run(q.repeat(seqs, 1), k, v, [table] * seqs, [n * i for i in range(seqs + 1)], [start] * seqs, n, window)
     assert torch.equal(many.view(seqs, n, hd), one.expand(seqs, n, hd))
+
+
+def _portions(lens, starts, nh, seed=5, hd=64):
+    """q, keys, values, tables, first rows of requests that bring ``lens`` rows; a start of -1 is a padding sequence."""
+    g = torch.Generator().manual_seed(seed)
+    need = [-(-(n + max(s, 0)) // 16) for n, s in zip(lens, starts)]
+    at, width = [sum(need[:i]) for i in range(len(need))], max(8, max(need))
+    tables = [[a + j if j < n and s >= 0 else -1 for j in range(width)] for a, n, s in zip(at, need, starts)]
+    k, v = (torch.randn(sum(need), 1, 16, hd, generator=g).to(DEV) for _ in range(2))
+    first = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    return torch.randn(sum(lens), nh * hd, generator=g).to(DEV), k, v, tables, first
+
+
+@pytest.mark.parametrize("nh, lens, starts", [
+    (1, [300, 1, 0, 65, 64, 2, 128, 20, 16, 16, 16, 16], [0, 3, 0, 0, 7, -1, 0, 0, 5, 0, 0, 0]),       # four groups for all tiles
+    (4, [200, 2, 65, 64] + [9] * 40 + [129, 0, 3], [0, -1] + [0] * 45),                                # first tiles apart
+    (13, [20] * 20 + [193, 64, 130] + [5] * 20, [300] + [0] * 42),                                     # ... with longer contexts
+])
+def test_the_bound_of_a_recorded_shape_gives_the_same_bits(nh, lens, starts):
+    data = _portions(lens, starts, nh)
+    q, first = data[0], data[4]
+    want = torch.zeros_like(q)
+    for s, (n, p) in enumerate(zip(lens, starts)):          # request by request
+        rows = slice(first[s], first[s + 1])
+        if n and p >= 0:
+            want[rows] = _run(q[rows], data[1], data[2], data[3][s:s + 1], [0, n], [p], n)
+    for bound in (max(lens), -(-sum(lens) // 128) * 128):
+        got = _run(*data[:4], first, starts, bound)
+        assert torch.equal(got, want), bound
+
+
+def test_the_bound_of_a_recorded_shape_costs_little():
+    """150 prompts of 16 tokens, of which a recorded step's shape tells only that no one has more than 2,432."""
+    from glassbox_b200 import kernels
+    q, k, v, tables, first = _portions([16] * 150, [0] * 150, 32)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    tables, first, start, status, out, times = i32(tables), i32(first), i32([0] * 150), i32([0]), torch.empty_like(q), []
+    for bound in (16, 2432):
+        spans = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(20):
+                kernels.attention_prefill_f32(q, out, k, v, tables, first, start, bound, 32, 1, 64, 16, 0.125, None, status)
+            b.record()
+            torch.cuda.synchronize()
+            spans.append(a.elapsed_time(b))
+        times.append(min(spans))
+    assert times[1] < 2 * times[0], times
