@@ -16,6 +16,9 @@
 //   delta_scan_kernel     a block per (request, head, 8 or 16 columns of S): U and S chunk after chunk, S in registers
 //   delta_out_kernel      every (chunk, head) side by side: O from the chunk's S_0 and U
 //
+// Each lets the next start only when it is about to end. A scanning block takes a multiprocessor's whole register file: when all three let
+// their successors in at once, blocks of the calls to come held most multiprocessors waiting, and the few blocks of a short prompt's
+// preparation and read-out ran two to a multiprocessor beside them (one request of 96 rows, 8 heads: 37.8 us; 28.6 so).
 // Everything is float32. The products run on the tensor cores with every float32 operand as three bfloat16 numbers whose sum it is
 // exactly, each what is left rounded to the nearest (Henry, Tang and Heinecke 2019), and six products of them, the largest in an
 // accumulator of its own: what is left out is below 2^-24 of a product and has either sign. Measured against 64 bits, random inputs
@@ -27,8 +30,8 @@
 // (movmatrix turns the accumulators into the next product's operand); the sums over the channels meet in shared memory. Operands come
 // in the order of the fragments, two chunks ahead, straight into registers. 16 columns a block where 8 would make more blocks than
 // multiprocessors: the operands' way counts once for both.
-// Measured, 2,048 tokens of one request, prepare + scan + read-out: 8 heads x 128 x 128 44 + 68 + 21 us (the chunk's products by FMA from
-// shared memory, read-out in the scan: 44 + 139), 16 heads 83 + 106 + 42 (85 + 215).
+// Measured, 2,048 tokens of one request, prepare + scan + read-out: 8 heads x 128 x 128 45 + 70 + 21 us (the chunk's products by FMA from
+// shared memory, read-out in the scan: 37 + 126), 16 heads 81 + 107 + 41 (78 + 200); 96 tokens, 8 heads, 16.5 + 5.0 + 7.1 (15.8 + 9.4).
 #include "common.cuh"
 
 constexpr int DC_C = 32;                            // tokens of a chunk
@@ -140,13 +143,11 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
     float* Q = dc_mem, *K = Q + DC_C * DC_RP, *G = K + DC_C * DC_RP;       // [32][136] each
     __shared__ __align__(16) float A[DC_C][DC_TP], B[DC_C][DC_TP];
     __shared__ float beta_s[DC_C];
-    gb_pdl_launch_dependents();
     gb_pdl_wait();
     const int chunk = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
-    if (p.seq_start_pos[seq] < 0) return;
-    const int r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];
+    const int start = p.seq_start_pos[seq], r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];      // (requested together)
     const int c0 = r0 + chunk * DC_C, nt = min(DC_C, r1 - c0);
-    if (nt <= 0) return;
+    if (start < 0 || nt <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int dk = p.dk, kvh = head / (p.heads / p.kv_heads), dc = p.decay_channels;
     float* ws = p.ws + dc_slot(r0, seq, chunk, p.heads, head);
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
     // A and B: a warp takes four rows, a lane four channels; walking j downwards, the decays between the tokens grow factor
     // by factor. The sums over the lanes go 32 at a time (four j of four rows and two matrices).
     {
-        const int i0 = warp * 4;
+        const int i0 = (warp < 4 ? warp : 11 - warp) * 4;  // (a scheduler's two warps have nine groups of four rows between them)
         dc_pair qi[4][2], ki[4][2], d[4][2];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunk
         }
     }
     __syncthreads();
+    gb_pdl_launch_dependents();
     // the operands in the order of the fragments
     const int g = lane >> 2, t4 = lane & 3;
     for (int it = warp; it < 52; it += DC_THREADS / 32) {
@@ -339,16 +341,14 @@ template <int NT>
 __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArgs p) {
     __shared__ float red[NT][8][DC_C][8];                    // T K P S by warp (16 channels each): [column group][warp][token][column]
     __shared__ __align__(16) unsigned short Ub[NT][3][8][DC_C];     // U's terms by column
-    gb_pdl_launch_dependents();
     gb_pdl_wait();
     const int head = blockIdx.y, seq = blockIdx.z;
-    if (p.seq_start_pos[seq] < 0) return;
-    const int slot = p.seq_slots[seq];
+    const int start = p.seq_start_pos[seq], slot = p.seq_slots[seq], r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];
+    if (start < 0) return;
     if (slot < 0 || slot >= p.num_slots) {
         if (threadIdx.x == 0) atomicOr(p.status, GB_STATUS_BAD_SLOT);
         return;
     }
-    const int r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];
     const int chunks = (r1 - r0 + DC_C - 1) / DC_C;
     if (chunks <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -455,6 +455,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArg
             step(chunk + i, o[i]);
         }
     }
+    gb_pdl_launch_dependents();
     if (p.write_state) {
 #pragma unroll
         for (int n = 0; n < NT; ++n)
@@ -469,14 +470,12 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArg
 // O = (Q P) S_0 + B U: a warp takes two groups of 8 columns.
 __global__ void __launch_bounds__(DC_THREADS, 2) delta_out_kernel(DeltaChunkArgs p) {
     __shared__ uint4 left[20 * DC_FRAG / 4];                 // the left operands: Q P, then B
-    gb_pdl_launch_dependents();
     gb_pdl_wait();
+    gb_pdl_launch_dependents();
     const int chunk = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
-    if (p.seq_start_pos[seq] < 0) return;
-    const int slot = p.seq_slots[seq];
-    if (slot < 0 || slot >= p.num_slots) return;
-    const int r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1], c0 = r0 + chunk * DC_C;
-    if (c0 >= r1) return;
+    const int start = p.seq_start_pos[seq], slot = p.seq_slots[seq], r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];
+    const int c0 = r0 + chunk * DC_C;
+    if (start < 0 || slot < 0 || slot >= p.num_slots || c0 >= r1) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const float* ws = p.ws + dc_slot(r0, seq, chunk, p.heads, head);
     for (int i = threadIdx.x; i < 20 * DC_FRAG / 4; i += DC_THREADS) dc_cp16(left + i, ws + DC_AT_QP + 4 * i);      // Q P and B

@@ -1554,17 +1554,18 @@ def channel_delta(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bia
 
 #: the delta rule runs in chunks of tokens instead of token by token from this many rows of a step on, and so many more for
 #: every request of the step
-DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 88, 7
+DELTA_CHUNKS_FROM, DELTA_CHUNKS_PER_REQUEST = 72, 7
 
 
 def delta_chunks_chosen(rows: int, num_seqs: int, dk: int) -> bool:
     """Whether the delta rule takes a step of ``rows`` rows in ``num_seqs`` requests in chunks of 32 tokens (key sizes up to 128).
     Both numbers are part of a recorded step's shape, which the longest portion is not. A request costs the chunks its state's way in and
     out, a row costs the walk its place in the chain. Measured, kernels alone, heads of 128 x 128, walk / chunks in us at 8 heads and at
-    16: one request of 64 rows 27 / 35 and 27 / 37, 96 rows 36 / 37 and 37 / 34, 200 rows 68 / 36 and 69 / 44; 8 requests of 64 rows in
-    all 27 / 38 and 48 / 52, 128 rows 42 / 38 and 74 / 52; 36 requests (prompts' ends) of 180 rows 85 / 79 and 166 / 159, of 324 rows 118
-    / 79 and 231 / 160; 35 single tokens beside a portion of 30 rows 76 / 78 and 138 / 160, of 100 rows 105 / 102 and 177 / 183, of 300
-    rows 173 / 118 and 276 / 206; 64 requests of 320 rows 149 / 149 and 294 / 290, of 1,024 rows 290 / 151 and 585 / 293."""
+    16: one request of 64 rows 27 / 27 and 28 / 28, 80 rows 32 / 27 and 33 / 30, 200 rows 69 / 32 and 70 / 40; two of 48 rows 23 / 28 and
+    43 / 32, of 64 rows 28 / 28 and 53 / 32; 8 requests of 64 rows in all 28 / 34 and 49 / 47, 128 rows 43 / 34 and 76 / 48; 36 requests
+    (prompts' ends) of 180 rows 86 / 77 and 167 / 157, of 324 rows 119 / 78 and 233 / 158; 35 single tokens beside a portion of 30 rows 77 / 77 and
+    139 / 158, of 100 rows 106 / 100 and 179 / 180, of 300 rows 174 / 114 and 278 / 202; 64 requests of 320 rows 150 / 147 and 296 / 285, of 1,024
+    rows 291 / 148 and 588 / 287."""
     return dk <= 128 and rows >= DELTA_CHUNKS_FROM + DELTA_CHUNKS_PER_REQUEST * num_seqs
 
 
