@@ -40,7 +40,7 @@ constexpr int DC_V = 128;                           // columns of S that one pas
 constexpr int DC_RP = DC_K + 8;                     // floats from row to row in shared memory: a fragment's 8-byte loads hit 32 banks
 constexpr int DC_TP = DC_C + 4;                     // ... of A and B
 constexpr int DC_THREADS = 256;
-// The workspace of a (chunk, head), in 32-bit words. Fragments of mma.m16n8k16, [tile][3 terms][32 lanes][4 words]:
+// The workspace of a (chunk, head), in 32-bit words (162 KB; with the operands as float32 and no S_0 it was 60). Fragments of mma.m16n8k16, [tile][3 terms][32 lanes][4 words]:
 //   T K P   [8 groups of 16 channels][2 groups of 16 tokens]       rows tokens, k channels
 //   K D     [8 groups of 16 channels][2 halves of each 8 tokens]   rows channels, k tokens (lane t of four: 8 t + 4 half ..)
 //   Q P     as T K P
@@ -68,8 +68,11 @@ struct DeltaChunkArgs {
     const int* seq_start_pos;
     const int* seq_slots;
     float* ws;
-    int heads, kv_heads, dk, dv, num_slots, write_state, decay_channels;
+    int heads, kv_heads, dk, dv, num_slots, write_state, decay_channels, num_seqs;
     int col0, cols;         // the columns of S of this pass: at most DC_V
+    int window, room;       // the chunks of this pass, by their places: `room` of them from `window` on
+    const float* from;      // S of the request that began in the pass before, [heads][128][128]
+    float* to;              // ... of the one that goes on in the next
     int* status;
 };
 
@@ -118,10 +121,36 @@ __device__ __forceinline__ void dc_mma_add(float (&c)[4], const uint4& a, uint32
 constexpr int DC_PRODUCTS = 6;
 __device__ constexpr int DC_A_TERM[DC_PRODUCTS] = {2, 0, 1, 1, 0, 0}, DC_B_TERM[DC_PRODUCTS] = {0, 2, 1, 0, 1, 0};
 
-// where a request's chunks lie in the workspace: requests own rows one after the other, so r0 / 32 + seq leaves room for
-// each one's last, ragged chunk
-__device__ __forceinline__ size_t dc_slot(int r0, int seq, int chunk, int heads, int head) {
-    return ((size_t)(r0 / DC_C + seq + chunk) * heads + head) * DC_WS;
+// A chunk's place: requests own rows one after the other, so r0 / 32 + seq leaves room for each one's last, ragged chunk. The workspace
+// holds the places of a pass.
+__device__ __forceinline__ size_t dc_slot(const DeltaChunkArgs& p, int r0, int seq, int chunk, int head) {
+    return ((size_t)(r0 / DC_C + seq + chunk - p.window) * p.heads + head) * DC_WS;
+}
+// What a block of prepare or read-out works on. SEARCH: x is a place of the pass, y the head, and a warp looks the request up, the last whose
+// first place is no higher; else x is the chunk and z the request.
+struct DcPlace {
+    int seq, chunk, start, slot, r0, r1;
+};
+template <bool SEARCH> __device__ __forceinline__ DcPlace dc_place(const DeltaChunkArgs& p) {
+    DcPlace at = {(int)blockIdx.z, (int)blockIdx.x, -1, -1, 0, 0};
+    if (!SEARCH) {
+        at.start = p.seq_start_pos[at.seq]; at.slot = p.seq_slots[at.seq];                                  // (requested together)
+        at.r0 = p.seq_first_row[at.seq]; at.r1 = p.seq_first_row[at.seq + 1];
+        return at;
+    }
+    const int lane = threadIdx.x & 31, place = p.window + (int)blockIdx.x;
+    for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
+        const int s = min(s0 + lane, p.num_seqs - 1), r0 = p.seq_first_row[s], r1 = p.seq_first_row[s + 1], start = p.seq_start_pos[s], slot = p.seq_slots[s];
+        const unsigned up_to = __ballot_sync(0xffffffffu, s0 + lane < p.num_seqs && r0 / DC_C + s <= place);
+        if (up_to == 0) break;
+        const int l = 31 - __clz(up_to);
+        at.seq = s0 + l;
+        at.start = __shfl_sync(0xffffffffu, start, l); at.slot = __shfl_sync(0xffffffffu, slot, l);
+        at.r0 = __shfl_sync(0xffffffffu, r0, l); at.r1 = __shfl_sync(0xffffffffu, r1, l);
+        if (up_to != 0xffffffffu) break;
+    }
+    at.chunk = place - (at.r0 / DC_C + at.seq);
+    return at;
 }
 
 // Sums v[0..31] over the warp's lanes; lane l receives the sum of v[l].
@@ -138,19 +167,19 @@ __device__ __forceinline__ float dc_transpose_sum(float (&v)[32], int lane) {
     return v[0];
 }
 
+template <bool SEARCH>
 __global__ void __launch_bounds__(DC_THREADS, 2) delta_prepare_kernel(DeltaChunkArgs p) {
     extern __shared__ __align__(16) float dc_mem[];
     float* Q = dc_mem, *K = Q + DC_C * DC_RP, *G = K + DC_C * DC_RP;       // [32][136] each
     __shared__ __align__(16) float A[DC_C][DC_TP], B[DC_C][DC_TP];
     __shared__ float beta_s[DC_C];
     gb_pdl_wait();
-    const int chunk = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
-    const int start = p.seq_start_pos[seq], r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];      // (requested together)
-    const int c0 = r0 + chunk * DC_C, nt = min(DC_C, r1 - c0);
-    if (start < 0 || nt <= 0) return;
+    const DcPlace at = dc_place<SEARCH>(p);
+    const int head = blockIdx.y, c0 = at.r0 + at.chunk * DC_C, nt = min(DC_C, at.r1 - c0);
+    if (at.start < 0 || nt <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int dk = p.dk, kvh = head / (p.heads / p.kv_heads), dc = p.decay_channels;
-    float* ws = p.ws + dc_slot(r0, seq, chunk, p.heads, head);
+    float* ws = p.ws + dc_slot(p, at.r0, at.seq, at.chunk, head);
     const float rate = expf(p.a_log[head]);
 
     // rows of the chunk: a token past its end is k = q = 0, decay 1, beta 0 and changes nothing
@@ -349,12 +378,14 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArg
         if (threadIdx.x == 0) atomicOr(p.status, GB_STATUS_BAD_SLOT);
         return;
     }
-    const int chunks = (r1 - r0 + DC_C - 1) / DC_C;
+    // its chunks in this pass
+    const int place = r0 / DC_C + seq, all = (r1 - r0 + DC_C - 1) / DC_C;
+    const int chunk0 = max(p.window - place, 0), chunks = min(all, p.window + p.room - place) - chunk0;
     if (chunks <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int dk = p.dk, dv = p.dv, col0 = blockIdx.x * 8 * NT;              // (of this pass)
     float* sbase = p.state + (size_t)slot * p.state_stride + (size_t)head * dk * dv + p.col0;
-    float* ws0 = p.ws + dc_slot(r0, seq, 0, p.heads, head);
+    float* ws0 = p.ws + dc_slot(p, r0, seq, chunk0, head);
     const size_t ws_step = (size_t)p.heads * DC_WS;
     const int ti = tid >> 3, tc = tid & 7;                   // a thread's token and column between the two products
     const int ch = warp * 16 + g;
@@ -365,7 +396,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArg
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int d = ch + 8 * (e >> 1), c = col0 + 8 * n + 2 * t4 + (e & 1);
-            S[n][e] = d < dk && c < p.cols ? sbase[(size_t)d * dv + c] : 0.f;
+            S[n][e] = d < dk && c < p.cols ? (chunk0 ? p.from[((size_t)head * DC_K + d) * DC_V + c] : sbase[(size_t)d * dv + c]) : 0.f;
         }
     auto load = [&](int chunk, DeltaOperands<NT>& o) {
         const float* ws = ws0 + chunk * ws_step;
@@ -456,28 +487,29 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArg
         }
     }
     gb_pdl_launch_dependents();
-    if (p.write_state) {
+    const bool goes_on = chunk0 + chunks < all;
+    if (goes_on || p.write_state) {
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int d = ch + 8 * (e >> 1), c = col0 + 8 * n + 2 * t4 + (e & 1);
-                if (d < dk && c < p.cols) sbase[(size_t)d * dv + c] = S[n][e];
+                if (d < dk && c < p.cols) *(goes_on ? p.to + ((size_t)head * DC_K + d) * DC_V + c : sbase + (size_t)d * dv + c) = S[n][e];
             }
     }
 }
 
 // O = (Q P) S_0 + B U: a warp takes two groups of 8 columns.
+template <bool SEARCH>
 __global__ void __launch_bounds__(DC_THREADS, 2) delta_out_kernel(DeltaChunkArgs p) {
     __shared__ uint4 left[20 * DC_FRAG / 4];                 // the left operands: Q P, then B
     gb_pdl_wait();
     gb_pdl_launch_dependents();
-    const int chunk = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
-    const int start = p.seq_start_pos[seq], slot = p.seq_slots[seq], r0 = p.seq_first_row[seq], r1 = p.seq_first_row[seq + 1];
-    const int c0 = r0 + chunk * DC_C;
-    if (start < 0 || slot < 0 || slot >= p.num_slots || c0 >= r1) return;
+    const DcPlace at = dc_place<SEARCH>(p);
+    const int head = blockIdx.y, c0 = at.r0 + at.chunk * DC_C, r1 = at.r1;
+    if (at.start < 0 || at.slot < 0 || at.slot >= p.num_slots || c0 >= r1) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-    const float* ws = p.ws + dc_slot(r0, seq, chunk, p.heads, head);
+    const float* ws = p.ws + dc_slot(p, at.r0, at.seq, at.chunk, head);
     for (int i = threadIdx.x; i < 20 * DC_FRAG / 4; i += DC_THREADS) dc_cp16(left + i, ws + DC_AT_QP + 4 * i);      // Q P and B
     asm volatile("cp.async.commit_group;");
     // (a group of columns past this pass's last has a slot, which nothing wrote: its sums are not stored)
@@ -581,43 +613,59 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_out_kernel(DeltaChunkArgs
 }
 
 GB_EXPORT int gb_delta_chunk_rows() { return DC_C; }
-GB_EXPORT int gb_delta_chunk_floats() { return DC_WS; }            // workspace of a (chunk, head)
+GB_EXPORT int gb_delta_chunk_floats() { return DC_WS; }                 // workspace of a (chunk, head)
+GB_EXPORT int gb_delta_carry_floats() { return 2 * DC_K * DC_V; }       // ... of a head beside the chunks', where a call takes several passes
 
-// As gb_channel_delta (delta_rule.cu) for key sizes up to 128 (value columns in passes of 128), with a workspace of n / 32 + S chunks of heads *
-// gb_delta_chunk_floats() numbers, 16-byte aligned. max_rows: the most rows that a request brings.
+// As gb_channel_delta (delta_rule.cu) for key sizes up to 128 (value columns in passes of 128), with a workspace of `room` chunks of heads *
+// gb_delta_chunk_floats() numbers, 16-byte aligned. A call of n rows in S requests has n / 32 + S places for chunks; where room is less,
+// it takes them in passes, one behind the other, and heads * gb_delta_carry_floats() numbers lie behind the chunks.
+// max_rows: the most rows that a request brings.
 GB_EXPORT int gb_channel_delta_chunks(const float* qkv, long long ldq, const float* beta, long long ldb, const float* a, long long lda,
                                       const float* dt_bias, const float* a_log, float* state, long long state_stride, float* out,
-                                      const int* seq_first_row, const int* seq_start_pos, const int* seq_slots, int S, int max_rows, int heads,
+                                      const int* seq_first_row, const int* seq_start_pos, const int* seq_slots, int n, int S, int max_rows, int heads,
                                       int kv_heads, int dk, int dv, int num_slots, int write_state, int* status, int decay_channels,
-                                      float* ws, cudaStream_t stream) {
-    GB_REQUIRE(S >= 0 && S <= 65535 && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0,
+                                      float* ws, int room, cudaStream_t stream) {
+    GB_REQUIRE(n >= 0 && S >= 0 && S <= 65535 && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0,
                "gb_channel_delta_chunks: heads %d must be a multiple of key heads %d", heads, kv_heads);
     GB_REQUIRE(decay_channels == 1 || decay_channels == dk, "gb_channel_delta_chunks: %d decays per head (one, or one per key channel)",
                decay_channels);
     GB_REQUIRE(dk > 0 && dk <= DC_K && dv > 0, "gb_channel_delta_chunks: a key size of %d is outside 1..%d", dk, DC_K);
-    GB_REQUIRE((uintptr_t)ws % 16 == 0, "gb_channel_delta_chunks: the workspace must be 16-byte aligned");
+    GB_REQUIRE((uintptr_t)ws % 16 == 0 && room > 0, "gb_channel_delta_chunks: the workspace must be 16-byte aligned and hold a chunk");
     if (S == 0 || max_rows <= 0) return 0;
     DeltaChunkArgs p = {qkv, ldq, beta, ldb, a, lda, dt_bias, a_log, state, state_stride, out, seq_first_row, seq_start_pos, seq_slots,
-                        ws, heads, kv_heads, dk, dv, num_slots, write_state, decay_channels, 0, 0, status};
+                        ws, heads, kv_heads, dk, dv, num_slots, write_state, decay_channels, S, 0, 0, 0, room, nullptr, nullptr, status};
+    const int places = n / DC_C + S, chunks = gb_ceil_div(max_rows, DC_C);
+    float* carry = ws + (size_t)room * heads * DC_WS;
+    // A recorded step gives its shape's longest possible portion, with which a grid of requests by chunks is mostly empty: beyond twice the
+    // places the request is looked up (8 heads, 32 prompts of 16 tokens as one step 90 us with that grid, 74 so; 64 of 64 394 and 254).
+    const bool search = places > room || (long long)S * chunks > 2LL * places;
+    auto prepare = search ? delta_prepare_kernel<true> : delta_prepare_kernel<false>;
+    auto read_out = search ? delta_out_kernel<true> : delta_out_kernel<false>;
     const int prepare_smem = 3 * DC_C * DC_RP * 4;
-    cudaError_t e = cudaFuncSetAttribute(delta_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_smem);
+    cudaError_t e = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_smem);
     GB_REQUIRE(e == cudaSuccess, "gb_channel_delta_chunks: %d bytes of shared memory refused: %s", prepare_smem, cudaGetErrorString(e));
-    const dim3 every(gb_ceil_div(max_rows, DC_C), heads, S);
     for (p.col0 = 0; p.col0 < dv; p.col0 += DC_V) {
         p.cols = dv - p.col0 < DC_V ? dv - p.col0 : DC_V;
-        gb_launch(GB_PDL_ATTENTION, delta_prepare_kernel, every, dim3(DC_THREADS), prepare_smem, stream, p);
-        int rc = gb_check_launch("gb_channel_delta_chunks (prepare)");
-        if (rc) return rc;
-        const long long narrow = (long long)gb_ceil_div(p.cols, 8) * heads * S;
-        if (narrow <= 148)
-            gb_launch(GB_PDL_ATTENTION, delta_scan_kernel<1>, dim3(gb_ceil_div(p.cols, 8), heads, S), dim3(DC_THREADS), 0, stream, p);
-        else
-            gb_launch(GB_PDL_ATTENTION, delta_scan_kernel<2>, dim3(gb_ceil_div(p.cols, 16), heads, S), dim3(DC_THREADS), 0, stream, p);
-        rc = gb_check_launch("gb_channel_delta_chunks (scan)");
-        if (rc) return rc;
-        gb_launch(GB_PDL_ATTENTION, delta_out_kernel, every, dim3(DC_THREADS), 0, stream, p);
-        rc = gb_check_launch("gb_channel_delta_chunks (read-out)");
-        if (rc) return rc;
+        int pass = 0;
+        for (p.window = 0; p.window < places; p.window += room, ++pass) {
+            const int here = places - p.window < room ? places - p.window : room;
+            const dim3 every = search ? dim3(here, heads) : dim3(chunks, heads, S);
+            p.from = carry + (size_t)((pass + 1) & 1) * heads * DC_K * DC_V;
+            p.to = carry + (size_t)(pass & 1) * heads * DC_K * DC_V;
+            gb_launch(GB_PDL_ATTENTION, prepare, every, dim3(DC_THREADS), prepare_smem, stream, p);
+            int rc = gb_check_launch("gb_channel_delta_chunks (prepare)");
+            if (rc) return rc;
+            const long long narrow = (long long)gb_ceil_div(p.cols, 8) * heads * S;
+            if (narrow <= 148)
+                gb_launch(GB_PDL_ATTENTION, delta_scan_kernel<1>, dim3(gb_ceil_div(p.cols, 8), heads, S), dim3(DC_THREADS), 0, stream, p);
+            else
+                gb_launch(GB_PDL_ATTENTION, delta_scan_kernel<2>, dim3(gb_ceil_div(p.cols, 16), heads, S), dim3(DC_THREADS), 0, stream, p);
+            rc = gb_check_launch("gb_channel_delta_chunks (scan)");
+            if (rc) return rc;
+            gb_launch(GB_PDL_ATTENTION, read_out, every, dim3(DC_THREADS), 0, stream, p);
+            rc = gb_check_launch("gb_channel_delta_chunks (read-out)");
+            if (rc) return rc;
+        }
     }
     return 0;
 }

@@ -131,9 +131,10 @@ _SIGNATURES = {
     "gb_talk_combine": [_P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _P],
     "gb_short_conv": [_P, _LL, _P, _P, _LL, _P, _LL, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "gb_channel_delta": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P],
-    "gb_channel_delta_chunks": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P],
+    "gb_channel_delta_chunks": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _P],
     "gb_delta_chunk_rows": [],
     "gb_delta_chunk_floats": [],
+    "gb_delta_carry_floats": [],
     "gb_channel_delta_decode_supported": [_I, _I],
     "gb_channel_delta_decode": [_P, _LL, _P, _LL, _P, _LL, _P, _P, _P, _LL, _P, _LL, _P, _F, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I,
                                 _I, _I, _P, _P, _LL, _P, _LL, _I, _I, _I, _I, _P, _P, _I, _I, _I, _P],
@@ -1578,13 +1579,27 @@ def delta_chunk_floats() -> int:
     return lib().gb_delta_chunk_floats()
 
 
+#: a step of more chunks takes them in passes: at 162 KB a chunk and head, 16 heads, 8,192 rows and 64 slots would hold a gigabyte, and hold 332
+#: MB so. Passes / one, us: 8 heads, one request of 4,096 rows 263 / 258, of 8,192 520 / 495, 64 of 64 rows 287 / 254; 16 heads 443 / 434, 881 / 855
+#: and 528 / 476
+DELTA_WORKSPACE_CHUNKS = 128
+
+
+def delta_workspace_floats(chunks: int, heads: int) -> int:
+    """Numbers of a workspace with which ``channel_delta_chunks`` takes any step that needs up to ``chunks`` chunks, in passes of
+    ``DELTA_WORKSPACE_CHUNKS`` where they are more."""
+    if chunks <= DELTA_WORKSPACE_CHUNKS:
+        return chunks * heads * delta_chunk_floats()
+    return heads * (DELTA_WORKSPACE_CHUNKS * delta_chunk_floats() + lib().gb_delta_carry_floats())
+
+
 def channel_delta_chunks(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
                          state: torch.Tensor, out: torch.Tensor, seq_first_row: torch.Tensor, seq_start_pos: torch.Tensor,
                          seq_slots: torch.Tensor, max_rows_per_seq: int, heads: int, kv_heads: int, dk: int, dv: int, write_state: bool,
                          status: torch.Tensor, workspace: torch.Tensor, decay_per_head: bool = False) -> None:
     """``channel_delta`` with the tokens of a request taken 32 at a time (the same sums in another order, float32
-    throughout). ``workspace`` float32 [chunks, heads * delta_chunk_floats()] is scratch, chunks = ``delta_chunks_needed``;
-    no request may bring more than ``max_rows_per_seq`` rows."""
+    throughout). ``workspace`` float32, ``delta_workspace_floats(delta_chunks_needed(n, S), heads)`` numbers or more, is scratch (fewer
+    make more passes); no request may bring more than ``max_rows_per_seq`` rows."""
     _cuda(qkv, beta, a, dt_bias, a_log, state, out, seq_first_row, seq_start_pos, seq_slots, status, workspace)
     n, S = qkv.shape[0], seq_start_pos.shape[0]
     dc = 1 if decay_per_head else dk
@@ -1594,12 +1609,16 @@ def channel_delta_chunks(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor,
     assert a.shape == (n, heads * dc) and a.stride(1) == 1 and beta.stride(1) == 1 and out.shape == (n, heads * dv)
     assert out.is_contiguous() and state.dim() == 2 and state.is_contiguous() and state.shape[1] >= heads * dk * dv
     assert dt_bias.numel() == heads * dc and a_log.numel() == heads
-    assert workspace.is_contiguous() and workspace.numel() >= delta_chunks_needed(n, S) * heads * delta_chunk_floats()
+    room = needed = delta_chunks_needed(n, S)
+    if workspace.numel() < needed * heads * delta_chunk_floats():
+        room = (workspace.numel() // heads - lib().gb_delta_carry_floats()) // delta_chunk_floats()
+    assert workspace.is_contiguous() and (room > 0 or needed == 0)
     _call("gb_channel_delta_chunks", _ptr(qkv), qkv.stride(0), _ptr(beta), beta.stride(0), _ptr(a), a.stride(0), _ptr(dt_bias),
-          _ptr(a_log), _ptr(state), state.stride(0), _ptr(out), _ptr(seq_first_row), _ptr(seq_start_pos), _ptr(seq_slots), S,
-          int(max_rows_per_seq), heads, kv_heads, dk, dv, state.shape[0], 1 if write_state else 0, _ptr(status), dc, _ptr(workspace), _stream())
+          _ptr(a_log), _ptr(state), state.stride(0), _ptr(out), _ptr(seq_first_row), _ptr(seq_start_pos), _ptr(seq_slots), n, S,
+          int(max_rows_per_seq), heads, kv_heads, dk, dv, state.shape[0], 1 if write_state else 0, _ptr(status), dc, _ptr(workspace),
+          max(room, 1), _stream())
     global launch_count
-    launch_count += 1
+    launch_count += 3 * -(-needed // max(room, 1)) * -(-dv // 128) - 1         # (three kernels a pass of chunks and 128 value columns)
 
 
 CD_SILU_INPUTS, CD_PLAIN, CD_GATE_SILU, CD_NO_NORM = 1, 2, 4, 8

@@ -34,7 +34,7 @@ def run_delta(ctx, qkv, beta, decay, params, state, out, heads: int, kv_heads: i
     # One workspace for all steps, recorded or not (they never overlap): what the largest step needs. A recorded step's sequences
     # are at most its single tokens rounded up to eight and its portions rounded up to a power of two, of one slot each.
     most = max(kernels.delta_chunks_needed(ctx.max_rows, 2 * state.shape[0] + 8), kernels.delta_chunks_needed(qkv.shape[0], ctx.seq_start_pos.shape[0]))
-    work = ctx.flat(f"delta_chunks_{heads}", most * heads * kernels.delta_chunk_floats(), torch.float32)
+    work = ctx.flat(f"delta_chunks_{heads}", kernels.delta_workspace_floats(most, heads), torch.float32)
     kernels.channel_delta_chunks(*args, ctx.max_rows_per_seq, heads, kv_heads, dk, dv, writes_cache, ctx.status, work,
                                  decay_per_head=decay_per_head)
 

@@ -44,8 +44,9 @@ def _truth(lens, H, KH, D, V, per_head, qkv, beta, a, dt_bias, a_log, states):
     return np.concatenate(outs), np.stack(after)
 
 
-def _run(chunked, lens, H, KH, D, V, per_head, qkv, beta, a, dt_bias, a_log, states, padding=False):
-    """Requests in slots in reverse order; with ``padding`` a padding sequence of two rows in front."""
+def _run(chunked, lens, H, KH, D, V, per_head, qkv, beta, a, dt_bias, a_log, states, padding=False, room=None, most=None):
+    """Requests in slots in reverse order; with ``padding`` a padding sequence of two rows in front. ``room``: the workspace's chunks, if fewer
+    than the step needs; ``most``: the bound of a request's rows, if more than they are."""
     from glassbox_b200 import kernels
     f = lambda x: torch.tensor(x.copy(), dtype=torch.float32, device=DEV)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
@@ -62,7 +63,9 @@ def _run(chunked, lens, H, KH, D, V, per_head, qkv, beta, a, dt_bias, a_log, sta
     args = (pad(qkv), pad(beta), pad(a), f(dt_bias), f(a_log), state, out, first, start, slots)
     if chunked:
         work = torch.full((kernels.delta_chunks_needed(sum(rows), len(rows)), H * kernels.delta_chunk_floats()), float("nan"), device=DEV)
-        kernels.channel_delta_chunks(*args, max(rows), H, KH, D, V, True, status, work, decay_per_head=per_head)
+        if room is not None:
+            work = torch.full((H * (room * kernels.delta_chunk_floats() + kernels.lib().gb_delta_carry_floats()),), float("nan"), device=DEV)
+        kernels.channel_delta_chunks(*args, most or max(rows), H, KH, D, V, True, status, work, decay_per_head=per_head)
     else:
         kernels.channel_delta(*args, H, KH, D, V, True, status, decay_per_head=per_head)
     assert int(status) == 0 and torch.all(state[S] == 3.0) and torch.all(state[:, H * D * V:] == 3.0)
@@ -194,3 +197,21 @@ def test_a_short_prompt_is_no_slower_in_chunks():
             spans.append(a.elapsed_time(b))
         times.append(min(spans))
     assert times[0] < 0.9 * times[1], times
+
+
+@pytest.mark.parametrize("padding", [False, True])
+@pytest.mark.parametrize("H, KH, D, V, lens", [(2, 1, 128, 128, [31, 200, 1, 33, 96]), (3, 3, 64, 150, [300]), (1, 1, 40, 24, [5] * 40 + [70, 64])])
+def test_passes_and_bounds_give_the_same_bits(H, KH, D, V, lens, padding):
+    """A workspace that holds a part of the chunks, down to one, and a bound of the rows that is far above them."""
+    data = _inputs(lens, H, KH, D, V, False, V)
+    want = _run(True, lens, H, KH, D, V, False, *data, padding=padding)
+    for room, most in ((None, 4096), (1, None), (3, 1000), (7, None)):
+        got = _run(True, lens, H, KH, D, V, False, *data, padding=padding, room=room, most=most)
+        assert all(np.array_equal(g, w) for g, w in zip(got, want)), (room, most)
+
+
+def test_the_workspace_stays_within_bounds():
+    from glassbox_b200 import kernels
+    for rows, slots, heads in ((2048, 8, 16), (8192, 64, 16), (1 << 17, 256, 32)):
+        floats = kernels.delta_workspace_floats(kernels.delta_chunks_needed(rows, 2 * slots + 8), heads)
+        assert floats * 4 <= heads * (24 << 20), (rows, slots)              # 128 chunks of 162 KB and the carried states
