@@ -368,7 +368,7 @@ template <int NT> struct DeltaOperands {                     // what a chunk bri
 
 template <int NT>
 __global__ void __launch_bounds__(DC_THREADS, 1) delta_scan_kernel(DeltaChunkArgs p) {
-    __shared__ float red[NT][8][DC_C][8];                    // T K P S by warp (16 channels each): [column group][warp][token][column]
+    __shared__ __align__(16) float red[NT][8][DC_C][8];      // T K P S by warp (16 channels each): [column group][warp][token][column]
     __shared__ __align__(16) unsigned short Ub[NT][3][8][DC_C];     // U's terms by column
     gb_pdl_wait();
     const int head = blockIdx.y, seq = blockIdx.z;
