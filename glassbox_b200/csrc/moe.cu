@@ -294,8 +294,9 @@ __global__ void __launch_bounds__(RB > 1 ? MOE_ROUTE_THREADS / 2 : MOE_ROUTE_THR
 }
 
 // The logits of many bfloat16 rows on the tensor cores (mma.sync): 16 rows a block, the K of their products dealt out to 16 warps in pieces
-// of 32, sums over the warps in shared memory, then a warp per row chooses. A router weight is the exact sum of three bfloat16 numbers; the
-// largest product of 16 channels has an accumulator of its own and is added in float32 (the tensor core cuts what it adds to).
+// of 32, sums over the warps in shared memory, then a warp per row chooses. A router weight is the exact sum of three bfloat16 numbers, all of
+// whose products with a row's are kept; the largest product of 16 channels has an accumulator of its own and is added in float32 (the
+// tensor core cuts what it adds to).
 // Operands come straight from memory in 16-byte loads: a lane's eight neighbouring channels stand for the fragment's pairs, the same way
 // on both sides. The FMA form brings every row through shared memory as float32 for every two experts: bound by those reads.
 // Measured, 16 experts, width 1,024, FMA / this, us: 300 rows 14.0 / 7.7, 2,048 rows 15.4 / 7.9;
@@ -430,7 +431,9 @@ GB_EXPORT int gb_moe_route(const void* h, int h_dtype, int d, const float* w_rou
     GB_REQUIRE(h_dtype == GB_F32 || h_dtype == GB_BF16, "gb_moe_route: unsupported dtype %d", h_dtype);
     if (n == 0) return 0;
     // From the rows on for which the FMA form takes eight rows a block: 256 rows, a row a block, 16 experts 5.7 us against 7.7, 128 experts
-    // 24 against 27.
+    // 24 against 27. The sums over K are taken in another order here, so a logit's low bits, and with them the choice between experts that
+    // are all but equal, depend on whether 256 rows or more are routed together (as a bfloat16 row's hidden numbers do on the products'
+    // forms, which are chosen by rows too).
     if (h_dtype == GB_BF16 && n > 256 && E <= MR_EMAX && d % 8 == 0 && (((uintptr_t)h | (uintptr_t)w_router | (uintptr_t)w_gate) & 15) == 0) {
         cudaError_t e = cudaFuncSetAttribute(moe_route_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MrShared));
         GB_REQUIRE(e == cudaSuccess, "gb_moe_route: %d bytes of shared memory refused: %s", (int)sizeof(MrShared), cudaGetErrorString(e));

@@ -46,3 +46,65 @@ def test_an_infinite_row_is_routed_as_by_fma():
         kernels.moe_route(rows, w, None, None, torch.arange(rows.shape[0], dtype=torch.int32, device=DEV), 2, 1, 1, 1.0, choice, weight, None)
         out.append((choice, weight))
     assert torch.equal(out[0][0][5], out[1][0][0]) and torch.equal(out[0][1][5], out[1][1][0])
+
+
+def _route64(z, top, groups, keep, correction, scoring, best):
+    """The chosen experts of one row by float64 logits, the scores, and the smallest difference on which a choice rested."""
+    score = torch.sigmoid(z) if scoring == "sigmoid" else torch.softmax(z, 0) if scoring == "softmax" else z
+    c, margin = score + correction, float("inf")
+    if groups > 1:
+        runs = c.view(groups, -1)
+        run = runs.amax(1) if best else runs.topk(2, 1).values.sum(1)
+        order = run.sort(descending=True)
+        margin = float(order.values[keep - 1] - order.values[keep])
+        c = torch.where(torch.isin(torch.arange(len(z)) // runs.shape[1], order.indices[:keep]), c, -float("inf"))
+    order = c.sort(descending=True)
+    margin = min(margin, float((order.values[:top] - order.values[1:top + 1]).min()))
+    return order.indices[:top], score, margin
+
+
+@pytest.mark.parametrize("E, top, d, scoring, groups, keep, options", [
+    (16, 4, 1024, "sigmoid", 4, 2, dict(correction=True, gate=True, renorm_eps=1e-20)),
+    (32, 3, 136, "softmax", 1, 1, dict(gate=True)),                       # (the gate is the first column of a turn of its own)
+    (40, 6, 72, "softmax", 8, 3, dict(group_best=True, renorm_eps=0.0)),
+    (128, 8, 520, "chosen", 1, 1, dict(bias=True)),
+    (31, 2, 2056, "chosen", 1, 1, dict(bias=True, gate=True)),
+])
+def test_both_forms_choose_alike(E, top, d, scoring, groups, keep, options):
+    """The same rows among 256 (by FMA) and among 257 and more (on the tensor cores): their sums are taken in another order, so that a
+    logit's low bits and with them the choice between all but equal experts differ; nothing else does."""
+    from glassbox_b200 import kernels
+    options, g, n = dict(options), torch.Generator().manual_seed(E), 272
+    h, w = torch.randn(n, d, generator=g).bfloat16().to(DEV), (torch.randn(E, d, generator=g) / d ** 0.5).to(DEV)
+    extra = torch.randn(E, generator=g) / 4
+    correction = extra.to(DEV) if options.pop("correction", False) else None
+    bias = extra.to(DEV) if options.pop("bias", False) else None
+    wg = (torch.randn(1, d, generator=g) / d ** 0.5).to(DEV) if options.pop("gate", False) else None
+    out = []
+    for step in (n, 257, 256):
+        parts = []
+        for at in range(0, n, step):
+            rows = h[at:at + step].contiguous()
+            m = rows.shape[0]
+            choice, weight, gate = torch.zeros(m, top, dtype=torch.int32, device=DEV), torch.zeros(m, top, device=DEV), torch.zeros(m, 1, device=DEV)
+            kernels.moe_route(rows, w, correction, wg, torch.arange(m, dtype=torch.int32, device=DEV), top, groups, keep, 1.0, choice, weight,
+                              gate if wg is not None else None, router_bias=bias, softmax_chosen=scoring == "chosen", softmax=scoring == "softmax", **options)
+            parts.append((choice.cpu(), weight.double().cpu(), gate.double().cpu()))
+        out.append([torch.cat(x) for x in zip(*parts)])
+    z = (h.double() @ w.double().T).cpu() + (extra.double() if bias is not None else 0.0)
+    clear = 0
+    for r in range(n):
+        want, score, margin = _route64(z[r], top, groups, keep, extra.double() if correction is not None else 0.0, scoring, options.get("group_best", False))
+        if margin < 2 ** -18:                               # (logits of up to four are off by some 2^-21 in either form)
+            continue
+        clear += 1
+        weight = torch.softmax(score[want], 0) if scoring == "chosen" else score[want]
+        if "renorm_eps" in options:
+            weight = weight / weight.sum()
+        for choice, weights, _ in out:
+            assert torch.equal(choice[r].long(), want), r
+            assert (weights[r] - weight).abs().max() <= 2 ** -20, r
+    assert clear > 0.9 * n
+    assert torch.equal(out[0][0][:257], out[1][0][:257]) and torch.equal(out[0][1][:257], out[1][1][:257])      # (one form: the same bits)
+    if wg is not None:
+        assert max(float((o[2] - torch.sigmoid(h.double() @ wg.double().T).cpu()).abs().max()) for o in out) <= 2 ** -20
