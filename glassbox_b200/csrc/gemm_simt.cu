@@ -1,8 +1,8 @@
 // C[M, N] (+)= A[M, K] * W[N, K]^T on the CUDA cores with float32 FMA only.
 //
-// This is the true 32-bit matrix product (no TF32, no tensor cores) and also the generic
-// fallback for any mix of float32 / bfloat16 operands at any size. The kernels:
-//   * register-tiled kernels with packed FMA for M > 8 (float32 activations, rows aligned to 16 bytes),
+// The generic product for any mix of float32 / bfloat16 operands at any size, and the one for up to eight float32 rows. (More of them run
+// gemm_f32_tc.cu where K is 64 or more and rows are whole 16-byte pieces.) The kernels:
+//   * register-tiled kernels with packed FMA for M > 8 (float32 activations, rows aligned to 16 bytes: the products of K below 64),
 //   * a 64x64x16 register-tiled kernel for every other M > 8,
 //   * weight-streaming kernels for M <= 8 (a block or a warp per four output columns, or a warp per column), which is what a
 //     decode step needs: every weight is read once, coalesced along K.

@@ -672,8 +672,8 @@ GB_EXPORT int gb_gemm_tcgen05_unit(const void* a, const void* w, void* c, int M,
                 : launch_tc<128, true>(ma, mw, c, TC_STORE_BF16, M, inter, K, ldc, inter, status, stream, TcQkv(), TcNorm(), unit);
 }
 
-// 1 if gb_gemm_tcgen05_qkv takes this head size: whole heads must tile the 128 columns of an output tile and half
-// a head must be a multiple of the 32 columns an epilogue thread reads at a time.
+// 1 if gb_gemm_tcgen05_qkv takes this head size: whole heads must tile the 128 columns of an output tile, and
+// the two warps that share a tile's rows take turns of 16 channels of half a head.
 GB_EXPORT int gb_gemm_tcgen05_qkv_supported(int hd) { return hd == 64 || hd == 128; }
 
 // Stacked QKV projection with rotary encoding and cache write in the epilogue: w = [q rows; k rows; v rows]

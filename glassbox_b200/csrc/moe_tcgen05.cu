@@ -3,7 +3,7 @@
 //
 // A tile is 128 of an expert's pairs x BN of its outputs; a block (one per SM) walks the tiles of all experts in turn, an
 // expert's tiles next to each other and its rows innermost, so that a piece of its matrix is read from memory once and from L2
-// by the expert's other row tiles. Six warps, as in the dense product (gemm_tcgen05.cu):
+// by the expert's other row tiles. Ten warps, as in the dense product (gemm_tcgen05.cu):
 //   warp 0     producer: per 64-wide k-block a TMA box of the expert's matrix and the 128 input rows. DOWN, and UP where the rows
 //              were gathered before (moe_gather_rows_kernel): the rows are the slots themselves, one box. UP otherwise: the rows of h
 //              lie anywhere (sorted[slot] / top); every lane fetches four of them by TMA gather, straight into the swizzled tile.
@@ -334,7 +334,7 @@ GB_EXPORT int gb_moe_grouped_gemm(const void* a, long long lda, int rows, const 
 #undef ME_CASE
 }
 
-// Rows of h in the order of the slots: out[slot, :] = h[sorted[slot] / top, :], a warp per row, four rows' pieces under way.
+// Rows of h in the order of the slots: out[slot, :] = h[sorted[slot] / top, :], a warp per row, four of a lane's 16-byte pieces under way.
 __global__ void __launch_bounds__(256) moe_gather_rows_kernel(const uint4* __restrict__ h, int pieces, const int* __restrict__ sorted,
                                                               const int* __restrict__ offsets, int E, int top, uint4* __restrict__ out) {
     gb_pdl_launch_dependents();

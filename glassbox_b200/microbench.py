@@ -712,17 +712,28 @@ def bench_babotar() -> None:
 
 
 def bench_float32() -> None:
-    """The kernels of the true 32-bit path at SmolLM2-135M shapes: FMA products for a 2,048-token prompt and for 8
-    decoded rows, split-key decode attention and one-warp-per-row attention over a float32 cache."""
+    """The kernels of the true 32-bit path at SmolLM2-135M shapes: products for a 2,048-token prompt (tensor cores) and for 8
+    decoded rows (FMA), prompt attention, split-key decode attention and one-warp-per-row attention over a float32 cache."""
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
     for name, m, n, k in [("135m qkv, 2048 rows", 2048, 960, 576), ("135m gate/up, 2048 rows", 2048, 3072, 576),
                           ("135m down, 2048 rows", 2048, 576, 1536), ("135m qkv, 8 rows", 8, 960, 576),
                           ("135m head, 8 rows", 8, 49152, 576)]:
         a, w, c = torch.randn(m, k, device=DEV), torch.randn(n, k, device=DEV), torch.empty(m, n, device=DEV)
-        t = graph_time(lambda: kernels.gemm_simt(a, w, c), reps=6)
-        print(f"gemm_simt {name:24s} {m} x {n} x {k}: {t:8.1f} us {2.0 * m * n * k / t / 1e6:6.2f} TFLOP/s "
+        product = kernels.gemm_f32_tc if kernels.gemm_f32_tc_chosen(a, w, c) else kernels.gemm_simt
+        t = graph_time(lambda: product(a, w, c), reps=6)
+        print(f"{product.__name__} {name:24s} {m} x {n} x {k}: {t:8.1f} us {2.0 * m * n * k / t / 1e6:6.2f} TFLOP/s "
               f"{(m * k + n * k + m * n) * 4 / t / 1e3:6.0f} GB/s", flush=True)
     nh, nkv, hd, ps, ctx = 9, 3, 64, 16, 4096
+    for lens, bound in (([2048], 2048), ([1000, 700, 347], 1000), ([16] * 32, 512)):
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        n, first = sum(lens), i32([sum(lens[:i]) for i in range(len(lens) + 1)])
+        per = -(-max(lens) // ps)
+        kc, q = torch.randn(per * len(lens), nkv, ps, hd, device=DEV), torch.randn(n, nh * hd, device=DEV)
+        vc, o, start = torch.randn_like(kc), torch.empty_like(q), i32([0] * len(lens))
+        tables = torch.arange(per * len(lens), dtype=torch.int32, device=DEV).view(len(lens), per)
+        t = graph_time(lambda: kernels.attention_prefill_f32(q, o, kc, vc, tables, first, start, bound, nh, nkv, hd, ps, hd ** -0.5, None, status))
+        print(f"attention_prefill_f32 {len(lens)} prompts of up to {max(lens)} rows (bound {bound}): {t:7.1f} us "
+              f"{sum(2.0 * k * k * nh * hd for k in lens) / t / 1e6:6.2f} TFLOP/s", flush=True)
     for m in (1, 8):
         per = ctx // ps
         kc = torch.randn(m * per + 4, nkv, ps, hd, device=DEV)

@@ -185,8 +185,9 @@ class GqaAttention(Mixer):
 #: otherwise add more 128-row tiles (one per request and head) than the GPU has SMs
 SPLIT_MIXED_ABOVE = 148
 
-#: up to this many tokens a request (cached and new) the one-warp kernel walks its few keys in less time than a 64 x 64 tile takes in
-#: float32: 32 prompts of 8 tokens at 32 heads 20 us against 30, at 9 heads 9 against 11; of 16 tokens 52 against 24 and 19 against 12
+#: up to this many tokens a request (cached and new) the one-warp kernel walks its few keys in less time than a tile of 64 rows takes in
+#: float32: 64 prompts of 8 tokens at 32 heads 31 us against 39, at 9 heads 12 against 15; 32 of 9 tokens 22 against 23 and 9.8 against 9.3,
+#: of 16 tokens 52 against 24 and 19 against 9.4
 FLASH_F32_MIN_CONTEXT = 8
 
 register_part("mixer", "gqa_attention", GqaAttention, replace=True)
