@@ -128,7 +128,8 @@ __device__ __forceinline__ float gb_gated_unit(float gate, float up, float limit
 
 // x and y as three bfloat16 each, every term what is left rounded to the nearest (8 + 8 + at most 8 bits: the terms' sum is the number, and
 // a term is below 2^-8 of the one before), packed with x in the low halves. A number that rounds to an infinity (from 2^128 - 2^119 on)
-// leaves a term that is no number, unless CLAMPED: its first term is then the largest bfloat16, and only infinities do.
+// leaves a term that is no number, unless CLAMPED: its first term is then the largest bfloat16, and only infinities do. Numbers below some
+// 2^-110 lose what lies under bfloat16's smallest number: 2^-134 at most.
 template <bool CLAMPED = false>
 __device__ __forceinline__ void gb_split_bf16(float x, float y, uint32_t (&term)[3]) {
 #pragma unroll
