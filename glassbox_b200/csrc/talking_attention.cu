@@ -13,7 +13,8 @@
 //                          channels (channel i with channel i + rot/2, a (cos, sin) table per position), q into the query
 //                          buffer, k and v into the paged cache at each row's slot
 //   talking_attention_rows one warp per (row, head), any row, both dtypes
-//   talking_attention_decode  single decoded tokens: a block of 8 warps per (row, heads of a group, share of the keys)
+//   talking_attention_decode  single decoded tokens: a block of 8 warps per (row, heads of a group, share of the keys); bfloat16 at the
+//                          sizes of talking_decode_mma.cu: the kernel there
 //   talking_attention_tiles   prompt portions in bfloat16 on the tensor cores (mma.sync), 64 rows x one head per block
 //   talk_combine           the mix of the heads' results (and the merge of the shares of the keys, if there are several)
 #include "common.cuh"
@@ -502,6 +503,11 @@ GB_EXPORT int gb_talking_attention_decode_plan(int H, int G, int V, int VG) {
     return 0;
 }
 
+int gb_talking_decode_mma(const void* q, float* out, float* ml, const void* kcache, const void* vcache, const int* block_tables,
+                          int max_pages, const int* row_seq, const int* positions, int n, int H, int G, int D, int V, int page_size,
+                          long long num_pages, float scale, float cap, float unit, int window, int shares, int* status, cudaStream_t stream);
+extern "C" int gb_talking_decode_mma_heads(int H, int G, int D, int V, int VG);
+
 // shares > 1: out is [shares][n][H][wide] and ml [shares][n][H][2], for talk_combine to merge; shares == 1: out is final
 GB_EXPORT int gb_talking_attention_decode(const void* q, float* out, float* ml, int dtype, const void* kcache, const void* vcache,
                                           const int* block_tables, int max_pages, const int* row_seq, const int* positions, int n, int H,
@@ -512,6 +518,12 @@ GB_EXPORT int gb_talking_attention_decode(const void* q, float* out, float* ml, 
     GB_REQUIRE(plan > 0, "gb_talking_attention_decode: %d value heads of %d channels are not built", VG, V);
     GB_REQUIRE(shares >= 1 && shares <= 64 && (shares == 1 || ml != nullptr), "gb_talking_attention_decode: %d shares", shares);
     if (n == 0) return 0;
+    // bfloat16 at the sizes it is built for: the tensor cores (its places in the pool are counted in 32 bits, its loads and stores 16 and
+    // 8 bytes wide)
+    if (dtype == GB_BF16 && gb_talking_decode_mma_heads(H, G, D, V, VG) > 0 && num_pages * G * page_size < (1LL << 31) &&
+        (((uintptr_t)q | (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0 && ((uintptr_t)out & 7) == 0)
+        return gb_talking_decode_mma(q, out, ml, kcache, vcache, block_tables, max_pages, row_seq, positions, n, H, G, D, V, page_size,
+                                     num_pages, scale, cap, unit, window, shares, status, stream);
     const int col_blocks = plan / 10000, R = plan % 10000 / 100, nc = plan % 100;
     const dim3 grid(n, H / R, shares * col_blocks);
     // (the vector form: bfloat16, a wide row of exactly 32 * nc channels, a lane's nc channels inside one value head)
@@ -867,6 +879,116 @@ __global__ void __launch_bounds__(256) talk_combine_kernel(const float* __restri
     }
 }
 
+// The same merge and mix where the results arrive in shares, four channels a thread. The block's loads of all shares (eight at a time
+// in flight) are asked for before the shares' weights are formed, a thread per (head, share), by way of shared memory. The form above
+// took one thread per head through three chains of dependent loads and two 4-byte loads at a time. 16 heads, 4 value heads of 64: 32 rows in
+// nine shares 8.5 -> 3.9 us, 16 rows in sixteen 8.7 -> 4.1.
+constexpr int TKS_FLY = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(256) talk_shares_kernel(const float* __restrict__ o, const float* __restrict__ ml,
+                                                          const float* __restrict__ talk, T* __restrict__ att,
+                                                          const int* __restrict__ positions, int n, int H, int G, int V, int shares,
+                                                          float unit, int quads) {
+    extern __shared__ __align__(16) float tks_smem[];
+    float* rows = tks_smem;                              // [H][4 * quads]: head g's merged result over this block's channels
+    float* s_m = rows + (size_t)H * quads * 4;           // [H][shares]: maxima, then weights of the shares
+    float* s_l = s_m + H * shares;                       // [H][shares]: denominators, then weighted ones
+    float* s_talk = s_l + H * shares;                    // [per][H]
+    gb_pdl_launch_dependents();
+    const int row = blockIdx.x, c = blockIdx.y, per = H / G, wide = G * V, ch0 = blockIdx.z * quads * 4;
+    for (int i = threadIdx.x; i < per * H; i += 256) s_talk[i] = talk[(size_t)c * per * H + i];      // (a weight)
+    if (positions[row] < 0) return;
+    gb_pdl_wait();
+    const int cells = H * quads;
+    const size_t stride = (size_t)n * H * wide;          // from a share to the next
+    const float* src0 = o + (size_t)row * H * wide + (size_t)c * V + ch0;
+    float4 x[TKS_FLY];
+    auto ask = [&](int cell, int z0) {
+        const float* src = src0 + (size_t)(cell / quads) * wide + cell % quads * 4;
+#pragma unroll
+        for (int u = 0; u < TKS_FLY; ++u)
+            if (z0 + u < shares) x[u] = *reinterpret_cast<const float4*>(src + (size_t)(z0 + u) * stride);
+    };
+    if (threadIdx.x < cells) ask(threadIdx.x, 0);
+    for (int i = threadIdx.x; i < H * shares; i += 256) {
+        const float2 v = *reinterpret_cast<const float2*>(ml + (((size_t)(i % shares) * n + row) * H + i / shares) * 2);
+        s_m[i] = v.x;
+        s_l[i] = v.y;
+    }
+    __syncthreads();
+    float f_mine[16];                                    // (H * shares <= 4096)
+    float d_mine[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        if (i >= H * shares) break;
+        float top = unit > 0.f ? 0.f : -INFINITY;
+        for (int z = 0; z < shares; ++z) top = fmaxf(top, s_m[i / shares * shares + z]);
+        const float m = s_m[i];
+        f_mine[k] = m == -INFINITY ? 0.f : expf(m - top);
+        d_mine[k] = s_l[i] * f_mine[k];
+        if (i % shares == 0 && unit > 0.f) d_mine[k] += unit * expf(-top);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        if (i >= H * shares) break;
+        s_m[i] = f_mine[k];
+        s_l[i] = d_mine[k];
+    }
+    __syncthreads();
+    for (int cell = threadIdx.x; cell < cells; cell += 256) {
+        const int g = cell / quads;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        float den = 0.f;
+        for (int z0 = 0; z0 < shares; z0 += TKS_FLY) {
+            if (z0 > 0 || cell != threadIdx.x) ask(cell, z0);
+#pragma unroll
+            for (int u = 0; u < TKS_FLY; ++u) {
+                if (z0 + u >= shares) break;
+                const float f = s_m[g * shares + z0 + u];
+                den += s_l[g * shares + z0 + u];
+                sum.x = fmaf(f, x[u].x, sum.x);
+                sum.y = fmaf(f, x[u].y, sum.y);
+                sum.z = fmaf(f, x[u].z, sum.z);
+                sum.w = fmaf(f, x[u].w, sum.w);
+            }
+        }
+        const float inv = den > 0.f ? 1.0f / den : 0.f;
+        *reinterpret_cast<float4*>(rows + cell * 4) = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, sum.w * inv);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < per * quads; t += 256) {
+        const int p = t / quads, quad = t % quads;
+        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int g = 0; g < H; ++g) {
+            const float w = s_talk[p * H + g];
+            const float4 v = *reinterpret_cast<const float4*>(rows + (g * quads + quad) * 4);
+            a0.x = fmaf(w, v.x, a0.x);
+            a0.y = fmaf(w, v.y, a0.y);
+            a0.z = fmaf(w, v.z, a0.z);
+            a0.w = fmaf(w, v.w, a0.w);
+        }
+        tk_store4<T>(att + ((size_t)row * H + c * per + p) * V + ch0 + quad * 4, a0);
+    }
+}
+
+template <typename T>
+static int tks_launch(const float* o, const float* ml, const float* talk, void* att, const int* positions, int n, int H, int G, int V,
+                      int shares, float unit, cudaStream_t stream) {
+    // a block's channels: a value head's, halved while the blocks are fewer than two a multiprocessor and a block has over 256 cells
+    int quads = V / 4;
+    while (quads % 2 == 0 && (H * quads > 256 || (long long)n * G * (V / 4 / quads) < 148) && H * quads > 64) quads /= 2;
+    const size_t smem = ((size_t)H * quads * 4 + (size_t)2 * H * shares + (size_t)H / G * H) * sizeof(float);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(talk_shares_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    gb_launch(GB_PDL_ELEMENTWISE, talk_shares_kernel<T>, dim3(n, G, V / 4 / quads), dim3(256), smem, stream, o, ml, talk, (T*)att, positions, n,
+              H, G, V, shares, unit, quads);
+    return gb_check_launch("gb_talk_combine");
+}
+
 // The mix of whole results (shares == 1) for steps of many rows: a thread has four channels of a (row, key/value head) and forms
 // all PER outputs of them, eight heads' 16-byte loads in flight at a time, no exchange between threads; the sums run in the
 // order of the form above (even heads, odd heads). That one brought 4 KB a block through shared memory behind two barriers, one
@@ -956,6 +1078,11 @@ GB_EXPORT int gb_talk_combine(const float* o, const float* ml, const float* talk
         (((uintptr_t)o | (uintptr_t)att) & 15) == 0) {
         if (dtype == GB_F32) return tkm_launch<float>(o, talk, att, positions, n, H, G, V, stream);
         if (dtype == GB_BF16) return tkm_launch<__nv_bfloat16>(o, talk, att, positions, n, H, G, V, stream);
+    }
+    if (talk != nullptr && shares > 1 && V % 4 == 0 && H <= 64 && H * shares <= 4096 &&
+        (((uintptr_t)o | (uintptr_t)att) & 15) == 0 && ((uintptr_t)ml & 7) == 0) {
+        if (dtype == GB_F32) return tks_launch<float>(o, ml, talk, att, positions, n, H, G, V, shares, unit, stream);
+        if (dtype == GB_BF16) return tks_launch<__nv_bfloat16>(o, ml, talk, att, positions, n, H, G, V, shares, unit, stream);
     }
     if (dtype == GB_F32) return tkc_launch<float>(o, ml, talk, att, positions, n, H, G, V, VG, shares, unit, stream);
     if (dtype == GB_BF16) return tkc_launch<__nv_bfloat16>(o, ml, talk, att, positions, n, H, G, V, VG, shares, unit, stream);

@@ -122,6 +122,7 @@ _SIGNATURES = {
     "gb_talking_attention_rows": [_P, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _F, _F, _I, _P, _P],
     "gb_talking_attention_decode": [_P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _F, _F, _I, _I, _P, _P],
     "gb_talking_attention_decode_plan": [_I, _I, _I, _I],
+    "gb_talking_decode_mma_heads": [_I, _I, _I, _I, _I],
     "gb_talking_attention_tiles": [_P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _F, _F, _I, _P, _P],
     "gb_talking_attention_tiles_columns": [_I, _I, _I],
     "gb_talking_attention_flash_supported": [_I, _I, _I, _I],
@@ -2243,12 +2244,23 @@ def talking_attention_decode_supported(dtype: torch.dtype, heads: int, kv_heads:
     return dtype in _DT and bool(lib().gb_talking_attention_decode_plan(heads, kv_heads, vdim, value_heads))
 
 
-def talking_decode_shares(n: int, heads: int, kv_heads: int, vdim: int, value_heads: int, reach: int) -> int:
+def talking_decode_shares(n: int, heads: int, kv_heads: int, vdim: int, value_heads: int, reach: int, dim: int = 0,
+                          dtype: Optional[torch.dtype] = None) -> int:
     """Into how many shares the decoding kernel cuts a row's keys: the count whose rounds of blocks (two per multiprocessor, 296
-    at once) take the least time, a round costing a block's keys and about 400 more for its start and merge; no share shorter
-    than 256 keys, at most 16. Measured (16 heads, 4 value heads of 64, contexts to 2,047), mixer with this rule / with the
-    smallest count that fills 296 blocks: 16 rows 46.2 us (4 shares) / 51.6 (5), 24 rows 55.9 (3) / 67.0 (4), 32 rows 70.3 (2) /
-    80.3 (3), 48 rows 92.0 (3) / 102.5 (2), 96 rows 160 (2) / 184 (1)."""
+    at once) take the least time, a round costing a block's keys and what its start and merge cost.
+
+    On the tensor cores (bfloat16 at the sizes it is built for; ``dim`` and ``dtype`` say so) that is about 200 keys' worth, and no share is
+    shorter than one step of the kernel. Attention and merge of 16 heads, 4 value heads of 64: 32 rows, contexts to 2,047, with 4 / 8 /
+    9 / 12 / 16 shares 33 / 19.7 / 20.2 / 26.8 / 22.3 us (9 chosen); 64 rows, contexts to 1,000, 4 / 8 / 12 19.6 / 21.6 / 29.5 (4 chosen).
+
+    By FMA it is about 400, no share is shorter than 256 keys. Measured (16 heads, 4 value heads of 64, contexts to 2,047), mixer with this
+    rule / with the smallest count that fills 296 blocks: 16 rows 46.2 us (4 shares) / 51.6 (5), 24 rows 55.9 (3) / 67.0 (4), 32 rows 70.3
+    (2) / 80.3 (3), 48 rows 92.0 (3) / 102.5 (2), 96 rows 160 (2) / 184 (1). At most 16 shares either way."""
+    per_block = lib().gb_talking_decode_mma_heads(heads, kv_heads, dim, vdim, value_heads) if dtype == torch.bfloat16 else 0
+    if per_block:
+        blocks = max(1, n * -(-heads // per_block))
+        most = max(1, min(16, reach // (64 if value_heads * vdim > 256 else 128), 4096 // heads))
+        return min(range(1, most + 1), key=lambda s: (-(-blocks * s // 296) * (200 + -(-reach // s)), s))
     plan = lib().gb_talking_attention_decode_plan(heads, kv_heads, vdim, value_heads)
     blocks = max(1, n * (heads // max(plan % 10000 // 100, 1)) * max(plan // 10000, 1))
     most = max(1, min(16, reach // 256, 4096 // heads))

@@ -93,7 +93,7 @@ class TalkingAttention(Mixer):
         if how == "decode":
             # few rows: the keys of a row are cut into shares, so that the blocks fill the chip; the mix merges the shares
             reach = min(ctx.max_context, s.window) if s.window else ctx.max_context
-            shares = kernels.talking_decode_shares(n, self.H, self.G, self.V, value_heads, reach)
+            shares = kernels.talking_decode_shares(n, self.H, self.G, self.V, value_heads, reach, self.D, q.dtype)
             wide = ctx.scratch("tk_wide_shares", (n, shares * cols), torch.float32, grow=True)
             ml = ctx.scratch("tk_ml", (n, shares * self.H * 2), torch.float32, grow=True) if shares > 1 else None
             kernels.talking_attention_decode(q, wide, cache.k, cache.v, cache.block_tables, ctx.row_seq, ctx.positions, shares=shares, ml=ml,
