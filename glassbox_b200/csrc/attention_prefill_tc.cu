@@ -3,7 +3,9 @@
 // their accumulators in tensor memory; queries, keys and values come into shared memory by TMA, the
 // keys and values page by page straight from the paged cache through the request's block table.
 //
-// One block = 128 consecutive query rows of one request for one query head, over tiles of 128 keys:
+// One block = 128 consecutive query rows of one request for one query head, over tiles of 128 keys (PAIR: two blocks, a cluster, work
+// on two such row tiles, the p-th and the p-th from the end; the second takes over the first key tiles of the later one, hands its
+// sums over through distributed shared memory, and goes on to the earlier one, so that both end at about the same time):
 //   warp 0, 10  producers of keys (and the query tile, once) and of values. For every key tile the lanes
 //               read the page ids from the block table (one tile ahead) and each issues the TMA load of
 //               one page (a page is `page_size` rows of one kv head: one box of the 2-D view
@@ -45,7 +47,7 @@ constexpr int AT_STAGES = 4;   // key tiles, and value tiles, in flight
 constexpr int AT_WARPS = 11;   // key producer, MMA issuer, eight softmax warps, value producer
 
 struct __align__(8) AtShared {
-    uint64_t q_full;                 // TMA -> MMA: the query tile has landed
+    uint64_t q_full[2];              // TMA -> MMA: an item's query tile has landed
     uint64_t k_full[AT_STAGES];      // TMA -> MMA: a stage's keys have landed
     uint64_t k_empty[AT_STAGES];     // MMA -> TMA: S = Q K^T has read the stage
     uint64_t v_full[AT_STAGES];      // TMA -> MMA: a stage's values have landed
@@ -54,27 +56,32 @@ struct __align__(8) AtShared {
     uint64_t s_free[2];              // softmax -> MMA: S_j has been read out of buffer j & 1
     uint64_t p_ready[2];             // softmax -> MMA: P_j is in TMEM buffer j & 1 (and O is rescaled)
     uint64_t pv_done[2];             // MMA -> softmax: O += P_j V_j is complete (P buffer j & 1 is free, O is current)
-    uint64_t x_ready;                // softmax <-> softmax: both groups have posted their final maximum and sum
+    uint64_t x_ready;                // softmax <-> softmax: both groups have posted their final maximum and sum (a phase per item)
+    uint64_t merged;                 // softmax <-> softmax: the first item's accumulators have been read (one phase)
+    uint64_t peer_done;              // PAIR, the other block's softmax -> softmax: its share of this block's tile has arrived (one phase)
     float row_stat[2][2][AT_BM];     // [group][maximum, sum][row]
     uint32_t tmem_base;
     int abort_flag;
     int issued[2];                   // key / value tiles whose TMA loads were issued
     int consumed[2];                 // key / value tiles whose full barrier the MMA thread has passed
-    int q_issued, q_consumed;
+    int q_issued, q_consumed;        // query tiles
 };
 
-template <int HD> struct AtGeometry {
+template <int HD, bool PAIR> struct AtGeometry {
     static constexpr int Q_BYTES = AT_BM * HD * 2, KV_BYTES = AT_BN * HD * 2;
-    static constexpr int K_OFF = Q_BYTES, V_OFF = K_OFF + AT_STAGES * KV_BYTES;
+    static constexpr int K_OFF = (PAIR ? 2 : 1) * Q_BYTES, V_OFF = K_OFF + AT_STAGES * KV_BYTES;
     static constexpr int SH_OFF = V_OFF + AT_STAGES * KV_BYTES;
     // (SINK: behind the barriers and row statistics, a table of distance biases per softmax warp)
     static constexpr int BIAS_OFF = SH_OFF + 2560, BIAS_WARP = 160;
-    static constexpr int SMEM = BIAS_OFF + 8 * BIAS_WARP * 4;
+    // (PAIR: a share of a row tile from the other block: float32 sums in pieces of four channels [HD / 4][rows], maxima, denominators)
+    static constexpr int SHARE_OFF = BIAS_OFF + 8 * BIAS_WARP * 4;
+    static constexpr int SMEM = SHARE_OFF + (PAIR ? AT_BM * HD * 4 + 2 * AT_BM * 4 : 0);
+    static_assert(SHARE_OFF % 16 == 0 && SMEM <= 227 * 1024, "the block does not fit");
     // tensor memory: two S buffers of 128 columns, two accumulators O_g of HD columns, two P buffers of 64
     // columns (128 bfloat16 keys, two per 32-bit column)
     static constexpr int O_COL = 2 * AT_BN, P_COL = O_COL + 2 * HD;
     static constexpr int TMEM_COLS = 512;
-    static_assert(P_COL + 2 * (AT_BN / 2) <= TMEM_COLS, "tensor memory layout");
+    static_assert(sizeof(AtShared) <= 2560 && P_COL + 2 * (AT_BN / 2) <= TMEM_COLS, "tensor memory layout");
 };
 
 // MN-major B operand (V: rows are keys, the head's channels contiguous) in 128-byte-swizzled rows:
@@ -130,14 +137,38 @@ struct AtSinkTerms {
     float cap;              // > 0: scores are capped as cap * tanh(score / cap) before the bias
 };
 
-template <int HD, bool SINK = false>
+// A warp's bounded wait for what the other block of a pair has written into this block's shared memory.
+__device__ __forceinline__ bool at_wait_peer(uint64_t* bar, volatile int* abort_flag, int* status) {
+    const long long t0 = clock64();
+    bool ok = true;
+    for (;;) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(smem_u32(bar)) : "memory");
+        if (done) break;
+        if (*abort_flag || clock64() - t0 > 2 * TC_WAIT_CYCLES) {           // (the other block's own waits run out first)
+            if (!*abort_flag) atomicOr(status, GB_STATUS_WAIT_TIMEOUT);
+            *abort_flag = 1;
+            ok = false;
+            break;
+        }
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+struct AtItem {
+    int q_lo, pos_lo, pos_hi, key_lo, kt_begin, ntiles;
+};
+constexpr int AT_ITEM_TILES = 2;      // what a second item costs a block beside its key tiles, in key tiles
+
+template <int HD, bool SINK, bool PAIR>
 __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, long long out_stride,
     const int* __restrict__ block_tables, int max_pages, const int* __restrict__ seq_first_row,
     const int* __restrict__ seq_start_pos, int nh, int nkv, int page_size, int page_shift, long long num_pages,
     float scale, int window, int* __restrict__ status, const AtSinkTerms terms) {
-    using G = AtGeometry<HD>;
+    using G = AtGeometry<HD, PAIR>;
     static_assert(HD == 64, "this kernel is built for head size 64");
     extern __shared__ __align__(1024) unsigned char at_smem[];
     unsigned char* Qs = at_smem;
@@ -146,11 +177,15 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
     AtShared& sh = *reinterpret_cast<AtShared*>(at_smem + G::SH_OFF);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int qt = gridDim.x - 1 - blockIdx.x;   // later tiles see more keys: start the longest blocks first
-    const int head = blockIdx.y, seq = blockIdx.z;
+    const int rank = PAIR ? (int)blockIdx.x & 1 : 0;
+    const int head = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, seq = blockIdx.y;
     const int row0 = seq_first_row[seq];
     const int nrows = seq_first_row[seq + 1] - row0;
-    if (qt * AT_BM >= nrows) return;              // uniform for the block, before anything is allocated
+    // Later tiles see more keys. One block a tile: the longest blocks start first, over all heads and requests (the tile is the
+    // slowest dimension of the grid). Two blocks a pair of tiles: the p-th from the end and the p-th.
+    const int row_tiles = (nrows + AT_BM - 1) / AT_BM;
+    const int qt = PAIR ? row_tiles - 1 - (int)blockIdx.z : (int)(gridDim.z - 1 - blockIdx.z), qt_low = blockIdx.z;
+    if (PAIR ? qt < qt_low : qt * AT_BM >= nrows) return;         // uniform for the block (the pair), before anything is allocated
     if (smem_u32(at_smem) & 1023u) {              // swizzled tiles want 1024-byte alignment: refuse rather than compute nonsense
         if (tid == 0) atomicOr(status, GB_STATUS_WAIT_TIMEOUT);
         return;
@@ -163,15 +198,40 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
         return;
     }
     const int kvh = head / (nh / nkv);
-    const int q_lo = qt * AT_BM;
-    const int pos_lo = start_pos + q_lo, pos_hi = start_pos + min(nrows, q_lo + AT_BM) - 1;
-    const int key_lo = gb_first_key(pos_lo, window);
-    const int kt_begin = key_lo / AT_BN, kt_end = pos_hi / AT_BN;   // inclusive
-    const int ntiles = kt_end - kt_begin + 1;
     const int* table = block_tables + (size_t)seq * max_pages;
+    // What this block works on, one item after the other: a row tile over a run of key tiles. The key tiles, the rings, the score
+    // buffers and the groups are counted through both items (tile j of the block belongs to group j & 1).
+    auto whole = [&](int tile) {
+        AtItem it;
+        it.q_lo = tile * AT_BM;
+        it.pos_lo = start_pos + it.q_lo;
+        it.pos_hi = start_pos + min(nrows, it.q_lo + AT_BM) - 1;
+        it.key_lo = gb_first_key(it.pos_lo, window);
+        it.kt_begin = it.key_lo / AT_BN;
+        it.ntiles = it.pos_hi / AT_BN - it.kt_begin + 1;
+        return it;
+    };
+    AtItem items[2];
+    int n_items = 1, share = 0;                   // share: key tiles of the later row tile that the second block takes over
+    items[0] = whole(qt);
+    if constexpr (PAIR) {
+        const bool middle = qt == qt_low;         // (an odd count: the tile in the middle has no partner)
+        items[1] = whole(qt_low);
+        share = middle ? (items[0].ntiles - 1) / 2 : max(0, (items[0].ntiles - items[1].ntiles - AT_ITEM_TILES) / 2);
+        if (rank == 0) {
+            items[0].kt_begin += share;
+            items[0].ntiles -= share;
+        } else {
+            items[0].ntiles = share;
+            if (share == 0) items[0] = items[1];
+            n_items = middle ? (share > 0 ? 1 : 0) : (share > 0 ? 2 : 1);
+        }
+    }
+    const int n_first = items[0].ntiles, total = n_items == 0 ? 0 : n_items == 1 ? n_first : n_first + items[1].ntiles;
 
     if (tid == 0) {
-        mbar_init(&sh.q_full, 1);
+        mbar_init(&sh.q_full[0], 1);
+        mbar_init(&sh.q_full[1], 1);
         for (int b = 0; b < AT_STAGES; ++b) {
             mbar_init(&sh.k_full[b], 1);
             mbar_init(&sh.k_empty[b], 1);
@@ -185,6 +245,8 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             mbar_init(&sh.pv_done[b], 1);
         }
         mbar_init(&sh.x_ready, 8);
+        mbar_init(&sh.merged, 8);
+        mbar_init(&sh.peer_done, 8);
         sh.abort_flag = 0;
         sh.issued[0] = sh.issued[1] = sh.consumed[0] = sh.consumed[1] = sh.q_issued = sh.q_consumed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -199,60 +261,69 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if constexpr (PAIR) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // (the barriers are set up)
     const uint32_t tmem = sh.tmem_base;
     volatile int* abort_flag = &sh.abort_flag;
     // the set-up above overlapped the tail of the kernel before; from here on its results are read
     gb_pdl_launch_dependents();
     gb_pdl_wait();
+    bool met = false;       // PAIR: this warp has seen that the other block is set up
 
     if (warp == 0 || warp == AT_WARPS - 1) {
         // ------------------------------------------------------------------------- producers
         // warp 0 loads the query tile and the keys, the last warp the values: keys are needed (and their
         // stages free again) earlier than values, so the two rings run at their own pace
         const int what = warp == 0 ? 0 : 1;
-        if (what == 0 && lane == 0) {
-            mbar_expect_tx(&sh.q_full, G::Q_BYTES);
-            tma_load_2d(Qs, &map_q, &sh.q_full, head * HD, row0 + q_lo);
-            sh.q_issued = 1;
-        }
         const int ppt = AT_BN >> page_shift;   // pages per key tile (1 .. 16)
         int bad = 0;
-        auto page_of = [&](int kt) -> long long {   // this lane's page of key tile kt
-            long long page = 0;
-            if (lane < ppt) {
-                const int pi = ((kt * AT_BN) >> page_shift) + lane;
-                page = pi < max_pages ? table[pi] : -1;
-                if (page < 0 || page >= num_pages) {
-                    // only a page that holds a key some row can see is missed
-                    const int first = pi << page_shift, last = first + page_size - 1;
-                    if (first <= pos_hi && last >= key_lo) bad = 1;
-                    page = 0;
-                }
-            }
-            return page;
-        };
         uint64_t* full = what == 0 ? sh.k_full : sh.v_full;
         uint64_t* empty = what == 0 ? sh.k_empty : sh.v_empty;
         unsigned char* ring = what == 0 ? Ks : Vs;
         const CUtensorMap* map = what == 0 ? &map_k : &map_v;
-        long long page = page_of(kt_begin);
-        for (int j = 0; j < ntiles; ++j) {
-            const int s = j % AT_STAGES;
-            const long long next_page = j + 1 < ntiles ? page_of(kt_begin + j + 1) : 0;   // in flight during the wait
-            int ok = 1;
-            if (lane == 0 && j >= AT_STAGES)
-                ok = mbar_wait(&empty[s], ((j / AT_STAGES) - 1) & 1, abort_flag, status) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) break;
-            if (lane == 0) mbar_expect_tx(&full[s], G::KV_BYTES);
-            __syncwarp();
-            if (lane < ppt) {
-                const int row = (int)((page * nkv + kvh) * page_size);
-                tma_load_2d(ring + s * G::KV_BYTES + lane * page_size * HD * 2, map, &full[s], 0, row);
+        int j = 0;
+        bool go = true;
+#pragma unroll
+        for (int item = 0; item < (PAIR ? 2 : 1); ++item) {
+            if (item >= n_items || !go) break;
+            const AtItem& it = items[item];
+            if (what == 0 && lane == 0) {
+                mbar_expect_tx(&sh.q_full[item], G::Q_BYTES);
+                tma_load_2d(Qs + item * G::Q_BYTES, &map_q, &sh.q_full[item], head * HD, row0 + it.q_lo);
+                sh.q_issued = item + 1;
             }
-            __syncwarp();
-            if (lane == 0) sh.issued[what] = j + 1;
-            page = next_page;
+            auto page_of = [&](int kt) -> long long {   // this lane's page of key tile kt
+                long long page = 0;
+                if (lane < ppt) {
+                    const int pi = ((kt * AT_BN) >> page_shift) + lane;
+                    page = pi < max_pages ? table[pi] : -1;
+                    if (page < 0 || page >= num_pages) {
+                        // only a page that holds a key some row can see is missed
+                        const int first = pi << page_shift, last = first + page_size - 1;
+                        if (first <= it.pos_hi && last >= it.key_lo) bad = 1;
+                        page = 0;
+                    }
+                }
+                return page;
+            };
+            long long page = page_of(it.kt_begin);
+            for (int t = 0; t < it.ntiles; ++t, ++j) {
+                const int s = j % AT_STAGES;
+                const long long next_page = t + 1 < it.ntiles ? page_of(it.kt_begin + t + 1) : 0;   // in flight during the wait
+                int ok = 1;
+                if (lane == 0 && j >= AT_STAGES)
+                    ok = mbar_wait(&empty[s], ((j / AT_STAGES) - 1) & 1, abort_flag, status) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) { go = false; break; }
+                if (lane == 0) mbar_expect_tx(&full[s], G::KV_BYTES);
+                __syncwarp();
+                if (lane < ppt) {
+                    const int row = (int)((page * nkv + kvh) * page_size);
+                    tma_load_2d(ring + s * G::KV_BYTES + lane * page_size * HD * 2, map, &full[s], 0, row);
+                }
+                __syncwarp();
+                if (lane == 0) sh.issued[what] = j + 1;
+                page = next_page;
+            }
         }
         if (bad && what == 0) atomicOr(status, GB_STATUS_BAD_SLOT);
     } else if (warp == 1) {
@@ -261,25 +332,26 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             const uint32_t idesc_qk = umma_idesc(AT_BM, AT_BN);
             const uint32_t idesc_pv = umma_idesc(AT_BM, HD) | (1u << 16);   // B is MN-major
             const uint64_t q_desc = umma_desc(smem_u32(Qs)), k_desc = umma_desc(smem_u32(Ks)), v_desc = umma_desc_mn(smem_u32(Vs), AT_BN * 128);
-            bool ok = mbar_wait(&sh.q_full, 0, abort_flag, status);
-            if (ok) sh.q_consumed = 1;
+            bool ok = true;
+            int q_have = 0;                       // query tiles that have landed
             // Whatever is ready is issued: S_j as soon as its keys have landed and its group has read S_{j-2} out of
             // the buffer (so S runs up to two tiles ahead and neither softmax group waits for the other), O += P_j V_j
             // as soon as P_j is written and its values have landed. The loop polls without blocking; the limit
             // counts from the first look that found nothing.
             int next_qk = 0, next_pv = 0;
             long long t_idle = 0;
-            while (ok && next_pv < ntiles) {
+            while (ok && next_pv < total) {
                 bool progressed = false;
-                if (next_qk < ntiles) {
-                    const int j = next_qk, st = j % AT_STAGES;
-                    if (mbar_test(&sh.k_full[st], (j / AT_STAGES) & 1) &&
+                if (next_qk < total) {
+                    const int j = next_qk, st = j % AT_STAGES, item = PAIR && j >= n_first ? 1 : 0;
+                    if (q_have == item && mbar_test(&sh.q_full[item], 0)) sh.q_consumed = q_have = item + 1;
+                    if (q_have > item && mbar_test(&sh.k_full[st], (j / AT_STAGES) & 1) &&
                         (j < 2 || mbar_test(&sh.s_free[j & 1], ((j >> 1) - 1) & 1))) {
                         tc_fence_after();
-                        const uint64_t kd = k_desc + (uint64_t)((st * G::KV_BYTES) >> 4);
+                        const uint64_t kd = k_desc + (uint64_t)((st * G::KV_BYTES) >> 4), qd = q_desc + (uint64_t)((item * G::Q_BYTES) >> 4);
 #pragma unroll
                         for (int k = 0; k < HD / 16; ++k)
-                            umma_bf16(tmem + (uint32_t)((j & 1) * AT_BN), q_desc + k * 2, kd + k * 2, idesc_qk, k ? 1u : 0u);
+                            umma_bf16(tmem + (uint32_t)((j & 1) * AT_BN), qd + k * 2, kd + k * 2, idesc_qk, k ? 1u : 0u);
                         umma_commit(&sh.s_full[j & 1]);
                         umma_commit(&sh.k_empty[st]);
                         ++next_qk;
@@ -292,10 +364,11 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
                         tc_fence_after();
                         const uint64_t vd = v_desc + (uint64_t)((st * G::KV_BYTES) >> 4);
                         const uint32_t pt = tmem + (uint32_t)(G::P_COL + (j & 1) * (AT_BN / 2));
+                        const bool onto = (PAIR && j >= n_first ? j - n_first : j) >= 2;      // (each group's first tile of an item starts anew)
 #pragma unroll
                         for (int kk = 0; kk < AT_BN / 16; ++kk)   // 16 keys per instruction: 8 columns of P
                             umma_bf16_ts(tmem + (uint32_t)(G::O_COL + (j & 1) * HD), pt + (uint32_t)(kk * 8),
-                                         vd + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, (j >= 2 || kk) ? 1u : 0u);
+                                         vd + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, (onto || kk) ? 1u : 0u);
                         umma_commit(&sh.pv_done[j & 1]);
                         umma_commit(&sh.v_empty[st]);
                         ++next_pv;
@@ -327,15 +400,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
         const int q = warp & 3;                        // the quarter of TMEM lanes this warp may read
         const int g = (warp - 2) >> 2;                 // the group: parity of its key tiles
         const int r = q * 32 + lane;                   // this thread's query row within the tile
-        const int pos = pos_lo + r;
         const float sl2 = scale * 1.4426950408889634f; // exp(x * scale) = exp2(x * sl2)
         const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
         const uint32_t o_col = (uint32_t)(G::O_COL + g * HD);
-        const int my_tiles = (ntiles - g + 1) >> 1;
-        float m_run = AT_NEG_BIG, l_run = 0.f;
         bool ok = true;
-        const int first = gb_first_key(pos, window), first_last = gb_first_key(pos_lo + AT_BM - 1, window);
-        auto visible = [&](int key) { return key <= pos && key >= first; };
         // SINK: the scores are brought into the base-2 domain and lose their bias before the maximum is taken, so what
         // follows scales them by one. The bias depends on the distance alone: the 32 rows of this warp and the 128 keys of a
         // tile are 159 distances apart, whose biases the warp writes into a table of its own per tile (five logarithms a
@@ -357,8 +425,18 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
                 b2 = terms.r2[head];
             }
         }
-        for (int i = 0; i < my_tiles; ++i) {
-            const int key0 = (kt_begin + 2 * i + g) * AT_BN;
+#pragma unroll 1
+        for (int item = 0; item < (PAIR ? n_items : 1) && ok; ++item) {
+        const AtItem it = PAIR && item ? items[1] : items[0];
+        const int base = PAIR && item ? n_first : 0, ntiles = it.ntiles, pos_lo = it.pos_lo, q_lo = it.q_lo;
+        const int pos = pos_lo + r;
+        float m_run = AT_NEG_BIG, l_run = 0.f;
+        const int first = gb_first_key(pos, window), first_last = gb_first_key(pos_lo + AT_BM - 1, window);
+        auto visible = [&](int key) { return key <= pos && key >= first; };
+        const int j_first = base + ((base ^ g) & 1);              // this group's first tile
+        for (int j = j_first; j < base + ntiles; j += 2) {
+            const int i = j >> 1;                                  // the group's tiles so far
+            const int key0 = (it.kt_begin + j - base) * AT_BN;
             if (!mbar_wait_warp(&sh.s_full[g], i & 1, abort_flag, status)) { ok = false; break; }
             tc_fence_after();
             uint32_t sv[AT_BN];
@@ -422,7 +500,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             if (i > 0 && !mbar_wait_warp(&sh.pv_done[g], (i - 1) & 1, abort_flag, status)) { ok = false; break; }
             // raise the running maximum only when it is exceeded by more than 2^8 in the exponent
             const bool raise = (mx - m_run) * slx > 8.0f;
-            if (i == 0) {
+            if (j == j_first) {
                 if (raise) m_run = mx;               // nothing is accumulated yet
             } else if (__any_sync(0xffffffffu, raise)) {
                 tc_fence_after();
@@ -457,6 +535,8 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             tmem_store64(lane_base + (uint32_t)(G::P_COL + g * (AT_BN / 2)), pw);
             tc_fence_before();
             __syncwarp();
+            // an accumulator is written anew only when both groups have read the item before out of both
+            if (PAIR && item == 1 && j == j_first && !mbar_wait_warp(&sh.merged, 0, abort_flag, status)) { ok = false; break; }
             if (lane == 0) mbar_arrive(&sh.p_ready[g]);
         }
         // merge: the groups post their maximum and sum per row, then each writes half of the channels
@@ -465,11 +545,14 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             sh.row_stat[g][1][r] = l_run;
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.x_ready);
-            ok = mbar_wait_warp(&sh.x_ready, 0, abort_flag, status);
+            ok = mbar_wait_warp(&sh.x_ready, item & 1, abort_flag, status);
         }
-        const int tiles_of[2] = {(ntiles + 1) >> 1, ntiles >> 1};
-        for (int gg = 0; gg < 2 && ok; ++gg)   // both accumulators must be final
-            if (tiles_of[gg] > 0) ok = mbar_wait_warp(&sh.pv_done[gg], (tiles_of[gg] - 1) & 1, abort_flag, status);
+        int tiles_of[2];
+        for (int gg = 0; gg < 2 && ok; ++gg) { // both accumulators must be final
+            const int last = base + ntiles - 1 - ((base + ntiles - 1 - gg) & 1);      // the group's last tile
+            tiles_of[gg] = last >= base ? 1 : 0;
+            if (last >= base) ok = mbar_wait_warp(&sh.pv_done[gg], (last >> 1) & 1, abort_flag, status);
+        }
         if (ok) {
             tc_fence_after();
             const float m0 = sh.row_stat[0][0][r], l0 = sh.row_stat[0][1][r];
@@ -486,15 +569,12 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             const float a1 = tiles_of[1] > 0 ? at_exp2((m1 - m) * slx) : 0.f;
             float l = l0 * a0 + l1 * a1;
             if constexpr (SINK) l += at_exp2(sink2 - m);
-            float inv = l > 0.f ? 1.0f / l : 0.f;
-            if constexpr (SINK) {
-                if (terms.gate != nullptr && !terms.gate_channels && q_lo + r < nrows)
-                    inv *= 1.0f / (1.0f + __expf(-terms.gate[(size_t)(row0 + q_lo + r) * terms.ld_gate + head]));
-            }
             constexpr int OC = HD / 2;                 // this thread's channels: g * OC ..
             static_assert(OC == 32, "one 32-column access per accumulator");
             float o[OC];
-            {
+#pragma unroll
+            for (int k = 0; k < OC; ++k) o[k] = 0.f;
+            if (tiles_of[0] > 0) {                      // uniform for the block
                 uint32_t ov[32];
                 tmem_load32(lane_base + (uint32_t)(G::O_COL + g * OC), ov);
 #pragma unroll
@@ -506,7 +586,58 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
 #pragma unroll
                 for (int k = 0; k < OC; ++k) o[k] = fmaf(__uint_as_float(ov[k]), a1, o[k]);
             }
-            if (q_lo + r < nrows) {
+            bool mine = true;                           // this block writes the tile's rows
+            if constexpr (PAIR) {
+                if (n_items == 2 && item == 0) {        // the accumulators and row statistics may be written anew
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.merged);
+                }
+                const uint32_t sums = smem_u32(at_smem + G::SHARE_OFF), stats = sums + AT_BM * HD * 4;
+                if (share > 0 && rank == 1 && item == 0) {
+                    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+                    met = true;
+                    // this share of the other block's tile goes into that block's shared memory, pieces of four channels, a row a lane
+                    uint32_t there, there_stats, there_bar;
+                    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(there) : "r"(sums));
+                    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(there_stats) : "r"(stats));
+                    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(there_bar) : "r"(smem_u32(&sh.peer_done)));
+#pragma unroll
+                    for (int k = 0; k < OC; k += 4)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(there + (uint32_t)((g * (OC / 4) + k / 4) * AT_BM + r) * 16),
+                                     "f"(o[k]), "f"(o[k + 1]), "f"(o[k + 2]), "f"(o[k + 3])
+                                     : "memory");
+                    if (g == 0) {
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there_stats + r * 4), "f"(m) : "memory");
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there_stats + (AT_BM + r) * 4), "f"(l) : "memory");
+                    }
+                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(there_bar) : "memory");
+                    mine = false;
+                } else if (share > 0 && rank == 0) {
+                    ok = at_wait_peer(&sh.peer_done, abort_flag, status);
+                    const float* sums_p = reinterpret_cast<const float*>(at_smem + G::SHARE_OFF);
+                    const float m2 = sums_p[AT_BM * HD + r], l2 = sums_p[AT_BM * HD + AT_BM + r];
+                    const float m_all = fmaxf(m, m2), b1 = at_exp2((m - m_all) * slx), b2 = at_exp2((m2 - m_all) * slx);
+                    l = l * b1 + l2 * b2;
+#pragma unroll
+                    for (int k = 0; k < OC; k += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(sums_p + ((g * (OC / 4) + k / 4) * AT_BM + r) * 4);
+                        o[k] = fmaf(v.x, b2, o[k] * b1);
+                        o[k + 1] = fmaf(v.y, b2, o[k + 1] * b1);
+                        o[k + 2] = fmaf(v.z, b2, o[k + 2] * b1);
+                        o[k + 3] = fmaf(v.w, b2, o[k + 3] * b1);
+                    }
+                    mine = ok;
+                }
+            }
+            float inv = l > 0.f ? 1.0f / l : 0.f;
+            if constexpr (SINK) {
+                if (terms.gate != nullptr && !terms.gate_channels && q_lo + r < nrows)
+                    inv *= 1.0f / (1.0f + __expf(-terms.gate[(size_t)(row0 + q_lo + r) * terms.ld_gate + head]));
+            }
+            if (mine && q_lo + r < nrows) {
                 __nv_bfloat16* dst = out + (size_t)(row0 + q_lo + r) * out_stride + (size_t)head * HD + g * OC;
                 if constexpr (SINK) {
                     if (terms.gate != nullptr && terms.gate_channels) {
@@ -535,17 +666,23 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
                 }
             }
         }
+        }
     }
 
     // ------------------------------------------------------------------------------- wind down
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) {   // (the first block's shared memory outlives what the second writes there; nobody writes to the second)
+        if (!met) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (rank == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     if (warp == 0) {
         if (lane == 0 && sh.abort_flag) {
             // copies that were issued but never consumed may still be in flight: wait for them (bounded)
-            if (sh.q_issued && !sh.q_consumed) {
+            for (int it = sh.q_consumed; it < sh.q_issued; ++it) {
                 const long long t0 = clock64();
-                while (!mbar_try_wait(&sh.q_full, 0) && clock64() - t0 < TC_WAIT_CYCLES) {}
+                while (!mbar_try_wait(&sh.q_full[it], 0) && clock64() - t0 < TC_WAIT_CYCLES) {}
             }
             for (int what = 0; what < 2; ++what)
                 for (int it = sh.consumed[what]; it < sh.issued[what]; ++it) {
@@ -562,6 +699,48 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
 GB_EXPORT int gb_attention_prefill_tc_supported(int nh, int nkv, int hd, int page_size) {
     if (nkv <= 0 || nh % nkv) return 0;
     return hd == 64 && page_size >= 8 && page_size <= AT_BN && (page_size & (page_size - 1)) == 0;
+}
+
+template <bool SINK, bool PAIR>
+static int prefill_tc_run(const void* q, long long q_stride, int n_rows, void* out, long long out_stride, const void* kcache,
+                          const void* vcache, const int* block_tables, int max_pages, const int* seq_first_row, const int* seq_start_pos,
+                          int num_seqs, int tiles, int nh, int nkv, int hd, int page_size, long long num_pages, float scale, int window,
+                          int* status, cudaStream_t stream, const AtSinkTerms& terms) {
+    using G = AtGeometry<64, PAIR>;
+    CUtensorMap mq, mk, mv;
+    if (tc_make_map_2d(&mq, q, n_rows, (long long)nh * hd, q_stride, AT_BM, 64, "gb_attention_prefill_tc")) return 1;
+    if (tc_make_map_2d(&mk, kcache, num_pages * nkv * page_size, hd, hd, page_size, 64, "gb_attention_prefill_tc")) return 1;
+    if (tc_make_map_2d(&mv, vcache, num_pages * nkv * page_size, hd, hd, page_size, 64, "gb_attention_prefill_tc")) return 1;
+    auto kernel = attention_prefill_tc_kernel<64, SINK, PAIR>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+        GB_REQUIRE(e == cudaSuccess, "gb_attention_prefill_tc: %d bytes of shared memory refused: %s", G::SMEM, cudaGetErrorString(e));
+        configured = true;
+    }
+    int page_shift = 0;
+    while ((1 << page_shift) < page_size) ++page_shift;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = PAIR ? dim3(2 * nh, num_seqs, (tiles + 1) / 2) : dim3(nh, num_seqs, tiles);
+    cfg.blockDim = dim3(AT_WARPS * 32);
+    cfg.dynamicSmemBytes = G::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    if (gb_pdl_enabled() & GB_PDL_ATTENTION) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (PAIR) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    cfg.attrs = attr;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, (__nv_bfloat16*)out, out_stride, block_tables, max_pages, seq_first_row,
+                                       seq_start_pos, nh, nkv, page_size, page_shift, num_pages, scale, window, status, terms);
+    GB_REQUIRE(e == cudaSuccess, "gb_attention_prefill_tc: launch failed: %s", cudaGetErrorString(e));
+    return gb_check_launch("gb_attention_prefill_tc");
 }
 
 // Rows of each request are consecutive: request s owns rows seq_first_row[s] .. seq_first_row[s+1]-1, at
@@ -583,28 +762,17 @@ static int prefill_tc_launch(const void* q, long long q_stride, int n_rows, void
                "gb_attention_prefill_tc: bad batch shape");
     GB_REQUIRE(num_pages * nkv * page_size < (1ll << 31), "gb_attention_prefill_tc: the cache layer has too many rows for a 32-bit TMA coordinate");
     if (num_seqs == 0 || max_rows_per_seq <= 0 || n_rows == 0) return 0;
-    using G = AtGeometry<64>;
-    CUtensorMap mq, mk, mv;
-    if (tc_make_map_2d(&mq, q, n_rows, (long long)nh * hd, q_stride, AT_BM, 64, "gb_attention_prefill_tc")) return 1;
-    if (tc_make_map_2d(&mk, kcache, num_pages * nkv * page_size, hd, hd, page_size, 64, "gb_attention_prefill_tc")) return 1;
-    if (tc_make_map_2d(&mv, vcache, num_pages * nkv * page_size, hd, hd, page_size, 64, "gb_attention_prefill_tc")) return 1;
-    auto kernel = attention_prefill_tc_kernel<64, SINK>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-        GB_REQUIRE(e == cudaSuccess, "gb_attention_prefill_tc: %d bytes of shared memory refused: %s", G::SMEM, cudaGetErrorString(e));
-        configured = true;
-    }
-    int page_shift = 0;
-    while ((1 << page_shift) < page_size) ++page_shift;
-    dim3 grid(gb_ceil_div(max_rows_per_seq, AT_BM), nh, num_seqs);
-    cudaError_t e = gb_launch(GB_PDL_ATTENTION, kernel, grid, dim3(AT_WARPS * 32), G::SMEM, stream, mq, mk, mv, (__nv_bfloat16*)out, out_stride,
-                              block_tables, max_pages, seq_first_row, seq_start_pos, nh, nkv, page_size, page_shift, num_pages,
-                              scale, window, status, terms);
-    GB_REQUIRE(e == cudaSuccess, "gb_attention_prefill_tc: launch failed: %s", cudaGetErrorString(e));
-    return gb_check_launch("gb_attention_prefill_tc");
+    const int tiles = gb_ceil_div(max_rows_per_seq, AT_BM);
+    // One request whose row tiles are all at work at once: two blocks a pair of tiles, where the tile that sees the most keys would keep the
+    // launch waiting long enough (what a pair costs is 1.5 us) - many fresh tiles, or one tile behind a long context. Block a tile / two
+    // blocks a pair, 9 heads, us: 256 rows 7.2 / 8.7, 1,024 12.8 / 13.0, 1,280 14.9 / 14.2, 1,536 16.7 / 15.4, 2,048 20.7 / 18.0; behind 1,000
+    // tokens 64 rows 13.5 / 11.1, 128 14.1 / 12.0, 256 15.2 / 16.1, 1,024 20.6 / 21.5, 1,500 24.2 / 23.7; 128 rows behind 2,000 21.4 / 15.6.
+    if (!SINK && num_seqs == 1 && tiles * nh <= 148 && (tiles >= 10 || (tiles == 1 && (long long)max_pages * page_size >= 2048)))
+        return prefill_tc_run<SINK, !SINK>(q, q_stride, n_rows, out, out_stride, kcache, vcache, block_tables, max_pages, seq_first_row,
+                                           seq_start_pos, num_seqs, tiles, nh, nkv, hd, page_size, num_pages, scale, window, status, stream, terms);
+    return prefill_tc_run<SINK, false>(q, q_stride, n_rows, out, out_stride, kcache, vcache, block_tables, max_pages, seq_first_row,
+                                       seq_start_pos, num_seqs, tiles, nh, nkv, hd, page_size, num_pages, scale, window, status, stream, terms);
 }
-
 GB_EXPORT int gb_attention_prefill_tc(const void* q, long long q_stride, int n_rows, void* out, long long out_stride,
                                       const void* kcache, const void* vcache, const int* block_tables, int max_pages,
                                       const int* seq_first_row, const int* seq_start_pos, int num_seqs,

@@ -1,0 +1,38 @@
+"""Prompt attention with two blocks a pair of row tiles (one request of many tiles, or of one tile behind a long context)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("nh, nkv, rows, past, window, page", [
+    (9, 3, 1153, 0, 0, 16), (9, 3, 1280, 0, 0, 16), (2, 1, 1281, 0, 0, 64), (3, 1, 1409, 37, 0, 16), (4, 2, 2048, 0, 0, 128), (1, 1, 2047, 1000, 0, 16),
+    (3, 3, 1500, 300, 300, 16), (2, 2, 1300, 700, 65, 8), (2, 1, 1400, 0, -512, 16), (9, 3, 128, 1990, 0, 16), (5, 5, 1, 1920, 0, 16), (3, 1, 77, 1025, 600, 32)])
+def test_pairs_of_row_tiles(nh, nkv, rows, past, window, page):
+    from glassbox_b200 import kernels
+    gen = torch.Generator(device=DEV).manual_seed(rows + past)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device=DEV).bfloat16()
+    total = rows + past
+    used = -(-total // page)
+    width = max(-(-2048 // page), used + 1)                       # (a table that reaches 2,048 keys: one tile takes the pairs too)
+    order = torch.randperm(used + 3, generator=torch.Generator().manual_seed(1))[:used].to(torch.int32)
+    table = torch.full((1, width), -1, dtype=torch.int32)
+    table[0, :used] = order
+    k, v, q = rand(used + 3, nkv, page, 64), rand(used + 3, nkv, page, 64), rand(rows, nh * 64)
+    out, status = torch.full((rows, nh * 64), 7.0, device=DEV, dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    kernels.attention_prefill_tc(q, out, k, v, table.to(DEV), i32([0, rows]), i32([past]), rows, nh, nkv, 64, page, 0.125, window, status)
+    assert int(status) == 0
+    keys, values = (t[order.long().to(DEV)].transpose(1, 2).flatten(0, 1)[:total].double() for t in (k, v))
+    at, pos = torch.arange(total, device=DEV)[None], past + torch.arange(rows, device=DEV)[:, None]
+    seen = at <= pos
+    if window > 0:
+        seen &= at > pos - window
+    elif window < 0:
+        seen &= at >= pos - pos % -window
+    for h in range(nh):
+        s = (q[:, h * 64:h * 64 + 64].double() @ keys[:, h // (nh // nkv)].T * 0.125).masked_fill(~seen, float("-inf"))
+        want = torch.softmax(s, -1) @ values[:, h // (nh // nkv)]
+        # weights in bfloat16 (2^-9 each, of either sign) and one rounding of the result: 2^-8 of values of a few
+        assert (out[:, h * 64:h * 64 + 64].double() - want).abs().max() < 2.0 ** -8 * 4, h
