@@ -254,7 +254,22 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
                     }
                 }
             };
-            if (!GATED && mode == TC_ADD_F32) load_old(first_col);
+            float4 gain = make_float4(0.f, 0.f, 0.f, 0.f);     // of the norm that reads the sums next, likewise
+            auto load_gain = [&](int col0) {
+                const int col = col0 + (lane & 7) * 4;
+                gain = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (col + 4 <= N) {
+                    gain = *reinterpret_cast<const float4*>(norm.gain + col);      // 16-byte aligned (checked by the host)
+                } else {
+                    if (col < N) gain.x = norm.gain[col];
+                    if (col + 1 < N) gain.y = norm.gain[col + 1];
+                    if (col + 2 < N) gain.z = norm.gain[col + 2];
+                }
+            };
+            if (!GATED && mode == TC_ADD_F32) {
+                load_old(first_col);
+                if (norm.gain != nullptr) load_gain(first_col);
+            }
             // mode TC_ROPE_QKV: this lane's row's position and slot, and the rotations of the channels that it will turn for the rows
             // 8 i + lane / 4, requested while the products run
             const bool is_qkv = !GATED && mode == TC_ROPE_QKV;
@@ -263,6 +278,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
             const int h_first = BN > hd ? part * hd : 0, h_step = BN > hd ? 2 * hd : hd;
             const int c_first = BN > hd ? 0 : part * 16, c_step = BN > hd ? 16 : 32;
             const int pos = is_qkv && row < M ? qkv.positions[row] : -1;
+            const long long slot = is_qkv && row < M ? qkv.slots[row] : -1;
             float4 (&cs)[8] = old;      // (a launch is one or the other)
             auto load_cs = [&](int c) {
 #pragma unroll
@@ -284,7 +300,6 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
                 // Stacked QKV (crates/glassbox-core/src/model.rs:266-276): a tile holds whole heads (BN is a multiple
                 // of the head size). Query and key heads are rotated, channel i with channel i + hd/2, from the
                 // float32 sums; queries go to C, rotated keys and the values to the row's cache slot.
-                const long long slot = (row < M && pos >= 0) ? qkv.slots[row] : -1;
                 const bool bad_pos = qkv.rope != nullptr && pos >= qkv.max_pos;
                 const bool bad_slot = qkv.write_kv && pos >= 0 && (slot < 0 || slot >= qkv.num_slots);
                 if (bad_pos) atomicOr(status, GB_STATUS_BAD_POSITION);
@@ -453,14 +468,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
                         // producer half of a split RMSNorm: the new residual values also leave as bfloat16(x * gain) and add their
                         // squares to their rows' sums (columns beyond N hold what the zero-filled weight rows gave: nothing is
                         // stored or summed for them)
-                        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (col + 4 <= N) {
-                            g = *reinterpret_cast<const float4*>(norm.gain + col);      // 16-byte aligned (checked by the host)
-                        } else {
-                            if (col < N) g.x = norm.gain[col];
-                            if (col + 1 < N) g.y = norm.gain[col + 1];
-                            if (col + 2 < N) g.z = norm.gain[col + 2];
-                        }
+                        const float4 g = gain;
                         const bool vec_pre = ((uintptr_t)norm.pre & 7) == 0 && (norm.ldp & 3) == 0 && col + 4 <= N;
                         __nv_bfloat16* pre = norm.pre + (size_t)(m0 + q * 32) * norm.ldp + col;
 #pragma unroll
@@ -485,7 +493,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tcgen05_kernel(const __grid_c
                             }
                         }
                     }
-                    if (c0 + 32 < (part + 1) * (BNO / 2)) load_old(col0 + 32);
+                    if (c0 + 32 < (part + 1) * (BNO / 2)) {
+                        load_old(col0 + 32);
+                        if (norm.gain != nullptr) load_gain(col0 + 32);
+                    }
                 } else {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
