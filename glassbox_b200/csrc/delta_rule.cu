@@ -120,6 +120,79 @@ __global__ void __launch_bounds__(256) short_conv_strip_kernel(const float* __re
     }
 }
 
+// ... and four channels of ROWS rows: 16-byte loads and stores, in the strip's order of sums. Measurements beside the rule in gb_short_conv.
+// Bound by the trip to memory of a block's loads and of its rows' lookups, three blocks an SM.
+template <int TAPS, int ROWS>
+__global__ void __launch_bounds__(256, 3) short_conv_strip4_kernel(const float* __restrict__ x, long long ldx, const float* __restrict__ w,
+                                                                float* __restrict__ y, long long ldy, const float* __restrict__ state,
+                                                                long long state_stride, long long state_off, const int* __restrict__ row_seq,
+                                                                const int* __restrict__ positions, const int* __restrict__ seq_first_row,
+                                                                const int* __restrict__ seq_slots, int n, int C, int num_slots,
+                                                                int* __restrict__ status) {
+    gb_pdl_launch_dependents();
+    gb_pdl_wait();
+    const int row0 = blockIdx.x * ROWS, ch = (blockIdx.y * 256 + threadIdx.x) * 4;
+    float4 in[ROWS + TAPS - 1];                    // rows row0 - (TAPS - 1) .. row0 + ROWS - 1
+#pragma unroll
+    for (int i = 0; i < ROWS + TAPS - 1; ++i) {
+        const int row = row0 - (TAPS - 1) + i;
+        in[i] = row >= 0 && row < n && ch < C ? *reinterpret_cast<const float4*>(x + (size_t)row * ldx + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float tap[4][TAPS];
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i) {                         // (4 * TAPS consecutive numbers)
+        const float4 v = ch < C ? *reinterpret_cast<const float4*>(w + (size_t)ch * TAPS + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tap[(4 * i + e) / TAPS][(4 * i + e) % TAPS] = f[e];
+    }
+    bool own = true;                               // (as above: a row a lane)
+    if ((threadIdx.x & 31) < ROWS) {
+        const int row = row0 + (threadIdx.x & 31);
+        own = row < n && positions[row] >= 0;
+        if (own) {
+            const int seq = row_seq[row], slot = seq_slots[seq];
+            own = slot >= 0 && slot < num_slots && row - (TAPS - 1) >= seq_first_row[seq];
+        }
+    }
+    const bool plain = __all_sync(0xffffffffu, own);
+    if (ch >= C) return;
+    auto silu = [](float v) { return gb_quotient(v, 1.0f + expf(-v)); };
+#pragma unroll
+    for (int t = 0; t < ROWS; ++t) {
+        const int row = row0 + t;
+        float4 v[TAPS];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) v[j] = in[t + j];
+        if (!plain) {
+            if (row >= n || positions[row] < 0) continue;
+            const int seq = row_seq[row], r0 = seq_first_row[seq], slot = seq_slots[seq];
+            if (slot < 0 || slot >= num_slots) {
+                atomicOr(status, GB_STATUS_BAD_SLOT);
+                continue;
+            }
+            const float* st = state + (size_t)slot * state_stride + state_off + ch;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const int src = row - (TAPS - 1) + j;
+                if (src < r0) {
+                    const float* s = st + (size_t)(TAPS - 1 - (r0 - src)) * C;
+                    v[j] = make_float4(s[0], s[1], s[2], s[3]);
+                }
+            }
+        }
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            acc.x = fmaf(tap[0][j], v[j].x, acc.x);
+            acc.y = fmaf(tap[1][j], v[j].y, acc.y);
+            acc.z = fmaf(tap[2][j], v[j].z, acc.z);
+            acc.w = fmaf(tap[3][j], v[j].w, acc.w);
+        }
+        *reinterpret_cast<float4*>(y + (size_t)row * ldy + ch) = make_float4(silu(acc.x), silu(acc.y), silu(acc.z), silu(acc.w));
+    }
+}
+
 // One thread per (sequence, channel): shift what the slot holds by the portion's length and append the portion's last inputs.
 __global__ void __launch_bounds__(256) short_conv_state_kernel(const float* __restrict__ x, long long ldx, float* __restrict__ state,
                                                                long long state_stride, long long state_off,
@@ -157,13 +230,35 @@ GB_EXPORT int gb_short_conv(const float* x, long long ldx, const float* w, float
     gb_launch(GB_PDL_ELEMENTWISE, short_conv_strip_kernel<TAPS>, strips, dim3(256), 0, stream, x, ldx, w, y, ldy, (const float*)state, \
               state_stride, state_off, row_seq, positions, seq_first_row, seq_slots, n, C, num_slots, status)
     const bool many = (long long)strips.x * strips.y >= 444;
-    if (many && taps == 4) SC_STRIPS(4);
+    // Four channels a thread where requests bring sixteen rows and more each on average (where they bring few, every strip looks every row's
+    // request up: 64 rows of as many requests 7.3 us by rows, 8.8 so) and there are 96 rows, in strips of four rows, of eight from
+    // five blocks an SM on. By rows or by the strips below / so, one request, with the state's update, us: 3,072 channels 70 rows 5.8 / 6.0,
+    // 128 6.6 / 6.3, 256 9.5 / 6.2, 512 14.9 / 6.8, 768 11.3 / 8.3, 1,024 13.8 / 9.9, 2,048 18.5 / 14.2 (strips of four 14.9); 6,144
+    // channels 128 9.5 / 6.5, 512 14.1 / 10.1, 2,048 32.1 / 26.0.
+    const bool fours = n >= 96 && n >= 16LL * S && taps >= 2 && taps <= 4 && C % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 &&
+                       (((uintptr_t)x | (uintptr_t)y | (uintptr_t)w) & 15) == 0;
+    const bool eight = (long long)gb_ceil_div(n, 8) * gb_ceil_div(C, 1024) >= 5 * 148;
+#define SC_FOURS(TAPS, ROWS)                                                                                                         \
+    gb_launch(GB_PDL_ELEMENTWISE, short_conv_strip4_kernel<TAPS, ROWS>, dim3(gb_ceil_div(n, ROWS), gb_ceil_div(C, 1024)), dim3(256), 0, \
+              stream, x, ldx, w, y, ldy, (const float*)state, state_stride, state_off, row_seq, positions, seq_first_row, seq_slots, n, C, \
+              num_slots, status)
+#define SC_FOURS_ROWS(TAPS)               \
+    {                                     \
+        if (eight) SC_FOURS(TAPS, 8);     \
+        else SC_FOURS(TAPS, 4);           \
+    }
+    if (fours && taps == 4) SC_FOURS_ROWS(4)
+    else if (fours && taps == 3) SC_FOURS_ROWS(3)
+    else if (fours) SC_FOURS_ROWS(2)
+    else if (many && taps == 4) SC_STRIPS(4);
     else if (many && taps == 3) SC_STRIPS(3);
     else if (many && taps == 2) SC_STRIPS(2);
     else
         gb_launch(GB_PDL_ELEMENTWISE, short_conv_kernel, grid, dim3(256), 0, stream, x, ldx, w, y, ldy, (const float*)state, state_stride,
                   state_off, row_seq, positions, seq_first_row, seq_slots, n, C, taps, num_slots, status);
 #undef SC_STRIPS
+#undef SC_FOURS_ROWS
+#undef SC_FOURS
     int rc = gb_check_launch("gb_short_conv");
     if (rc || !update_state || taps == 1) return rc;
     dim3 grid2(S, gb_ceil_div(C, 256));

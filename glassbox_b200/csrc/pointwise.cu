@@ -349,6 +349,70 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __res
     }
 }
 
+// The same with four numbers a lane and two (row, head) a warp, all loads asked for before the first sum: a number a lane and load took a
+// (row, head) in two dependent trips to memory, 4 bytes a lane at a time. 2,048 rows of 8 heads of 128 12.2 -> 5.1 us (20 MB).
+__device__ __forceinline__ void ghn_store(float* dst, const float4& v) { *reinterpret_cast<float4*>(dst) = v; }
+__device__ __forceinline__ void ghn_store(__nv_bfloat16* dst, const float4& v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+template <typename T, int QUADS>          // QUADS: of four numbers, a lane's share of v
+__global__ void __launch_bounds__(128) gated_head_norm4_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long ldg,
+                                                               const float* __restrict__ w, T* __restrict__ out, int n, int heads, int v,
+                                                               float eps, int gate_silu) {
+    constexpr int TASKS = 2;
+    gb_pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 wv[QUADS];
+#pragma unroll
+    for (int k = 0; k < QUADS; ++k) wv[k] = (lane + 32 * k) * 4 < v ? *reinterpret_cast<const float4*>(w + (lane + 32 * k) * 4) : none;   // (a weight)
+    gb_pdl_wait();
+    const long long task0 = ((long long)blockIdx.x * 4 + warp) * TASKS, tasks = (long long)n * heads;
+    float4 x[TASKS][QUADS], g[TASKS][QUADS];
+#pragma unroll
+    for (int t = 0; t < TASKS; ++t) {
+        const long long task = task0 + t, row = task / heads;
+        const int head = (int)(task - row * heads);
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k) {
+            const int j = (lane + 32 * k) * 4;
+            const bool in = task < tasks && j < v;
+            x[t][k] = in ? *reinterpret_cast<const float4*>(o + task * v + j) : none;
+            g[t][k] = in ? *reinterpret_cast<const float4*>(gate + row * ldg + (long long)head * v + j) : none;
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TASKS; ++t) {
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k)
+            ss = fmaf(x[t][k].x, x[t][k].x, fmaf(x[t][k].y, x[t][k].y, fmaf(x[t][k].z, x[t][k].z, fmaf(x[t][k].w, x[t][k].w, ss))));
+        ss = gb_warp_sum(ss);
+        const float s = 1.0f / sqrtf(ss / (float)v + eps);
+        auto one = [&](float a, float z, float c) {
+            const float d = 1.0f + expf(-z);
+            return a * s * c * (gate_silu ? gb_quotient(z, d) : gb_quotient(1.0f, d));
+        };
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k) {
+            const int j = (lane + 32 * k) * 4;
+            if (task0 + t < tasks && j < v)
+                ghn_store(out + (task0 + t) * v + j, make_float4(one(x[t][k].x, g[t][k].x, wv[k].x), one(x[t][k].y, g[t][k].y, wv[k].y),
+                                                                one(x[t][k].z, g[t][k].z, wv[k].z), one(x[t][k].w, g[t][k].w, wv[k].w)));
+        }
+    }
+}
+
+template <typename T>
+static int ghn4_launch(const float* o, const float* gate, long long ldg, const float* w, T* out, int n, int heads, int v, float eps, int gate_silu,
+                       cudaStream_t stream) {
+    const dim3 grid((unsigned)(((long long)n * heads + 7) / 8));
+    if (v <= 128) gb_launch(GB_PDL_ELEMENTWISE, gated_head_norm4_kernel<T, 1>, grid, dim3(128), 0, stream, o, gate, ldg, w, out, n, heads, v, eps, gate_silu);
+    else gb_launch(GB_PDL_ELEMENTWISE, gated_head_norm4_kernel<T, 2>, grid, dim3(128), 0, stream, o, gate, ldg, w, out, n, heads, v, eps, gate_silu);
+    return gb_check_launch("gb_gated_head_norm");
+}
+
 // The same for long rows (a norm that spans all heads): one block per (row, head), the sum of squares meets in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(256) gated_head_norm_wide_kernel(const float* __restrict__ o, const float* __restrict__ gate,
@@ -390,6 +454,11 @@ GB_EXPORT int gb_gated_head_norm(const float* o, const float* gate, long long ld
         else
             GB_REQUIRE(false, "gb_gated_head_norm: unsupported output dtype %d", out_dtype);
         return gb_check_launch("gb_gated_head_norm");
+    }
+    if (v % 4 == 0 && ldg % 4 == 0 && (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)w) & 15) == 0) {
+        if (out_dtype == GB_F32 && ((uintptr_t)out & 15) == 0) return ghn4_launch(o, gate, ldg, w, (float*)out, n, heads, v, eps, gate_silu, stream);
+        if (out_dtype == GB_BF16 && ((uintptr_t)out & 7) == 0)
+            return ghn4_launch(o, gate, ldg, w, (__nv_bfloat16*)out, n, heads, v, eps, gate_silu, stream);
     }
     const int blocks = gb_ceil_div((long long)n * heads, 4);
     if (out_dtype == GB_F32)
