@@ -47,7 +47,7 @@ template <int BN, bool GATED>
 __global__ void __launch_bounds__(128) head_linear_kernel(const __nv_bfloat16* __restrict__ a, long long lda, long long a_head,
                                                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                           long long ldc, long long c_head, int n, int N, int K,
-                                                          const void* __restrict__ gate, long long ld_gate, int gate_kind, HlTurn turn) {
+                                                          const void* __restrict__ gate, long long ld_gate, int gate_kind, int vec, HlTurn turn) {
     extern __shared__ __align__(128) unsigned char hl_smem[];
     gb_pdl_launch_dependents();
     const int KS = K + 8;                                    // padded row, elements
@@ -136,16 +136,40 @@ __global__ void __launch_bounds__(128) head_linear_kernel(const __nv_bfloat16* _
             dst[k + turn.half] = __float2bfloat16_rn(v * cs + u * sn);
         }
     }
-    __nv_bfloat16* oh = out + (size_t)head * c_head + n0;
+    if constexpr (GATED) {
 #pragma unroll
-    for (int nt = 0; nt < BN / 8; ++nt) {
-        const int col = nt * 8 + 2 * t;
-        if constexpr (GATED) {
+        for (int nt = 0; nt < BN / 8; ++nt) {
             acc[nt][0] = hl_open(acc[nt][0], gate_a[nt].x);
             acc[nt][1] = hl_open(acc[nt][1], gate_a[nt].y);
             acc[nt][2] = hl_open(acc[nt][2], gate_b[nt].x);
             acc[nt][3] = hl_open(acc[nt][3], gate_b[nt].y);
         }
+    }
+    __nv_bfloat16* oh = out + (size_t)head * c_head + n0;
+    if (vec) {
+        // a warp's 16 rows turn over in shared memory, where the operands were: a store writes whole rows and not 16 bytes in each of
+        // eight (1,500 rows of 32 heads: N 128, K 64 10.4 -> 7.3 us, N 64, K 128 7.4 -> 6.4; 8 rows 3.0 -> 2.5 and 2.3 -> 2.2)
+        constexpr int LD = BN + 8;
+        __syncthreads();
+        __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(hl_smem) + warp * 16 * LD;
+#pragma unroll
+        for (int nt = 0; nt < BN / 8; ++nt) {
+            *reinterpret_cast<__nv_bfloat162*>(tile + g * LD + nt * 8 + 2 * t) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
+            *reinterpret_cast<__nv_bfloat162*>(tile + (g + 8) * LD + nt * 8 + 2 * t) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
+        }
+        __syncwarp();
+        const int row0 = m0 + warp * 16;
+#pragma unroll
+        for (int i = 0; i < BN / 16; ++i) {                    // 16 rows of BN / 8 pieces
+            const int piece = (i * 32 + lane) % (BN / 8), r = (i * 32 + lane) / (BN / 8);
+            if (row0 + r < n && piece * 8 < cols)
+                *reinterpret_cast<uint4*>(oh + (size_t)(row0 + r) * ldc + piece * 8) = *reinterpret_cast<const uint4*>(tile + r * LD + piece * 8);
+        }
+        return;
+    }
+#pragma unroll
+    for (int nt = 0; nt < BN / 8; ++nt) {
+        const int col = nt * 8 + 2 * t;
         if (col < cols) {      // (N is even: a pair never straddles the edge)
             if (row_a < n) {
                 __nv_bfloat162 v = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
@@ -179,9 +203,11 @@ GB_EXPORT int gb_head_linear(const void* a, long long lda, long long a_head, con
     // narrow heads take the narrow tile: half the registers and less shared memory, so more blocks at once
     const bool narrow = N <= HL_BN / 2;
     const int bn = narrow ? HL_BN / 2 : HL_BN;
-    const size_t smem = (size_t)(HL_BM + bn) * (K + 8) * sizeof(__nv_bfloat16);
+    const size_t operands = (size_t)(HL_BM + bn) * (K + 8) * sizeof(__nv_bfloat16), turned = (size_t)HL_BM * (bn + 8) * sizeof(__nv_bfloat16);
+    const size_t smem = operands > turned ? operands : turned;
+    const int vec = N % 8 == 0 && ldc % 8 == 0 && c_head % 8 == 0 && (uintptr_t)out % 16 == 0;
     void (*kernel)(const __nv_bfloat16*, long long, long long, const __nv_bfloat16*, __nv_bfloat16*, long long, long long, int, int, int, const void*,
-                   long long, int, HlTurn) = narrow ? (gate ? head_linear_kernel<HL_BN / 2, true> : head_linear_kernel<HL_BN / 2, false>)
+                   long long, int, int, HlTurn) = narrow ? (gate ? head_linear_kernel<HL_BN / 2, true> : head_linear_kernel<HL_BN / 2, false>)
                                             : (gate ? head_linear_kernel<HL_BN, true> : head_linear_kernel<HL_BN, false>);
     static size_t allowed[4] = {48 * 1024, 48 * 1024, 48 * 1024, 48 * 1024};
     size_t& have = allowed[(narrow ? 2 : 0) + (gate ? 1 : 0)];
@@ -191,7 +217,7 @@ GB_EXPORT int gb_head_linear(const void* a, long long lda, long long a_head, con
     }
     dim3 grid(gb_ceil_div(n, HL_BM), heads, gb_ceil_div(N, bn));
     cudaError_t e = gb_launch(GB_PDL_GEMM, kernel, grid, dim3(128), smem, stream, (const __nv_bfloat16*)a, lda, a_head, (const __nv_bfloat16*)w,
-                              (__nv_bfloat16*)out, ldc, c_head, n, N, K, gate, ld_gate, kind, HlTurn{positions, inv_freq, magnitude, rot_dims / 2, dims});
+                              (__nv_bfloat16*)out, ldc, c_head, n, N, K, gate, ld_gate, kind, vec, HlTurn{positions, inv_freq, magnitude, rot_dims / 2, dims});
     if (e != cudaSuccess) {
         gb_set_error("gb_head_linear: launch failed: %s", cudaGetErrorString(e));
         return 2;
