@@ -13,8 +13,9 @@
 // Rows past an expert's last pair are loaded (another row's numbers) and never stored. A k-block takes 1.4 us with 32 gathers, 0.3 with
 // a box of rows (the products 0.26), so a pass that brings the rows into slot order (16.8 MB: 4 us) pays from 64 pairs per expert
 // on; with fewer a tile needs only a gather or two and the pass would cost its launch. Measured, 2,048 rows, 16 experts, four per
-// token (1024 -> 2 x 1024 -> 1024): up half 101 us with gathers, 47 + 4 with the pass; down half 38 -> 23 with the epilogue of eight warps
-// and 16-byte stores. With few pairs per expert it is bound by reading every expert's matrices once.
+// token (1024 -> 2 x 1024 -> 1024): up half 101 us with gathers, 47 + 4 with the pass, 35 + 4 since the epilogue's units are told apart once
+// (me_units); down half 38 -> 23 with the epilogue of eight warps and 16-byte stores. The up half's four rounds of tiles take 700 cycles a
+// k-block of 48 KB where the products take 540, behind 7,000 of start. With few pairs per expert it is bound by reading every expert's matrices once.
 //
 // Every wait is bounded, as in the dense product: on a timeout the block records GB_STATUS_WAIT_TIMEOUT, waits (bounded) for its
 // copies, frees its tensor memory and returns. No multicast.
@@ -43,13 +44,26 @@ __device__ __forceinline__ void me_gather4(void* dst, const CUtensorMap* map, ui
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
 
-// One gated unit with the numbers of gb_gated_unit.
-__device__ __forceinline__ float me_unit(float gate, float up, float limit, float slope) {
+// Gated units with the numbers of gb_gated_unit: v holds 16 pairs of a gate sum and an up sum. Which unit it is is asked once for all of them:
+// asked for every pair, in code unrolled over the pairs, the three kinds made an epilogue of 77 KB of instructions that came from
+// memory for every tile (16,600 cycles a tile of 128 x 256 sums, whose products take 10,000).
+__device__ __forceinline__ void me_units(const uint32_t (&v)[32], uint32_t* u, float limit, float slope) {
     if (slope > 0.f) {
-        const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-        return gb_quotient(g, 1.0f + expf(-slope * g)) * (u + 1.0f);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float g = fminf(__uint_as_float(v[2 * j]), limit), up = fminf(fmaxf(__uint_as_float(v[2 * j + 1]), -limit), limit);
+            u[j] = __float_as_uint(gb_quotient(g, 1.0f + expf(-slope * g)) * (up + 1.0f));
+        }
+    } else if (slope < 0.f) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(gb_gelu_tanh(__uint_as_float(v[2 * j])) * __uint_as_float(v[2 * j + 1]));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float g = __uint_as_float(v[2 * j]);
+            u[j] = __float_as_uint(gb_quotient(g, 1.0f + expf(-g)) * __uint_as_float(v[2 * j + 1]));
+        }
     }
-    return slope < 0.f ? gb_gelu_tanh(gate) * up : gb_quotient(gate, 1.0f + expf(-gate)) * up;
 }
 
 template <int BN, bool UP>
@@ -218,15 +232,18 @@ __global__ void __launch_bounds__(ME_THREADS) moe_tcgen05_kernel(const __grid_co
                         // neighbouring outputs are the gate sum and the up sum of one unit
                         col0 >>= 1;
                         cols >>= 1;
-                        uint32_t u[32];
+                        // (32 units of a row are 64 bytes: two pieces of each half of the turned tile, as tc_turn_put_bf16 lays them)
+#pragma unroll 1
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t u[16];
+                            if (h) tmem_load32(t_base + (uint32_t)(c0 + 32), v);
+                            me_units(v, u, limit, slope);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            u[j] = __float_as_uint(me_unit(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), limit, slope));
-                        tmem_load32(t_base + (uint32_t)(c0 + 32), v);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            u[16 + j] = __float_as_uint(me_unit(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), limit, slope));
-                        tc_turn_put_bf16(stage, lane, u);
+                            for (int c = 0; c < 2; ++c)
+                                stage[lane * 4 + ((2 * h + c) ^ ((lane >> 1) & 3))] =
+                                    make_uint4(pack2(u[8 * c], u[8 * c + 1]), pack2(u[8 * c + 2], u[8 * c + 3]), pack2(u[8 * c + 4], u[8 * c + 5]),
+                                               pack2(u[8 * c + 6], u[8 * c + 7]));
+                        }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
