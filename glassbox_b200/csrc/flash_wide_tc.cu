@@ -41,6 +41,7 @@ struct FwArgs {
     int window, wide, vdim;    // channels of a row's output in all; of a value head
     int key_steps;             // 16-channel steps of a key row
     int col_blocks;            // blocks of DV channels that a row's output is cut into
+    int merged;                // a page's values of all the block's heads come as one copy (see fw_values_merged)
     int* status;
 };
 
@@ -114,9 +115,9 @@ __device__ __forceinline__ void fw_tanh(uint32_t (&s)[64], float in) {
         s[k + 1] = __float_as_uint(w.y);
     }
 }
-// MN-major B operand (rows are keys, 64-channel column blocks FW_BLOCK apart), 128-byte-swizzled rows
-__device__ __forceinline__ uint64_t fw_desc_mn(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)(FW_BLOCK >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
+// MN-major B operand (rows are keys, 64-channel column blocks `block` bytes apart), 128-byte-swizzled rows
+__device__ __forceinline__ uint64_t fw_desc_mn(uint32_t smem_addr, int block) {
+    return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)(block >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
            (uint64_t)2 << 61;
 }
 __device__ __forceinline__ void fw_tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
@@ -157,6 +158,12 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
     const int key_lo = gb_first_key(pos_lo, a.window);
     const int kt_begin = key_lo / FW_BN, ntiles = pos_hi / FW_BN - kt_begin + 1;
     const int* table = a.block_tables + (size_t)seq * a.max_pages;
+    // Where a key's values lie in a tile: column blocks of all 128 keys one behind the other, or (merged) a page's column blocks together
+    const bool merged = !LATENT && a.merged;
+    const int v_block = merged ? a.page_size * 128 : FW_BLOCK;
+    auto value_at = [&](int block, int key) {
+        return merged ? (key >> a.page_shift) * (DV / 64) * v_block + block * v_block + (key & (a.page_size - 1)) * 128 : block * FW_BLOCK + key * 128;
+    };
 
     if (tid == 0) {
         mbar_init(&sh.q_full, 1);
@@ -198,7 +205,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         const int keys = front + max(FW_BN - 1 - hi, 0);
         for (int i = lane; i < keys * (DV / 8); i += 32) {      // 16-byte pieces of a key's values, eight a column block
             const int k = i / (DV / 8), piece = i % (DV / 8), key = k < front ? k : hi + 1 + k - front;
-            *reinterpret_cast<uint4*>(values + (piece >> 3) * FW_BLOCK + key * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(values + value_at(piece >> 3, key) + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -243,8 +250,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             if (lane < ppt) {
                 const bool there = entry >= 0 && entry < a.num_pages;
                 if (!there && entry != UNSEEN) bad = 1;
-                unsigned char* dst = ring + s * bytes + lane * a.page_size * 128;
-                for (int b = 0; b < boxes; ++b) {
+                unsigned char* dst = ring + s * bytes + lane * a.page_size * 128 * (what == 1 && merged ? boxes : 1);
+                if (what == 1 && merged)
+                    tma_load_2d(dst, &map_v, &full[s], 0, there ? (entry * a.kv_heads + col0 / 64) * a.page_size : nowhere);
+                else for (int b = 0; b < boxes; ++b) {
                     if (what == 0) {
                         tma_load_2d(dst + b * FW_BLOCK, &map_k, &full[s], b * 64, there ? (entry * a.kv_heads + kvh) * a.page_size : nowhere);
                     } else {
@@ -268,7 +277,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         // ------------------------------------------------------------------------- MMA issuer
         if (elect_one()) {
             const uint32_t idesc_qk = umma_idesc(FW_BM, FW_BN), idesc_pv = umma_idesc(FW_BM, DV) | (1u << 16);     // (B is MN-major)
-            const uint64_t q_desc = umma_desc(smem_u32(Qs)), k_desc = umma_desc(smem_u32(Ks)), v_desc = fw_desc_mn(smem_u32(Vs));
+            const uint64_t q_desc = umma_desc(smem_u32(Qs)), k_desc = umma_desc(smem_u32(Ks)), v_desc = fw_desc_mn(smem_u32(Vs), v_block);
+            uint32_t v_step[FW_BN / 16];                        // where 16 keys' values start, in the descriptor's units
+#pragma unroll
+            for (int kk = 0; kk < FW_BN / 16; ++kk) v_step[kk] = (uint32_t)value_at(0, kk * 16) >> 4;
             bool ok = mbar_wait(&sh.q_full, 0, abort_flag, a.status);
             if (ok) sh.q_consumed = 1;
             auto scores = [&](int j) {
@@ -299,7 +311,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 const uint64_t vd = v_desc + (uint64_t)((s * (LATENT ? G::K_BYTES : G::V_BYTES)) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < FW_BN / 16; ++kk)         // 16 keys an instruction: 8 columns of P, 16 rows of the values
-                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + kk * 8), vd + (uint64_t)((kk * 16 * 128) >> 4), idesc_pv,
+                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + kk * 8), vd + v_step[kk], idesc_pv,
                                  (j | kk) ? 1u : 0u);
                 umma_commit(&sh.pv_done);
                 umma_commit(LATENT ? &sh.k_empty[s] : &sh.v_empty[s]);
@@ -402,28 +414,37 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
             const float top = fmaxf(m2, sink2), corr = fw_exp2(m2 - top);
             l = l * corr + fw_exp2(sink2 - top);
             const float inv = l > 0.f ? corr / l : 0.f;
-            const size_t row = (size_t)(row0 + q_lo + r);
+            // Rows turn over where the keys were (all products are done, nothing is on its way there): a store writes 128 bytes of four rows,
+            // of bfloat16 64 of eight, and not 16 bytes in each of 32 (float32, 256 channels: 10,800 cycles a block, 2,600 so).
+            uint4* stage = reinterpret_cast<uint4*>(Ks) + (warp - 2) * (32 * 8);
+            const int live = min(32, nrows - q_lo - q * 32);
+            const size_t row0w = (size_t)(row0 + q_lo + q * 32);
 #pragma unroll 1
             for (int c = h * (DV / 2); c < (h + 1) * (DV / 2); c += 32) {
                 uint32_t ov[32];
                 tmem_load32(lane_base + (uint32_t)(G::O_COL + c), ov);
-                if (q_lo + r < nrows) {
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * inv);
-                    if (LATENT) {
-                        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
+                for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * inv);
+                if (LATENT) {
+                    tc_turn_put_bf16(stage, lane, ov);
+                    __syncwarp();
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + (row0w * a.H + head) * a.wide + col0 + c + 8 * (lane & 3);
 #pragma unroll
-                        for (int k = 0; k < 32; k += 8)
-                            *reinterpret_cast<uint4*>(dst + k) = make_uint4(pack2(ov[k], ov[k + 1]), pack2(ov[k + 2], ov[k + 3]),
-                                                                            pack2(ov[k + 4], ov[k + 5]), pack2(ov[k + 6], ov[k + 7]));
-                    } else {
-                        float* dst = reinterpret_cast<float*>(a.out) + (row * a.H + head) * a.wide + col0 + c;
+                    for (int i = 0; i < 4; ++i) {
+                        const int rr = 8 * i + (lane >> 2);
+                        if (rr < live) *reinterpret_cast<uint4*>(dst + (size_t)rr * a.H * a.wide) = tc_turn_get_bf16(stage, lane, i);
+                    }
+                } else {
+                    tc_turn_put_f32(stage, lane, ov);
+                    __syncwarp();
+                    float* dst = reinterpret_cast<float*>(a.out) + (row0w * a.H + head) * a.wide + col0 + c + 4 * (lane & 7);
 #pragma unroll
-                        for (int k = 0; k < 32; k += 4)
-                            *reinterpret_cast<uint4*>(dst + k) = make_uint4(ov[k], ov[k + 1], ov[k + 2], ov[k + 3]);
+                    for (int i = 0; i < 8; ++i) {
+                        const int rr = 4 * i + (lane >> 3);
+                        if (rr < live) *reinterpret_cast<float4*>(dst + (size_t)rr * a.H * a.wide) = tc_turn_get_f32(stage, lane, i);
                     }
                 }
-                __syncwarp();      // the next load is the whole warp's; lanes past the last row have taken the other way here
+                __syncwarp();      // (the tile is read before it is written again; the next load is the whole warp's)
             }
         }
     } else if (LATENT) {
@@ -463,6 +484,11 @@ static int fw_map_q(CUtensorMap* map, const void* q, long long n, int H, int dim
     return 0;
 }
 
+// Value heads of 64 lie one behind the other in a page: a block's heads come in one copy of up to 256 rows, where 16 keys of a product lie in
+// one page. A copy a page and head (32 of 2 KB a tile of 256 channels and pages of 16) cost more than the tile's products: 2,048 tokens,
+// 16/4 heads, pages of 16 / 32 / 64 / 128 tokens 56.9 / 50.8 / 47.9 / 47.8 us; with this and whole rows stored 41.2 at all of them.
+static int fw_values_merged(int vdim, int dv, int page_size) { return vdim == 64 && page_size >= 16 && page_size * (dv / 64) <= 256; }
+
 template <int KB, int DV, bool LATENT>
 static int fw_launch(const void* q, const void* kcache, const void* vcache, int n, int dim, int num_seqs, int max_rows, const FwArgs& a,
                      cudaStream_t stream, const char* who) {
@@ -471,7 +497,8 @@ static int fw_launch(const void* q, const void* kcache, const void* vcache, int 
     if (fw_map_q(&mq, q, n, a.H, dim, who)) return 1;
     if (tc_make_map_2d(&mk, kcache, a.num_pages * a.kv_heads * a.page_size, dim, dim, a.page_size, 64, who)) return 1;
     if (LATENT) mv = mk;
-    else if (tc_make_map_2d(&mv, vcache, a.num_pages * a.kv_heads * a.page_size, a.vdim, a.vdim, a.page_size, 64, who)) return 1;
+    else if (tc_make_map_2d(&mv, vcache, a.num_pages * a.kv_heads * a.page_size, a.vdim, a.vdim, a.merged ? a.page_size * (DV / 64) : a.page_size, 64,
+                            who)) return 1;
     auto kernel = flash_wide_kernel<KB, DV, LATENT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
     GB_REQUIRE(e == cudaSuccess, "%s: %d bytes of shared memory refused: %s", who, G::SMEM, cudaGetErrorString(e));
@@ -508,12 +535,14 @@ GB_EXPORT int gb_talking_attention_flash(const void* q, float* out, const void* 
     if (n == 0 || num_seqs == 0 || max_rows_per_seq <= 0) return 0;
     const int wide = G * V;
     FwArgs a = {out, block_tables, max_pages, seq_first_row, seq_start_pos, nullptr, H, G, page_size, fw_page_shift(page_size), num_pages, scale, cap,
-                unit, window, wide, V, 4, 1, status};
+                unit, window, wide, V, 4, 1, 0, status};
     if (wide % 256 == 0) {
         a.col_blocks = wide / 256;
+        a.merged = fw_values_merged(V, 256, page_size);
         return fw_launch<1, 256, false>(q, kcache, vcache, n, 64, num_seqs, max_rows_per_seq, a, stream, "gb_talking_attention_flash");
     }
     a.col_blocks = wide / 128;
+    a.merged = fw_values_merged(V, 128, page_size);
     return fw_launch<1, 128, false>(q, kcache, vcache, n, 64, num_seqs, max_rows_per_seq, a, stream, "gb_talking_attention_flash");
 }
 
@@ -532,6 +561,6 @@ GB_EXPORT int gb_latent_flash(const void* q, void* out, const void* cache, const
     GB_REQUIRE(n >= 0 && num_seqs >= 0 && max_pages > 0 && num_pages * page_size < (1ll << 31), "gb_latent_flash: bad batch shape");
     if (n == 0 || num_seqs == 0 || max_rows_per_seq <= 0) return 0;
     FwArgs a = {out, block_tables, max_pages, seq_first_row, seq_start_pos, sink, H, 1, page_size, fw_page_shift(page_size), num_pages, scale, 0.f,
-                0, window, 128, 128, (c + r) / 16, 1, status};
+                0, window, 128, 128, (c + r) / 16, 1, 0, status};
     return fw_launch<3, 128, true>(q, cache, cache, n, c + r, num_seqs, max_rows_per_seq, a, stream, "gb_latent_flash");
 }
