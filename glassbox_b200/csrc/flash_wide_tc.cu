@@ -67,7 +67,7 @@ __device__ __forceinline__ float fw_exp2(float x) {
 }
 // s <- tanh(s * in) for a warp's scores, as exactly as a call of tanhf (at most 1.1 units in the last place below 1, two beyond; NaN
 // stays NaN). The tanh of y is y + y t c(t), t = y^2, with c the interpolation of (tanh(sqrt t) / sqrt t - 1) / t at Chebyshev nodes: of
-// [0, 0.36] for a warp whose scores all lie within 0.6 of the cap (most do), of [0, 1] otherwise, fused multiply-adds of two
+// [0, 0.0625] for a warp whose scores all lie within a quarter of the cap (most do), of [0, 0.36] and [0, 1] otherwise, fused multiply-adds of two
 // scores at a time and no special function. Where a score lies beyond the cap, 1 - 2 / (1 + e^(2|y|)).
 __device__ __forceinline__ void fw_tanh(uint32_t (&s)[64], float in) {
     float tops[4] = {0.f, 0.f, 0.f, 0.f};
@@ -81,6 +81,18 @@ __device__ __forceinline__ void fw_tanh(uint32_t (&s)[64], float in) {
     }
     const float top = fmaxf(fmaxf(tops[0], tops[1]), fmaxf(tops[2], tops[3]));
     auto both = [](float c) { return make_float2(c, c); };
+    if (!__any_sync(0xffffffffu, top >= 0.25f)) {
+#pragma unroll
+        for (int k = 0; k < 64; k += 2) {
+            const float2 y = make_float2(__uint_as_float(s[k]), __uint_as_float(s[k + 1])), t = __fmul2_rn(y, y);
+            float2 w = __ffma2_rn(both(-0.051974945f), t, both(0.13328698f));
+            w = __ffma2_rn(w, t, both(-0.33333316f));
+            w = __ffma2_rn(y, __fmul2_rn(w, t), y);
+            s[k] = __float_as_uint(w.x);
+            s[k + 1] = __float_as_uint(w.y);
+        }
+        return;
+    }
     if (!__any_sync(0xffffffffu, top >= 0.6f)) {
 #pragma unroll
         for (int k = 0; k < 64; k += 2) {
@@ -311,7 +323,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 const uint64_t vd = v_desc + (uint64_t)((s * (LATENT ? G::K_BYTES : G::V_BYTES)) >> 4);
 #pragma unroll
                 for (int kk = 0; kk < FW_BN / 16; ++kk)         // 16 keys an instruction: 8 columns of P, 16 rows of the values
-                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + kk * 8), vd + v_step[kk], idesc_pv,
+                    umma_bf16_ts(tmem + (uint32_t)G::O_COL, tmem + (uint32_t)((j & 1) * FW_BN + (kk >> 2) * 64 + (kk & 3) * 8), vd + v_step[kk], idesc_pv,
                                  (j | kk) ? 1u : 0u);
                 umma_commit(&sh.pv_done);
                 umma_commit(LATENT ? &sh.k_empty[s] : &sh.v_empty[s]);
@@ -329,6 +341,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? a.scale / a.cap : 0.f;
         const float slx = cap2 > 0.f ? cap2 : sl2;              // what is left to scale
         const int first = gb_first_key(pos, a.window), first_last = gb_first_key(pos_lo + FW_BM - 1, a.window);
+        const bool bounded = a.cap > 0.f && a.cap <= 32.f && first_last == 0;      // (and every row sees a key of the first tile)
         float m_run = FW_NEG_BIG, l_run = 0.f;
         bool ok = true;
         for (int j = 0; j < ntiles; ++j) {
@@ -344,36 +357,40 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 for (int k = 0; k < 64; ++k)
                     if (!(key0 + k <= pos && key0 + k >= first)) sv[k] = __float_as_uint(FW_NEG_BIG);
             }
-            float mx4[4] = {FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG};
+            // Scores that a cap bounds: the first tile's maximum stays, or -16 (a weight is then at most e^48), and the two halves of a row go
+            // their own ways, one's caps beside the other's exponentials.
+            if (j == 0 || !bounded) {
+                float mx4[4] = {FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG};
 #pragma unroll
-            for (int k = 0; k < 64; k += 8)
+                for (int k = 0; k < 64; k += 8)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) asm("max.f32 %0, %0, %1, %2;" : "+f"(mx4[u]) : "f"(__uint_as_float(sv[k + 2 * u])), "f"(__uint_as_float(sv[k + 2 * u + 1])));
-            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            // the partner's maximum. Once both have met here, both have also read their scores: P may take their place
-            sh.stat[b][h][r] = mx;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.x_bar[q]);
-            if (!mbar_wait_warp(&sh.x_bar[q], j & 1, abort_flag, a.status)) { ok = false; break; }
-            mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
-            const bool raise = (mx - m_run) * slx > 8.0f;
-            if (j == 0) {
-                if (raise) m_run = mx;                          // nothing is accumulated yet
-            } else if (__any_sync(0xffffffffu, raise)) {
-                // (S_j was issued after O += P_(j-2) V_(j-2) was done: the phase of P_(j-1) V_(j-1) is the one to wait for)
-                if (!mbar_wait_warp(&sh.pv_done, (j - 1) & 1, abort_flag, a.status)) { ok = false; break; }
-                tc_fence_after();
-                const float corr = raise ? fw_exp2((m_run - mx) * slx) : 1.0f;
-                if (raise) m_run = mx;
-                l_run *= corr;
+                    for (int u = 0; u < 4; ++u) asm("max.f32 %0, %0, %1, %2;" : "+f"(mx4[u]) : "f"(__uint_as_float(sv[k + 2 * u])), "f"(__uint_as_float(sv[k + 2 * u + 1])));
+                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                // the partner's maximum
+                sh.stat[b][h][r] = mx;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.x_bar[q]);
+                if (!mbar_wait_warp(&sh.x_bar[q], j & 1, abort_flag, a.status)) { ok = false; break; }
+                mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
+                const bool raise = (mx - m_run) * slx > 8.0f;
+                if (j == 0) {
+                    if (raise) m_run = bounded ? fmaxf(mx, -16.0f / a.cap) : mx;      // nothing is accumulated yet (scores are in units of the cap)
+                } else if (__any_sync(0xffffffffu, raise)) {
+                    // (S_j was issued after O += P_(j-2) V_(j-2) was done: the phase of P_(j-1) V_(j-1) is the one to wait for)
+                    if (!mbar_wait_warp(&sh.pv_done, (j - 1) & 1, abort_flag, a.status)) { ok = false; break; }
+                    tc_fence_after();
+                    const float corr = raise ? fw_exp2((m_run - mx) * slx) : 1.0f;
+                    if (raise) m_run = mx;
+                    l_run *= corr;
 #pragma unroll 1
-                for (int c = 0; c < DV / 2; c += 32) {
-                    uint32_t ov[32];
-                    const uint32_t at = lane_base + (uint32_t)(G::O_COL + h * (DV / 2) + c);
-                    tmem_load32(at, ov);
+                    for (int c = 0; c < DV / 2; c += 32) {
+                        uint32_t ov[32];
+                        const uint32_t at = lane_base + (uint32_t)(G::O_COL + h * (DV / 2) + c);
+                        tmem_load32(at, ov);
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * corr);
-                    tmem_store32(at, ov);
+                        for (int k = 0; k < 32; ++k) ov[k] = __float_as_uint(__uint_as_float(ov[k]) * corr);
+                        tmem_store32(at, ov);
+                    }
                 }
             }
             // a masked key holds -1e30 and comes out as exactly 0; a row that has seen no key yet must not cancel that
@@ -390,16 +407,17 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
             }
             l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
-            tmem_store32(lane_base + (uint32_t)(b * FW_BN + h * 32), pw);
+            tmem_store32(lane_base + (uint32_t)(b * FW_BN + h * 64), pw);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.p_ready[b]);
         }
         if (ok) {                                               // the halves' sums
-            sh.stat[ntiles & 1][h][r] = l_run;
+            const int turn = bounded ? 1 : ntiles;              // exchanges of the halves so far
+            sh.stat[turn & 1][h][r] = l_run;
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.x_bar[q]);
-            ok = mbar_wait_warp(&sh.x_bar[q], ntiles & 1, abort_flag, a.status);
+            ok = mbar_wait_warp(&sh.x_bar[q], turn & 1, abort_flag, a.status);
             // A barrier of its own, with one phase, says that all products are done: nothing orders this look against the last two
             // phases of pv_done, and a parity tells an open phase from its neighbours only (with both complete, the wait for the
             // last but one would take the next, open phase for it and never pass).
@@ -407,7 +425,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         }
         if (ok) {
             tc_fence_after();
-            float l = l_run + sh.stat[ntiles & 1][h ^ 1][r], m2 = m_run <= FW_NEG_BIG ? FW_NEG_BIG : m_run * slx;
+            float l = l_run + sh.stat[(bounded ? 1 : ntiles) & 1][h ^ 1][r], m2 = m_run <= FW_NEG_BIG ? FW_NEG_BIG : m_run * slx;
             float sink2 = FW_NEG_BIG;
             if (LATENT && a.sink != nullptr) sink2 = a.sink[head] * FW_LOG2E;
             if (a.unit) sink2 = 0.f;
