@@ -25,7 +25,7 @@
 template <int HD, int BK, int NW, bool CLUSTER, bool SINK = false>
 __global__ void __launch_bounds__(NW * 32) attention_decode_mma_kernel(const DecodeAttnArgs a) {
     __shared__ DecodeAttnSmem sm;
-    extern __shared__ __align__(16) float cluster_part[];   // CLUSTER: the first block's copy receives every warp's partial result
+    extern __shared__ __align__(16) float cluster_part[];   // merges in a cluster: the partial results (see the body)
     GbPdlSync sync;
     attention_decode_mma_body<HD, BK, GbPdlSync, NW, CLUSTER, SINK>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, sm, sync, cluster_part);
 }
@@ -41,12 +41,13 @@ struct DecodeSinkTerms {
     float cap;
 };
 
-// The merge runs inside a thread-block cluster in the variant for large batches (16 keys per iteration: small
-// blocks, several per SM), when the splits of a (row, kv head) fit one cluster (at most 8 blocks) and their partial
-// results fit the first block's shared memory. Measured at 9/3 heads, context 4096: batch 32 24.8 -> 23.2 us,
-// batch 64 43.0 -> 41.0 us. The small-batch variants keep the merge through global memory: their blocks fill an SM
-// each, clusters of 6 then no longer all find room in one wave (batch 8: 12.5 -> 19.5 us), and at batch 1 the
-// cluster's barrier is no faster than the counter (11.2 -> 12.0 us).
+// The merge runs inside a thread-block cluster wherever the splits of a (row, kv head) are at most 8 (a portable cluster), their results
+// fit shared memory, and either the blocks are small (16 keys per iteration and four warps: several an SM) or all clusters find room at
+// once: a processing cluster of at least 16 SMs (there are eight) holds 16 blocks of eight warps, or 32 of four warps with 32 keys per
+// iteration. One split needs no partner at all. Through global memory (a store, a fence, the counter, a load, one after the
+// other) / in the cluster, us: 9/3 heads, one row, contexts 100 / 1,024 / 4,000 5.1 / 3.0, 5.4 / 3.2, 8.0 / 6.1; four rows of 1,024 6.0 /
+// 3.7; 32/32 heads, one row of 1,024 5.7 / 4.5. With every warp sending its own result to the first block: 24 rows of 15/5 heads, 1,500
+// keys 13.6, the block's warps added up first 12.2; 40 rows of 9/3, 600 keys 9.1 and 8.1; 64 rows of 32/32, 4,000 keys 347 and 345.
 constexpr int MMA_CLUSTER_SMEM_MAX = 96 * 1024;
 
 template <int HD, int BK, int NW, bool SINK = false>
@@ -68,7 +69,8 @@ static int launch_mma(const void* q, long long q_stride, void* out, long long ou
     a.late_release = 1;   // (135M decode step at batch 1: 0.646 -> 0.630 ms; no difference at batch 64)
     const int group = nh / nkv;
     const int cluster_bytes = decode_attn_cluster_floats<HD>(group, splits, NW) * (int)sizeof(float);
-    const bool in_cluster = BK == 16 && NW == 4 && splits <= 8 && cluster_bytes <= MMA_CLUSTER_SMEM_MAX && group * splits * NW <= MMA_MAX_MERGE;
+    const bool room = (BK == 16 && NW == 4) || splits == 1 || (long long)n * nkv <= 8 * ((NW == 8 ? 16 : 32) / splits);
+    const bool in_cluster = splits <= 8 && room && cluster_bytes <= MMA_CLUSTER_SMEM_MAX;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, nkv, n);
     cfg.blockDim = dim3(NW * 32);

@@ -112,17 +112,16 @@ struct __align__(16) DecodeAttnSmem {   // (a multiple of 16 bytes, so that arra
 
 // NW warps (NW * 32 threads) work on one virtual block: 4, or 8 where few blocks would otherwise leave the chip's
 // memory system idle (a small batch): each warp then has half as many blocks of keys to walk through.
-// Floats of shared memory that the merge inside a thread-block cluster needs in the cluster's first block: one
-// (output row, maximum, sum) per head of the group and per warp of every split.
+// Floats of shared memory that the merge inside a thread-block cluster needs in every block: one (output row, maximum, sum) per head of
+// the group and per warp of its own, then (in the first block) per split.
 template <int HD>
-__host__ __device__ constexpr int decode_attn_cluster_floats(int group, int splits, int warps) { return group * splits * warps * (HD + 2); }
+__host__ __device__ constexpr int decode_attn_cluster_floats(int group, int splits, int warps) { return group * (splits + warps) * (HD + 2); }
 
-// CLUSTER: the blocks of one (row, kv head), one per split, are one thread-block cluster (the caller launches them
-// so). Their warps then put their partial results straight into the shared memory of the cluster's first block
-// (`cluster_part`, decode_attn_cluster_floats<HD>() floats, the same offset in every block), meet at the cluster's
-// barrier, and the first block merges from its own shared memory: no trip through global memory, no counter, no
-// second pass over what other blocks wrote. Otherwise the partial results go through `part_acc` / `part_ml` and the
-// block that arrives last at `counters` merges them.
+// CLUSTER: the blocks of one (row, kv head), one per split, are one thread-block cluster (the caller launches them so; one block may
+// stand alone). A block adds up its warps' partial results in its own shared memory (`cluster_part`, decode_attn_cluster_floats<HD>()
+// floats, the same offset in every block) and puts one result into the first block's; they meet at the cluster's barrier, and the
+// first block merges the splits: no trip through global memory, no counter, no second pass over what other blocks wrote. Otherwise
+// the warps' partial results go through `part_acc` / `part_ml` and the block that arrives last at `counters` merges them.
 template <int HD, int BK, class Sync, int NW = 4, bool CLUSTER = false, bool SINK = false>
 __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& a, const int split, const int kvh, const int row,
                                                           DecodeAttnSmem& sm, Sync& sync, float* cluster_part = nullptr) {
@@ -393,14 +392,12 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
     if constexpr (CLUSTER) {
         namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
-        // [head of the group][sub-split][HD channels, maximum, sum] in the first block's shared memory
-        float* first = cluster.map_shared_rank(cluster_part, 0);
-        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        float* first = cluster.map_shared_rank(cluster_part, 0) + (size_t)NW * G * (HD + 2);       // [split][head][HD channels, maximum, sum]
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int hi = g + 8 * h;
             if (hi < G) {
-                float* pa = first + ((size_t)hi * S4 + sub) * (HD + 2);
+                float* pa = cluster_part + ((size_t)warp * G + hi) * (HD + 2);
                 if (t == 0) {
                     pa[HD] = m_run[h];
                     pa[HD + 1] = l_run[h];
@@ -412,36 +409,49 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
                 }
             }
         }
-        cluster.sync();                       // (release / acquire: the first block sees what the others stored)
-        if (cluster.block_rank() != 0) return;
-        // one warp per head turns the (maximum, sum) pairs into normalised weights; then every thread adds up its channel
-        for (int hi = warp; hi < G; hi += NW) {
-            const float* ph = cluster_part + (size_t)hi * S4 * (HD + 2);
-            float m = MMA_NEG_BIG;
-            for (int sidx = lane; sidx < S4; sidx += 32) m = fmaxf(m, ph[sidx * (HD + 2) + HD]);
-            const float sk = sink_logit(head0 + hi);
-            m = fmaxf(gb_warp_max(m), sk);
-            float l = 0.f;
-            for (int sidx = lane; sidx < S4; sidx += 32) {
-                const float w = __expf(ph[sidx * (HD + 2) + HD] - m);
-                weights[hi * S4 + sidx] = w;
-                l = fmaf(ph[sidx * (HD + 2) + HD + 1], w, l);
+        // a head's channel over `parts` results `step` floats apart: its sum, their maximum and their sum (the weights formed by every thread)
+        auto merge = [&](const float* pa, int parts, int step, int d, float top, float& m, float& l) {
+            m = top;
+            for (int i = 0; i < parts; ++i) m = fmaxf(m, pa[i * step + HD]);
+            float v = 0.f;
+            l = 0.f;
+#pragma unroll 8
+            for (int i = 0; i < parts; ++i) {
+                const float w = __expf(pa[i * step + HD] - m);
+                l = fmaf(pa[i * step + HD + 1], w, l);
+                v = fmaf(pa[i * step + d], w, v);
             }
-            l = gb_warp_sum(l) + (SINK ? __expf(sk - m) : 0.f);
-            const float inv = (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head0 + hi);
-            __syncwarp();
-            for (int sidx = lane; sidx < S4; sidx += 32) weights[hi * S4 + sidx] *= inv;
-        }
+            return v;
+        };
+        auto finish = [&](const float* pa, int parts, int i) {
+            const int hi = i / HD, d = i % HD;
+            const float sk = sink_logit(head0 + hi);
+            float m, l;
+            float v = merge(pa + (size_t)hi * (HD + 2), parts, G * (HD + 2), d, sk, m, l);
+            if constexpr (SINK) l += __expf(sk - m);
+            v *= (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head0 + hi);
+            orow[(head0 + hi) * HD + d] = __float2bfloat16_rn(SINK ? v * channel_gate(head0 + hi, d) : v);
+        };
         sync.group_barrier();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        if (splits == 1) {
+            for (int i = tid; i < G * HD; i += NTHREADS) finish(cluster_part, NW, i);
+            return;
+        }
         for (int i = tid; i < G * HD; i += NTHREADS) {
             const int hi = i / HD, d = i % HD;
-            const float* pa = cluster_part + (size_t)hi * S4 * (HD + 2) + d;
-            const float* w = weights + hi * S4;
-            float v = 0.f;
-#pragma unroll 8
-            for (int sidx = 0; sidx < S4; ++sidx) v = fmaf(pa[(size_t)sidx * (HD + 2)], w[sidx], v);
-            orow[(head0 + hi) * HD + d] = __float2bfloat16_rn(SINK ? v * channel_gate(head0 + hi, d) : v);
+            float m, l;
+            const float v = merge(cluster_part + (size_t)hi * (HD + 2), NW, G * (HD + 2), d, MMA_NEG_BIG, m, l);
+            float* to = first + ((size_t)split * G + hi) * (HD + 2);
+            to[d] = v;
+            if (d == 0) {
+                to[HD] = m;
+                to[HD + 1] = l;
+            }
         }
+        cluster.sync();                       // (release / acquire: the first block sees what the others stored)
+        if (cluster.block_rank() != 0) return;
+        for (int i = tid; i < G * HD; i += NTHREADS) finish(cluster_part + (size_t)NW * G * (HD + 2), splits, i);
         return;
     }
 #pragma unroll

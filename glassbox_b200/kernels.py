@@ -902,7 +902,12 @@ def decode_mma_plan(n: int, nkv: int, hd: int, max_context: int):
         # take the same time; in a 135M decode step: batch 1 0.73 -> 0.65 ms, batch 8 0.80 -> 0.78 ms)
         # (with more than 1,024 keys per block the longer loop of the 16-key variant costs more than the room gains:
         # 360M shapes at batch 8, three splits of 1,365 keys: 1.23 ms with 32 keys per iteration, 1.27 ms with 16)
-        splits = max(1, min(148 // pairs, 8, -(-max_context // 256)))
+        # Of the splits whose clusters find room at once (their merge stays on the chip: attention_decode_mma.cu) and those that fill
+        # one wave (theirs goes through global memory: 2 us more) whichever ends sooner, at 7.5 us a thousand keys of a block.
+        # 9/3 heads, context 1,024: 8 rows 5 splits / 6 through memory 3.9 / 5.9 us.
+        most = -(-max_context // 256)
+        wide, near = max(1, min(148 // pairs, 8, most)), max(1, min(16 // -(-pairs // 8), 8, most))
+        splits = near if 0.0075 * max_context / near <= 2.0 + 0.0075 * max_context / wide else wide
         return splits, (16 if max_context <= 1024 * splits else 0), 8
     return max(1, min(-(-148 // pairs), most)), 0, 4
 
