@@ -67,8 +67,6 @@ _SIGNATURES = {
     "gb_attention_decode_mma": [_P, _LL, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _LL, _F, _I, _I, _P, _P, _P,
                                 _P, _P],
     "gb_attention_decode_mma_supported": [_I, _I, _I],
-    "gb_stream_marker": [_P],
-    "gb_kv_prefetch": [_P, _P, _P, _I, _P, _P, _I, _I, _I, _LL, _LL, _I, _I, _P],
     "gb_attention_prefill": [_P, _LL, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P],
     "gb_attention_prefill_supported": [_I, _I, _I, _I],
     "gb_attention_prefill_f32": [_P, _LL, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P],
@@ -902,12 +900,12 @@ def decode_mma_plan(n: int, nkv: int, hd: int, max_context: int):
         # take the same time; in a 135M decode step: batch 1 0.73 -> 0.65 ms, batch 8 0.80 -> 0.78 ms)
         # (with more than 1,024 keys per block the longer loop of the 16-key variant costs more than the room gains:
         # 360M shapes at batch 8, three splits of 1,365 keys: 1.23 ms with 32 keys per iteration, 1.27 ms with 16)
-        # Of the splits whose clusters find room at once (their merge stays on the chip: attention_decode_mma.cu) and those that fill
-        # one wave (theirs goes through global memory: 2 us more) whichever ends sooner, at 7.5 us a thousand keys of a block.
-        # 9/3 heads, context 1,024: 8 rows 5 splits / 6 through memory 3.9 / 5.9 us.
+        # Splits whose clusters find room at once merge on the chip (attention_decode_mma.cu), those that fill one wave through global
+        # memory, 2 us more: the former as long as a block has at most 512 keys. 9/3 heads, context 1,024: 6 rows 5 splits 4.2 us (8 through
+        # memory 5.7), 8 rows 5 / 4.6 (6: 5.9), 12 rows 3 / 5.2 (4: 6.5).
         most = -(-max_context // 256)
         wide, near = max(1, min(148 // pairs, 8, most)), max(1, min(16 // -(-pairs // 8), 8, most))
-        splits = near if 0.0075 * max_context / near <= 2.0 + 0.0075 * max_context / wide else wide
+        splits = near if max_context <= 512 * near else wide
         return splits, (16 if max_context <= 1024 * splits else 0), 8
     return max(1, min(-(-148 // pairs), most)), 0, 4
 
@@ -1042,24 +1040,6 @@ def attention_prefill_f32(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tens
     _call("gb_attention_prefill_f32", _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(kcache), _ptr(vcache),
           _ptr(block_tables), block_tables.shape[1], _ptr(seq_first_row), _ptr(seq_start_pos), q.shape[0], S, int(max_rows_per_seq),
           nh, nkv, hd, page_size, kcache.shape[0], float(scale), int(window or 0), _ptr(status), _stream())
-
-
-def kv_prefetch(kcache: torch.Tensor, vcache: torch.Tensor, block_tables: torch.Tensor, row_seq: torch.Tensor,
-                positions: torch.Tensor, nkv: int, hd: int, page_size: int, window: Optional[int],
-                blocks_per_row: int) -> None:
-    """Ask the memory system to bring the pages that each row's attention will read into L2."""
-    _cuda(kcache, vcache, block_tables, row_seq, positions)
-    tile_bytes = page_size * hd * kcache.element_size()
-    if tile_bytes % 128:
-        return
-    _call("gb_kv_prefetch", _ptr(kcache), _ptr(vcache), _ptr(block_tables), block_tables.shape[1], _ptr(row_seq),
-          _ptr(positions), positions.shape[0], nkv, page_size, kcache.shape[0], tile_bytes, int(window or 0),
-          int(blocks_per_row), _stream())
-
-
-def stream_marker() -> None:
-    """An empty kernel on the current stream: a node of its own in a recorded step (see ``GqaAttention.prefetch``)."""
-    _call("gb_stream_marker", _stream())
 
 
 def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.Tensor] = None,
