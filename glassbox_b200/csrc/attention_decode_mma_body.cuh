@@ -483,9 +483,49 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
     sync.group_barrier();
     if (!is_last) return;
     __threadfence();
-    // Merge: one warp per head turns the (maximum, sum) pairs of all sub-splits into normalised
-    // weights in shared memory; then every thread adds up its channel over the sub-splits with
-    // independent loads.
+    // Merge, in the order of the cluster's (a split's warps first, then the splits), so that both give the same bits: one warp per head
+    // turns the (maximum, sum) pairs into each warp's weight within its split (`weights`), each split's weight (`tops`, over the page ids,
+    // which nothing reads any more) and the head's scale; then every thread adds up its channel with independent loads.
+    float2* tops = reinterpret_cast<float2*>(sm.pages);      // [head of the pass][split]: weight, sum (of split 0: the head's scale, once known)
+    static_assert(sizeof(sm.pages) >= 2 * sizeof(float) * (MMA_MAX_MERGE / NW), "a pass's splits must fit the page ids' place");
+    auto weigh = [&](int hi, int head) {
+        const float2* ml = reinterpret_cast<const float2*>(part_ml + ((size_t)row * nh + head) * S4 * 2);
+        const float sk = sink_logit(head);
+        float m = sk, l = 0.f;
+        for (int sp = lane; sp < splits; sp += 32) {
+            float2 p[NW];
+            float ms = MMA_NEG_BIG, ls = 0.f;
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                p[i] = __ldcg(ml + sp * NW + i);
+                ms = fmaxf(ms, p[i].x);
+            }
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                const float w = __expf(p[i].x - ms);
+                weights[hi * S4 + sp * NW + i] = w;
+                ls = fmaf(p[i].y, w, ls);
+            }
+            tops[hi * splits + sp] = make_float2(ms, ls);
+            m = fmaxf(m, ms);
+        }
+        m = gb_warp_max(m);
+        for (int sp = lane; sp < splits; sp += 32) {
+            float2& top = tops[hi * splits + sp];
+            top.x = __expf(top.x - m);
+            l = fmaf(top.y, top.x, l);
+        }
+        __syncwarp();
+        if (splits <= 8) {
+            l = 0.f;
+            for (int sp = 0; sp < splits; ++sp) l = fmaf(tops[hi * splits + sp].y, tops[hi * splits + sp].x, l);
+        } else {                                             // (more than a cluster holds: any order)
+            l = gb_warp_sum(l);
+        }
+        if constexpr (SINK) l += __expf(sk - m);
+        __syncwarp();
+        if (lane == 0) tops[hi * splits].y = (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head);
+    };
     if (G * HD <= NTHREADS && S4 <= 64) {
         // The usual case (every output channel of the group has a thread of its own, at most 64 partial results per
         // head): a thread asks for its channel of every partial result at once, before the weights exist, and a lane
@@ -499,25 +539,20 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
 #pragma unroll
             for (int sidx = 0; sidx < MAXP; ++sidx) pv[sidx] = sidx < S4 ? __ldcg(pa + (size_t)sidx * HD) : 0.f;
         }
-        for (int hi = warp; hi < G; hi += NW) {
-            const float2* ml = reinterpret_cast<const float2*>(part_ml + ((size_t)row * nh + head0 + hi) * S4 * 2);
-            const float2 p0 = lane < S4 ? __ldcg(ml + lane) : make_float2(MMA_NEG_BIG, 0.f);
-            const float2 p1 = lane + 32 < S4 ? __ldcg(ml + lane + 32) : make_float2(MMA_NEG_BIG, 0.f);
-            const float sk = sink_logit(head0 + hi);
-            const float m = fmaxf(gb_warp_max(fmaxf(p0.x, p1.x)), sk);
-            const float w0 = __expf(p0.x - m), w1 = __expf(p1.x - m);
-            const float l = gb_warp_sum(fmaf(p0.y, w0, p1.y * w1)) + (SINK ? __expf(sk - m) : 0.f);
-            const float inv = (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head0 + hi);
-            if (lane < S4) weights[hi * S4 + lane] = w0 * inv;
-            if (lane + 32 < S4) weights[hi * S4 + lane + 32] = w1 * inv;
-        }
+        for (int hi = warp; hi < G; hi += NW) weigh(hi, head0 + hi);
         sync.group_barrier();
         if (tid < G * HD) {
             const float* w = weights + hi_o * S4;
             float v = 0.f;
 #pragma unroll
-            for (int sidx = 0; sidx < MAXP; ++sidx)
-                if (sidx < S4) v = fmaf(pv[sidx], w[sidx], v);
+            for (int sp = 0; sp < MAXP / NW; ++sp)
+                if (sp < splits) {
+                    float part = 0.f;
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) part = fmaf(pv[sp * NW + i], w[sp * NW + i], part);
+                    v = fmaf(part, tops[hi_o * splits + sp].x, v);
+                }
+            v *= tops[hi_o * splits].y;
             orow[(head0 + hi_o) * HD + d_o] = __float2bfloat16_rn(SINK ? v * gch : v);
         }
         return;
@@ -525,34 +560,23 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
     const int per_pass = MMA_MAX_MERGE / S4;                 // heads whose weights fit at once
     for (int h0 = 0; h0 < G; h0 += per_pass) {
         const int hcount = min(per_pass, G - h0);
-        for (int hi = warp; hi < hcount; hi += NW) {
-            const float* ml = part_ml + ((size_t)row * nh + head0 + h0 + hi) * S4 * 2;
-            float m = MMA_NEG_BIG;
-            for (int sidx = lane; sidx < S4; sidx += 32) m = fmaxf(m, __ldcg(ml + 2 * sidx));
-            const float sk = sink_logit(head0 + h0 + hi);
-            m = fmaxf(gb_warp_max(m), sk);
-            float l = 0.f;
-            for (int sidx = lane; sidx < S4; sidx += 32) {
-                const float w = __expf(__ldcg(ml + 2 * sidx) - m);
-                weights[hi * S4 + sidx] = w;
-                l = fmaf(__ldcg(ml + 2 * sidx + 1), w, l);
-            }
-            l = gb_warp_sum(l) + (SINK ? __expf(sk - m) : 0.f);
-            const float inv = (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head0 + h0 + hi);
-            __syncwarp();
-            for (int sidx = lane; sidx < S4; sidx += 32) weights[hi * S4 + sidx] *= inv;
-        }
+        for (int hi = warp; hi < hcount; hi += NW) weigh(hi, head0 + h0 + hi);
         sync.group_barrier();
         for (int i = tid; i < hcount * HD; i += NTHREADS) {
             const int hi = i / HD, d = i % HD;
             const float* pa = part_acc + ((size_t)row * nh + head0 + h0 + hi) * S4 * HD + d;
             const float* w = weights + hi * S4;
             float v = 0.f;
-#pragma unroll 8
-            for (int sidx = 0; sidx < S4; ++sidx) v = fmaf(__ldcg(pa + (size_t)sidx * HD), w[sidx], v);
+#pragma unroll 2
+            for (int sp = 0; sp < splits; ++sp) {
+                float part = 0.f;
+#pragma unroll
+                for (int k = 0; k < NW; ++k) part = fmaf(__ldcg(pa + (size_t)(sp * NW + k) * HD), w[sp * NW + k], part);
+                v = fmaf(part, tops[hi * splits + sp].x, v);
+            }
+            v *= tops[hi * splits].y;
             orow[(head0 + h0 + hi) * HD + d] = __float2bfloat16_rn(SINK ? v * channel_gate(head0 + h0 + hi, d) : v);
         }
         sync.group_barrier();
     }
 }
-
