@@ -15,6 +15,7 @@
 // kernel leaves it zero again).
 #include "common.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_pipeline.h>
 
 // Keys per tile (DK) is 64, 32 or 16, chosen so that the tiles fit in shared memory whatever the
@@ -355,13 +356,19 @@ static int launch_decode(const void* q, long long q_stride, void* out, long long
 // memory. A warp takes 16 loads of 16 bytes a lane of keys and as many of values at once (HD 64: 32 keys, two a load; HD 128:
 // 16 keys), all requested before the first product, so a block's 256 (128) keys cost one latency; the partial dot products of a
 // key's lanes come together by a transposing reduction (15 shuffles for 16 keys and head), which leaves each lane the score of
-// one key. Scores, exponentials (expf), sums and the merge are float32 as above. What bounds it is that latency: page table, keys,
-// block merge, split merge. The tiles above take the keys 64 at a time through shared memory, four barriers a tile, and the
-// split rule's 592 blocks of 64 KB are two waves. Measured, 8 rows of 9 / 3 heads, contexts to 2,041: 34.4 -> 14.2 us.
+// one key. Scores, exponentials (expf), sums and the merge are float32 as above. What bounds it is that latency: keys, block
+// merge, split merge (positions and page table are read while the kernel before still runs). The tiles above take the keys 64 at a
+// time through shared memory, four barriers a tile, and the split rule's 592 blocks of 64 KB are two waves.
+// The grid has no more blocks than a row can have rounds of keys (a block fills an SM's registers, and the split rule alone asked
+// for three times as many, which came and went in between), and the splits come together in a cluster where all clusters find
+// room at once. Measured, us, tiles / splits by the rule alone, merged through global memory / this: 8 rows of 9/3 heads, contexts to
+// 2,041 34.4 / 15.6 / 9.9; one row of 1,024 - / 8.3 / 4.8; of 8,000 - / 13.3 / 11.4; 64 rows of 1,500 - / 64.9 / 60.9.
 // ----------------------------------------------------------------------------------------------
 constexpr int DF_WARPS = 8;
+constexpr int DF_CLUSTER = 8;    // splits whose results come together in a cluster's shared memory (a portable cluster)
+constexpr int DF_AT_ONCE = 16;   // splits' results that a thread of the merge asks for at once
 
-template <int HD, int GT>
+template <int HD, int GT, bool CLUSTER>
 __global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
     const float* __restrict__ q, long long q_stride, float* __restrict__ out, long long out_stride,
     const float* __restrict__ kcache, const float* __restrict__ vcache, const int* __restrict__ block_tables, int max_pages,
@@ -370,33 +377,54 @@ __global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
     float* __restrict__ part_ml, int* __restrict__ counters, int* __restrict__ status) {
     constexpr int LPK = HD / 4, KPS = 32 / LPK, STEPS = 16, CK = STEPS * KPS;   // lanes a key, keys a load, loads, keys a chunk
     __shared__ float wacc[DF_WARPS][GT][HD], wm[DF_WARPS][GT], wl[DF_WARPS][GT];
+    __shared__ float parts[CLUSTER ? DF_CLUSTER : 1][GT][HD + 2];     // CLUSTER, the first block's: each split's channels, maximum and sum
     __shared__ int is_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int split = blockIdx.x, row = blockIdx.z;
     const int G = nh / nkv, subgroups = (G + GT - 1) / GT;
     const int kvh = blockIdx.y / subgroups, sg = blockIdx.y % subgroups;
     const int head0 = kvh * G + sg * GT, gcount = min(GT, G - sg * GT);
-    gb_pdl_launch_dependents();
-    gb_pdl_wait();
+    // The positions and the block table are the step's and written by no kernel of it: read before the wait, so that only
+    // the queries, keys and values are left to ask for after it.
     int pos = positions[row];
-    if (pos >= 0 && pos / page_size >= max_pages) {   // a position the block table does not reach: reported, and the
-        if (tid == 0) atomicOr(status, GB_STATUS_BAD_POSITION);   // row is treated as padding (nothing is read)
-        pos = -1;
-    }
+    const int* table = block_tables + (size_t)row_seq[row] * max_pages;
+    const bool out_of_table = pos >= 0 && pos / page_size >= max_pages;   // a position the block table does not reach: reported, and
+    if (out_of_table) pos = -1;                                           // the row is treated as padding (nothing is read)
     float* orow = out + (size_t)row * out_stride;
     if (pos < 0) {  // padding row
+        gb_pdl_wait();
+        gb_pdl_launch_dependents();
+        if (out_of_table && tid == 0) atomicOr(status, GB_STATUS_BAD_POSITION);
         if (split == 0)
             for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) orow[head0 * HD + i] = 0.f;
         return;
     }
-    const int* table = block_tables + (size_t)row_seq[row] * max_pages;
     const int first = (window > 0 && pos + 1 > window) ? pos + 1 - window : 0;
     const int total = pos + 1 - first;
     // a split is whole rounds of the block's warps; the splits that get keys take part in the merge, the others leave
     const int round = DF_WARPS * CK, chunk = ((total + splits - 1) / splits + round - 1) / round * round;
     const int active = (total + chunk - 1) / chunk;
-    if (split >= active) return;
+    if constexpr (CLUSTER) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its shared memory exists
+    if (split >= active) {
+        if constexpr (CLUSTER) {
+            asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+        return;
+    }
     const int k_begin = first + split * chunk, k_end = min(pos + 1, k_begin + chunk);
+    // after the reduction lane l has key KPS * (l % 16) + (l / 16 at HD 64) of the chunk; (HD 128: both halves the same key)
+    const int mine = KPS == 2 ? 2 * (lane & 15) + (lane >> 4) : (lane & 15);
+    const bool counted = KPS == 2 || lane < 16;
+    auto offset = [&](int key) -> long long {       // of this lane's key in the cache, in elements; -1: no key, -2: a page that is none
+        if (key >= k_end) return -1;
+        const long long page = table[key / page_size];
+        return page < 0 || page >= num_pages ? -2 : ((page * nkv + kvh) * page_size + key % page_size) * HD;
+    };
+    long long off = offset(k_begin + warp * CK + mine);
+    gb_pdl_wait();
+    gb_pdl_launch_dependents();
 
     float4 qv[GT];
 #pragma unroll
@@ -411,17 +439,9 @@ __global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
         l_run[g] = 0.f;
         acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    // after the reduction lane l has key KPS * (l % 16) + (l / 16 at HD 64) of the chunk; (HD 128: both halves the same key)
-    const int mine = KPS == 2 ? 2 * (lane & 15) + (lane >> 4) : (lane & 15);
-    const bool counted = KPS == 2 || lane < 16;
     for (int base = k_begin + warp * CK; base < k_end; base += round) {
-        const int key = base + mine;
-        long long off = -1;
-        if (key < k_end) {
-            const long long page = table[key / page_size];
-            if (page < 0 || page >= num_pages) atomicOr(status, GB_STATUS_BAD_SLOT);
-            else off = ((page * nkv + kvh) * page_size + key % page_size) * HD;
-        }
+        if (base != k_begin + warp * CK) off = offset(base + mine);
+        if (off == -2) atomicOr(status, GB_STATUS_BAD_SLOT);
         float4 kr[STEPS], vr[STEPS];
 #pragma unroll
         for (int i = 0; i < STEPS; ++i) {
@@ -484,6 +504,7 @@ __global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
         }
     }
     __syncthreads();
+    if constexpr (CLUSTER) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) {
         const int g = i / HD, d = i % HD;
         float m = wm[0][g], l = 0.f, v = 0.f;
@@ -497,41 +518,78 @@ __global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
         }
         if (active == 1) {
             orow[(head0 + g) * HD + d] = l > 0.f ? v / l : 0.f;
+        } else if constexpr (CLUSTER) {
+            float* to = cooperative_groups::this_cluster().map_shared_rank(&parts[split][g][0], 0);
+            to[d] = v;
+            if (d == 0) {
+                to[HD] = m;
+                to[HD + 1] = l;
+            }
         } else {
             part_acc[(((size_t)row * nh + head0 + g) * splits + split) * HD + d] = v;
-            if (d == 0) {
-                float* ml = part_ml + (((size_t)row * nh + head0 + g) * splits + split) * 2;
-                ml[0] = m;
-                ml[1] = l;
-            }
+            if (d == 0) *reinterpret_cast<float2*>(part_ml + (((size_t)row * nh + head0 + g) * splits + split) * 2) = make_float2(m, l);
         }
+    }
+    if constexpr (CLUSTER) {
+        cooperative_groups::this_cluster().sync();       // (release / acquire: the first block sees what the others stored)
+        if (active == 1 || split != 0) return;
+        for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) {
+            const int g = i / HD, d = i % HD;
+            float m = NEG_BIG, l = 0.f, v = 0.f;
+            for (int sidx = 0; sidx < active; ++sidx) m = fmaxf(m, parts[sidx][g][HD]);
+            for (int sidx = 0; sidx < active; ++sidx) {
+                const float w = expf(parts[sidx][g][HD] - m);
+                l = fmaf(parts[sidx][g][HD + 1], w, l);
+                v = fmaf(parts[sidx][g][d], w, v);
+            }
+            orow[(head0 + g) * HD + d] = l > 0.f ? v / l : 0.f;
+        }
+        return;
     }
     if (active == 1) return;
     // the block that arrives last merges the splits
-    __threadfence();
     __syncthreads();
     if (tid == 0) {
         int* counter = counters + (size_t)row * gridDim.y + blockIdx.y;
+        __threadfence();              // (after the barrier: the block's stores above come before the count)
         const int prev = atomicAdd(counter, 1);
         is_last = (prev == active - 1);
         if (is_last) *counter = 0;  // ready for the next launch
+        __threadfence();
     }
     __syncthreads();
     if (!is_last) return;
-    __threadfence();
     for (int i = tid; i < gcount * HD; i += DF_WARPS * 32) {
         const int g = i / HD, d = i % HD;
-        const float* ml = part_ml + ((size_t)row * nh + head0 + g) * splits * 2;
-        const float* pa = part_acc + ((size_t)row * nh + head0 + g) * splits * HD;
-        float m = NEG_BIG;
+        const float2* ml = reinterpret_cast<const float2*>(part_ml + ((size_t)row * nh + head0 + g) * splits * 2);
+        const float* pa = part_acc + ((size_t)row * nh + head0 + g) * splits * HD + d;
+        float m = NEG_BIG, l = 0.f, v = 0.f;
+        if (active <= DF_AT_ONCE) {   // all asked for before the first is used: one trip to L2
+            float2 mls[DF_AT_ONCE];
+            float pv[DF_AT_ONCE];
+#pragma unroll
+            for (int sidx = 0; sidx < DF_AT_ONCE; ++sidx) {
+                mls[sidx] = sidx < active ? __ldcg(ml + sidx) : make_float2(NEG_BIG, 0.f);
+                pv[sidx] = sidx < active ? __ldcg(pa + (size_t)sidx * HD) : 0.f;
+                m = fmaxf(m, mls[sidx].x);
+            }
+#pragma unroll
+            for (int sidx = 0; sidx < DF_AT_ONCE; ++sidx)
+                if (sidx < active) {
+                    const float w = expf(mls[sidx].x - m);
+                    l = fmaf(mls[sidx].y, w, l);
+                    v = fmaf(pv[sidx], w, v);
+                }
+        } else {
 #pragma unroll 8
-        for (int sidx = 0; sidx < active; ++sidx) m = fmaxf(m, __ldcg(ml + 2 * sidx));
-        float l = 0.f, v = 0.f;
+            for (int sidx = 0; sidx < active; ++sidx) m = fmaxf(m, __ldcg(ml + sidx).x);
 #pragma unroll 8
-        for (int sidx = 0; sidx < active; ++sidx) {
-            const float w = expf(__ldcg(ml + 2 * sidx) - m);
-            l = fmaf(__ldcg(ml + 2 * sidx + 1), w, l);
-            v = fmaf(__ldcg(pa + (size_t)sidx * HD + d), w, v);
+            for (int sidx = 0; sidx < active; ++sidx) {
+                const float2 p = __ldcg(ml + sidx);
+                const float w = expf(p.x - m);
+                l = fmaf(p.y, w, l);
+                v = fmaf(__ldcg(pa + (size_t)sidx * HD), w, v);
+            }
         }
         orow[(head0 + g) * HD + d] = l > 0.f ? v / l : 0.f;
     }
@@ -543,9 +601,40 @@ static int launch_decode_f32(const float* q, long long q_stride, float* out, lon
                              int page_size, long long num_pages, float scale, int window, int splits, float* part_acc,
                              float* part_ml, int* counters, int* status, cudaStream_t stream) {
     const int subgroups = (nh / nkv + GT - 1) / GT;
-    gb_launch(GB_PDL_ATTENTION, attention_decode_f32_kernel<HD, GT>, dim3(splits, nkv * subgroups, n), dim3(DF_WARPS * 32), 0, stream, q,
-              q_stride, out, out_stride, kcache, vcache, block_tables, max_pages, row_seq, positions, nh, nkv, page_size, num_pages, scale,
-              window, splits, part_acc, part_ml, counters, status);
+    // no more blocks than rounds of keys that a row can see: one that gets no keys still takes an SM's registers until it has read its
+    // row's position
+    constexpr int round = DF_WARPS * 16 * (32 / (HD / 4));
+    const long long most = window > 0 && window < (long long)max_pages * page_size ? window : (long long)max_pages * page_size;
+    const int blocks = (int)((most + round - 1) / round < splits ? (most + round - 1) / round : splits);
+    // one block an SM: a processing cluster of at least 16 SMs (there are eight) holds 16 / blocks clusters
+    const bool in_cluster = blocks <= DF_CLUSTER && (blocks == 1 || (long long)n * nkv * subgroups <= 8 * (16 / blocks));
+    const dim3 grid(blocks, nkv * subgroups, n);
+    cudaError_t e;
+    if (in_cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(DF_WARPS * 32);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = (gb_pdl_enabled() & GB_PDL_ATTENTION) ? 2 : 1;
+        e = cudaLaunchKernelEx(&cfg, attention_decode_f32_kernel<HD, GT, true>, q, q_stride, out, out_stride, kcache, vcache, block_tables,
+                               max_pages, row_seq, positions, nh, nkv, page_size, num_pages, scale, window, splits, part_acc, part_ml,
+                               counters, status);
+    } else {
+        e = gb_launch(GB_PDL_ATTENTION, attention_decode_f32_kernel<HD, GT, false>, grid, dim3(DF_WARPS * 32), 0, stream, q, q_stride, out,
+                      out_stride, kcache, vcache, block_tables, max_pages, row_seq, positions, nh, nkv, page_size, num_pages, scale, window,
+                      splits, part_acc, part_ml, counters, status);
+    }
+    if (e != cudaSuccess) {
+        gb_set_error("gb_attention_decode: launch failed: %s", cudaGetErrorString(e));
+        return 2;
+    }
     return gb_check_launch("gb_attention_decode");
 }
 
