@@ -25,12 +25,16 @@
 constexpr int GF_BM = 128, GF_BK = 128, GF_ROWS = 64, GF_STAGES = 4, GF_THREADS = 192;
 constexpr int GF_W_BYTES = GF_BM * GF_BK * 2, GF_X_BYTES = GF_ROWS * GF_BK * 2, GF_STAGE = GF_W_BYTES + GF_X_BYTES;
 constexpr int GF_PITCH = GF_BM + 4;                      // floats from row to row of the partial sums
+// k-blocks of a block's slice that are asked for into L2 before the wait: a slice of up to GF_WHOLE whole, of a longer one two past the ring
+constexpr int GF_WHOLE = 12, GF_AHEAD = GF_STAGES + 2;
 constexpr int GF_SMEM = GF_STAGES * GF_STAGE + 1024;
 static_assert(GF_ROWS * GF_PITCH * 4 <= GF_STAGES * GF_STAGE, "the partial sums fit where the stages were");
 
 enum { GF_STORE_BF16 = 0, GF_STORE_F32 = 1, GF_ADD_F32 = 2, GF_GLU_BF16 = 3, GF_ROPE_QKV = 4, GF_RELU2_BF16 = 5, GF_GELU_BF16 = 7 };
 
 struct GfArgs {
+    const __nv_bfloat16* w;       // the matrix that map_w describes, its rows ldw numbers apart (read only to ask for it early)
+    long long w_rows, ldw;
     void* C;
     long long ldc;
     int mode, M, N, K, split, slice;      // slice: 128-wide k-blocks of a block
@@ -159,6 +163,14 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_few_kernel(const __grid_const
             sh.consumed = consumed;
         }
     } else {
+        // A row of the tile a thread: weights beyond the first stages' are asked for into L2 now, a row's part in one piece (the boxes take
+        // 256 bytes of each of 128 rows at a time). Weights from memory, 40 rows, us: 2048 x 8192 (slices of 10) 9.9 -> 9.0, 6144 x 2048 8.9 ->
+        // 8.4; a long slice whole runs ahead of the ring's own requests: 2 x 8192 x 2048 gated (16) 16.9 -> 18.2, two past the ring 16.7.
+        const int r = (warp - 2) * 32 + lane, begin = (kb0 + GF_STAGES) * GF_BK, end = min(a.K, (kb0 + (kblocks <= GF_WHOLE ? kblocks : GF_AHEAD)) * GF_BK);
+        const long long row = gated && r >= 64 ? a.gate_rows + n0 + r - 64 : n0 + r, rows = gated && r < 64 ? a.gate_rows : a.w_rows;
+        const int bytes = (end - begin) * 2 / 16 * 16;
+        if (row < rows && bytes > 0)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.w + row * a.ldw + begin), "r"(bytes) : "memory");
         gb_pdl_wait();
         const int q = warp & 3;                                   // the quarter of the tensor-memory lanes (outputs) of this warp
         if (mbar_wait_warp(&sh.tfull, 0, abort_flag, a.status)) {
@@ -303,6 +315,9 @@ static int gf_launch(GfArgs a, const void* x, long long ldx, const void* w, long
     a.slice = gb_ceil_div(kb, a.split);
     a.split = gb_ceil_div(kb, a.slice);                          // (no block without work)
     a.x_rows = (a.M + 15) / 16 * 16;
+    a.w = (const __nv_bfloat16*)w;
+    a.w_rows = w_rows;
+    a.ldw = ldw;
     CUtensorMap mw, mx;
     if (tc_make_map_2d(&mw, w, w_rows, a.K, ldw, a.mode == GF_GLU_BF16 ? 64 : GF_BM, 64, "gb_gemm_few")) return 1;
     if (tc_make_map_2d(&mx, x, a.M, a.K, ldx, a.x_rows, 64, "gb_gemm_few")) return 1;
