@@ -362,7 +362,7 @@ static int launch_decode(const void* q, long long q_stride, void* out, long long
 // The grid has no more blocks than a row can have rounds of keys (a block fills an SM's registers, and the split rule alone asked
 // for three times as many, which came and went in between), and the splits come together in a cluster where all clusters find
 // room at once. Measured, us, tiles / splits by the rule alone, merged through global memory / this: 8 rows of 9/3 heads, contexts to
-// 2,041 34.4 / 15.6 / 9.9; one row of 1,024 - / 8.3 / 4.8; of 8,000 - / 13.3 / 11.4; 64 rows of 1,500 - / 64.9 / 60.9.
+// 2,041 34.4 / 15.6 / 9.9 (8.4 with what is asked for into L2); one row of 1,024 - / 8.3 / 4.8; of 8,000 - / 13.3 / 11.4; 64 rows of 1,500 - / 64.9 / 60.9.
 // ----------------------------------------------------------------------------------------------
 constexpr int DF_WARPS = 8;
 constexpr int DF_CLUSTER = 8;    // splits whose results come together in a cluster's shared memory (a portable cluster)
@@ -423,6 +423,17 @@ __global__ void __launch_bounds__(DF_WARPS * 32) attention_decode_f32_kernel(
         return page < 0 || page >= num_pages ? -2 : ((page * nkv + kvh) * page_size + key % page_size) * HD;
     };
     long long off = offset(k_begin + warp * CK + mine);
+    // Where blocks fill the chip their keys and values are asked for into L2 at once, whole rows: two instructions a lane for each, where
+    // the loads below, 32 a warp, take 4,000 to 12,000 cycles to go out. (What the kernel before writes of them is read after the wait.) With
+    // blocks for a part of the chip (4 rows of 600 5.8 -> 6.2), and at 128 channels, where a load has whole rows, it gains nothing. Us: 8 rows of 9/3
+    // heads, contexts to 2,041 9.9 -> 8.4, 64 rows of 1,500 60.9 -> 56.3, of 200 15.2 -> 12.8, 8 rows of 32/32
+    // heads to 2,041 46.9 -> 41.5.
+    if (HD == 64 && off >= 0 && gridDim.x * gridDim.y * gridDim.z > 148) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(kcache + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(vcache + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(kcache + off + 32));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(vcache + off + 32));
+    }
     gb_pdl_wait();
     gb_pdl_launch_dependents();
 

@@ -262,7 +262,7 @@ __global__ void rope_kv_write_kernel(T* __restrict__ qkv, const float2* __restri
 // The same four channels of a head at a time: a thread has one unit of a row (four pairs of a query or key head, four channels that
 // are not rotated, four of a value), asks for all of it at once and stores it in 16-byte (bfloat16: 8-byte) pieces, where the form
 // above has a chain of up to five loads and stores of single numbers. What a row's place is comes from memory while the product
-// before still runs; the kernel after starts when this one has ended (see above). Bound by its few trips to memory where
+// before still runs; a bfloat16 kernel after starts when this one has ended (see above). Bound by its few trips to memory where
 // rows are few and by the bytes where many. Us, float32 rows of 9/3 heads of 64 channels, 8 / 2,047 / 6,141 rows: 3.2 -> 1.7, 5.6 -> 4.1,
 // 16.8 -> 12.5; bfloat16 3.3 -> 1.9, 5.8 -> 4.1, 13.8 -> 8.9.
 template <typename T> struct Four;
@@ -299,6 +299,7 @@ __global__ void rope_kv_write4_kernel(T* __restrict__ qkv, const float2* __restr
     const int pairs = half / 4, plain = (hd - rot) / 4, per_k = pairs + plain;    // units of a head
     const int nq = rotate ? nh * pairs : 0, nk = nkv * per_k, nv = store ? kvd / 4 : 0;
     gb_pdl_wait();
+    if (sizeof(T) == 4) gb_pdl_launch_dependents();     // (the float32 attention's blocks read their places and ask for their keys meanwhile)
     if (pos < 0) return;   // a padding row of a fixed-shape batch: nothing to rotate, nothing to store
     if (threadIdx.x == 0 && (bad_pos || bad_slot)) atomicOr(status, (bad_pos ? GB_STATUS_BAD_POSITION : 0) | (bad_slot ? GB_STATUS_BAD_SLOT : 0));
     for (int u = threadIdx.x; u < nq + nk + nv; u += blockDim.x) {
