@@ -57,7 +57,7 @@ struct __align__(8) AtShared {
     uint64_t p_ready[2];             // softmax -> MMA: P_j is in TMEM buffer j & 1 (and O is rescaled)
     uint64_t pv_done[2];             // MMA -> softmax: O += P_j V_j is complete (P buffer j & 1 is free, O is current)
     uint64_t x_ready;                // softmax <-> softmax: both groups have posted their final maximum and sum (a phase per item)
-    uint64_t merged;                 // softmax <-> softmax: the first item's accumulators have been read (one phase)
+    uint64_t merged;                 // softmax <-> softmax: the first item's accumulators and row statistics have been read (one phase)
     uint64_t peer_done;              // PAIR, the other block's softmax -> softmax: its share of this block's tile has arrived (one phase)
     float row_stat[2][2][AT_BM];     // [group][maximum, sum][row]
     uint32_t tmem_base;
@@ -539,7 +539,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
             if (PAIR && item == 1 && j == j_first && !mbar_wait_warp(&sh.merged, 0, abort_flag, status)) { ok = false; break; }
             if (lane == 0) mbar_arrive(&sh.p_ready[g]);
         }
-        // merge: the groups post their maximum and sum per row, then each writes half of the channels
+        // merge: the groups post their maximum and sum per row, then each writes half of the channels. The second item's statistics take
+        // the place of the first's: all warps have read those when `merged` completes. (A group without a key tile in the second
+        // item, which is so of every fresh prompt's first row tile, has not waited for it above.)
+        if (PAIR && item == 1 && ok) ok = mbar_wait_warp(&sh.merged, 0, abort_flag, status);
         if (ok) {
             sh.row_stat[g][0][r] = m_run;
             sh.row_stat[g][1][r] = l_run;

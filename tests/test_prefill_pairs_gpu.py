@@ -36,3 +36,21 @@ def test_pairs_of_row_tiles(nh, nkv, rows, past, window, page):
         want = torch.softmax(s, -1) @ values[:, h // (nh // nkv)]
         # weights in bfloat16 (2^-9 each, of either sign) and one rounding of the result: 2^-8 of values of a few
         assert (out[:, h * 64:h * 64 + 64].double() - want).abs().max() < 2.0 ** -8 * 4, h
+
+
+@pytest.mark.parametrize("nh, nkv, rows, past", [(9, 3, 1153, 0), (9, 3, 2048, 0), (4, 2, 1500, 0), (2, 1, 1290, 40)])
+def test_second_items_of_one_key_tile_repeat_their_bits(nh, nkv, rows, past):
+    """The first row tile of a fresh prompt sees one key tile: one softmax group has none there and must not post that item's row
+    statistics before the other group has read the first item's. What orders them is `merged` in the kernel; a late reader would
+    lose half of a share, so every launch has to give the same bits."""
+    from glassbox_b200 import kernels
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device=DEV).bfloat16()
+    pages = -(-(rows + past) // 16)
+    k, v, q = rand(pages, nkv, 16, 64), rand(pages, nkv, 16, 64), rand(rows, nh * 64)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    table, first, start, status = i32([list(range(pages))]), i32([0, rows]), i32([past]), i32([0])
+    outs = [torch.empty_like(q) for _ in range(50)]
+    for out in outs:
+        kernels.attention_prefill_tc(q, out, k, v, table, first, start, rows, nh, nkv, 64, 16, 0.125, 0, status)
+    assert int(status) == 0 and all(torch.equal(out, outs[0]) for out in outs)
