@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(TDM_THREADS, 2) talking_decode_mma_kernel(
                 for (int h = 0; h < NH; ++h)
 #pragma unroll
                     for (int i = 0; i < KL; ++i) {
-                        const float y = s[h][i] * inv_cap;
-                        most = y == -INFINITY ? most : !(fabsf(y) < 0.6f) ? 1.f : most;
+                        const float y = s[h][i] * inv_cap;                  // (a key is masked by `seen`: the score of one that is may be -infinity too)
+                        most = seen[i] && !(fabsf(y) < 0.6f) ? 1.f : most;
                     }
                 const bool small = !__any_sync(0xffffffffu, most > 0.f);
 #pragma unroll
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(TDM_THREADS, 2) talking_decode_mma_kernel(
 #pragma unroll
                     for (int i = 0; i < KL; ++i) {
                         const float y = s[h][i] * inv_cap;
-                        if (y != -INFINITY) s[h][i] = cap * (small ? tdm_tanh_small(y) : tanhf(y));
+                        if (seen[i]) s[h][i] = cap * (small ? tdm_tanh_small(y) : tanhf(y));
                     }
             }
             float top[NH], sum[NH];

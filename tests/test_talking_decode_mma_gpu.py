@@ -92,3 +92,19 @@ def test_numbers_that_are_not_finite_stay_where_they_are_seen():
     c["tables"][3, 1] = 10 ** 6
     got, _, status = _run(kernels, c, H, G, D, V, 2, 30.0, True, None)
     assert status == 2 and torch.equal(got[1:3], clean[1:3]) and got[3].isfinite().all()
+
+
+@pytest.mark.parametrize("shares, cap, unit, window", [(1, 2.0, True, None), (2, 2.0, False, None), (3, 3.0, True, 200), (1, 30.0, False, 17)])
+def test_scores_of_minus_infinity_take_the_cap(shares, cap, unit, window):
+    """A key that is seen is capped whatever its score: an infinite key weighs exp(+-cap) as in every other kernel, and is not taken for a
+    masked one where its score is -infinity."""
+    from glassbox_b200 import kernels
+    H, G, D, V = 16, 4, 64, 64
+    c = _case(H, G, D, V, [1, 40, 130, 300], 8)
+    for i, pos, g, channel in ((0, 0, 1, 3), (1, 39, 0, 0), (1, 30, 3, 5), (2, 129, 2, 63), (2, 120, 2, 1), (3, 170, 1, 9), (3, 299, 0, 33)):
+        c["k"][int(c["tables"][i][pos // 16]), g, pos % 16, channel] = float("inf")       # (the sign of a score is the query's)
+    att, talk, status = _run(kernels, c, H, G, D, V, shares, cap, unit, window)
+    want = _exact(c, H, G, D, V, talk, cap, unit, window)
+    assert status == 0 and want.isfinite().all()
+    # as above; a score of 30 in float32 adds 30 units of 6e-8 to a weight's relative error
+    assert (att.double() - want).abs().max() < 4e-6 * H ** 0.5 * 4 and (att.double() - want).norm() < 2e-6 * want.norm()
