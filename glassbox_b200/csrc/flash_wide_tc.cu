@@ -341,7 +341,12 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? a.scale / a.cap : 0.f;
         const float slx = cap2 > 0.f ? cap2 : sl2;              // what is left to scale
         const int first = gb_first_key(pos, a.window), first_last = gb_first_key(pos_lo + FW_BM - 1, a.window);
-        const bool bounded = a.cap > 0.f && a.cap <= 32.f && first_last == 0;      // (and every row sees a key of the first tile)
+        // Scores that a cap bounds: what a row subtracts is chosen after the first tile (every row must see a key of it) and stays, and the two
+        // halves of a row go their own ways, one's caps beside the other's exponentials. It is the tile's maximum, at least what 2^8 lies
+        // below the cap, so that no weight grows above 2^8, as none does where the maximum is followed. Rows whose first tile lies 2^60
+        // below that are left to the general form: their weights could become too small for sums in float32.
+        bool bounded = a.cap > 0.f && a.cap <= 32.f && first_last == 0;
+        const float least = 1.0f - 8.0f / cap2;                 // (scores are in units of the cap)
         float m_run = FW_NEG_BIG, l_run = 0.f;
         bool ok = true;
         for (int j = 0; j < ntiles; ++j) {
@@ -357,8 +362,6 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 for (int k = 0; k < 64; ++k)
                     if (!(key0 + k <= pos && key0 + k >= first)) sv[k] = __float_as_uint(FW_NEG_BIG);
             }
-            // Scores that a cap bounds: the first tile's maximum stays, or -16 (a weight is then at most e^48), and the two halves of a row go
-            // their own ways, one's caps beside the other's exponentials.
             if (j == 0 || !bounded) {
                 float mx4[4] = {FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG};
 #pragma unroll
@@ -374,7 +377,8 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
                 const bool raise = (mx - m_run) * slx > 8.0f;
                 if (j == 0) {
-                    if (raise) m_run = bounded ? fmaxf(mx, -16.0f / a.cap) : mx;      // nothing is accumulated yet (scores are in units of the cap)
+                    bounded = bounded && __all_sync(0xffffffffu, mx >= least - 60.0f / cap2);      // (both halves have the same maxima)
+                    if (raise) m_run = bounded ? fmaxf(mx, least) : mx;      // nothing is accumulated yet
                 } else if (__any_sync(0xffffffffu, raise)) {
                     // (S_j was issued after O += P_(j-2) V_(j-2) was done: the phase of P_(j-1) V_(j-1) is the one to wait for)
                     if (!mbar_wait_warp(&sh.pv_done, (j - 1) & 1, abort_flag, a.status)) { ok = false; break; }
