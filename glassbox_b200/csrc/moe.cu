@@ -909,10 +909,13 @@ GB_EXPORT int gb_moe_sort(const int* choice, const int* positions, int n, int E,
     GB_REQUIRE(n >= 0 && E > 0 && E <= MOE_MAX_EXPERTS && top > 0, "gb_moe_sort: bad sizes");
     if (n == 0) return 0;
     if (E <= MS_FEW && (long long)n * top <= (long long)MS_KEEP * MS_THREADS) {
+        // (the limit is the most that any sizes need: a kernel has one, and a thread with few pairs must not lower it under another's launch)
+        constexpr int most = MS_FEW * MS_THREADS * (int)sizeof(unsigned short) + MS_KEEP * MS_THREADS * (int)sizeof(int);
         const int smem = E * MS_THREADS * (int)sizeof(unsigned short) + n * top * (int)sizeof(int);
-        cudaError_t e = cudaFuncSetAttribute(moe_sort_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem > 48 * 1024 ? smem : 48 * 1024);
-        GB_REQUIRE(e == cudaSuccess, "gb_moe_sort: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-        gb_launch(GB_PDL_ELEMENTWISE, moe_sort_columns_kernel, dim3(1), dim3(MS_THREADS), smem, stream, choice, positions, n, E, top, offsets, sorted);
+        cudaError_t e = cudaFuncSetAttribute(moe_sort_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        GB_REQUIRE(e == cudaSuccess, "gb_moe_sort: %d bytes of shared memory refused: %s", most, cudaGetErrorString(e));
+        e = gb_launch(GB_PDL_ELEMENTWISE, moe_sort_columns_kernel, dim3(1), dim3(MS_THREADS), smem, stream, choice, positions, n, E, top, offsets, sorted);
+        GB_REQUIRE(e == cudaSuccess, "gb_moe_sort: launch failed: %s", cudaGetErrorString(e));
         return gb_check_launch("gb_moe_sort");
     }
     gb_launch(GB_PDL_ELEMENTWISE, moe_sort_kernel, dim3(1), dim3(MS_THREADS), 0, stream, choice, positions, n, E, top, offsets, sorted);

@@ -27,3 +27,29 @@ def test_every_live_pair_has_a_slot_of_its_expert(n, E, top):
     used = order[:len(live)]
     assert torch.equal(used.sort().values.long(), live) and (order[len(live):] == -1).all()
     assert torch.equal(expert[used.long()].long(), torch.repeat_interleave(torch.arange(E, device=DEV), counts))
+
+
+def test_threads_with_few_and_many_pairs_do_not_disturb_each_other():
+    """The kernel's limit of shared memory is one for all threads of a process: a small sort beside a large one must not lower it."""
+    import threading
+    from glassbox_b200 import kernels
+    failures = []
+
+    def work(n, E, top):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                choice = (torch.arange(n * top, device=DEV) % E).to(torch.int32)
+                positions, offsets, order = (torch.zeros(size, dtype=torch.int32, device=DEV) for size in (n, E + 1, n * top))
+                for _ in range(3000):
+                    kernels._call("gb_moe_sort", choice.data_ptr(), positions.data_ptr(), n, E, top, offsets.data_ptr(), order.data_ptr(),
+                                  kernels._stream())
+                torch.cuda.current_stream().synchronize()
+                assert offsets.tolist() == [i * n * top // E for i in range(E + 1)]
+        except Exception as e:      # noqa: BLE001 (reported by the thread that asserts)
+            failures.append(repr(e))
+    threads = [threading.Thread(target=work, args=shape) for shape in ((16, 16, 4), (4096, 64, 4), (64, 16, 2), (4096, 64, 4))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
