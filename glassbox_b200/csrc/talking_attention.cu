@@ -976,16 +976,30 @@ __global__ void __launch_bounds__(256) talk_shares_kernel(const float* __restric
     }
 }
 
+// Most dynamic shared memory of the merging kernels below; their limit is this whatever a call needs (a kernel has one limit, and a
+// small call must not lower it under another thread's launch).
+constexpr int TKC_SMEM_MAX = 200 * 1024;
+
+// Channels of a block in fours: a value head's, halved while a block has over 256 cells or there are fewer blocks than
+// multiprocessors, as long as a block keeps more than 64 cells.
+static int tks_quads(int n, int H, int G, int V) {
+    int quads = V / 4;
+    while (quads % 2 == 0 && (H * quads > 256 || (long long)n * G * (V / 4 / quads) < 148) && H * quads > 64) quads /= 2;
+    return quads;
+}
+static size_t tks_smem_bytes(int H, int G, int shares, int quads) {
+    return ((size_t)H * quads * 4 + (size_t)2 * H * shares + (size_t)H / G * H) * sizeof(float);
+}
+
 template <typename T>
 static int tks_launch(const float* o, const float* ml, const float* talk, void* att, const int* positions, int n, int H, int G, int V,
                       int shares, float unit, cudaStream_t stream) {
-    // a block's channels: a value head's, halved while the blocks are fewer than two a multiprocessor and a block has over 256 cells
-    int quads = V / 4;
-    while (quads % 2 == 0 && (H * quads > 256 || (long long)n * G * (V / 4 / quads) < 148) && H * quads > 64) quads /= 2;
-    const size_t smem = ((size_t)H * quads * 4 + (size_t)2 * H * shares + (size_t)H / G * H) * sizeof(float);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(talk_shares_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gb_launch(GB_PDL_ELEMENTWISE, talk_shares_kernel<T>, dim3(n, G, V / 4 / quads), dim3(256), smem, stream, o, ml, talk, (T*)att, positions, n,
-              H, G, V, shares, unit, quads);
+    const int quads = tks_quads(n, H, G, V);
+    cudaError_t e = cudaFuncSetAttribute(talk_shares_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, TKC_SMEM_MAX);
+    GB_REQUIRE(e == cudaSuccess, "gb_talk_combine: %d bytes of shared memory refused: %s", TKC_SMEM_MAX, cudaGetErrorString(e));
+    e = gb_launch(GB_PDL_ELEMENTWISE, talk_shares_kernel<T>, dim3(n, G, V / 4 / quads), dim3(256), tks_smem_bytes(H, G, shares, quads), stream, o, ml,
+                  talk, (T*)att, positions, n, H, G, V, shares, unit, quads);
+    GB_REQUIRE(e == cudaSuccess, "gb_talk_combine: launch failed: %s", cudaGetErrorString(e));
     return gb_check_launch("gb_talk_combine");
 }
 
@@ -1059,8 +1073,9 @@ template <typename T>
 static int tkc_launch(const float* o, const float* ml, const float* talk, void* att, const int* positions, int n, int H, int G, int V,
                       int VG, int shares, float unit, cudaStream_t stream) {
     const size_t smem = ((size_t)H * V + (size_t)H * shares) * sizeof(float);
-    GB_REQUIRE(smem <= 200 * 1024, "gb_talk_combine: %d heads of %d channels in %d shares do not fit a block's shared memory", H, V, shares);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(talk_combine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    GB_REQUIRE(smem <= TKC_SMEM_MAX, "gb_talk_combine: %d heads of %d channels in %d shares do not fit a block's shared memory", H, V, shares);
+    cudaError_t e = cudaFuncSetAttribute(talk_combine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, TKC_SMEM_MAX);
+    GB_REQUIRE(e == cudaSuccess, "gb_talk_combine: %d bytes of shared memory refused: %s", TKC_SMEM_MAX, cudaGetErrorString(e));
     const int cuts = (long long)n * G >= 296 ? 1 : (int)min((long long)gb_ceil_div(V, 16), (long long)gb_ceil_div(296, (long long)n * G));
     gb_launch(GB_PDL_ELEMENTWISE, talk_combine_kernel<T>, dim3(n, G, cuts), dim3(256), smem, stream, o, ml, talk, (T*)att, positions, n, H, G,
               V, VG, shares, unit);
@@ -1080,7 +1095,7 @@ GB_EXPORT int gb_talk_combine(const float* o, const float* ml, const float* talk
         if (dtype == GB_BF16) return tkm_launch<__nv_bfloat16>(o, talk, att, positions, n, H, G, V, stream);
     }
     if (talk != nullptr && shares > 1 && V % 4 == 0 && H <= 64 && H * shares <= 4096 &&
-        (((uintptr_t)o | (uintptr_t)att) & 15) == 0 && ((uintptr_t)ml & 7) == 0) {
+        tks_smem_bytes(H, G, shares, tks_quads(n, H, G, V)) <= TKC_SMEM_MAX && (((uintptr_t)o | (uintptr_t)att) & 15) == 0 && ((uintptr_t)ml & 7) == 0) {
         if (dtype == GB_F32) return tks_launch<float>(o, ml, talk, att, positions, n, H, G, V, shares, unit, stream);
         if (dtype == GB_BF16) return tks_launch<__nv_bfloat16>(o, ml, talk, att, positions, n, H, G, V, shares, unit, stream);
     }

@@ -108,3 +108,47 @@ def test_scores_of_minus_infinity_take_the_cap(shares, cap, unit, window):
     assert status == 0 and want.isfinite().all()
     # as above; a score of 30 in float32 adds 30 units of 6e-8 to a weight's relative error
     assert (att.double() - want).abs().max() < 4e-6 * H ** 0.5 * 4 and (att.double() - want).norm() < 2e-6 * want.norm()
+
+
+def _merge(kernels, H, V, shares, launches=1):
+    gen = torch.Generator(device=DEV).manual_seed(V)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device=DEV)
+    wide, ml, talk = rand(shares * 1, H * V), rand(shares * 1, H * 2), rand(H, H)
+    ml[:, 1::2] = ml[:, 1::2].abs() + 1.0
+    att, positions = torch.zeros(1, H * V, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    for _ in range(launches):
+        kernels.talk_combine(wide, talk, att, positions, H, 1, V, 1, shares=shares, ml=ml, unit_sink=False)
+    return wide, ml, talk, att
+
+
+def test_merges_of_any_size_in_several_threads():
+    """The merging kernel's limit of shared memory is one for all threads: 64 heads of 252 channels beside 64 heads of 508."""
+    import threading
+    from glassbox_b200 import kernels
+    failures = []
+
+    def work(V):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                wide, ml, talk, att = _merge(kernels, 64, V, 2, launches=2000)
+                torch.cuda.current_stream().synchronize()
+                m, l = ml.double().view(2, 64, 2).unbind(-1)
+                f = torch.exp(m - m.amax(0))
+                rows = (wide.double().view(2, 64, V) * f[..., None]).sum(0) / (l * f).sum(0)[:, None]
+                want = talk.double() @ rows
+                # float32 sums of 64 products
+                assert (att.double().view(64, V) - want).norm() < 2e-6 * want.norm()
+        except Exception as e:      # noqa: BLE001 (reported by the thread that asserts)
+            failures.append(repr(e))
+    threads = [threading.Thread(target=work, args=(V,)) for V in (252, 508, 252, 508)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+
+
+def test_a_merge_that_no_block_can_hold_says_so():
+    from glassbox_b200 import kernels
+    with pytest.raises(kernels.KernelError, match="do not fit a block's shared memory"):
+        _merge(kernels, 64, 1020, 2)
