@@ -12,13 +12,13 @@
 //     column n of channel tile j stands for channel (HD/8)*n + j, so a thread needs HD/8 consecutive
 //     channels of its four value rows (one 16-byte load at HD 64) and ends up owning 2*HD/8
 //     consecutive output channels.
-// Softmax statistics and accumulators are float32. Every warp writes its partial result (maximum,
-// sum, unnormalised output) and the block that finishes last merges all of them.
+// Softmax statistics and accumulators are float32. A block adds up its warps' results (maximum, sum,
+// unnormalised output) and, where there are several splits, one block merges theirs.
 // Semantics as crates/glassbox-core/src/model.rs:278-317 (keys max(0, p-window+1) .. p).
 // The cache must hold finite numbers everywhere (it is zero-filled when allocated): rows of a page
 // beyond a request's length are loaded and then masked, not skipped.
 //
-// Scratch: part_acc float32 [rows, heads, 4*splits, HD], part_ml float32 [rows, heads, 4*splits, 2],
+// Scratch: part_acc float32 [rows, heads, splits, HD], part_ml float32 [rows, heads, splits, 2] (callers give room for every warp's),
 // counters int32 [rows * kv heads], zero on entry and left zero.
 #include "attention_decode_mma_body.cuh"
 
@@ -138,7 +138,7 @@ static int decode_mma_dispatch(const void* q, long long q_stride, void* out, lon
     GB_REQUIRE(max_pages > 0 && splits >= 1 && part_acc && part_ml && counters,
                "gb_attention_decode_mma: bad page geometry, split count or scratch");
     GB_REQUIRE(warps == 4 || (warps == 8 && hd == 64), "gb_attention_decode_mma: %d warps per block are not built for this variant (4; 8 at head size 64)", warps);
-    GB_REQUIRE(n <= 65535 && splits <= MMA_MAX_MERGE / warps, "gb_attention_decode_mma: too many rows or splits for one launch");
+    GB_REQUIRE(n <= 65535 && splits <= MMA_MAX_PARTS / warps, "gb_attention_decode_mma: too many rows or splits for one launch");
     GB_REQUIRE(q_stride % 4 == 0 && (uintptr_t)q % 8 == 0, "gb_attention_decode_mma: q must be 8-byte aligned");
     if (n == 0) return 0;
 #define GB_MMA(HH, BB) GB_MMAW(HH, BB, 4)

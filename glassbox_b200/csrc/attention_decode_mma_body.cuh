@@ -44,8 +44,9 @@ struct DecodeAttnArgs {
 };
 
 constexpr float MMA_NEG_BIG = -1.0e30f;
-constexpr int MMA_MAX_MERGE = 2048;   // weights of (heads x sub-splits) merged per pass
+constexpr int MMA_MAX_PARTS = 2048;   // partial results of a head (splits x warps) at most
 constexpr int MMA_MAX_PAGES = 1024;   // page ids of one block's key range kept in shared memory
+constexpr int MMA_SCRATCH = 3072;     // floats in which a block's warps add up their results
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
@@ -105,8 +106,10 @@ template <> struct RowLoad<8> {
 // one). Queries, which another block of the same launch may have written, are read past L1.
 // Shared memory of the body, provided by the caller.
 struct __align__(16) DecodeAttnSmem {   // (a multiple of 16 bytes, so that arrays of it keep what follows aligned)
-    int pages[MMA_MAX_PAGES];
-    float weights[MMA_MAX_MERGE];
+    union {
+        int pages[MMA_MAX_PAGES];
+        float scratch[MMA_SCRATCH];   // once no page id is needed any more
+    };
     int is_last;
 };
 
@@ -121,7 +124,7 @@ __host__ __device__ constexpr int decode_attn_cluster_floats(int group, int spli
 // stand alone). A block adds up its warps' partial results in its own shared memory (`cluster_part`, decode_attn_cluster_floats<HD>()
 // floats, the same offset in every block) and puts one result into the first block's; they meet at the cluster's barrier, and the
 // first block merges the splits: no trip through global memory, no counter, no second pass over what other blocks wrote. Otherwise
-// the warps' partial results go through `part_acc` / `part_ml` and the block that arrives last at `counters` merges them.
+// the blocks' results go through `part_acc` / `part_ml` and the block that arrives last at `counters` merges them.
 template <int HD, int BK, class Sync, int NW = 4, bool CLUSTER = false, bool SINK = false>
 __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& a, const int split, const int kvh, const int row,
                                                           DecodeAttnSmem& sm, Sync& sync, float* cluster_part = nullptr) {
@@ -152,7 +155,6 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
     const int g = lane >> 2, t = lane & 3;
     const int G = nh / nkv;
     const int head0 = kvh * G;
-    const int S4 = splits * NW;   // partial results per head: one per warp of every split
     int& is_last = sm.is_last;
     // SINK: the distance bias of this thread's two heads (rows g and g + 8 of the score tile), and what a merged head's
     // denominator and output still need: the sink's logit joins the maximum and the sum, the gate scales the result
@@ -387,62 +389,65 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
     }
-    const int sub = split * NW + warp;
-    float* weights = sm.weights;
+    // What a block's warps found comes together in shared memory first, then what the splits found: the same sums in the same order in both
+    // ways of merging, so that both give the same bits.
+    constexpr int PITCH = HD + 2;                 // a result: HD channels, maximum, sum
+    auto put = [&](float* to, int h) {            // this warp's result of its head g + 8 h
+        if (t == 0) {
+            to[HD] = m_run[h];
+            to[HD + 1] = l_run[h];
+        }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            to[NT * (2 * t) + j] = acc[j][2 * h];
+            to[NT * (2 * t + 1) + j] = acc[j][2 * h + 1];
+        }
+    };
+    // a head's channel over `parts` results `step` floats apart: its sum, their maximum and their sum (the weights formed by every thread)
+    auto merge = [&](const float* pa, int parts, int step, int d, float top, float& m, float& l) {
+        m = top;
+        for (int i = 0; i < parts; ++i) m = fmaxf(m, pa[i * step + HD]);
+        float v = 0.f;
+        l = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < parts; ++i) {
+            const float w = __expf(pa[i * step + HD] - m);
+            l = fmaf(pa[i * step + HD + 1], w, l);
+            v = fmaf(pa[i * step + d], w, v);
+        }
+        return v;
+    };
+    // the head's result from its channel's sum v, the maximum m (the sink's logit sk among what it is of) and the sum l
+    auto finish = [&](int hi, int d, float sk, float m, float l, float v) {
+        if constexpr (SINK) l += __expf(sk - m);
+        v *= (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head0 + hi);
+        orow[(head0 + hi) * HD + d] = __float2bfloat16_rn(SINK ? v * channel_gate(head0 + hi, d) : v);
+    };
     if constexpr (CLUSTER) {
         namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
-        float* first = cluster.map_shared_rank(cluster_part, 0) + (size_t)NW * G * (HD + 2);       // [split][head][HD channels, maximum, sum]
+        float* first = cluster.map_shared_rank(cluster_part, 0) + (size_t)NW * G * PITCH;       // [split][head][HD channels, maximum, sum]
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int hi = g + 8 * h;
-            if (hi < G) {
-                float* pa = cluster_part + ((size_t)warp * G + hi) * (HD + 2);
-                if (t == 0) {
-                    pa[HD] = m_run[h];
-                    pa[HD + 1] = l_run[h];
-                }
-#pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    pa[NT * (2 * t) + j] = acc[j][2 * h];
-                    pa[NT * (2 * t + 1) + j] = acc[j][2 * h + 1];
-                }
-            }
-        }
-        // a head's channel over `parts` results `step` floats apart: its sum, their maximum and their sum (the weights formed by every thread)
-        auto merge = [&](const float* pa, int parts, int step, int d, float top, float& m, float& l) {
-            m = top;
-            for (int i = 0; i < parts; ++i) m = fmaxf(m, pa[i * step + HD]);
-            float v = 0.f;
-            l = 0.f;
-#pragma unroll 8
-            for (int i = 0; i < parts; ++i) {
-                const float w = __expf(pa[i * step + HD] - m);
-                l = fmaf(pa[i * step + HD + 1], w, l);
-                v = fmaf(pa[i * step + d], w, v);
-            }
-            return v;
-        };
-        auto finish = [&](const float* pa, int parts, int i) {
+        for (int h = 0; h < 2; ++h)
+            if (g + 8 * h < G) put(cluster_part + ((size_t)warp * G + g + 8 * h) * PITCH, h);
+        auto last = [&](const float* pa, int parts, int i) {
             const int hi = i / HD, d = i % HD;
             const float sk = sink_logit(head0 + hi);
             float m, l;
-            float v = merge(pa + (size_t)hi * (HD + 2), parts, G * (HD + 2), d, sk, m, l);
-            if constexpr (SINK) l += __expf(sk - m);
-            v *= (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head0 + hi);
-            orow[(head0 + hi) * HD + d] = __float2bfloat16_rn(SINK ? v * channel_gate(head0 + hi, d) : v);
+            const float v = merge(pa + (size_t)hi * PITCH, parts, G * PITCH, d, sk, m, l);
+            finish(hi, d, sk, m, l, v);
         };
         sync.group_barrier();
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
         if (splits == 1) {
-            for (int i = tid; i < G * HD; i += NTHREADS) finish(cluster_part, NW, i);
+            for (int i = tid; i < G * HD; i += NTHREADS) last(cluster_part, NW, i);
             return;
         }
         for (int i = tid; i < G * HD; i += NTHREADS) {
             const int hi = i / HD, d = i % HD;
             float m, l;
-            const float v = merge(cluster_part + (size_t)hi * (HD + 2), NW, G * (HD + 2), d, MMA_NEG_BIG, m, l);
-            float* to = first + ((size_t)split * G + hi) * (HD + 2);
+            const float v = merge(cluster_part + (size_t)hi * PITCH, NW, G * PITCH, d, MMA_NEG_BIG, m, l);
+            float* to = first + ((size_t)split * G + hi) * PITCH;
             to[d] = v;
             if (d == 0) {
                 to[HD] = m;
@@ -451,27 +456,40 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
         }
         cluster.sync();                       // (release / acquire: the first block sees what the others stored)
         if (cluster.block_rank() != 0) return;
-        for (int i = tid; i < G * HD; i += NTHREADS) finish(cluster_part + (size_t)NW * G * (HD + 2), splits, i);
+        for (int i = tid; i < G * HD; i += NTHREADS) last(cluster_part + (size_t)NW * G * PITCH, splits, i);
         return;
     }
+    // Through global memory: the block's results, as many heads at a time as the scratch holds, one for every split; the block that arrives
+    // last merges them. With every warp's result stored, 48 of them for the last block to merge, 8 rows of 9/3 heads behind 4,000 keys took
+    // 10.7 us with a lane a warp for the weights (sums in another order) and 11.1 with a lane a split, 10.4 so; a 135M step of them 751, 763
+    // and 734, of 16 such rows 919, 927 and 902.
+    constexpr int HEADS = MMA_SCRATCH / (NW * PITCH) < 16 ? MMA_SCRATCH / (NW * PITCH) : 16;
+    static_assert(HEADS >= 1, "a head's results of all warps must fit the scratch");
+    float* own = sm.scratch;                      // [warp][head of the pass][HD channels, maximum, sum], where the page ids were
+    for (int h0 = 0; h0 < G; h0 += HEADS) {
+        const int count = min(HEADS, G - h0);
+        sync.group_barrier();                     // (the page ids, or the pass before, have been read)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int hi = g + 8 * h;
-        if (hi < G) {
-            const size_t slot = ((size_t)row * nh + head0 + hi) * S4 + sub;
-            if (t == 0) {
-                part_ml[slot * 2] = m_run[h];
-                part_ml[slot * 2 + 1] = l_run[h];
+        for (int h = 0; h < 2; ++h) {
+            const int hi = g + 8 * h - h0;
+            if (hi >= 0 && hi < count) put(own + (warp * count + hi) * PITCH, h);
+        }
+        sync.group_barrier();
+        for (int i = tid; i < count * HD; i += NTHREADS) {
+            const int hi = i / HD, d = i % HD;
+            const float sk = splits == 1 ? sink_logit(head0 + h0 + hi) : MMA_NEG_BIG;
+            float m, l;
+            const float v = merge(own + hi * PITCH, NW, count * PITCH, d, sk, m, l);
+            if (splits == 1) {
+                finish(h0 + hi, d, sk, m, l, v);
+                continue;
             }
-            float* pa = part_acc + slot * HD;
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                pa[NT * (2 * t) + j] = acc[j][2 * h];
-                pa[NT * (2 * t + 1) + j] = acc[j][2 * h + 1];
-            }
+            const size_t slot = ((size_t)row * nh + head0 + h0 + hi) * splits + split;
+            part_acc[slot * HD + d] = v;
+            if (d == 0) *reinterpret_cast<float2*>(part_ml + slot * 2) = make_float2(m, l);
         }
     }
-    // ---- the block that arrives last merges every warp of every split
+    if (splits == 1) return;
     __threadfence();
     sync.group_barrier();
     if (tid == 0) {
@@ -483,100 +501,40 @@ __device__ __forceinline__ void attention_decode_mma_body(const DecodeAttnArgs& 
     sync.group_barrier();
     if (!is_last) return;
     __threadfence();
-    // Merge, in the order of the cluster's (a split's warps first, then the splits), so that both give the same bits: one warp per head
-    // turns the (maximum, sum) pairs into each warp's weight within its split (`weights`), each split's weight (`tops`, over the page ids,
-    // which nothing reads any more) and the head's scale; then every thread adds up its channel with independent loads.
-    float2* tops = reinterpret_cast<float2*>(sm.pages);      // [head of the pass][split]: weight, sum (of split 0: the head's scale, once known)
-    static_assert(sizeof(sm.pages) >= 2 * sizeof(float) * (MMA_MAX_MERGE / NW), "a pass's splits must fit the page ids' place");
-    auto weigh = [&](int hi, int head) {
-        const float2* ml = reinterpret_cast<const float2*>(part_ml + ((size_t)row * nh + head) * S4 * 2);
-        const float sk = sink_logit(head);
-        float m = sk, l = 0.f;
-        for (int sp = lane; sp < splits; sp += 32) {
-            float2 p[NW];
-            float ms = MMA_NEG_BIG, ls = 0.f;
+    for (int i = tid; i < G * HD; i += NTHREADS) {
+        const int hi = i / HD, d = i % HD;
+        const float* pa = part_acc + ((size_t)row * nh + head0 + hi) * splits * HD + d;
+        const float2* ml = reinterpret_cast<const float2*>(part_ml) + ((size_t)row * nh + head0 + hi) * splits;
+        const float sk = sink_logit(head0 + hi);
+        float m = sk, l = 0.f, v = 0.f;
+        if (splits <= 8) {                        // all asked for before the first is used: one trip to L2
+            float2 p[8];
+            float pv[8];
 #pragma unroll
-            for (int i = 0; i < NW; ++i) {
-                p[i] = __ldcg(ml + sp * NW + i);
-                ms = fmaxf(ms, p[i].x);
+            for (int sp = 0; sp < 8; ++sp) {
+                p[sp] = sp < splits ? __ldcg(ml + sp) : make_float2(MMA_NEG_BIG, 0.f);
+                pv[sp] = sp < splits ? __ldcg(pa + (size_t)sp * HD) : 0.f;
             }
 #pragma unroll
-            for (int i = 0; i < NW; ++i) {
-                const float w = __expf(p[i].x - ms);
-                weights[hi * S4 + sp * NW + i] = w;
-                ls = fmaf(p[i].y, w, ls);
-            }
-            tops[hi * splits + sp] = make_float2(ms, ls);
-            m = fmaxf(m, ms);
-        }
-        m = gb_warp_max(m);
-        for (int sp = lane; sp < splits; sp += 32) {
-            float2& top = tops[hi * splits + sp];
-            top.x = __expf(top.x - m);
-            l = fmaf(top.y, top.x, l);
-        }
-        __syncwarp();
-        if (splits <= 8) {
-            l = 0.f;
-            for (int sp = 0; sp < splits; ++sp) l = fmaf(tops[hi * splits + sp].y, tops[hi * splits + sp].x, l);
-        } else {                                             // (more than a cluster holds: any order)
-            l = gb_warp_sum(l);
-        }
-        if constexpr (SINK) l += __expf(sk - m);
-        __syncwarp();
-        if (lane == 0) tops[hi * splits].y = (l > 0.f ? 1.0f / l : 0.f) * gate_factor(head);
-    };
-    if (G * HD <= NTHREADS && S4 <= 64) {
-        // The usual case (every output channel of the group has a thread of its own, at most 64 partial results per
-        // head): a thread asks for its channel of every partial result at once, before the weights exist, and a lane
-        // reads its (maximum, sum) pairs once; the merge is then two trips to L2 that overlap instead of four in a row.
-        constexpr int MAXP = 64;
-        const int hi_o = tid / HD, d_o = tid % HD;
-        float pv[MAXP];
-        const float gch = tid < G * HD ? channel_gate(head0 + hi_o, d_o) : 1.0f;
-        if (tid < G * HD) {
-            const float* pa = part_acc + ((size_t)row * nh + head0 + hi_o) * S4 * HD + d_o;
+            for (int sp = 0; sp < 8; ++sp) m = fmaxf(m, p[sp].x);
 #pragma unroll
-            for (int sidx = 0; sidx < MAXP; ++sidx) pv[sidx] = sidx < S4 ? __ldcg(pa + (size_t)sidx * HD) : 0.f;
-        }
-        for (int hi = warp; hi < G; hi += NW) weigh(hi, head0 + hi);
-        sync.group_barrier();
-        if (tid < G * HD) {
-            const float* w = weights + hi_o * S4;
-            float v = 0.f;
-#pragma unroll
-            for (int sp = 0; sp < MAXP / NW; ++sp)
+            for (int sp = 0; sp < 8; ++sp)
                 if (sp < splits) {
-                    float part = 0.f;
-#pragma unroll
-                    for (int i = 0; i < NW; ++i) part = fmaf(pv[sp * NW + i], w[sp * NW + i], part);
-                    v = fmaf(part, tops[hi_o * splits + sp].x, v);
+                    const float w = __expf(p[sp].x - m);
+                    l = fmaf(p[sp].y, w, l);
+                    v = fmaf(pv[sp], w, v);
                 }
-            v *= tops[hi_o * splits].y;
-            orow[(head0 + hi_o) * HD + d_o] = __float2bfloat16_rn(SINK ? v * gch : v);
-        }
-        return;
-    }
-    const int per_pass = MMA_MAX_MERGE / S4;                 // heads whose weights fit at once
-    for (int h0 = 0; h0 < G; h0 += per_pass) {
-        const int hcount = min(per_pass, G - h0);
-        for (int hi = warp; hi < hcount; hi += NW) weigh(hi, head0 + h0 + hi);
-        sync.group_barrier();
-        for (int i = tid; i < hcount * HD; i += NTHREADS) {
-            const int hi = i / HD, d = i % HD;
-            const float* pa = part_acc + ((size_t)row * nh + head0 + h0 + hi) * S4 * HD + d;
-            const float* w = weights + hi * S4;
-            float v = 0.f;
-#pragma unroll 2
+        } else {
+#pragma unroll 8
+            for (int sp = 0; sp < splits; ++sp) m = fmaxf(m, __ldcg(ml + sp).x);
+#pragma unroll 8
             for (int sp = 0; sp < splits; ++sp) {
-                float part = 0.f;
-#pragma unroll
-                for (int k = 0; k < NW; ++k) part = fmaf(__ldcg(pa + (size_t)(sp * NW + k) * HD), w[sp * NW + k], part);
-                v = fmaf(part, tops[hi * splits + sp].x, v);
+                const float2 p = __ldcg(ml + sp);
+                const float w = __expf(p.x - m);
+                l = fmaf(p.y, w, l);
+                v = fmaf(__ldcg(pa + (size_t)sp * HD), w, v);
             }
-            v *= tops[hi * splits].y;
-            orow[(head0 + h0 + hi) * HD + d] = __float2bfloat16_rn(SINK ? v * channel_gate(head0 + h0 + hi, d) : v);
         }
-        sync.group_barrier();
+        finish(hi, d, sk, m, l, v);
     }
 }

@@ -562,7 +562,7 @@ GB_EXPORT int gb_program_encode_attention(void* op, const void* q, long long q_s
     GB_REQUIRE(nkv > 0 && nh % nkv == 0 && nh / nkv <= 16, "gb_program_encode_attention: %d heads per kv head are not built", nkv > 0 ? nh / nkv : 0);
     GB_REQUIRE(page_size >= 16 && (page_size & (page_size - 1)) == 0, "gb_program_encode_attention: page size %d must be a power of two >= 16", page_size);
     GB_REQUIRE((long long)num_pages * nkv * page_size < (1ll << 31), "gb_program_encode_attention: the cache has too many rows");
-    GB_REQUIRE(max_pages > 0 && splits >= 1 && splits <= MMA_MAX_MERGE / 4 && part_acc && part_ml && counters && status,
+    GB_REQUIRE(max_pages > 0 && splits >= 1 && splits <= MMA_MAX_PARTS / 4 && part_acc && part_ml && counters && status,
                "gb_program_encode_attention: bad page geometry, split count or scratch");
     GB_REQUIRE(n >= 1 && n <= 16, "gb_program_encode_attention: %d rows are outside a program's range", n);
     GB_REQUIRE(q_stride % 4 == 0 && (uintptr_t)q % 8 == 0, "gb_program_encode_attention: q must be 8-byte aligned");

@@ -39,3 +39,37 @@ def test_splits_merge_in_a_cluster(nh, nkv, hd, splits, block_keys, warps, windo
         want = torch.einsum("hk,khd->hd", torch.softmax(s, -1), values)
         # weights and result in bfloat16: 2^-8 of values of a few
         assert (out[i].double().view(nh, hd) - want).abs().max() < 2.0 ** -8 * 4, i
+
+
+@pytest.mark.parametrize("nh, nkv, hd, warps", [(9, 3, 64, 8), (16, 1, 64, 8), (24, 2, 128, 4), (32, 4, 96, 4), (16, 1, 16, 4), (5, 1, 64, 4)])
+@pytest.mark.parametrize("splits, many", [(2, 100), (6, 64), (8, 64), (3, 160), (13, 3), (30, 3)])
+def test_both_ways_of_merging_give_the_same_bits(nh, nkv, hd, warps, splits, many):
+    """A few rows merge on the chip, as many as find no room there through global memory (whose scratch may take a large group's heads in
+    several passes), as do more splits than a cluster has blocks: the same order of sums, so the same bits."""
+    from glassbox_b200 import kernels
+    gen = torch.Generator(device=DEV).manual_seed(nh + splits)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device=DEV).bfloat16()
+    context, page = 1500, 16
+    pages = -(-context // page)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    k, v, q = rand(pages, nkv, page, hd), rand(pages, nkv, page, hd), rand(many, nh * hd)
+    tables = i32([list(range(pages))] * many)
+    scratch = lambda n: (torch.full((n * nh * warps * splits * hd,), float("nan"), device=DEV), torch.full((n * nh * warps * splits * 2,), float("nan"), device=DEV))
+    status, counters = i32([0]), i32([0] * (many * nkv))
+    positions = i32([(context - 1 - 37 * i) % context for i in range(many)])
+
+    def run(n, keys):
+        out = torch.full((n, nh * hd), 7.0, device=DEV, dtype=torch.bfloat16)
+        part, ml = scratch(n)
+        kernels.attention_decode_mma(q[:n], out, k, v, tables[:n], i32(range(n)), positions[:n], nh, nkv, hd, page, hd ** -0.5, None, splits, part, ml,
+                                     counters, status, keys, warps)
+        return out
+    keys = 16 if warps == 8 else 0
+    all_rows = run(many, keys)
+    assert int(status) == 0 and not counters.any()
+    assert torch.equal(all_rows[:2], run(2, keys))
+    for i in range(min(many, 3)):
+        c = int(positions[i]) + 1
+        kk, vv = (t.transpose(1, 2).flatten(0, 1)[:c].double().repeat_interleave(nh // nkv, dim=1) for t in (k, v))
+        want = torch.einsum("hk,khd->hd", torch.softmax(torch.einsum("hd,khd->hk", q[i].double().view(nh, hd), kk) * hd ** -0.5, -1), vv)
+        assert (all_rows[i].double().view(nh, hd) - want).abs().max() < 2.0 ** -8 * 4, i
