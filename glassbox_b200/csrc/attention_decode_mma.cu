@@ -20,6 +20,8 @@
 //
 // Scratch: part_acc float32 [rows, heads, splits, HD], part_ml float32 [rows, heads, splits, 2] (callers give room for every warp's),
 // counters int32 [rows * kv heads], zero on entry and left zero.
+#include <atomic>
+
 #include "attention_decode_mma_body.cuh"
 
 template <int HD, int BK, int NW, bool CLUSTER, bool SINK = false>
@@ -43,12 +45,24 @@ struct DecodeSinkTerms {
 
 // The merge runs inside a thread-block cluster wherever the splits of a (row, kv head) are at most 8 (a portable cluster), their results
 // fit shared memory, and either the blocks are small (16 keys per iteration and four warps: several an SM) or all clusters find room at
-// once: a processing cluster of at least 16 SMs (there are eight) holds 16 blocks of eight warps, or 32 of four warps with 32 keys per
-// iteration. One split needs no partner at all. Through global memory (a store, a fence, the counter, a load, one after the
+// once: eight processing clusters with 16 SMs each, of one block of eight warps or two of four warps with 32 keys per iteration, and
+// no more than the GPU says that it holds. Neither is enough alone. Of clusters of eight one card holds 15: with 16 the last starts when
+// the others have ended (32/8 heads, two rows of 4,000 / 8,000 keys 12.9 / 20.1 us, through global memory 8.7 / 12.5). And it names 45
+// of three and 26 of five that do not run at once (45 rows and heads of 4,000 keys 18.0, through global memory 14.6). One split needs no partner at all. Through global memory (a store, a fence, the counter, a load, one after the
 // other) / in the cluster, us: 9/3 heads, one row, contexts 100 / 1,024 / 4,000 5.1 / 3.0, 5.4 / 3.2, 8.0 / 6.1; four rows of 1,024 6.0 /
 // 3.7; 32/32 heads, one row of 1,024 5.7 / 4.5. With every warp sending its own result to the first block: 24 rows of 15/5 heads, 1,500
 // keys 13.6, the block's warps added up first 12.2; 40 rows of 9/3, 600 keys 9.1 and 8.1; 64 rows of 32/32, 4,000 keys 347 and 345.
 constexpr int MMA_CLUSTER_SMEM_MAX = 96 * 1024;
+
+// Clusters of a kernel's blocks that find room at once, asked once for every size and group.
+template <int HD, int BK, int NW, bool SINK>
+static int mma_clusters(int splits, int group, int bytes) {
+    static std::atomic<int> known[9][17];         // (+ 1: 0 is not asked yet)
+    std::atomic<int>& n = known[splits][group];
+    if (n.load(std::memory_order_relaxed) == 0)
+        n.store(gb_clusters_at_once(attention_decode_mma_kernel<HD, BK, NW, true, SINK>, splits, NW * 32, bytes) + 1, std::memory_order_relaxed);
+    return n.load(std::memory_order_relaxed) - 1;
+}
 
 template <int HD, int BK, int NW, bool SINK = false>
 static int launch_mma(const void* q, long long q_stride, void* out, long long out_stride, const void* kcache,
@@ -69,8 +83,15 @@ static int launch_mma(const void* q, long long q_stride, void* out, long long ou
     a.late_release = 1;   // (135M decode step at batch 1: 0.646 -> 0.630 ms; no difference at batch 64)
     const int group = nh / nkv;
     const int cluster_bytes = decode_attn_cluster_floats<HD>(group, splits, NW) * (int)sizeof(float);
-    const bool room = (BK == 16 && NW == 4) || splits == 1 || (long long)n * nkv <= 8 * ((NW == 8 ? 16 : 32) / splits);
-    const bool in_cluster = splits <= 8 && room && cluster_bytes <= MMA_CLUSTER_SMEM_MAX;
+    cudaError_t e;
+    bool in_cluster = splits <= 8 && cluster_bytes <= MMA_CLUSTER_SMEM_MAX;
+    if (in_cluster) {
+        e = cudaFuncSetAttribute(attention_decode_mma_kernel<HD, BK, NW, true, SINK>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_CLUSTER_SMEM_MAX);
+        GB_REQUIRE(e == cudaSuccess, "gb_attention_decode_mma: %d bytes of shared memory refused: %s", MMA_CLUSTER_SMEM_MAX, cudaGetErrorString(e));
+        const long long pairs = (long long)n * nkv;
+        in_cluster = (BK == 16 && NW == 4) || splits == 1 ||
+                     (pairs <= 8 * ((NW == 8 ? 16 : 32) / splits) && pairs <= mma_clusters<HD, BK, NW, SINK>(splits, group, cluster_bytes));
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, nkv, n);
     cfg.blockDim = dim3(NW * 32);
@@ -82,14 +103,7 @@ static int launch_mma(const void* q, long long q_stride, void* out, long long ou
         attr[na].val.programmaticStreamSerializationAllowed = 1;
         ++na;
     }
-    cudaError_t e;
     if (in_cluster) {
-        static int configured = 0;
-        if (cluster_bytes > configured) {
-            e = cudaFuncSetAttribute(attention_decode_mma_kernel<HD, BK, NW, true, SINK>, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_CLUSTER_SMEM_MAX);
-            GB_REQUIRE(e == cudaSuccess, "gb_attention_decode_mma: %d bytes of shared memory refused: %s", MMA_CLUSTER_SMEM_MAX, cudaGetErrorString(e));
-            configured = MMA_CLUSTER_SMEM_MAX;
-        }
         attr[na].id = cudaLaunchAttributeClusterDimension;
         attr[na].val.clusterDim.x = splits;
         attr[na].val.clusterDim.y = 1;

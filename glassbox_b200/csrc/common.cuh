@@ -196,3 +196,25 @@ static inline cudaError_t gb_launch(int family, void (*kernel)(KArgs...), dim3 g
     cfg.numAttrs = (gb_pdl_enabled() & family) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+// How many clusters of `size` blocks of a kernel find room on the GPU at once (0 where that cannot be asked). No constant says it: the
+// processing clusters of one chip differ in their multiprocessors, and those of two chips from each other.
+template <typename... KArgs>
+static inline int gb_clusters_at_once(void (*kernel)(KArgs...), int size, int threads, size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return n;
+}
