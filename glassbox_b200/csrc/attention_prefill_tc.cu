@@ -746,6 +746,25 @@ static int prefill_tc_run(const void* q, long long q_stride, int n_rows, void* o
     return gb_check_launch("gb_attention_prefill_tc");
 }
 
+// Whether a launch takes two blocks a pair of row tiles: one request whose row tiles are all at work at once, where the tile that sees the
+// most keys would keep the launch waiting long enough (what a pair costs is 1.5 us) - many fresh tiles, or one tile behind a long
+// context. `reach`: the keys that the table covers (where it is wide for another request's sake, one fresh tile takes 8.2 us as a pair and
+// 6.6 by itself; a 135M step of eight decoded rows behind 4,000 tokens and a fresh prompt of 100 shows no difference).
+// Block a tile / two blocks a pair, 9 heads, us: 256 rows 7.2 / 8.7, 1,024 12.8 / 13.0, 1,280 14.7 / 14.2, 1,536 16.7 / 15.4, 2,048 20.6 /
+// 18.1; behind 1,000 tokens 64 rows 13.5 / 10.9, 128 14.1 / 12.0, 256 15.2 / 16.1, 1,024 20.6 / 21.5, 1,500 24.0 / 23.4; 128 rows behind
+// 1,900 20.5 / 15.6.
+// A window makes the tiles alike and leaves little to share. 2,048 fresh rows, windows of 300 / 1,024 / 1,300 / 1,600 10.5 / 13.3, 15.8 / 18.1, 18.1 /
+// 19.3, 20.0 / 18.9, chunks of 1,024 13.1 / 15.5; 1,500 rows behind 1,000, window of 2,000 22.8 / 24.5: many tiles take pairs where it is no
+// window to them. One tile behind 1,900: windows of 300 / 600 / 1,024 9.7 / 9.9, 11.6 / 10.3, 15.3 / 12.0, a chunk of 1,024 12.7 / 11.1.
+GB_EXPORT int gb_attention_prefill_tc_pairs(int num_seqs, int max_rows_per_seq, int nh, int window, long long reach) {
+    const long long tiles = gb_ceil_div(max_rows_per_seq, AT_BM);
+    if (num_seqs != 1 || tiles * nh > 148) return 0;
+    long long up = 1;                             // (a power of two, as the tables of recorded steps are: both go the same way)
+    while (up < reach) up *= 2;
+    if (tiles == 1) return up >= 2048 && (window == 0 || window >= 512 || window <= -1024);
+    return tiles >= 10 && (window == 0 || llabs((long long)window) >= up);
+}
+
 // Rows of each request are consecutive: request s owns rows seq_first_row[s] .. seq_first_row[s+1]-1, at
 // positions seq_start_pos[s] + local index. q [n_rows, >= nh*hd] and out are bfloat16 with 16-byte aligned
 // rows; kcache and vcache are one layer of the paged cache, [num_pages, nkv, page_size, hd] contiguous.
@@ -766,11 +785,7 @@ static int prefill_tc_launch(const void* q, long long q_stride, int n_rows, void
     GB_REQUIRE(num_pages * nkv * page_size < (1ll << 31), "gb_attention_prefill_tc: the cache layer has too many rows for a 32-bit TMA coordinate");
     if (num_seqs == 0 || max_rows_per_seq <= 0 || n_rows == 0) return 0;
     const int tiles = gb_ceil_div(max_rows_per_seq, AT_BM);
-    // One request whose row tiles are all at work at once: two blocks a pair of tiles, where the tile that sees the most keys would keep the
-    // launch waiting long enough (what a pair costs is 1.5 us) - many fresh tiles, or one tile behind a long context. Block a tile / two
-    // blocks a pair, 9 heads, us: 256 rows 7.2 / 8.7, 1,024 12.8 / 13.0, 1,280 14.9 / 14.2, 1,536 16.7 / 15.4, 2,048 20.7 / 18.0; behind 1,000
-    // tokens 64 rows 13.5 / 11.1, 128 14.1 / 12.0, 256 15.2 / 16.1, 1,024 20.6 / 21.5, 1,500 24.2 / 23.7; 128 rows behind 2,000 21.4 / 15.6.
-    if (!SINK && num_seqs == 1 && tiles * nh <= 148 && (tiles >= 10 || (tiles == 1 && (long long)max_pages * page_size >= 2048)))
+    if (!SINK && gb_attention_prefill_tc_pairs(num_seqs, max_rows_per_seq, nh, window, (long long)max_pages * page_size))
         return prefill_tc_run<SINK, !SINK>(q, q_stride, n_rows, out, out_stride, kcache, vcache, block_tables, max_pages, seq_first_row,
                                            seq_start_pos, num_seqs, tiles, nh, nkv, hd, page_size, num_pages, scale, window, status, stream, terms);
     return prefill_tc_run<SINK, false>(q, q_stride, n_rows, out, out_stride, kcache, vcache, block_tables, max_pages, seq_first_row,

@@ -78,6 +78,7 @@ _SIGNATURES = {
     "gb_attention_prefill_tc_sink": [_P, _LL, _I, _P, _LL, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _LL, _F, _I, _P, _P, _P,
                                      _P, _P, _LL, _I, _F, _P],
     "gb_attention_prefill_tc_supported": [_I, _I, _I, _I],
+    "gb_attention_prefill_tc_pairs": [_I, _I, _I, _I, _LL],
     "gb_gemm_tcgen05": [_P, _P, _P, _I, _I, _I, _I, _LL, _LL, _LL, _P, _P, _P, _P, _LL, _P, _P, _I, _F],
     "gb_gemm_tcgen05_column_tiles": [_I, _I, _I],
     "gb_gemm_tcgen05_supported": [_P, _P, _I, _I, _I, _LL, _LL],

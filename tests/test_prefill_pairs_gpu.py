@@ -54,3 +54,16 @@ def test_second_items_of_one_key_tile_repeat_their_bits(nh, nkv, rows, past):
     for out in outs:
         kernels.attention_prefill_tc(q, out, k, v, table, first, start, rows, nh, nkv, 64, 16, 0.125, 0, status)
     assert int(status) == 0 and all(torch.equal(out, outs[0]) for out in outs)
+
+
+@pytest.mark.parametrize("pairs, num_seqs, rows, nh, window, reach", [
+    (1, 1, 2048, 9, 0, 2048), (1, 1, 1153, 9, 0, 1153), (0, 1, 1152, 9, 0, 2048), (0, 2, 2048, 9, 0, 2048), (0, 1, 2176, 9, 0, 4096),
+    # a window or chunk that ends within what the rows see: tiles see about the same
+    (0, 1, 2048, 9, 300, 2048), (0, 1, 2048, 9, 1300, 2048), (0, 1, 2048, 9, -1024, 2048), (1, 1, 2048, 9, 2048, 2048), (1, 1, 2048, 9, 4096, 2048),
+    (0, 1, 2048, 9, 2048, 4096), (0, 1, 1500, 9, 2000, 2500),
+    # one tile: behind a context that may be long
+    (1, 1, 128, 9, 0, 1025), (0, 1, 128, 9, 0, 1024), (0, 1, 129, 9, 0, 4096), (0, 1, 77, 3, 300, 4096), (1, 1, 77, 3, 600, 4096),
+    (0, 1, 77, 3, -512, 4096), (1, 1, 1, 148, 0, 2048), (0, 1, 1, 149, 0, 2048)])
+def test_which_launches_take_pairs(pairs, num_seqs, rows, nh, window, reach):
+    from glassbox_b200 import kernels
+    assert kernels.lib().gb_attention_prefill_tc_pairs(num_seqs, rows, nh, window, reach) == pairs
