@@ -129,7 +129,7 @@ class StepContext:
         self.token_slots = None           # int32 [rows]: state slot of the rows whose token the device supplies itself, else -1
         self.want_slots = None            # int32 [wanted rows]: state slot of the rows that are sampled from their own state, else -1
         self.weight_order: Optional[WeightOrder] = None
-        self.side_stream = None           # a second CUDA stream for work beside the main chain (prefetch, one of two mixers)
+        self.side_stream = None           # a second CUDA stream for work beside the main chain (one of two mixers)
         self.scratch_prefix = ""          # set while a part runs on the second stream: its buffers must be its own
         self.program = None               # a kernels.Program: decode steps of few rows run as one persistent kernel
         # An RMSNorm may be split between the product that completes the residual rows and the product that reads

@@ -15,7 +15,7 @@ from .. import kernels
 from ..config.specs import ModelConfig
 from ..parts import build_block, build_part
 from ..parts.block import collapse_streams
-from ..parts.base import Mixer, Part
+from ..parts.base import Part
 from ..weights.binding import ParamSpec
 
 
@@ -115,12 +115,12 @@ class DecoderModel:
         if program is not None:
             kernels.program_begin(program, ctx.status)
         try:
-            return self._forward(ctx, x, program is not None)
+            return self._forward(ctx, x)
         finally:
             if program is not None:
                 kernels.program_end()
 
-    def _forward(self, ctx, x, in_program: bool) -> torch.Tensor:
+    def _forward(self, ctx, x) -> torch.Tensor:
         n, d = ctx.n, self.config.hidden_size
         ctx.next_norm = ctx.norm_after_layer = ctx.prepared_norm = ctx.pending_fold = ctx.residual_copy = None
         self.embed.forward(ctx, ctx.tokens, x)
@@ -131,32 +131,11 @@ class DecoderModel:
             embedded, x = x, ctx.scratch("x_streams", (n, streams * d), torch.float32)
             kernels.streams_broadcast(embedded, x, streams)
         schedule = self.config.schedule
-        # (a program's persistent kernel asks for the next layer's keys and values itself)
-        side = ctx.side_stream if ctx.decode_only and not in_program else None
-        pending = False
         for i, run in enumerate(schedule):
-            hook = None
-            if side is not None and i + 1 < len(schedule):
-                nxt = schedule[i + 1]
-                mixer = getattr(self.layers[nxt.layer], "mixer", None)
-                if mixer is not None and type(mixer).prefetch is not Mixer.prefetch:
-                    def hook(mixer=mixer, cache_layer=nxt.cache):
-                        # beside this layer's feed-forward, on a second stream: the next mixer's prefetch
-                        main = torch.cuda.current_stream()
-                        side.wait_stream(main)
-                        with torch.cuda.stream(side):
-                            mixer.prefetch(ctx, ctx.cache_view(cache_layer))
-            if pending:
-                torch.cuda.current_stream().wait_stream(side)   # the prefetch kernel must not outlive the step
-                pending = False
             # which norm reads x after this layer: the next layer's first one, if it says which that is
             entry = getattr(self.layers[schedule[i + 1].layer], "entry_norm", None) if i + 1 < len(schedule) else None
             ctx.norm_after_layer = entry() if entry is not None else None
-            self.layers[run.layer].forward(ctx, x, ctx.cache_view(run.cache), run.writes_cache, after_mixer=hook) \
-                if hook is not None else self.layers[run.layer].forward(ctx, x, ctx.cache_view(run.cache), run.writes_cache)
-            pending = hook is not None
-        if pending:
-            torch.cuda.current_stream().wait_stream(side)
+            self.layers[run.layer].forward(ctx, x, ctx.cache_view(run.cache), run.writes_cache)
         ctx.norm_after_layer = None
         w = ctx.num_wanted
         logits = ctx.scratch("logits", (w, self.config.vocab_size), torch.float32, grow=True)

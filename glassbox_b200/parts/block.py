@@ -44,8 +44,8 @@ class PreNormBlock(Part):
         return self.mixer_norm
 
     def forward(self, ctx, x, cache, writes_cache: bool, after_mixer=None) -> None:
-        """``after_mixer`` (optional) is called once the mixer's kernels are launched: the model uses it
-        to let the next layer's mixer start its prefetch beside this layer's feed-forward.
+        """``after_mixer`` (optional) is called once the mixer's kernels are launched, for a caller with work of its own to
+        launch before the feed-forward's.
         ``ctx.norm_after_layer`` (optional) is the norm that will read ``x`` after this layer."""
         after_layer = getattr(ctx, "norm_after_layer", None)
         h = DeferredNorm(ctx, self.mixer_norm, x)
