@@ -2230,12 +2230,12 @@ def talking_attention_decode_supported(dtype: torch.dtype, heads: int, kv_heads:
     return dtype in _DT and bool(lib().gb_talking_attention_decode_plan(heads, kv_heads, vdim, value_heads))
 
 
-def talking_decode_shares(n: int, heads: int, kv_heads: int, vdim: int, value_heads: int, reach: int, dim: int = 0,
-                          dtype: Optional[torch.dtype] = None) -> int:
+def talking_decode_shares(n: int, heads: int, kv_heads: int, vdim: int, value_heads: int, reach: int, dim: int,
+                          dtype: torch.dtype) -> int:
     """Into how many shares the decoding kernel cuts a row's keys: the count whose rounds of blocks (two per multiprocessor, 296
     at once) take the least time, a round costing a block's keys and what its start and merge cost.
 
-    On the tensor cores (bfloat16 at the sizes it is built for; ``dim`` and ``dtype`` say so) that is about 200 keys' worth, and no share is
+    On the tensor cores (bfloat16 at the sizes it is built for; the key size ``dim`` and ``dtype`` say so) that is about 200 keys' worth, and no share is
     shorter than one step of the kernel. Attention and merge of 16 heads, 4 value heads of 64: 32 rows, contexts to 2,047, with 4 / 8 /
     9 / 12 / 16 shares 33 / 19.7 / 20.2 / 26.8 / 22.3 us (9 chosen); 64 rows, contexts to 1,000, 4 / 8 / 12 19.6 / 21.6 / 29.5 (4 chosen).
 

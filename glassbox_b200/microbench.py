@@ -623,7 +623,7 @@ def bench_babotar() -> None:
             od = torch.empty_like(qd)
             wd = torch.empty(m, H * G * hd, device=DEV)
             nbytes = m * ctx * G * hd * 2 * 2
-            shares = kernels.talking_decode_shares(m, H, G, hd, G, ctx)
+            shares = kernels.talking_decode_shares(m, H, G, hd, G, ctx, hd, qd.dtype)
             wd = torch.empty(shares * m, H * G * hd, device=DEV)
             mld = torch.empty(shares * m, H * 2, device=DEV)
             t = graph_time(lambda: kernels.talking_attention_decode(qd, wd, kd, vd, tb, row_seq, pd, shares=shares, ml=mld, **own))

@@ -146,3 +146,9 @@ def test_the_few_rows_projection_leaves_unaligned_tables_and_caches_to_the_other
     assert not kernels.gemm_few_qkv_supported(q, q, 64, q, odd, even, None)
     assert not kernels.gemm_few_qkv_supported(q, q, 64, q, even, odd, None)
     assert not kernels.gemm_few_qkv_supported(q, q, 64, q, even, even, table[1:])
+
+
+def test_talking_decode_shares_are_asked_for_one_kernel():
+    """The tensor-core kernel and the one by FMA cut a row's keys by rules of their own: which of them a call takes has to be said."""
+    with pytest.raises(TypeError):
+        kernels.talking_decode_shares(32, 16, 4, 64, 4, 2048)
