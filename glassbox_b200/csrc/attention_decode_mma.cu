@@ -48,10 +48,10 @@ struct DecodeSinkTerms {
 // once: eight processing clusters with 16 SMs each, of one block of eight warps or two of four warps with 32 keys per iteration, and
 // no more than the GPU says that it holds. Neither is enough alone. Of clusters of eight one card holds 15: with 16 the last starts when
 // the others have ended (32/8 heads, two rows of 4,000 / 8,000 keys 12.9 / 20.1 us, through global memory 8.7 / 12.5). And it names 45
-// of three and 26 of five that do not run at once (45 rows and heads of 4,000 keys 18.0, through global memory 14.6). One split needs no partner at all. Through global memory (a store, a fence, the counter, a load, one after the
-// other) / in the cluster, us: 9/3 heads, one row, contexts 100 / 1,024 / 4,000 5.1 / 3.0, 5.4 / 3.2, 8.0 / 6.1; four rows of 1,024 6.0 /
-// 3.7; 32/32 heads, one row of 1,024 5.7 / 4.5. With every warp sending its own result to the first block: 24 rows of 15/5 heads, 1,500
-// keys 13.6, the block's warps added up first 12.2; 40 rows of 9/3, 600 keys 9.1 and 8.1; 64 rows of 32/32, 4,000 keys 347 and 345.
+// of three and 26 of five that do not run at once (45 rows and heads of 4,000 keys 18.0, through global memory 14.6). One split needs
+// no partner at all. Through global memory (a store, a fence, the counter, a load, one after the other) / in the cluster, us: 9/3 heads, one
+// row, contexts 1,024 / 4,000 5.5 / 4.2 and 7.6 / 6.0; four rows of 1,024 5.5 / 4.4; 32/32 heads, one row of 1,024 6.2 / 5.3; 24 rows of
+// 15/5 heads, 1,500 keys 14.5 / 12.6; 40 rows of 9/3, 600 keys 10.1 / 8.3; 64 rows of 9/3, 4,000 keys 40.4 / 38.2.
 constexpr int MMA_CLUSTER_SMEM_MAX = 96 * 1024;
 
 // Clusters of a kernel's blocks that find room at once, asked once for every size and group.

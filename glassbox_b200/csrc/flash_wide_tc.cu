@@ -545,7 +545,7 @@ GB_EXPORT int gb_talking_attention_flash_supported(int D, int V, int VG, int pag
 }
 
 // As gb_talking_attention_tiles (talking_attention.cu), VG == G. q bfloat16 [n, H, 64], out float32 [n, H, G * V].
-// Measured, 2,048 tokens, 16/4 heads of 64, capped: 402 us in tiles of mma.sync, 58 us here.
+// Measured, 2,048 tokens, 16/4 heads of 64, capped: 395 us in tiles of mma.sync, 37 us here.
 GB_EXPORT int gb_talking_attention_flash(const void* q, float* out, const void* kcache, const void* vcache, const int* block_tables, int max_pages,
                                          const int* seq_first_row, const int* seq_start_pos, int n, int num_seqs, int max_rows_per_seq, int H, int G,
                                          int V, int page_size, long long num_pages, float scale, float cap, int unit, int window, int* status,
@@ -574,7 +574,7 @@ GB_EXPORT int gb_latent_flash_supported(int c, int r, int page_size) {
 
 // Attention of prompt portions over a latent cache [pages, page_size, 128 + r]: q bfloat16 [n, H, 128 + r], out bfloat16
 // [n, H, 128]; arguments as gb_latent_attention_mma. Measured, two portions of 1,500 tokens in all
-// behind up to 900, 32 heads, 128 + 64: 197 us in tiles of mma.sync, 65 us here.
+// behind up to 900, 32 heads, 128 + 64: 197 us in tiles of mma.sync, 60 us here.
 GB_EXPORT int gb_latent_flash(const void* q, void* out, const void* cache, const int* block_tables, int max_pages, const int* seq_first_row,
                               const int* seq_start_pos, const float* sink, int n, int num_seqs, int max_rows_per_seq, int H, int c, int r,
                               int page_size, long long num_pages, float scale, int window, int* status, cudaStream_t stream) {

@@ -878,12 +878,12 @@ def decode_mma_plan(n: int, nkv: int, hd: int, max_context: int):
     if hd == 64 and pairs >= 96:
         # Blocks of the 16-key variant run three to an SM, in waves: all blocks of a wave take as long as one of them.
         # A block costs about 5.7 us of start, merge and hand-over and 14.7 ns a key; a wave holds about 410 blocks
-        # (432 no longer fit one; without clusters, at one split, 416 still do: 71.3 us, 3 splits 92.0). The split count that this estimate likes best, among 1 to 4 (clusters of 5 and 7
-        # place badly), is the one measured best at context 4096 for 96 to 2,048 pairs, within 1 %: 128 pairs 3 splits
-        # 26.8 us (2: 34.6, 4: 37.3); 144 pairs 2 splits 35.6 (3: 45.6); 256 pairs 3 splits 51.6 (1: 66.1, 2: 66.3,
-        # 4: 57.7); 320 pairs 1 split 68.4 (2: 72.9, 4: 79.0); 512 pairs 3 splits 99.0 (1: 123.1, 4: 98.2); 2,048 pairs
-        # 1 split 338.7 (2: 354.7). (Filling two blocks per SM once, the rule before, took 2 splits at 256 pairs: a 1.7B
-        # decode step at batch 8 2.85 ms, with 3 splits 2.56 ms.)
+        # (432 no longer fit one; without clusters, at one split, 416 still do: 70.7 us, 3 splits 89.0). The split count that this
+        # estimate likes best, among 1 to 4 (clusters of 5 and 7 place badly), is the one measured best at context 4,096
+        # for 96 to 2,048 pairs, within 1 %: 96 pairs 4 splits 21.7 us (3: 25.7); 128 pairs 3 27.3 (2: 34.5, 4: 37.7); 144
+        # pairs 2 35.6 (3: 45.3, 4: 39.6); 256 pairs 3 51.8 (1: 63.6, 2: 65.7, 4: 57.9); 320 pairs 1 67.1 (2: 71.9, 4: 74.2);
+        # 512 pairs 3 100.1 (1: 121.3, 4: 99.3); 2,048 pairs 1 333.9 (2: 352.7). (Filling two blocks per SM once, the rule before,
+        # took 2 splits at 256 pairs: a 1.7B decode step at batch 8 2.85 ms, with 3 splits 2.56 ms.)
         best, best_cost = 1, None
         for splits in range(1, min(4, most) + 1):
             waves = -(-pairs * splits // (DECODE_MMA_WAVE_BLOCKS if splits > 1 else DECODE_MMA_WAVE_SINGLE))
@@ -902,8 +902,8 @@ def decode_mma_plan(n: int, nkv: int, hd: int, max_context: int):
         # (with more than 1,024 keys per block the longer loop of the 16-key variant costs more than the room gains:
         # 360M shapes at batch 8, three splits of 1,365 keys: 1.23 ms with 32 keys per iteration, 1.27 ms with 16)
         # Splits whose clusters find room at once merge on the chip (attention_decode_mma.cu), those that fill one wave through global
-        # memory, 2 us more: the former as long as a block has at most 512 keys. 9/3 heads, context 1,024: 6 rows 5 splits 4.2 us (8 through
-        # memory 5.7), 8 rows 5 / 4.6 (6: 5.9), 12 rows 3 / 5.2 (4: 6.5).
+        # memory, 1 to 2 us more: the former as long as a block has at most 512 keys. 9/3 heads: 8 rows of 1,024 keys 4 splits 4.9 us
+        # (6 through memory 6.1), of 2,048 5 / 6.9 (6: 7.7), of 4,096 5 / 10.1 (6: 10.3); 12 rows of 1,024 3 / 5.9 (4: 6.6).
         most = -(-max_context // 256)
         wide, near = max(1, min(148 // pairs, 8, most)), max(1, min(16 // -(-pairs // 8), 8, most))
         splits = near if max_context <= 512 * near else wide
