@@ -341,13 +341,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         const float cap2 = a.cap > 0.f ? a.cap * FW_LOG2E : 0.f, cap_in = a.cap > 0.f ? a.scale / a.cap : 0.f;
         const float slx = cap2 > 0.f ? cap2 : sl2;              // what is left to scale
         const int first = gb_first_key(pos, a.window), first_last = gb_first_key(pos_lo + FW_BM - 1, a.window);
-        // Scores that a cap bounds: what a row subtracts is chosen after the first tile (every row must see a key of it) and stays, and the two
-        // halves of a row go their own ways, one's caps beside the other's exponentials. It is the tile's maximum, at least what 2^8 lies
-        // below the cap, so that no weight grows above 2^8, as none does where the maximum is followed. Rows whose first tile lies 2^60
-        // below that are left to the general form: their weights could become too small for sums in float32.
-        bool bounded = a.cap > 0.f && a.cap <= 32.f && first_last == 0;
-        const float least = 1.0f - 8.0f / cap2;                 // (scores are in units of the cap)
+        const bool bounded = a.cap > 0.f && a.cap <= 32.f && first_last == 0;      // (and every row sees a key of the first tile)
         float m_run = FW_NEG_BIG, l_run = 0.f;
+        float down = 1.0f;          // weights and their sums are held at `down` times themselves
         bool ok = true;
         for (int j = 0; j < ntiles; ++j) {
             const int b = j & 1, key0 = (kt_begin + j) * FW_BN + h * 64;
@@ -362,6 +358,11 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 for (int k = 0; k < 64; ++k)
                     if (!(key0 + k <= pos && key0 + k >= first)) sv[k] = __float_as_uint(FW_NEG_BIG);
             }
+            // Scores that a cap bounds: the first tile's maximum stays, or -16, and the two halves of a row go their own ways, one's caps
+            // beside the other's exponentials. A weight may then grow to e^48: the row's weights are held at a power of two times
+            // themselves, which changes no bit of them and lets none exceed 2^8, as none does where the maximum is followed. (Where the
+            // first tile lies below -4 under a cap of 32, less: the sums have to hold the first tile's weights as well as the last one's.
+            // Values from 1e-18 to 1e27 keep their precision whatever the scores do.)
             if (j == 0 || !bounded) {
                 float mx4[4] = {FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG, FW_NEG_BIG};
 #pragma unroll
@@ -377,8 +378,8 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
                 mx = fmaxf(mx, sh.stat[b][h ^ 1][r]);
                 const bool raise = (mx - m_run) * slx > 8.0f;
                 if (j == 0) {
-                    bounded = bounded && __all_sync(0xffffffffu, mx >= least - 60.0f / cap2);      // (both halves have the same maxima)
-                    if (raise) m_run = bounded ? fmaxf(mx, least) : mx;      // nothing is accumulated yet
+                    if (raise) m_run = bounded ? fmaxf(mx, -16.0f / a.cap) : mx;      // nothing is accumulated yet (scores are in units of the cap)
+                    if (!LATENT && bounded) down = __int_as_float((127 - (int)ceilf(fminf(fmaxf(cap2 - m_run * slx - 8.0f, 0.f), 44.f))) << 23);
                 } else if (__any_sync(0xffffffffu, raise)) {
                     // (S_j was issued after O += P_(j-2) V_(j-2) was done: the phase of P_(j-1) V_(j-1) is the one to wait for)
                     if (!mbar_wait_warp(&sh.pv_done, (j - 1) & 1, abort_flag, a.status)) { ok = false; break; }
@@ -405,7 +406,8 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
 #pragma unroll
             for (int c = 0; c < 64; c += 2) {
                 const float2 y = __ffma2_rn(make_float2(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), scale2, off2);
-                const float2 pp = make_float2(fw_exp2(y.x), fw_exp2(y.y));
+                float2 pp = make_float2(fw_exp2(y.x), fw_exp2(y.y));
+                if (!LATENT) pp = __fmul2_rn(pp, make_float2(down, down));
                 // the denominator sums what the product uses: the weights as rounded to bfloat16
                 const uint32_t both = pw[c >> 1] = pack2(__float_as_uint(pp.x), __float_as_uint(pp.y));
                 l2[(c >> 1) & 1] = __fadd2_rn(l2[(c >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
@@ -429,13 +431,14 @@ __global__ void __launch_bounds__(FW_WARPS * 32) flash_wide_kernel(const __grid_
         }
         if (ok) {
             tc_fence_after();
-            float l = l_run + sh.stat[(bounded ? 1 : ntiles) & 1][h ^ 1][r], m2 = m_run <= FW_NEG_BIG ? FW_NEG_BIG : m_run * slx;
+            const float up = 1.0f / down;                       // (a power of two)
+            float l = (l_run + sh.stat[(bounded ? 1 : ntiles) & 1][h ^ 1][r]) * up, m2 = m_run <= FW_NEG_BIG ? FW_NEG_BIG : m_run * slx;
             float sink2 = FW_NEG_BIG;
             if (LATENT && a.sink != nullptr) sink2 = a.sink[head] * FW_LOG2E;
             if (a.unit) sink2 = 0.f;
             const float top = fmaxf(m2, sink2), corr = fw_exp2(m2 - top);
             l = l * corr + fw_exp2(sink2 - top);
-            const float inv = l > 0.f ? corr / l : 0.f;
+            const float inv = l > 0.f ? corr / l * up : 0.f;
             // Rows turn over where the keys were (all products are done, nothing is on its way there): a store writes 128 bytes of four rows,
             // of bfloat16 64 of eight, and not 16 bytes in each of 32 (float32, 256 channels: 10,800 cycles a block, 2,600 so).
             uint4* stage = reinterpret_cast<uint4*>(Ks) + (warp - 2) * (32 * 8);

@@ -14,10 +14,11 @@ def test_scores_that_climb_across_the_cap(cap, low, high, window, G, page):
     _climb(cap, low, high, window, G, page, 1e6)
 
 
-@pytest.mark.parametrize("size", [1e30, 1e-15])
+@pytest.mark.parametrize("size", [1e27, 1e-15, 1e-18])
 @pytest.mark.parametrize("cap, low, high", [(8.0, -1.0, 1.0), (30.0, -1.0, 1.0), (32.0, -1.0, 1.0), (30.0, 1.0, -1.0), (32.0, -0.1, 1.0)])
 def test_values_keep_their_range_whatever_the_scores_do(cap, low, high, size):
-    """Large values meet no weight above 2^8 and small ones none that the sums could lose, wherever in the cap the first keys lie."""
+    """Large values meet no weight that makes their sums overflow and small ones none that the sums could lose, wherever in the cap the
+    first keys lie."""
     _climb(cap, low, high, None, 4, 16, size)
 
 
