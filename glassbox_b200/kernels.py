@@ -462,7 +462,8 @@ def copy_pages(kcache: torch.Tensor, vcache: torch.Tensor, pairs: torch.Tensor) 
 
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, accumulate: bool = False) -> None:
-    """c[M, N] (+)= a[M, K] @ w[N, K]^T with float32 FMA on the CUDA cores (rows may be strided)."""
+    """c[M, N] (+)= a[M, K] @ w[N, K]^T with float32 FMA on the CUDA cores (rows may be strided). ``w`` is a weight, as in every
+    product here: no kernel launched just before may still be writing it (it is asked for before the wait for those)."""
     _cuda(a, w, c)
     M, K = a.shape
     N = w.shape[0]
