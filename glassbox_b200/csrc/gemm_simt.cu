@@ -291,15 +291,19 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const TA* __restrict__
 // column: latency, a tenth of the copy rate at best. Measured, 8 rows float32: N 960, K 576 10.8 -> 2.3 us (split); N 576, K
 // 1536 22.5 -> 3.3 (split); N 3072, K 576 12.1 -> 6.9; N 49152, K 576 62.7 -> 38.1 (113 MB). With the weights ahead of the wait and
 // of the products, and (no split) two warps a block, which spread N 3072 over every SM: 2.3 -> 2.0, 3.3 -> 2.8, 6.9 -> 6.5, 38.0 -> 34.0;
-// N 3072, K 2048 18.2 -> 17.4. (The activations one round ahead as well: N 8192 7.3 -> 11.6 for want of warps.)
+// N 3072, K 2048 18.2 -> 17.4. (The activations one round ahead as well: N 8192 7.3 -> 11.6 for want of warps.) Weights of 16 bits, whose
+// conversions then stand between the requests, gain nothing so and keep eight warps a block and no round ahead: 8 rows, N 1600, K 960 4.3 ->
+// 4.0; N 8192, K 2048 20.4 -> 19.7.
+template <typename TW> constexpr bool SK4_EARLY = sizeof(TW) == 4;
 template <typename TA, typename TW, typename TC, bool SPLIT>
-__global__ void __launch_bounds__(SPLIT ? 256 : 64) gemm_skinny4_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, int M, int N,
+__global__ void __launch_bounds__(SPLIT || !SK4_EARLY<TW> ? 256 : 64) gemm_skinny4_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, int M, int N,
                                                            int K, long long lda, long long ldw, long long ldc, int mode) {
     __shared__ float part[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = (SPLIT ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + warp) * 4;
     gb_pdl_launch_dependents();
-    // The weights, which no kernel of a step writes, are asked for before the wait for the kernel before, and those of the next
+    // EARLY: the weights, which no kernel of a step writes, are asked for before the wait for the kernel before, and those of the next
     // round before this one's products.
+    constexpr bool EARLY = SK4_EARLY<TW>;
     constexpr int STEP = SPLIT ? 1024 : 128;
     float wn[4][4];
     auto weights = [&](int k) {
@@ -310,18 +314,19 @@ __global__ void __launch_bounds__(SPLIT ? 256 : 64) gemm_skinny4_kernel(const TA
         }
     };
     const int k0 = (SPLIT ? warp * 128 : 0) + lane * 4;
-    weights(k0);
+    if (EARLY) weights(k0);
     gb_pdl_wait();
     float acc[32];                                      // [row][column]
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
     for (int k = k0; k < K; k += STEP) {
         float w[4][4], a[8][4];
+        if (!EARLY) weights(k);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
             for (int e = 0; e < 4; ++e) w[c][e] = wn[c][e];
-        if (k + STEP < K) weights(k + STEP);
+        if (EARLY && k + STEP < K) weights(k + STEP);
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
             if (m < M) Vec4Load<TA>::load(A + (size_t)m * lda + k, a[m]);
@@ -380,7 +385,7 @@ static int launch_gemm(const void* a, const void* w, void* c, int M, int N, int 
         if (vec && N <= 2048)
             gb_launch(GB_PDL_GEMM, gemm_skinny4_kernel<TA, TW, TC, true>, dim3(gb_ceil_div(N, 4)), dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, mode);
         else if (vec && M > (sizeof(TA) == 4 ? 2 : 4))
-            gb_launch(GB_PDL_GEMM, gemm_skinny4_kernel<TA, TW, TC, false>, dim3(gb_ceil_div(N, 8)), dim3(64), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, mode);
+            gb_launch(GB_PDL_GEMM, gemm_skinny4_kernel<TA, TW, TC, false>, dim3(gb_ceil_div(N, SK4_EARLY<TW> ? 8 : 32)), dim3(SK4_EARLY<TW> ? 64 : 256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, mode);
         else if (vec) gemm_skinny_kernel<TA, TW, TC, true><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
         else gemm_skinny_kernel<TA, TW, TC, false><<<grid, warps * 32, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, mode);
     } else {
