@@ -813,8 +813,11 @@ __global__ void __launch_bounds__(MS_THREADS) moe_sort_kernel(const int* __restr
 
 // The same for up to MS_FEW experts and MS_KEEP pairs a thread, without two pairs ever meeting at one counter: a thread counts its own pairs in
 // a column of its own, a warp per expert turns the counts of its row into the threads' first slots, and the thread deals them out. (8,192
-// pairs of 16 experts were 2 x 256 additions of 32 lanes to a handful of addresses, a division a pair and scattered stores: 9.0 us, 6.9 so.) An expert's pairs come in a fixed order.
-constexpr int MS_FEW = 64;
+// pairs of 16 experts were 2 x 256 additions of 32 lanes to a handful of addresses, a division a pair and scattered stores: 7.8 us, 6.0 so.) An expert's pairs come in a fixed order.
+// What it costs whatever the pairs (columns to clear and to add up) pays from 3,072 pairs on, of more than 32 experts from 96 an expert. By
+// additions / by columns, us: 16 experts 256 pairs 3.3 / 4.4, 2,048 4.3 / 4.5, 3,072 4.9 / 4.7, 16,384 13.2 / 8.4; 32 experts 2,048 4.5 /
+// 5.0, 3,072 5.6 / 5.2; 64 experts 512 3.4 / 6.0, 4,096 6.5 / 6.8, 6,144 8.4 / 7.0, 8,192 10.0 / 7.7.
+constexpr int MS_FEW = 64, MS_MANY = 3072;
 
 __global__ void __launch_bounds__(MS_THREADS) moe_sort_columns_kernel(const int* __restrict__ choice, const int* __restrict__ positions, int n,
                                                                       int E, int top, int* __restrict__ offsets, int* __restrict__ sorted) {
@@ -908,7 +911,8 @@ __global__ void __launch_bounds__(MS_THREADS) moe_sort_columns_kernel(const int*
 GB_EXPORT int gb_moe_sort(const int* choice, const int* positions, int n, int E, int top, int* offsets, int* sorted, cudaStream_t stream) {
     GB_REQUIRE(n >= 0 && E > 0 && E <= MOE_MAX_EXPERTS && top > 0, "gb_moe_sort: bad sizes");
     if (n == 0) return 0;
-    if (E <= MS_FEW && (long long)n * top <= (long long)MS_KEEP * MS_THREADS) {
+    const long long pairs = (long long)n * top;
+    if (E <= MS_FEW && pairs <= (long long)MS_KEEP * MS_THREADS && pairs >= MS_MANY && pairs >= 96 * E) {
         // (the limit is the most that any sizes need: a kernel has one, and a thread with few pairs must not lower it under another's launch)
         constexpr int most = MS_FEW * MS_THREADS * (int)sizeof(unsigned short) + MS_KEEP * MS_THREADS * (int)sizeof(int);
         const int smem = E * MS_THREADS * (int)sizeof(unsigned short) + n * top * (int)sizeof(int);

@@ -29,6 +29,12 @@ def test_every_live_pair_has_a_slot_of_its_expert(n, E, top):
     assert torch.equal(expert[used.long()].long(), torch.repeat_interleave(torch.arange(E, device=DEV), counts))
 
 
+@pytest.mark.parametrize("n, E, top", [(3071, 16, 1), (3072, 16, 1), (1024, 32, 3), (1535, 64, 4), (1536, 64, 4), (3073, 1, 1), (8192, 7, 2), (16385, 16, 1)])
+def test_both_sides_of_the_line_sort(n, E, top):
+    """Counters of all pairs below 3,072 of them (and 96 an expert) and above what a block's columns hold, columns between."""
+    test_every_live_pair_has_a_slot_of_its_expert(n, E, top)
+
+
 def test_threads_with_few_and_many_pairs_do_not_disturb_each_other():
     """The kernel's limit of shared memory is one for all threads of a process: a small sort beside a large one must not lower it."""
     import threading
@@ -47,7 +53,7 @@ def test_threads_with_few_and_many_pairs_do_not_disturb_each_other():
                 assert offsets.tolist() == [i * n * top // E for i in range(E + 1)]
         except Exception as e:      # noqa: BLE001 (reported by the thread that asserts)
             failures.append(repr(e))
-    threads = [threading.Thread(target=work, args=shape) for shape in ((16, 16, 4), (4096, 64, 4), (64, 16, 2), (4096, 64, 4))]
+    threads = [threading.Thread(target=work, args=shape) for shape in ((768, 16, 4), (4096, 64, 4), (3072, 1, 1), (4096, 64, 4))]
     for t in threads:
         t.start()
     for t in threads:
