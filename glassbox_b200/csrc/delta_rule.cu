@@ -231,11 +231,12 @@ GB_EXPORT int gb_short_conv(const float* x, long long ldx, const float* w, float
               state_stride, state_off, row_seq, positions, seq_first_row, seq_slots, n, C, num_slots, status)
     const bool many = (long long)strips.x * strips.y >= 444;
     // Four channels a thread where requests bring sixteen rows and more each on average (where they bring few, every strip looks every row's
-    // request up: 64 rows of as many requests 7.3 us by rows, 8.8 so) and there are 96 rows, in strips of four rows, of eight from
-    // five blocks an SM on. By rows or by the strips below / so, one request, with the state's update, us: 3,072 channels 70 rows 5.8 / 6.0,
-    // 128 6.6 / 6.3, 256 9.5 / 6.2, 512 14.9 / 6.8, 768 11.3 / 8.3, 1,024 13.8 / 9.9, 2,048 18.5 / 14.2 (strips of four 14.9); 6,144
-    // channels 128 9.5 / 6.5, 512 14.1 / 10.1, 2,048 32.1 / 26.0.
-    const bool fours = n >= 96 && n >= 16LL * S && taps >= 2 && taps <= 4 && C % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 &&
+    // request up: 64 rows of as many requests 7.3 us by rows, 8.8 so), there are 96 rows, and 384 K numbers (several requests: 512 K) give
+    // a block enough to ask for; in strips of four rows, of eight from five blocks an SM on. By rows or by the strips above / so, with the
+    // state's update, us, one request: 1,024 channels 96 rows 4.6 / 6.0, 256 5.7 / 6.0, 384 6.6 / 6.2, 1,024 11.3 / 6.5; 3,072 channels 96 rows 5.8 / 6.2, 128
+    // 6.6 / 6.3, 512 15.0 / 6.7, 2,048 18.7 / 14.1 (strips of four 14.9); 6,144 channels 128 9.5 / 6.4, 2,048 32.3 / 25.8; requests of 16 rows: 1,536 channels
+    // 256 rows 6.9 / 7.2, 2,048 channels 7.8 / 7.7.
+    const bool fours = n >= 96 && n >= 16LL * S && (long long)n * C >= (S == 1 ? 384 : 512) * 1024 && taps >= 2 && taps <= 4 && C % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 &&
                        (((uintptr_t)x | (uintptr_t)y | (uintptr_t)w) & 15) == 0;
     const bool eight = (long long)gb_ceil_div(n, 8) * gb_ceil_div(C, 1024) >= 5 * 148;
 #define SC_FOURS(TAPS, ROWS)                                                                                                         \

@@ -33,6 +33,11 @@ def test_convolution_of_four_channels_a_thread_gives_the_bits_of_one(lengths, C,
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("lengths, C, taps", [([96], 4100, 4), ([97, 1], 5380, 4), ([131, 2, 60], 2724, 3), ([64, 1, 1, 33], 5300, 2), ([4096], 96, 4)])
+def test_the_smallest_that_take_four_channels(lengths, C, taps):
+    test_convolution_of_four_channels_a_thread_gives_the_bits_of_one(lengths, C, taps)
+
+
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n, heads, v, silu", [(1, 1, 4, False), (7, 3, 60, True), (33, 8, 128, False), (5, 2, 132, True), (129, 3, 256, False)])
 def test_head_norm_of_four_numbers_a_lane(n, heads, v, silu, dt):
