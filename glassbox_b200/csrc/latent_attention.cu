@@ -219,8 +219,13 @@ __global__ void __launch_bounds__(128, 11) latent_kv_write8_kernel(const __nv_bf
     if (mine_k) put(dst + c, tid, ka, kb);
 }
 
-static bool lat_eights(const void* proj, long long ldp, int kv_col, const void* qabs, const void* cache, int dq, int r, int c, int rot_dims,
+// Where a row brings enough of them: with few numbers most of the block's threads have none of the items of eight (of sixteen with
+// partners) and wait. A number a thread / eight, us, 128 latent numbers, 2,048 rows unless said: neighbours in pairs, 8 heads of 32 5.3 / 6.4, 16 of 32 6.0 /
+// 6.4, 24 of 32 6.9 / 6.5, 32 of 64 10.8 / 7.5, 300 rows of 8 heads of 64 3.2 / 3.1; halves in pairs, 16 heads of 32 6.0 / 7.1, 24 of 32 6.8 / 7.2, 16 of 64
+// 7.6 / 7.4, 64 of 16 7.6 / 9.4; 512 latent numbers, 8 heads of 32 7.3 / 7.0 and 7.3 / 7.5.
+static bool lat_eights(const void* proj, long long ldp, int kv_col, const void* qabs, const void* cache, int H, int dq, int r, int c, int rot_dims,
                        int write_kv, int half_pairs) {
+    if (H * r + (write_kv ? 2 * c : 0) < (half_pairs ? 1280 : 1024) || (half_pairs && r < 32)) return false;
     return dq % 8 == 0 && r % 8 == 0 && r <= 1024 && c % 8 == 0 && c <= 1024 && ldp % 8 == 0 && rot_dims % (half_pairs ? 16 : 8) == 0 &&
            (!write_kv || (kv_col % 8 == 0 && ((uintptr_t)cache & 15) == 0)) && (((uintptr_t)proj | (uintptr_t)qabs) & 15) == 0;
 }
@@ -237,7 +242,7 @@ GB_EXPORT int gb_latent_kv_write(const void* proj, long long ldp, int kv_col, vo
         gb_launch(GB_PDL_ELEMENTWISE, latent_kv_write_kernel<float>, dim3(n), dim3(128), 0, stream, (const float*)proj, ldp, kv_col,
                   (float*)qabs, (float*)cache, latent_gain, inv_freq, positions, slots, n, H, dq, r, c, rot_dims, num_slots, eps,
                   write_kv, half_pairs, magnitude, status);
-    else if (dtype == GB_BF16 && lat_eights(proj, ldp, kv_col, qabs, cache, dq, r, c, rot_dims, write_kv, half_pairs))
+    else if (dtype == GB_BF16 && lat_eights(proj, ldp, kv_col, qabs, cache, H, dq, r, c, rot_dims, write_kv, half_pairs))
         gb_launch(GB_PDL_ELEMENTWISE, latent_kv_write8_kernel, dim3(n), dim3(128), 0, stream, (const __nv_bfloat16*)proj, ldp, kv_col,
                   (__nv_bfloat16*)qabs, (__nv_bfloat16*)cache, latent_gain, inv_freq, positions, slots, n, H, dq, r, c, rot_dims, num_slots,
                   eps, write_kv, half_pairs, magnitude, status);

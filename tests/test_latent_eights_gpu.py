@@ -37,6 +37,13 @@ def test_cache_write_of_eight_numbers_a_thread(n, H, dq, r, c, rot, half, write)
     assert write == bool((outs[0][1] != 7.0).any()) and (outs[0][0][:, c:] != 7.0).any()
 
 
+@pytest.mark.parametrize("n, H, dq, r, c, rot, half, write", [
+    (1, 96, 8, 8, 128, 8, False, True), (33, 127, 16, 8, 8, 8, False, True), (9, 40, 16, 32, 64, 16, True, True), (5, 30, 8, 40, 96, 0, True, True),
+    (300, 40, 64, 32, 128, 32, True, False), (7, 1, 0, 1024, 1024, 1024, False, True)])
+def test_the_smallest_rows_that_take_eight_numbers_a_thread(n, H, dq, r, c, rot, half, write):
+    test_cache_write_of_eight_numbers_a_thread(n, H, dq, r, c, rot, half, write)
+
+
 @pytest.mark.parametrize("n, heads, N, K, gated", [(1, 1, 8, 16, False), (65, 3, 128, 64, False), (200, 2, 64, 128, True), (63, 5, 72, 16, True), (17, 4, 136, 256, False),
                                                    (130, 2, 192, 48, True)])
 def test_per_head_product_with_whole_rows_stored(n, heads, N, K, gated):
