@@ -67,7 +67,9 @@ __device__ __forceinline__ float4 gf_peer_load(uint32_t addr, uint32_t rank) {  
     return v;
 }
 
-__global__ void __launch_bounds__(GF_THREADS) gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+// (One block a multiprocessor, by its shared memory, and said so: without it the compiler keeps to 63 registers, and the merge of the
+// splits loses its loads under way: 64 rows, N 1024, K 1024 4.6 -> 4.8 us.)
+__global__ void __launch_bounds__(GF_THREADS, 1) gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                               const GfArgs a) {
     extern __shared__ __align__(16) unsigned char gf_dyn[];
     unsigned char* stages = gf_dyn + ((1024u - (smem_u32(gf_dyn) & 1023u)) & 1023u);      // swizzled tiles: 1024-byte aligned
