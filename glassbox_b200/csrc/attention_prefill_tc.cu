@@ -750,9 +750,9 @@ static int prefill_tc_run(const void* q, long long q_stride, int n_rows, void* o
 // most keys would keep the launch waiting long enough (what a pair costs is 1.5 us) - many fresh tiles, or one tile behind a long
 // context. `reach`: the keys that the table covers (where it is wide for another request's sake, one fresh tile takes 8.2 us as a pair and
 // 6.6 by itself; a 135M step of eight decoded rows behind 4,000 tokens and a fresh prompt of 100 shows no difference).
-// Block a tile / two blocks a pair, 9 heads, us: 256 rows 7.2 / 8.7, 1,024 12.8 / 13.0, 1,280 14.7 / 14.2, 1,536 16.7 / 15.4, 2,048 20.6 /
-// 18.1; behind 1,000 tokens 64 rows 13.5 / 10.9, 128 14.1 / 12.0, 256 15.2 / 16.1, 1,024 20.6 / 21.5, 1,500 24.0 / 23.4; 128 rows behind
-// 1,900 20.5 / 15.6.
+// Block a tile / two blocks a pair, 9 heads, us: 256 rows 7.2 / 8.7, 1,024 12.8 / 13.0, 1,280 14.7 / 14.2, 1,536 16.7 / 15.3, 2,048 20.5 /
+// 18.1; behind 300 tokens 1,220 rows 17.2 / 17.6, 1,348 18.0 / 18.7, 1,476 19.0 / 18.8; behind 1,000 64 rows 13.5 / 10.9, 128 14.1 / 12.0, 256 15.2 /
+// 16.1, 1,348 23.0 / 23.3, 1,476 23.9 / 23.4, 2,048 28.3 / 25.7; 128 rows behind 1,900 20.5 / 15.6. From twelve tiles on no context loses.
 // A window makes the tiles alike and leaves little to share. 2,048 fresh rows, windows of 300 / 1,024 / 1,300 / 1,600 10.5 / 13.3, 15.8 / 18.1, 18.1 /
 // 19.3, 20.0 / 18.9, chunks of 1,024 13.1 / 15.5; 1,500 rows behind 1,000, window of 2,000 22.8 / 24.5: many tiles take pairs where it is no
 // window to them. One tile behind 1,900: windows of 300 / 600 / 1,024 9.7 / 9.9, 11.6 / 10.3, 15.3 / 12.0, a chunk of 1,024 12.7 / 11.1.
@@ -762,7 +762,7 @@ GB_EXPORT int gb_attention_prefill_tc_pairs(int num_seqs, int max_rows_per_seq, 
     long long up = 1;                             // (a power of two, as the tables of recorded steps are: both go the same way)
     while (up < reach) up *= 2;
     if (tiles == 1) return up >= 2048 && (window == 0 || window >= 512 || window <= -1024);
-    return tiles >= 10 && (window == 0 || llabs((long long)window) >= up);
+    return tiles >= 12 && (window == 0 || llabs((long long)window) >= up);
 }
 
 // Rows of each request are consecutive: request s owns rows seq_first_row[s] .. seq_first_row[s+1]-1, at

@@ -38,7 +38,7 @@ def test_pairs_of_row_tiles(nh, nkv, rows, past, window, page):
         assert (out[:, h * 64:h * 64 + 64].double() - want).abs().max() < 2.0 ** -8 * 4, h
 
 
-@pytest.mark.parametrize("nh, nkv, rows, past", [(9, 3, 1153, 0), (9, 3, 2048, 0), (4, 2, 1500, 0), (2, 1, 1290, 40)])
+@pytest.mark.parametrize("nh, nkv, rows, past", [(9, 3, 1409, 0), (9, 3, 2048, 0), (4, 2, 1600, 0), (2, 1, 1700, 40)])
 def test_second_items_of_one_key_tile_repeat_their_bits(nh, nkv, rows, past):
     """The first row tile of a fresh prompt sees one key tile: one softmax group has none there and must not post that item's row
     statistics before the other group has read the first item's. What orders them is `merged` in the kernel; a late reader would
@@ -56,8 +56,14 @@ def test_second_items_of_one_key_tile_repeat_their_bits(nh, nkv, rows, past):
     assert int(status) == 0 and all(torch.equal(out, outs[0]) for out in outs)
 
 
+@pytest.mark.parametrize("nh, nkv, rows, past, page", [(9, 3, 1409, 0, 16), (2, 1, 1537, 0, 64), (9, 3, 1600, 0, 16), (2, 2, 1665, 700, 8), (2, 1, 1800, 0, 16)])
+def test_odd_and_even_counts_of_row_tiles(nh, nkv, rows, past, page):
+    """The tile in the middle of an odd count has no partner; the last tile may have one row."""
+    test_pairs_of_row_tiles(nh, nkv, rows, past, 0, page)
+
+
 @pytest.mark.parametrize("pairs, num_seqs, rows, nh, window, reach", [
-    (1, 1, 2048, 9, 0, 2048), (1, 1, 1153, 9, 0, 1153), (0, 1, 1152, 9, 0, 2048), (0, 2, 2048, 9, 0, 2048), (0, 1, 2176, 9, 0, 4096),
+    (1, 1, 2048, 9, 0, 2048), (1, 1, 1409, 9, 0, 1409), (0, 1, 1408, 9, 0, 2048), (0, 2, 2048, 9, 0, 2048), (0, 1, 2176, 9, 0, 4096),
     # a window or chunk that ends within what the rows see: tiles see about the same
     (0, 1, 2048, 9, 300, 2048), (0, 1, 2048, 9, 1300, 2048), (0, 1, 2048, 9, -1024, 2048), (1, 1, 2048, 9, 2048, 2048), (1, 1, 2048, 9, 4096, 2048),
     (0, 1, 2048, 9, 2048, 4096), (0, 1, 1500, 9, 2000, 2500),
