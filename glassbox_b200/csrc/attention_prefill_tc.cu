@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, long long out_stride,
     const int* __restrict__ block_tables, int max_pages, const int* __restrict__ seq_first_row,
     const int* __restrict__ seq_start_pos, int nh, int nkv, int page_size, int page_shift, long long num_pages,
-    float scale, int window, int* __restrict__ status, const AtSinkTerms terms) {
+    float scale, int window, int by_tile, int* __restrict__ status, const AtSinkTerms terms) {
     using G = AtGeometry<HD, PAIR>;
     static_assert(HD == 64, "this kernel is built for head size 64");
     extern __shared__ __align__(1024) unsigned char at_smem[];
@@ -178,13 +178,15 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attention_prefill_tc_kernel(
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = PAIR ? (int)blockIdx.x & 1 : 0;
-    const int head = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, seq = blockIdx.y;
+    // The grid: heads (PAIR: twice), requests, row tiles; by_tile: row tiles, requests, heads
+    const int head = PAIR ? (int)blockIdx.x >> 1 : by_tile ? (int)blockIdx.z : (int)blockIdx.x, seq = blockIdx.y;
+    const int at_tile = !PAIR && by_tile ? (int)blockIdx.x : (int)blockIdx.z, tiles = !PAIR && by_tile ? (int)gridDim.x : (int)gridDim.z;
     const int row0 = seq_first_row[seq];
     const int nrows = seq_first_row[seq + 1] - row0;
-    // Later tiles see more keys. One block a tile: the longest blocks start first, over all heads and requests (the tile is the
-    // slowest dimension of the grid). Two blocks a pair of tiles: the p-th from the end and the p-th.
+    // Later tiles see more keys. One block a tile: the longest blocks start first. Two blocks a pair of tiles: the p-th from the end
+    // and the p-th.
     const int row_tiles = (nrows + AT_BM - 1) / AT_BM;
-    const int qt = PAIR ? row_tiles - 1 - (int)blockIdx.z : (int)(gridDim.z - 1 - blockIdx.z), qt_low = blockIdx.z;
+    const int qt = PAIR ? row_tiles - 1 - at_tile : tiles - 1 - at_tile, qt_low = at_tile;
     if (PAIR ? qt < qt_low : qt * AT_BM >= nrows) return;         // uniform for the block (the pair), before anything is allocated
     if (smem_u32(at_smem) & 1023u) {              // swizzled tiles want 1024-byte alignment: refuse rather than compute nonsense
         if (tid == 0) atomicOr(status, GB_STATUS_WAIT_TIMEOUT);
@@ -724,7 +726,13 @@ static int prefill_tc_run(const void* q, long long q_stride, int n_rows, void* o
     int page_shift = 0;
     while ((1 << page_shift) < page_size) ++page_shift;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = PAIR ? dim3(2 * nh, num_seqs, (tiles + 1) / 2) : dim3(nh, num_seqs, tiles);
+    // The order of the blocks. Where they come in rounds, the longest first, over all heads; the same where they fill the chip once. Blocks
+    // for at most every other multiprocessor: a head's tiles one after the other, as measured; why was not found out. (By itself the
+    // launch does not show it; in a step, where the next kernels' blocks wait beside it, it does. 135M step, longest
+    // first / by head, us: 512 rows (36 blocks) 1,292 / 1,255, 681 (54) 1,386 / 1,360, 1,000 (72) 1,560 / 1,546, 1,300 (99) 1,521 / 1,541; a 360M layer
+    // of 512 (60) 54.5 / 54.0, of 1,000 (120) 62.2 / 63.0, of 2,048 (240) 96 / 105.)
+    const bool by_tile = !PAIR && (long long)nh * num_seqs * tiles <= 74;
+    cfg.gridDim = PAIR ? dim3(2 * nh, num_seqs, (tiles + 1) / 2) : by_tile ? dim3(tiles, num_seqs, nh) : dim3(nh, num_seqs, tiles);
     cfg.blockDim = dim3(AT_WARPS * 32);
     cfg.dynamicSmemBytes = G::SMEM;
     cfg.stream = stream;
@@ -741,7 +749,7 @@ static int prefill_tc_run(const void* q, long long q_stride, int n_rows, void* o
     }
     cfg.attrs = attr;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, (__nv_bfloat16*)out, out_stride, block_tables, max_pages, seq_first_row,
-                                       seq_start_pos, nh, nkv, page_size, page_shift, num_pages, scale, window, status, terms);
+                                       seq_start_pos, nh, nkv, page_size, page_shift, num_pages, scale, window, by_tile ? 1 : 0, status, terms);
     GB_REQUIRE(e == cudaSuccess, "gb_attention_prefill_tc: launch failed: %s", cudaGetErrorString(e));
     return gb_check_launch("gb_attention_prefill_tc");
 }
